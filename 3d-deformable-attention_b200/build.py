@@ -1,9 +1,9 @@
-"""Build libdfa3d_b200.so (CUDA kernels + C ABI) and libdfa3d_rates.so (memory-primitive rate probes,
-measurement code) in-tree with nvcc for sm_100a.
+"""Build libdfa3d_b200.so (CUDA kernels + C ABI), libdfa3d_rates.so (memory-primitive rate probes,
+measurement code) and _native.so (host path of the autograd Functions) in-tree, for sm_100a.
 
-No torch headers are involved: the library is plain CUDA C++ behind an ``extern "C"`` interface
-(include/dfa3d_b200.h).  The result is written next to the Python package
-(``dfa3d_b200/libdfa3d_b200.so``) so that it is found without any install step.
+The library is plain CUDA C++ behind an ``extern "C"`` interface (include/dfa3d_b200.h) without torch
+headers; only _native.so, which contains no kernels, is compiled against torch.  The results are written
+next to the Python package (``dfa3d_b200/``) so that they are found without any install step.
 """
 import os
 import subprocess
@@ -16,6 +16,8 @@ SOURCES = ["dfa3d_forward.cu", "dfa3d_backward.cu", "dfa3d_rebatch.cu", "dfa3d_d
            "dfa3d_fp64.cu", "dfa3d_layer_ops.cu", "dfa3d_capi.cu"]
 RATES_SRC = os.path.join(CSRC, "rates", "dfa3d_rates.cu")
 RATES_OUT = os.path.join(HERE, "dfa3d_b200", "libdfa3d_rates.so")
+NATIVE_SRC = os.path.join(CSRC, "binding", "dfa3d_torch.cpp")
+NATIVE_OUT = os.path.join(HERE, "dfa3d_b200", "_native.so")
 INCLUDE = os.path.join(HERE, "..", "include")
 NVCC_FLAGS = ["-O3", "-I", INCLUDE, "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -28,10 +30,25 @@ def _nvcc():
     return "nvcc"
 
 
+def _native_command():
+    """g++ command of the torch binding: header and library folders come from the installed torch."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+    lib = os.path.join(root, "lib")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
+            *[a for i in inc for a in ("-isystem", i)], NATIVE_SRC, "-o", NATIVE_OUT, "-L", lib,
+            "-Wl,-rpath," + lib, "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+
+
 def needs_build():
-    if not os.path.exists(OUT) or not os.path.exists(RATES_OUT):
+    outs = (OUT, RATES_OUT, NATIVE_OUT)
+    if not all(os.path.exists(o) for o in outs):
         return True
-    t = min(os.path.getmtime(OUT), os.path.getmtime(RATES_OUT))
+    t = min(os.path.getmtime(o) for o in outs)
     deps = [os.path.join(d, f) for d, _, fs in os.walk(CSRC) for f in fs]
     deps.append(os.path.join(HERE, "..", "include", "dfa3d_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
@@ -51,6 +68,7 @@ def build(force=False, verbose=False):
                                                  text=True)))
     rates = subprocess.Popen([_nvcc(), *NVCC_FLAGS, "-shared", "-cudart", "shared", RATES_SRC, "-o", RATES_OUT],
                              stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    native = subprocess.Popen(_native_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     objs = []
     for src, obj, pr in procs:
         log, _ = pr.communicate()
@@ -71,6 +89,9 @@ def build(force=False, verbose=False):
         f.write(log)
     if rates.returncode != 0:
         raise RuntimeError(f"nvcc failed on dfa3d_rates.cu:\n{log[-4000:]}")
+    log, _ = native.communicate()
+    if native.returncode != 0:
+        raise RuntimeError(f"g++ failed on dfa3d_torch.cpp:\n{log[-4000:]}")
     return OUT
 
 

@@ -525,6 +525,14 @@ int dfa3d_column_sum(const float *src, int64_t rows, int32_t cols, float *dst, v
   return finish(dfa3d::launch_column_sum(src, rows, cols, dst, (cudaStream_t)stream), "dfa3d_column_sum launch");
 }
 
+int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream) {
+  if (na < 0 || nb < 0)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "element counts must be >= 0 (got %lld, %lld)", (long long)na, (long long)nb);
+  if (na > 0) { REQUIRE_PTR(a); REQUIRE_ALIGNED(a); }
+  if (nb > 0) { REQUIRE_PTR(b); REQUIRE_ALIGNED(b); }
+  return finish(dfa3d::launch_zero_two(a, na, b, nb, (cudaStream_t)stream), "dfa3d_zero_two launch");
+}
+
 // ---- double precision -------------------------------------------------------------------------
 // Same checks as check_problem(); both dtype fields must say DFA3D_DTYPE_F64 and dist must be laid out
 // like value (no single-map option in double).

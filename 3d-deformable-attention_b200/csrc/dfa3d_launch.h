@@ -62,4 +62,5 @@ cudaError_t launch_layer_norm_backward(const float *grad_y, const float *in, con
                                        float *grad_in, float *grad_gamma, float *grad_beta,
                                        cudaStream_t s);
 cudaError_t launch_column_sum(const float *src, long long rows, int cols, float *dst, cudaStream_t s);
+cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cudaStream_t s);
 }  // namespace dfa3d

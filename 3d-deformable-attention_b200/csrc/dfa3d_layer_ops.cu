@@ -235,6 +235,17 @@ column_sum_kernel(const float *__restrict__ src, long long rows, int cols, float
   }
 }
 
+// Zeroes two buffers with one launch (a backward zeroes the two gradients it accumulates into; for a small
+// problem a second fill is a launch gap longer than the fill).  16-byte stores, the ragged ends one by one.
+__global__ void __launch_bounds__(256) zero_two_kernel(float *a, long long na, float *b, long long nb) {
+  const long long va = na >> 2, vb = nb >> 2, step = (long long)gridDim.x * blockDim.x;
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long t = t0; t < va + vb; t += step)
+    st4(t < va ? a + t * 4 : b + (t - va) * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+  if (t0 < (na & 3)) a[va * 4 + t0] = 0.f;
+  if (t0 < (nb & 3)) b[vb * 4 + t0] = 0.f;
+}
+
 unsigned row_grid(long long rows) {
   const long long want = (rows + kLnWarps - 1) / kLnWarps;
   const long long cap = (long long)kSms * kCtasPerSm;
@@ -298,6 +309,13 @@ cudaError_t launch_column_sum(const float *src, long long rows, int cols, float 
   if (gx > most) gx = most;
   if (gx < 1) gx = 1;
   column_sum_kernel<<<dim3((unsigned)gx, bands, 1), kCsThreads, 0, s>>>(src, rows, cols, dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cudaStream_t s) {
+  const long long groups = (na + nb + 3) / 4, want = (groups + 255) / 256, cap = (long long)kSms * 8;
+  if (na + nb == 0) return cudaSuccess;
+  zero_two_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(a, na, b, nb);
   return cudaGetLastError();
 }
 

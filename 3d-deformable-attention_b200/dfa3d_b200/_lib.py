@@ -77,11 +77,21 @@ PLAIN_ENTRY_POINTS = {
     "dfa3d_add_layer_norm_forward": [ctypes.c_void_p] * 4 + [_I64, _I32, ctypes.c_float] + [ctypes.c_void_p] * 5,
     "dfa3d_layer_norm_backward": [ctypes.c_void_p] * 5 + [_I64, _I32] + [ctypes.c_void_p] * 4,
     "dfa3d_column_sum": [ctypes.c_void_p, _I64, _I32, ctypes.c_void_p, ctypes.c_void_p],
+    "dfa3d_zero_two": [ctypes.c_void_p, _I64, ctypes.c_void_p, _I64, ctypes.c_void_p],
 }
 ACT_SOFTMAX, ACT_SIGMOID = 0, 1
 
 _lib = None
-calls = 0      # successful entry-point calls so far (each launches at least one kernel)
+_native = None
+_calls = 0      # successful entry-point calls made from Python so far
+
+
+def __getattr__(name):
+    # `calls`: successful entry-point calls so far, from Python and from the native host path (each launches
+    # at least one kernel)
+    if name == "calls":
+        return _calls + (_native.calls() if _native is not None else 0)
+    raise AttributeError(name)
 
 
 def load():
@@ -117,6 +127,21 @@ def load():
     return lib
 
 
+def native():
+    """The native host path (csrc/binding): built beside the library, bound to the library's entry points."""
+    global _native
+    if _native is None:
+        lib = load()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise ImportError(f"{e}: build it with `python 3d-deformable-attention_b200/build.py`. dfa3d_b200 has no "
+                              "fallback implementation.") from e
+        mod.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in mod.entries()})
+        _native = mod
+    return _native
+
+
 def call_plain(name, *args):
     """Invoke an entry point that takes no problem descriptor."""
     lib = load()
@@ -124,8 +149,8 @@ def call_plain(name, *args):
     if rc != 0:
         msg = lib.dfa3d_last_error().decode("utf-8", "replace")
         raise RuntimeError(f"{name} failed ({ERROR_NAMES.get(rc, rc)}): {msg}")
-    global calls
-    calls += 1
+    global _calls
+    _calls += 1
 
 
 def call(name, problem, *ptrs):
@@ -135,5 +160,5 @@ def call(name, problem, *ptrs):
     if rc != 0:
         msg = lib.dfa3d_last_error().decode("utf-8", "replace")
         raise RuntimeError(f"{name} failed ({ERROR_NAMES.get(rc, rc)}): {msg}")
-    global calls
-    calls += 1
+    global _calls
+    _calls += 1

@@ -31,6 +31,7 @@ def _check(logits, shapes, lsi):
 
 
 _DTYPES = {torch.float32: _lib.DTYPE_F32, torch.bfloat16: _lib.DTYPE_BF16, torch.float16: _lib.DTYPE_F16}
+_ACTS = {"softmax": _lib.ACT_SOFTMAX, "sigmoid": _lib.ACT_SIGMOID}
 
 
 class DepthDistributionFunction(Function):
@@ -68,6 +69,16 @@ class DepthDistributionFunction(Function):
                             shapes.data_ptr(), shapes.shape[1], lsi.data_ptr(), shapes.shape[0], ctx.N,
                             ctx.act, grad_dist.data_ptr(), grad_logits.data_ptr(), _stream(logits))
         return grad_logits, None, None, None, None, None
+
+    @classmethod
+    def apply(cls, logits, spatial_shapes, level_start_index, num_pixels, activation="softmax",
+              dtype=torch.float32):
+        if cls is DepthDistributionFunction and activation in _ACTS and dtype in _DTYPES:
+            out = _lib.native().dist_from_logits(logits, spatial_shapes, level_start_index, num_pixels,
+                                                 _ACTS[activation], _DTYPES[dtype])
+            if out is not NotImplemented:
+                return out
+        return super().apply(logits, spatial_shapes, level_start_index, num_pixels, activation, dtype)
 
 
 def depth_distribution(logits, spatial_shapes=None, level_start_index=None, num_pixels=None,

@@ -27,7 +27,35 @@ that recomputes the depth scores instead of re-reading them.
 import torch
 from torch.autograd.function import Function, once_differentiable
 
+from . import _lib
 from . import ext as ext_module
+
+
+def _native_apply(name):
+    """Class decorator: ``apply`` first offers the call to the native host path (csrc/binding/dfa3d_torch.cpp),
+    which takes the plain case -- CUDA tensors of the usual types and layouts, no autocast, no functorch -- and
+    answers NotImplemented to anything else; the Python Function then runs, with its checks and messages.
+    Measured on 512 queries, forward + backward: 190 us a pass through the Python Function, of which 34 us are
+    kernels."""
+
+    def wrap(cls):
+        python_apply = cls.apply.__func__
+        fast = None
+
+        def apply(c, *args):
+            nonlocal fast
+            if c is cls:                        # a subclass may have overridden forward or backward
+                if fast is None:
+                    fast = getattr(_lib.native(), name)
+                out = fast(*args)
+                if out is not NotImplemented:
+                    return out
+            return python_apply(c, *args)
+
+        cls.apply = classmethod(apply)
+        return cls
+
+    return wrap
 
 
 def _grad_dtype(t):
@@ -35,6 +63,7 @@ def _grad_dtype(t):
     return torch.float64 if t.dtype == torch.float64 else torch.float32
 
 
+@_native_apply("depth_score")
 class MultiScaleDepthScoreSampleFunction(Function):
     @staticmethod
     def forward(ctx, value, value_spatial_shapes, value_level_start_index, sampling_locations,
@@ -60,6 +89,7 @@ class MultiScaleDepthScoreSampleFunction(Function):
         return grad_value, None, None, grad_sampling_loc, None
 
 
+@_native_apply("wms")
 class WeightedMultiScaleDeformableAttnFunction(Function):
     @staticmethod
     def forward(ctx, value, value_spatial_shapes, value_level_start_index, sampling_locations,
@@ -88,6 +118,7 @@ class WeightedMultiScaleDeformableAttnFunction(Function):
         return grad_value, None, None, grad_sampling_loc, grad_attn_weight, grad_depth_score, None
 
 
+@_native_apply("fused")
 class MultiScale3DDeformableAttnFunction(Function):
     @staticmethod
     def forward(ctx, value, value_dpt_dist, value_spatial_shapes, value_level_start_index,
@@ -130,6 +161,7 @@ class MultiScale3DDeformableAttnFunction(Function):
         return grad_value, grad_dist, None, None, grad_sampling_loc, grad_attn_weight, None, None, None
 
 
+@_native_apply("msda")
 class MultiScaleDeformableAttnFunction(Function):
     """Plain 2-D multi-scale deformable attention with the call signature BEVFormer_DFA3D uses for its
     temporal self-attention and decoder (…/bevformer/modules/multi_scale_deformable_attn_function.py:
@@ -161,6 +193,7 @@ class MultiScaleDeformableAttnFunction(Function):
         return grad_value, None, None, grad_sampling_loc, grad_attn_weight, None
 
 
+@_native_apply("attn3d")
 class DeformableAttn3DFromOffsetsFunction(Function):
     """The one-stage operator fed with what the attention module's Linear layers produce: reference
     points, raw sampling offsets (pixels / depth bins) and raw attention logits.  The division by the
@@ -198,6 +231,7 @@ class DeformableAttn3DFromOffsetsFunction(Function):
         return grad_value, grad_dist, None, None, None, grad_uv, grad_d, grad_logits, None
 
 
+@_native_apply("fused_ragged")
 class MultiScale3DDeformableAttnRaggedFunction(Function):
     """The one-stage operator for cameras with different numbers of queries: sampling_locations
     (R,H,L,P,3) and attention_weights (R,H,L,P) are packed rows, camera b owning rows
@@ -239,6 +273,7 @@ class MultiScale3DDeformableAttnRaggedFunction(Function):
                 None)
 
 
+@_native_apply("attn3d_ragged")
 class DeformableAttn3DFromOffsetsRaggedFunction(Function):
     """DeformableAttn3DFromOffsetsFunction on packed rows: reference_points (R,Z,3),
     sampling_offsets_uv (R,H,L,P,2), sampling_offsets_depth (R,H,L,P), attention_logits (R,H,L*P);
@@ -275,30 +310,31 @@ class DeformableAttn3DFromOffsetsRaggedFunction(Function):
         return grad_value, grad_dist, None, None, None, grad_uv, grad_d, grad_logits, None, None, None
 
 
-def _fp32_variant(cls, name):
+def _fp32_variant(cls, name, native):
     """Same Function with inputs cast to float32 when autocast is active."""
     fwd = torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float32)(cls.forward)
     bwd = torch.amp.custom_bwd(device_type="cuda")(cls.backward)
-    return type(name, (Function,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)})
+    return _native_apply(native)(
+        type(name, (Function,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)}))
 
 
 MultiScaleDepthScoreSampleFunction_fp32 = _fp32_variant(
-    MultiScaleDepthScoreSampleFunction, "MultiScaleDepthScoreSampleFunction_fp32")
+    MultiScaleDepthScoreSampleFunction, "MultiScaleDepthScoreSampleFunction_fp32", "depth_score")
 WeightedMultiScaleDeformableAttnFunction_fp32 = _fp32_variant(
-    WeightedMultiScaleDeformableAttnFunction, "WeightedMultiScaleDeformableAttnFunction_fp32")
+    WeightedMultiScaleDeformableAttnFunction, "WeightedMultiScaleDeformableAttnFunction_fp32", "wms")
 MultiScale3DDeformableAttnFunction_fp32 = _fp32_variant(
-    MultiScale3DDeformableAttnFunction, "MultiScale3DDeformableAttnFunction_fp32")
+    MultiScale3DDeformableAttnFunction, "MultiScale3DDeformableAttnFunction_fp32", "fused")
 MultiScaleDeformableAttnFunction_fp32 = _fp32_variant(
-    MultiScaleDeformableAttnFunction, "MultiScaleDeformableAttnFunction_fp32")
+    MultiScaleDeformableAttnFunction, "MultiScaleDeformableAttnFunction_fp32", "msda")
 DeformableAttn3DFromOffsetsFunction_fp32 = _fp32_variant(
-    DeformableAttn3DFromOffsetsFunction, "DeformableAttn3DFromOffsetsFunction_fp32")
+    DeformableAttn3DFromOffsetsFunction, "DeformableAttn3DFromOffsetsFunction_fp32", "attn3d")
 MultiScale3DDeformableAttnRaggedFunction_fp32 = _fp32_variant(
-    MultiScale3DDeformableAttnRaggedFunction, "MultiScale3DDeformableAttnRaggedFunction_fp32")
+    MultiScale3DDeformableAttnRaggedFunction, "MultiScale3DDeformableAttnRaggedFunction_fp32", "fused_ragged")
 DeformableAttn3DFromOffsetsRaggedFunction_fp32 = _fp32_variant(
-    DeformableAttn3DFromOffsetsRaggedFunction, "DeformableAttn3DFromOffsetsRaggedFunction_fp32")
+    DeformableAttn3DFromOffsetsRaggedFunction, "DeformableAttn3DFromOffsetsRaggedFunction_fp32", "attn3d_ragged")
 
 
-def _fp16_variant(cls, name, storage):
+def _fp16_variant(cls, name, storage, native=None):
     """Half-precision variant of `cls`.  `storage` = positions of the tensors that stay half for the kernels
     (value, value_dpt_dist); every other half tensor is widened to float32 first, and when any argument was
     half the outputs are returned as half.  Gradients are computed in float32; autograd casts them to the
@@ -327,14 +363,16 @@ def _fp16_variant(cls, name, storage):
 
     fwd = torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float16)(forward)
     bwd = torch.amp.custom_bwd(device_type="cuda")(backward)
-    return type(name, (Function,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)})
+    variant = type(name, (Function,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)})
+    return variant if native is None else _native_apply(native)(variant)
 
 
 MultiScaleDepthScoreSampleFunction_fp16 = _fp16_variant(
     MultiScaleDepthScoreSampleFunction, "MultiScaleDepthScoreSampleFunction_fp16", (0,))
 WeightedMultiScaleDeformableAttnFunction_fp16 = _fp16_variant(
-    WeightedMultiScaleDeformableAttnFunction, "WeightedMultiScaleDeformableAttnFunction_fp16", (0,))
+    WeightedMultiScaleDeformableAttnFunction, "WeightedMultiScaleDeformableAttnFunction_fp16", (0,),
+    "wms_fp16")
 MultiScale3DDeformableAttnFunction_fp16 = _fp16_variant(
-    MultiScale3DDeformableAttnFunction, "MultiScale3DDeformableAttnFunction_fp16", (0, 1))
+    MultiScale3DDeformableAttnFunction, "MultiScale3DDeformableAttnFunction_fp16", (0, 1), "fused_fp16")
 MultiScaleDeformableAttnFunction_fp16 = _fp16_variant(
-    MultiScaleDeformableAttnFunction, "MultiScaleDeformableAttnFunction_fp16", (0,))
+    MultiScaleDeformableAttnFunction, "MultiScaleDeformableAttnFunction_fp16", (0,), "msda_fp16")

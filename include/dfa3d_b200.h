@@ -322,6 +322,10 @@ int dfa3d_layer_norm_backward(const float *grad_y, const float *in, const float 
  * aligned like src. */
 int dfa3d_column_sum(const float *src, int64_t rows, int32_t cols, float *dst, void *stream);
 
+/* a[0..na) = 0 and b[0..nb) = 0 with one launch: the two gradients a backward accumulates into.  Either
+ * count may be 0 (its pointer is then not looked at); pointers 16-byte aligned. */
+int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
