@@ -45,7 +45,7 @@ using torch::autograd::variable_list;
   X(dfa3d_wms_attn_forward) X(dfa3d_wms_attn_backward) X(dfa3d_fused_forward) X(dfa3d_fused_backward)    \
   X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward) X(dfa3d_attn3d_backward)          \
   X(dfa3d_fused_forward_ragged) X(dfa3d_fused_backward_ragged) X(dfa3d_attn3d_forward_ragged)            \
-  X(dfa3d_attn3d_backward_ragged) X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward)           \
+  X(dfa3d_attn3d_backward_ragged) X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward_typed)           \
   X(dfa3d_zero_two)
 
 struct Abi {
@@ -464,12 +464,12 @@ struct DistFn : torch::autograd::Function<DistFn> {
     const Tensor &logits = v[0];
     const auto a = c10::static_intrusive_pointer_cast<DistArgs>(ctx->saved_data.at("x").toCapsule());
     c10::cuda::CUDAGuard guard(logits.device());
-    const Tensor go = f32(grads[0]);
+    const Tensor go = storage_type(grads[0].scalar_type()) ? grads[0].contiguous() : f32(grads[0]);
     Tensor gl = at::empty_like(logits);
-    check(abi.dfa3d_dist_from_logits_backward(fp(logits), (int32_t)logits.size(0), (int32_t)logits.size(1),
+    check(abi.dfa3d_dist_from_logits_backward_typed(fp(logits), (int32_t)logits.size(0), (int32_t)logits.size(1),
                                               (int32_t)logits.size(2), (int32_t)logits.size(3), lp(v[1]),
                                               (int32_t)v[1].size(1), lp(v[2]), (int32_t)v[1].size(0), a->N, a->act,
-                                              fp(go), fpm(gl), stream_of(logits)),
+                                              dtype_code(go), go.const_data_ptr(), fpm(gl), stream_of(logits)),
           "dfa3d_dist_from_logits_backward");
     return once({gl, Tensor(), Tensor(), Tensor(), Tensor()}, grads);
   }

@@ -459,20 +459,31 @@ int dfa3d_dist_from_logits(const float *logits, int32_t B, int32_t D, int32_t ma
                 "dfa3d_dist_from_logits launch");
 }
 
+int dfa3d_dist_from_logits_backward_typed(const float *logits, int32_t B, int32_t D, int32_t map_h, int32_t map_w,
+                                          const int64_t *spatial_shapes, int32_t shape_stride,
+                                          const int64_t *level_start, int32_t L, int32_t N, int32_t activation,
+                                          int32_t grad_dtype, const void *grad_dist, float *grad_logits,
+                                          void *stream) {
+  if (int rc = check_producer(B, D, map_h, map_w, shape_stride, L, N, activation)) return rc;
+  if (grad_dtype != DFA3D_DTYPE_F32 && grad_dtype != DFA3D_DTYPE_BF16 && grad_dtype != DFA3D_DTYPE_F16)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "grad_dtype %d is not a DFA3D_DTYPE_*", grad_dtype);
+  if (B == 0) return DFA3D_OK;
+  REQUIRE_PTR(logits); REQUIRE_PTR(spatial_shapes); REQUIRE_PTR(level_start); REQUIRE_PTR(grad_logits);
+  if (N > 0) REQUIRE_PTR(grad_dist);
+  return finish(dfa3d::launch_dist_from_logits_backward(logits, spatial_shapes, shape_stride, level_start,
+                                                        grad_dist, grad_dtype, grad_logits, B, D, map_h, map_w, N, L,
+                                                        activation == DFA3D_ACT_SIGMOID,
+                                                        (cudaStream_t)stream),
+                "dfa3d_dist_from_logits_backward launch");
+}
+
 int dfa3d_dist_from_logits_backward(const float *logits, int32_t B, int32_t D, int32_t map_h,
                                     int32_t map_w, const int64_t *spatial_shapes, int32_t shape_stride,
                                     const int64_t *level_start, int32_t L, int32_t N,
                                     int32_t activation, const float *grad_dist, float *grad_logits,
                                     void *stream) {
-  if (int rc = check_producer(B, D, map_h, map_w, shape_stride, L, N, activation)) return rc;
-  if (B == 0) return DFA3D_OK;
-  REQUIRE_PTR(logits); REQUIRE_PTR(spatial_shapes); REQUIRE_PTR(level_start); REQUIRE_PTR(grad_logits);
-  if (N > 0) REQUIRE_PTR(grad_dist);
-  return finish(dfa3d::launch_dist_from_logits_backward(logits, spatial_shapes, shape_stride, level_start,
-                                                        grad_dist, grad_logits, B, D, map_h, map_w, N, L,
-                                                        activation == DFA3D_ACT_SIGMOID,
-                                                        (cudaStream_t)stream),
-                "dfa3d_dist_from_logits_backward launch");
+  return dfa3d_dist_from_logits_backward_typed(logits, B, D, map_h, map_w, spatial_shapes, shape_stride, level_start, L,
+                                               N, activation, DFA3D_DTYPE_F32, grad_dist, grad_logits, stream);
 }
 
 // ---- encoder-layer row operations --------------------------------------------------------------

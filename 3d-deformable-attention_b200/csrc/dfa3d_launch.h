@@ -48,7 +48,7 @@ cudaError_t launch_dist_from_logits(const float *logits, const int64_t *shapes, 
                                     const int64_t *lsi, void *dist, int dist_dtype, int B, int D, int hs,
                                     int ws, int N, int L, bool sigmoid, cudaStream_t s);
 cudaError_t launch_dist_from_logits_backward(const float *logits, const int64_t *shapes, int shape_stride,
-                                             const int64_t *lsi, const float *grad_dist,
+                                             const int64_t *lsi, const void *grad_dist, int grad_dtype,
                                              float *grad_logits, int B, int D, int hs, int ws, int N,
                                              int L, bool sigmoid, cudaStream_t s);
 // encoder-layer row operations (dfa3d_layer_ops.cu); E = columns of a row, a multiple of 4 up to 1024

@@ -74,6 +74,9 @@ PLAIN_ENTRY_POINTS = {
                               + [_I32] * 4 + [ctypes.c_void_p] * 2,
     "dfa3d_dist_from_logits_backward": [ctypes.c_void_p] + [_I32] * 4 + [ctypes.c_void_p, _I32, ctypes.c_void_p]
                                        + [_I32] * 3 + [ctypes.c_void_p] * 3,
+    "dfa3d_dist_from_logits_backward_typed": [ctypes.c_void_p] + [_I32] * 4
+                                             + [ctypes.c_void_p, _I32, ctypes.c_void_p] + [_I32] * 4
+                                             + [ctypes.c_void_p] * 3,
     "dfa3d_add_layer_norm_forward": [ctypes.c_void_p] * 4 + [_I64, _I32, ctypes.c_float] + [ctypes.c_void_p] * 5,
     "dfa3d_layer_norm_backward": [ctypes.c_void_p] * 5 + [_I64, _I32] + [ctypes.c_void_p] * 4,
     "dfa3d_column_sum": [ctypes.c_void_p, _I64, _I32, ctypes.c_void_p, ctypes.c_void_p],

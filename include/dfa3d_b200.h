@@ -264,6 +264,13 @@ int dfa3d_dist_from_logits_backward(const float *logits, int32_t B, int32_t D, i
                                     int32_t activation, const float *grad_dist, float *grad_logits,
                                     void *stream);
 
+/* The same with grad_dist in any storage type of dist (grad_dtype: DFA3D_DTYPE_F32, _BF16 or _F16). */
+int dfa3d_dist_from_logits_backward_typed(const float *logits, int32_t B, int32_t D, int32_t map_h, int32_t map_w,
+                                          const int64_t *spatial_shapes, int32_t shape_stride,
+                                          const int64_t *level_start, int32_t L, int32_t N, int32_t activation,
+                                          int32_t grad_dtype, const void *grad_dist, float *grad_logits,
+                                          void *stream);
+
 /* Double precision.  The reference instantiates its kernels for float and double
  * (AT_DISPATCH_FLOATING_TYPES, DFA3D/dfa3D/ops/csrc/cuda/wms_deform_attn_cuda.cu:267,344 and
  * cuda/ms_depth_score_sample_cuda.cu:94,184).  The *_f64 entry points are the double instantiations of
