@@ -16,7 +16,7 @@ SOURCES = ["dfa3d_forward.cu", "dfa3d_backward.cu", "dfa3d_rebatch.cu", "dfa3d_d
            "dfa3d_fp64.cu", "dfa3d_layer_ops.cu", "dfa3d_capi.cu"]
 RATES_SRC = os.path.join(CSRC, "rates", "dfa3d_rates.cu")
 RATES_OUT = os.path.join(HERE, "dfa3d_b200", "libdfa3d_rates.so")
-NATIVE_SRC = os.path.join(CSRC, "binding", "dfa3d_torch.cpp")
+NATIVE_SRC = [os.path.join(CSRC, "binding", f) for f in ("dfa3d_torch.cpp", "dfa3d_torch_layers.cpp")]
 NATIVE_OUT = os.path.join(HERE, "dfa3d_b200", "_native.so")
 INCLUDE = os.path.join(HERE, "..", "include")
 NVCC_FLAGS = ["-O3", "-I", INCLUDE, "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,7 +40,7 @@ def _native_command():
     lib = os.path.join(root, "lib")
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
-            *[a for i in inc for a in ("-isystem", i)], NATIVE_SRC, "-o", NATIVE_OUT, "-L", lib,
+            *[a for i in inc for a in ("-isystem", i)], *NATIVE_SRC, "-o", NATIVE_OUT, "-L", lib,
             "-Wl,-rpath," + lib, "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
@@ -91,7 +91,7 @@ def build(force=False, verbose=False):
         raise RuntimeError(f"nvcc failed on dfa3d_rates.cu:\n{log[-4000:]}")
     log, _ = native.communicate()
     if native.returncode != 0:
-        raise RuntimeError(f"g++ failed on dfa3d_torch.cpp:\n{log[-4000:]}")
+        raise RuntimeError(f"g++ failed on csrc/binding:\n{log[-4000:]}")
     return OUT
 
 

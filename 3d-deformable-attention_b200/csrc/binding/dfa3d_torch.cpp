@@ -13,199 +13,11 @@
 //
 // Kernels are reached through the C ABI (include/dfa3d_b200.h) of the library the Python side has loaded:
 // bind() receives the entry points' addresses.
-#include <torch/csrc/autograd/custom_function.h>
-#include <torch/csrc/autograd/functions/basic_ops.h>
-#include <torch/csrc/autograd/python_variable.h>
-#include <torch/csrc/Exceptions.h>
-#include <torch/csrc/utils/pybind.h>
+#include "dfa3d_torch.h"
 
-#include <ATen/ATen.h>
-#include <ATen/autocast_mode.h>
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/core/impl/LocalDispatchKeySet.h>
-#include <c10/core/impl/TorchDispatchModeTLS.h>
-#include <c10/cuda/CUDAGuard.h>
-
-#include <atomic>
-#include <optional>
-
-#include "dfa3d_b200.h"
+using namespace dfa3d_torch;
 
 namespace {
-
-using at::Tensor;
-using torch::autograd::AutogradContext;
-using torch::autograd::variable_list;
-
-// ------------------------------------------------------------------------------------------------
-// the C ABI
-// ------------------------------------------------------------------------------------------------
-#define DFA3D_ENTRIES(X)                                                                                 \
-  X(dfa3d_last_error) X(dfa3d_depth_score_forward) X(dfa3d_depth_score_backward)                         \
-  X(dfa3d_wms_attn_forward) X(dfa3d_wms_attn_backward) X(dfa3d_fused_forward) X(dfa3d_fused_backward)    \
-  X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward) X(dfa3d_attn3d_backward)          \
-  X(dfa3d_fused_forward_ragged) X(dfa3d_fused_backward_ragged) X(dfa3d_attn3d_forward_ragged)            \
-  X(dfa3d_attn3d_backward_ragged) X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward_typed)           \
-  X(dfa3d_zero_two)
-
-struct Abi {
-#define X(name) decltype(&::name) name = nullptr;
-  DFA3D_ENTRIES(X)
-#undef X
-} abi;
-
-bool bound = false;
-std::atomic<long long> calls{0};      // successful entry-point calls
-
-void check(int rc, const char *what) {
-  if (rc == DFA3D_OK) {
-    calls.fetch_add(1, std::memory_order_relaxed);
-    return;
-  }
-  const char *kind = rc == DFA3D_ERR_INVALID_ARGUMENT ? "invalid argument"
-                     : rc == DFA3D_ERR_UNSUPPORTED    ? "unsupported"
-                                                      : "CUDA error";
-  TORCH_CHECK(false, what, " failed (", kind, "): ", abi.dfa3d_last_error());
-}
-
-void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-
-// ------------------------------------------------------------------------------------------------
-// arguments
-// ------------------------------------------------------------------------------------------------
-// Modes in which the Python Function does something of its own.
-bool plain_mode() {
-  return bound && !at::autocast::is_autocast_enabled(at::kCUDA) &&
-         !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
-         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
-}
-
-bool storage_type(at::ScalarType t) { return t == at::kFloat || t == at::kBFloat16 || t == at::kHalf; }
-
-int dtype_code(const Tensor &t) {
-  return t.scalar_type() == at::kHalf ? DFA3D_DTYPE_F16 : t.scalar_type() == at::kBFloat16 ? DFA3D_DTYPE_BF16 : DFA3D_DTYPE_F32;
-}
-
-// A plain contiguous CUDA tensor without forward-mode tangent.
-bool plain_tensor(PyObject *o, Tensor &t) {
-  if (!THPVariable_Check(o)) return false;
-  t = THPVariable_Unpack(o);
-  return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
-         !t._fw_grad(0).defined();
-}
-
-bool float_tensor(PyObject *o, Tensor &t, int64_t dim) {
-  return plain_tensor(o, t) && t.scalar_type() == at::kFloat && (dim < 0 || t.dim() == dim);
-}
-
-bool long_tensor(PyObject *o, Tensor &t, int64_t dim) {
-  return plain_tensor(o, t) && t.scalar_type() == at::kLong && t.dim() == dim;
-}
-
-bool integer(PyObject *o, int64_t &v) {
-  if (!PyLong_CheckExact(o)) return false;
-  v = PyLong_AsLongLong(o);
-  if (v == -1 && PyErr_Occurred()) {
-    PyErr_Clear();
-    return false;
-  }
-  return true;
-}
-
-// None, or a pair of positive integers
-bool map_argument(PyObject *o, int64_t &h, int64_t &w) {
-  h = w = 0;
-  if (o == Py_None) return true;
-  return PyTuple_CheckExact(o) && PyTuple_GET_SIZE(o) == 2 && integer(PyTuple_GET_ITEM(o, 0), h) &&
-         integer(PyTuple_GET_ITEM(o, 1), w) && h > 0 && w > 0 && h < (1 << 24) && w < (1 << 24);
-}
-
-// `batch % min(batch, im2col_step)`, as the reference demands
-bool step_divides(PyObject *o, int64_t batch) {
-  int64_t step;
-  if (!integer(o, step) || step <= 0) return false;
-  return batch == 0 || batch % std::min(batch, step) == 0;
-}
-
-bool small(const Tensor &t) {      // every size fits the descriptor's int32 fields
-  for (int64_t s : t.sizes())
-    if (s >= (int64_t(1) << 31)) return false;
-  return true;
-}
-
-template <typename... T>
-bool one_device(const Tensor &a, const T &...more) {
-  return ((more.device() == a.device()) && ...);
-}
-
-bool sizes_are(const Tensor &t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s); }
-
-// value (B,N,H,C) and dist (B,Nd,H,D) | (B,Nd,D): fills the descriptor's fields that follow from them.
-bool describe_dist(const Tensor &dist, int64_t B, int64_t N, int64_t H, int64_t mh, int64_t mw, dfa3d_problem &p) {
-  if (dist.dim() != 3 && dist.dim() != 4) return false;
-  if (dist.dim() == 4 && dist.size(2) != H) return false;
-  const int64_t D = dist.size(-1);
-  if (dist.size(0) != B || dist.size(1) != (mh ? mh * mw : N)) return false;
-  p.D = (int32_t)D;
-  p.dist_dtype = dtype_code(dist);
-  p.dist_head_stride = dist.dim() == 4 ? D : 0;
-  p.dist_map_h = (int32_t)mh;
-  p.dist_map_w = (int32_t)mw;
-  return true;
-}
-
-void describe_value(const Tensor &value, dfa3d_problem &p) {
-  p.B = (int32_t)value.size(0); p.N = (int32_t)value.size(1);
-  p.H = (int32_t)value.size(2); p.C = (int32_t)value.size(3);
-  p.value_dtype = dtype_code(value);
-}
-
-Tensor empty_f32(at::IntArrayRef sizes, const Tensor &like) {
-  return at::empty(sizes, like.options().dtype(at::kFloat));
-}
-
-// Two zeroed float32 gradients (the second may be undefined), one launch for both.
-void zero_two(const Tensor &a, const Tensor &b, void *s) {
-  check(abi.dfa3d_zero_two(a.data_ptr<float>(), a.numel(), b.defined() ? b.data_ptr<float>() : nullptr,
-                           b.defined() ? b.numel() : 0, s),
-        "dfa3d_zero_two");
-  calls.fetch_sub(1, std::memory_order_relaxed);
-}
-
-const float *fp(const Tensor &t) { return static_cast<const float *>(t.const_data_ptr()); }
-float *fpm(const Tensor &t) { return static_cast<float *>(t.mutable_data_ptr()); }
-const int64_t *lp(const Tensor &t) { return static_cast<const int64_t *>(t.const_data_ptr()); }
-const int32_t *ip(const Tensor &t) { return static_cast<const int32_t *>(t.const_data_ptr()); }
-
-// float32 and contiguous, whatever the consumer of the result handed back
-Tensor f32(const Tensor &g) { return (g.scalar_type() == at::kFloat ? g : g.to(at::kFloat)).contiguous(); }
-
-// Gradients of a backward that must not be differentiated again: with create_graph the results get a node that
-// says so when it is reached (torch.autograd.function.once_differentiable does the same).
-variable_list once(variable_list out, const variable_list &grads) {
-  if (!at::GradMode::is_enabled()) return out;
-  bool any = false;
-  for (const auto &g : grads) any |= g.defined() && g.requires_grad();
-  if (!any) return out;
-  std::vector<size_t> where;
-  variable_list in;
-  for (size_t i = 0; i < out.size(); ++i)
-    if (out[i].defined()) {
-      where.push_back(i);
-      in.push_back(out[i].detach().requires_grad_(true));
-    }
-  auto err = std::make_shared<torch::autograd::DelayedError>(
-      "trying to differentiate twice a function that was marked with @once_differentiable", (int64_t)in.size());
-  auto res = (*err)(std::move(in));
-  for (size_t i = 0; i < where.size(); ++i) out[where[i]] = res[i];
-  return out;
-}
-
-// A gradient that flows into the returned depth_score is not supported (as in the reference): zero is tolerated.
-void refuse_score_gradient(const Tensor &g) {
-  TORCH_CHECK_NOT_IMPLEMENTED(!g.defined() || g.sum().item<double>() == 0.0,
-                              "no gradient can flow into the returned depth_score");
-}
 
 // ------------------------------------------------------------------------------------------------
 // autograd nodes; what they keep beside their tensors travels in one capsule
@@ -241,11 +53,11 @@ variable_list fused_forward(const dfa3d_problem &p, const Tensor &value, const T
   void *s = stream_of(value);
   float *ds = need_score ? fpm(score) : nullptr;
   if (ragged)
-    check(abi.dfa3d_fused_forward_ragged(&p, ip(q_off), value.const_data_ptr(), dist.const_data_ptr(), lp(shapes),
+    check(lib.dfa3d_fused_forward_ragged(&p, ip(q_off), value.const_data_ptr(), dist.const_data_ptr(), lp(shapes),
                                          lp(lsi), fp(loc), fp(attn), fpm(out), ds, s),
           "dfa3d_fused_forward_ragged");
   else
-    check(abi.dfa3d_fused_forward(&p, value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(loc),
+    check(lib.dfa3d_fused_forward(&p, value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(loc),
                                   fp(attn), fpm(out), ds, s),
           "dfa3d_fused_forward");
   return {out, score};
@@ -280,11 +92,11 @@ struct FusedFn : torch::autograd::Function<FusedFn> {
     void *s = stream_of(value);
     zero_two(gv, gd, s);
     if (q_off.defined())
-      check(abi.dfa3d_fused_backward_ragged(&x->p, ip(q_off), value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]),
+      check(lib.dfa3d_fused_backward_ragged(&x->p, ip(q_off), value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]),
                                             lp(v[3]), fp(loc), fp(attn), fp(go), fpm(gv), fpm(gd), fpm(gl), fpm(ga), s),
             "dfa3d_fused_backward_ragged");
     else
-      check(abi.dfa3d_fused_backward(&x->p, value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(loc),
+      check(lib.dfa3d_fused_backward(&x->p, value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(loc),
                                      fp(attn), fp(go), fpm(gv), fpm(gd), fpm(gl), fpm(ga), s),
             "dfa3d_fused_backward");
     return once({gv, gd, Tensor(), Tensor(), gl, ga, Tensor(), Tensor(), Tensor()}, grads);
@@ -301,14 +113,10 @@ Tensor attn3d_forward(const Extra &x, const Tensor &value, const Tensor &dist, c
   Tensor out = ragged ? empty_f32({uv.size(0), (int64_t)p.H * p.C}, value)
                       : empty_f32({uv.size(0), uv.size(1), (int64_t)p.H * p.C}, value);
   void *s = stream_of(value);
-  if (ragged)
-    check(abi.dfa3d_attn3d_forward_ragged(&p, (int32_t)x.Z, ip(q_off), value.const_data_ptr(), dist.const_data_ptr(),
-                                          lp(shapes), lp(lsi), fp(ref), fp(uv), fp(od), fp(logits), fpm(out), s),
-          "dfa3d_attn3d_forward_ragged");
-  else
-    check(abi.dfa3d_attn3d_forward(&p, (int32_t)x.Z, value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi),
-                                   fp(ref), fp(uv), fp(od), fp(logits), fpm(out), s),
-          "dfa3d_attn3d_forward");
+  check(lib.dfa3d_attn3d_forward_levels(&p, (int32_t)x.Z, (int32_t)shapes.size(1), ragged ? ip(q_off) : nullptr,
+                                        value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(uv),
+                                        fp(od), fp(logits), fpm(out), s),
+        "dfa3d_attn3d_forward");
   return out;
 }
 
@@ -333,16 +141,11 @@ struct Attn3dFn : torch::autograd::Function<Attn3dFn> {
     Tensor guv = at::empty_like(uv), god = at::empty_like(od), gl = at::empty_like(logits);
     void *s = stream_of(value);
     zero_two(gv, gd, s);
-    if (q_off.defined())
-      check(abi.dfa3d_attn3d_backward_ragged(&x->p, (int32_t)x->Z, ip(q_off), value.const_data_ptr(),
-                                             dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(v[4]), fp(uv), fp(od),
-                                             fp(logits), fp(go), fpm(gv), fpm(gd), fpm(guv), fpm(god), fpm(gl), s),
-            "dfa3d_attn3d_backward_ragged");
-    else
-      check(abi.dfa3d_attn3d_backward(&x->p, (int32_t)x->Z, value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]),
-                                      lp(v[3]), fp(v[4]), fp(uv), fp(od), fp(logits), fp(go), fpm(gv), fpm(gd),
-                                      fpm(guv), fpm(god), fpm(gl), s),
-            "dfa3d_attn3d_backward");
+    check(lib.dfa3d_attn3d_backward_levels(&x->p, (int32_t)x->Z, (int32_t)v[2].size(1), q_off.defined() ? ip(q_off) : nullptr,
+                                           value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(v[4]),
+                                           fp(uv), fp(od), fp(logits), fp(go), fpm(gv), fpm(gd), fpm(guv), fpm(god), fpm(gl),
+                                           s),
+          "dfa3d_attn3d_backward");
     return once({gv, gd, Tensor(), Tensor(), Tensor(), guv, god, gl, Tensor(), Tensor()}, grads);
   }
 };
@@ -354,11 +157,11 @@ Tensor attn2d_forward(const dfa3d_problem &p, const Tensor &value, const Tensor 
   Tensor out = empty_f32({loc.size(0), loc.size(1), (int64_t)p.H * p.C}, value);
   void *s = stream_of(value);
   if (score.defined())
-    check(abi.dfa3d_wms_attn_forward(&p, value.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fp(attn), fp(score),
+    check(lib.dfa3d_wms_attn_forward(&p, value.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fp(attn), fp(score),
                                      fpm(out), s),
           "dfa3d_wms_attn_forward");
   else
-    check(abi.dfa3d_msda_forward(&p, value.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fp(attn), fpm(out), s),
+    check(lib.dfa3d_msda_forward(&p, value.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fp(attn), fpm(out), s),
           "dfa3d_msda_forward");
   return out;
 }
@@ -385,11 +188,11 @@ struct Attn2dFn : torch::autograd::Function<Attn2dFn> {
     zero_two(gv, Tensor(), s);
     if (score.defined()) {
       gs = at::empty_like(score);
-      check(abi.dfa3d_wms_attn_backward(&x->p, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(attn), fp(score),
+      check(lib.dfa3d_wms_attn_backward(&x->p, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(attn), fp(score),
                                         fp(go), fpm(gv), fpm(gl), fpm(ga), fpm(gs), s),
             "dfa3d_wms_attn_backward");
     } else {
-      check(abi.dfa3d_msda_backward(&x->p, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(attn), fp(go),
+      check(lib.dfa3d_msda_backward(&x->p, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(attn), fp(go),
                                     fpm(gv), fpm(gl), fpm(ga), s),
             "dfa3d_msda_backward");
     }
@@ -404,7 +207,7 @@ Tensor depth_score_forward(const dfa3d_problem &p, const Tensor &dist, const Ten
   std::vector<int64_t> sz(loc.sizes().begin(), loc.sizes().end());
   sz.back() = 4;
   Tensor out = empty_f32(sz, dist);
-  check(abi.dfa3d_depth_score_forward(&p, dist.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fpm(out),
+  check(lib.dfa3d_depth_score_forward(&p, dist.const_data_ptr(), lp(shapes), lp(lsi), fp(loc), fpm(out),
                                       stream_of(dist)),
         "dfa3d_depth_score_forward");
   return out;
@@ -427,7 +230,7 @@ struct DepthScoreFn : torch::autograd::Function<DepthScoreFn> {
     Tensor gd = empty_f32(dist.sizes(), dist), gl = at::empty_like(loc);
     void *s = stream_of(dist);
     zero_two(gd, Tensor(), s);
-    check(abi.dfa3d_depth_score_backward(&x->p, dist.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(go), fpm(gd),
+    check(lib.dfa3d_depth_score_backward(&x->p, dist.const_data_ptr(), lp(v[1]), lp(v[2]), fp(loc), fp(go), fpm(gd),
                                          fpm(gl), s),
           "dfa3d_depth_score_backward");
     return once({gd, Tensor(), Tensor(), gl, Tensor()}, grads);
@@ -444,7 +247,7 @@ Tensor dist_forward(const DistArgs &a, const Tensor &logits, const Tensor &shape
   c10::cuda::CUDAGuard guard(logits.device());
   const int32_t B = (int32_t)logits.size(0), D = (int32_t)logits.size(1);
   Tensor dist = at::empty({B, a.N, D}, logits.options().dtype(type));
-  check(abi.dfa3d_dist_from_logits(fp(logits), B, D, (int32_t)logits.size(2), (int32_t)logits.size(3), lp(shapes),
+  check(lib.dfa3d_dist_from_logits(fp(logits), B, D, (int32_t)logits.size(2), (int32_t)logits.size(3), lp(shapes),
                                    (int32_t)shapes.size(1), lp(lsi), (int32_t)shapes.size(0), a.N, a.act, a.dtype,
                                    dist.mutable_data_ptr(), stream_of(logits)),
         "dfa3d_dist_from_logits");
@@ -466,7 +269,7 @@ struct DistFn : torch::autograd::Function<DistFn> {
     c10::cuda::CUDAGuard guard(logits.device());
     const Tensor go = storage_type(grads[0].scalar_type()) ? grads[0].contiguous() : f32(grads[0]);
     Tensor gl = at::empty_like(logits);
-    check(abi.dfa3d_dist_from_logits_backward_typed(fp(logits), (int32_t)logits.size(0), (int32_t)logits.size(1),
+    check(lib.dfa3d_dist_from_logits_backward_typed(fp(logits), (int32_t)logits.size(0), (int32_t)logits.size(1),
                                               (int32_t)logits.size(2), (int32_t)logits.size(3), lp(v[1]),
                                               (int32_t)v[1].size(1), lp(v[2]), (int32_t)v[1].size(0), a->N, a->act,
                                               dtype_code(go), go.const_data_ptr(), fpm(gl), stream_of(logits)),
@@ -480,13 +283,6 @@ struct DistFn : torch::autograd::Function<DistFn> {
 // ------------------------------------------------------------------------------------------------
 // torch::autograd::Function takes tensors that may be absent as optionals
 std::optional<Tensor> given(const Tensor &t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; }
-
-PyObject *not_plain() { Py_RETURN_NOTIMPLEMENTED; }
-
-template <typename... T>
-bool wants_grad(const T &...t) {
-  return at::GradMode::is_enabled() && (t.requires_grad() || ...);
-}
 
 // (out, score or None)
 PyObject *pair(const variable_list &r) {
@@ -571,7 +367,8 @@ PyObject *run_fused(PyObject *const *a, Py_ssize_t n, bool ragged, bool fp16) {
   return pair(r);
 }
 
-PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged) {
+// flat: the level table may also be (L, 2), D bins in every level (what the attention module holds)
+PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged, bool flat) {
   // value, dist, shapes, lsi, ref, off_uv, off_d, logits [, q_off, max_queries] [, dist_map]
   const Py_ssize_t fixed = ragged ? 10 : 8;
   if (n < fixed || n > fixed + 1 || !plain_mode()) return not_plain();
@@ -588,8 +385,8 @@ PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged) {
     return not_plain();
   const int64_t B = value.size(0), H = value.size(2), L = uv.size(k + 1), P = uv.size(k + 2), Z = ref.size(k);
   const int64_t pts = uv.numel() / 2;
-  if (uv.size(-1) != 2 || uv.size(k) != H || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 || !sizes_are(shapes, {L, 3}) ||
-      lsi.size(0) != L || od.numel() != pts || logits.numel() != pts || ref.size(0) != uv.size(0))
+  if (uv.size(-1) != 2 || uv.size(k) != H || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 ||
+      !(sizes_are(shapes, {L, 3}) || (flat && sizes_are(shapes, {L, 2}))) || lsi.size(0) != L || od.numel() != pts || logits.numel() != pts || ref.size(0) != uv.size(0))
     return not_plain();
   auto x = c10::make_intrusive<Extra>();
   dfa3d_problem &p = x->p;
@@ -715,7 +512,7 @@ PyObject *py_bind(PyObject *, PyObject *table) {
     TORCH_CHECK(o != nullptr, "bind(): no address of ", name);
     return PyLong_AsVoidPtr(o);
   };
-#define X(name) abi.name = reinterpret_cast<decltype(abi.name)>(get(#name));
+#define X(name) lib.name = reinterpret_cast<decltype(lib.name)>(get(#name));
   DFA3D_ENTRIES(X)
 #undef X
   bound = true;
@@ -745,8 +542,10 @@ PyObject *py_calls(PyObject *, PyObject *) { return PyLong_FromLongLong(calls.lo
 FAST(fused, run_fused(a, n, false, false))
 FAST(fused_fp16, run_fused(a, n, false, true))
 FAST(fused_ragged, run_fused(a, n, true, false))
-FAST(attn3d, run_attn3d(a, n, false))
-FAST(attn3d_ragged, run_attn3d(a, n, true))
+FAST(attn3d, run_attn3d(a, n, false, false))
+FAST(attn3d_ragged, run_attn3d(a, n, true, false))
+FAST(attn3d_flat, run_attn3d(a, n, false, true))
+FAST(attn3d_ragged_flat, run_attn3d(a, n, true, true))
 FAST(wms, run_attn2d(a, n, true, false))
 FAST(wms_fp16, run_attn2d(a, n, true, true))
 FAST(msda, run_attn2d(a, n, false, false))
@@ -760,7 +559,7 @@ PyMethodDef methods[] = {
     {"bind", py_bind, METH_O, nullptr},
     {"entries", py_entries, METH_NOARGS, nullptr},
     {"calls", py_calls, METH_NOARGS, nullptr},
-    FAST(fused), FAST(fused_fp16), FAST(fused_ragged), FAST(attn3d), FAST(attn3d_ragged), FAST(wms), FAST(wms_fp16),
+    FAST(fused), FAST(fused_fp16), FAST(fused_ragged), FAST(attn3d), FAST(attn3d_ragged), FAST(attn3d_flat), FAST(attn3d_ragged_flat), FAST(wms), FAST(wms_fp16),
     FAST(msda), FAST(msda_fp16), FAST(depth_score), FAST(dist_from_logits),
     {nullptr, nullptr, 0, nullptr},
 };
@@ -770,4 +569,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native(void) {
+  PyObject *m = PyModule_Create(&module);
+  if (m && PyModule_AddFunctions(m, dfa3d_torch::layer_methods) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -1,0 +1,211 @@
+// What the two halves of the native host path share: the C ABI's entry points, argument checks and small helpers
+// (dfa3d_torch.cpp: the operator; dfa3d_torch_layers.cpp: the layer around it).
+#pragma once
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include <atomic>
+#include <optional>
+
+#include "dfa3d_b200.h"
+
+namespace dfa3d_torch {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// ------------------------------------------------------------------------------------------------
+// the C ABI
+// ------------------------------------------------------------------------------------------------
+#define DFA3D_ENTRIES(X)                                                                                 \
+  X(dfa3d_last_error) X(dfa3d_depth_score_forward) X(dfa3d_depth_score_backward)                         \
+  X(dfa3d_wms_attn_forward) X(dfa3d_wms_attn_backward) X(dfa3d_fused_forward) X(dfa3d_fused_backward)    \
+  X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward_levels) X(dfa3d_attn3d_backward_levels)          \
+  X(dfa3d_fused_forward_ragged) X(dfa3d_fused_backward_ragged) \
+  X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward_typed)           \
+  X(dfa3d_zero_two) X(dfa3d_attn2d_supported) X(dfa3d_attn2d_forward) X(dfa3d_attn2d_backward)           \
+  X(dfa3d_rebatch_gather) X(dfa3d_rebatch_combine) X(dfa3d_add_layer_norm_forward)                       \
+  X(dfa3d_add_layer_norm_infer) X(dfa3d_layer_norm_backward) X(dfa3d_column_sum)                         \
+  X(dfa3d_relu_backward_column_sum)
+
+struct Abi {
+#define X(name) decltype(&::name) name = nullptr;
+  DFA3D_ENTRIES(X)
+#undef X
+};
+inline Abi lib;
+
+inline bool bound = false;
+inline std::atomic<long long> calls{0};      // successful entry-point calls
+
+inline void check(int rc, const char *what) {
+  if (rc == DFA3D_OK) {
+    calls.fetch_add(1, std::memory_order_relaxed);
+    return;
+  }
+  const char *kind = rc == DFA3D_ERR_INVALID_ARGUMENT ? "invalid argument"
+                     : rc == DFA3D_ERR_UNSUPPORTED    ? "unsupported"
+                                                      : "CUDA error";
+  TORCH_CHECK(false, what, " failed (", kind, "): ", lib.dfa3d_last_error());
+}
+
+inline void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// ------------------------------------------------------------------------------------------------
+// arguments
+// ------------------------------------------------------------------------------------------------
+// Modes in which the Python Function does something of its own.
+inline bool plain_mode() {
+  return bound && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+         !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
+inline bool storage_type(at::ScalarType t) { return t == at::kFloat || t == at::kBFloat16 || t == at::kHalf; }
+
+inline int dtype_code(const Tensor &t) {
+  return t.scalar_type() == at::kHalf ? DFA3D_DTYPE_F16 : t.scalar_type() == at::kBFloat16 ? DFA3D_DTYPE_BF16 : DFA3D_DTYPE_F32;
+}
+
+// A plain contiguous CUDA tensor without forward-mode tangent.
+inline bool plain_tensor(PyObject *o, Tensor &t) {
+  if (!THPVariable_Check(o)) return false;
+  t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
+         !t._fw_grad(0).defined();
+}
+
+inline bool float_tensor(PyObject *o, Tensor &t, int64_t dim) {
+  return plain_tensor(o, t) && t.scalar_type() == at::kFloat && (dim < 0 || t.dim() == dim);
+}
+
+inline bool long_tensor(PyObject *o, Tensor &t, int64_t dim) {
+  return plain_tensor(o, t) && t.scalar_type() == at::kLong && t.dim() == dim;
+}
+
+inline bool integer(PyObject *o, int64_t &v) {
+  if (!PyLong_CheckExact(o)) return false;
+  v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
+  return true;
+}
+
+// None, or a pair of positive integers
+inline bool map_argument(PyObject *o, int64_t &h, int64_t &w) {
+  h = w = 0;
+  if (o == Py_None) return true;
+  return PyTuple_CheckExact(o) && PyTuple_GET_SIZE(o) == 2 && integer(PyTuple_GET_ITEM(o, 0), h) &&
+         integer(PyTuple_GET_ITEM(o, 1), w) && h > 0 && w > 0 && h < (1 << 24) && w < (1 << 24);
+}
+
+// `batch % min(batch, im2col_step)`, as the reference demands
+inline bool step_divides(PyObject *o, int64_t batch) {
+  int64_t step;
+  if (!integer(o, step) || step <= 0) return false;
+  return batch == 0 || batch % std::min(batch, step) == 0;
+}
+
+inline bool small(const Tensor &t) {      // every size fits the descriptor's int32 fields
+  for (int64_t s : t.sizes())
+    if (s >= (int64_t(1) << 31)) return false;
+  return true;
+}
+
+template <typename... T>
+bool one_device(const Tensor &a, const T &...more) {
+  return ((more.device() == a.device()) && ...);
+}
+
+inline bool sizes_are(const Tensor &t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s); }
+
+// value (B,N,H,C) and dist (B,Nd,H,D) | (B,Nd,D): fills the descriptor's fields that follow from them.
+inline bool describe_dist(const Tensor &dist, int64_t B, int64_t N, int64_t H, int64_t mh, int64_t mw, dfa3d_problem &p) {
+  if (dist.dim() != 3 && dist.dim() != 4) return false;
+  if (dist.dim() == 4 && dist.size(2) != H) return false;
+  const int64_t D = dist.size(-1);
+  if (dist.size(0) != B || dist.size(1) != (mh ? mh * mw : N)) return false;
+  p.D = (int32_t)D;
+  p.dist_dtype = dtype_code(dist);
+  p.dist_head_stride = dist.dim() == 4 ? D : 0;
+  p.dist_map_h = (int32_t)mh;
+  p.dist_map_w = (int32_t)mw;
+  return true;
+}
+
+inline void describe_value(const Tensor &value, dfa3d_problem &p) {
+  p.B = (int32_t)value.size(0); p.N = (int32_t)value.size(1);
+  p.H = (int32_t)value.size(2); p.C = (int32_t)value.size(3);
+  p.value_dtype = dtype_code(value);
+}
+
+inline Tensor empty_f32(at::IntArrayRef sizes, const Tensor &like) {
+  return at::empty(sizes, like.options().dtype(at::kFloat));
+}
+
+// Two zeroed float32 gradients (the second may be undefined), one launch for both.
+inline void zero_two(const Tensor &a, const Tensor &b, void *s) {
+  check(lib.dfa3d_zero_two(a.data_ptr<float>(), a.numel(), b.defined() ? b.data_ptr<float>() : nullptr,
+                           b.defined() ? b.numel() : 0, s),
+        "dfa3d_zero_two");
+  calls.fetch_sub(1, std::memory_order_relaxed);
+}
+
+inline const float *fp(const Tensor &t) { return static_cast<const float *>(t.const_data_ptr()); }
+inline float *fpm(const Tensor &t) { return static_cast<float *>(t.mutable_data_ptr()); }
+inline const int64_t *lp(const Tensor &t) { return static_cast<const int64_t *>(t.const_data_ptr()); }
+inline const int32_t *ip(const Tensor &t) { return static_cast<const int32_t *>(t.const_data_ptr()); }
+
+// float32 and contiguous, whatever the consumer of the result handed back
+inline Tensor f32(const Tensor &g) { return (g.scalar_type() == at::kFloat ? g : g.to(at::kFloat)).contiguous(); }
+
+// Gradients of a backward that must not be differentiated again: with create_graph the results get a node that
+// says so when it is reached (torch.autograd.function.once_differentiable does the same).
+inline variable_list once(variable_list out, const variable_list &grads) {
+  if (!at::GradMode::is_enabled()) return out;
+  bool any = false;
+  for (const auto &g : grads) any |= g.defined() && g.requires_grad();
+  if (!any) return out;
+  std::vector<size_t> where;
+  variable_list in;
+  for (size_t i = 0; i < out.size(); ++i)
+    if (out[i].defined()) {
+      where.push_back(i);
+      in.push_back(out[i].detach().requires_grad_(true));
+    }
+  auto err = std::make_shared<torch::autograd::DelayedError>(
+      "trying to differentiate twice a function that was marked with @once_differentiable", (int64_t)in.size());
+  auto res = (*err)(std::move(in));
+  for (size_t i = 0; i < where.size(); ++i) out[where[i]] = res[i];
+  return out;
+}
+
+// A gradient that flows into the returned depth_score is not supported (as in the reference): zero is tolerated.
+inline void refuse_score_gradient(const Tensor &g) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!g.defined() || g.sum().item<double>() == 0.0,
+                              "no gradient can flow into the returned depth_score");
+}
+
+template <typename... T>
+bool wants_grad(const T &...t) {
+  return at::GradMode::is_enabled() && (t.requires_grad() || ...);
+}
+
+inline PyObject *not_plain() { Py_RETURN_NOTIMPLEMENTED; }
+
+extern PyMethodDef layer_methods[];      // dfa3d_torch_layers.cpp, ends in a null entry
+
+}  // namespace dfa3d_torch

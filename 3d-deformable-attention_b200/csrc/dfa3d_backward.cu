@@ -118,14 +118,14 @@ __device__ __forceinline__ float bwd_point_epilogue(const KArgs &a, const ItemCt
       g_z = (float)s.g.Dd * acc;
     }
   }
-  if (MODE == kCallerFused) {
+  if (mode_from_offsets(MODE)) {
     // d loc / d offset = 1 / (W, H, D); the logit gradient needs the whole item's dot product and is
     // finished by finish_logit_grads(): park the attention gradient in its slot for now
     a.grad_logits[pt] = g_attn;
     float *gu = a.grad_off_uv + pt * 2;
     gu[0] = s.live ? __fdiv_rn(g_x, (float)s.g.W) : 0.f;
     gu[1] = s.live ? __fdiv_rn(g_y, (float)s.g.Hh) : 0.f;
-    a.grad_off_d[pt] = __fdiv_rn(g_z, (float)a.D);
+    if (MODE == kCallerFused) a.grad_off_d[pt] = __fdiv_rn(g_z, (float)a.D);
     return s.aw * g_attn;
   }
   a.grad_attn[pt] = g_attn;
@@ -361,14 +361,14 @@ dfa3d_backward_packed_kernel(const KArgs a) {
     c.attn = a.attn + c.pt0;
     const int j = live ? lane % LP : a.LP;       // a.LP: no such point, the lane stays idle
     SoftmaxStats sm{0.f, 1.f};
-    if (MODE == kCallerFused) {                  // softmax over the item's LP logits: its own LP lanes
+    // lanes of a softmax: the item's LP, in 2-D those of one map
+    const int half = (MODE == kCallerFused2D ? LP / a.maps : LP) / 2;
+    if (mode_from_offsets(MODE)) {
       const float lg = live ? __ldg(a.logits + c.pt0 + j) : -INFINITY;
       float mx = lg;
-#pragma unroll
-      for (int s = LP / 2; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+      for (int s = half; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
       float sum = live ? expf(lg - mx) : 0.f;
-#pragma unroll
-      for (int s = LP / 2; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+      for (int s = half; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
       sm = SoftmaxStats{mx, sum};
     }
     PointState st;
@@ -440,11 +440,11 @@ dfa3d_backward_packed_kernel(const KArgs a) {
     const float4 tq = reinterpret_cast<const float4 *>(dot_slots)[lane];
     const float tt[4] = {tq.x, tq.y, tq.z, tq.w};
     float part = bwd_point_epilogue<DT, MODE>(a, c, j, st, tt);
-    if (MODE == kCallerFused) {
-      // softmax backward, grad_logit_j = a_j * (g_j - sum_k a_k g_k): the sum runs over the item's LP lanes;
-      // g_j was parked in grad_logits by the epilogue
-#pragma unroll
-      for (int s = LP / 2; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
+    if (mode_from_offsets(MODE)) {
+      // softmax backward, grad_logit_j = a_j * (g_j - sum_k a_k g_k): the sum runs over the softmax's lanes; g_j was
+      // parked in grad_logits by the epilogue.  2-D: the weight in hand is a_j / maps.
+      for (int s = half; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
+      if (MODE == kCallerFused2D) part *= (float)a.maps;
       if (live) a.grad_logits[c.pt0 + j] = st.aw * (a.grad_logits[c.pt0 + j] - part);
     }
     __syncwarp();
@@ -634,6 +634,14 @@ cudaError_t launch_backward(const KArgs &a, int value_dtype, int dist_dtype, int
     if (value_dtype == kDtypeF16) return launch_backward_vd<__half, float, kGivenDepthScore>(a, s);
     return value_dtype == kDtypeBF16 ? launch_backward_vd<__nv_bfloat16, float, kGivenDepthScore>(a, s)
                                      : launch_backward_vd<float, float, kGivenDepthScore>(a, s);
+  }
+  if (mode == kCallerFused2D) {     // packed kernels only (attn2d_supported)
+    for (int b0 = 0; b0 < a.B; b0 += 65535) {
+      KArgs c = a;
+      c.b0 = b0;
+      if (!launch_backward_packed<kCallerFused2D>(c, min(65535, a.B - b0), s)) return cudaErrorNotSupported;
+    }
+    return cudaGetLastError();
   }
   if (mode == kCallerFused) return launch_backward_m<kCallerFused>(a, value_dtype, dist_dtype, s);
   return launch_backward_m<kFused>(a, value_dtype, dist_dtype, s);

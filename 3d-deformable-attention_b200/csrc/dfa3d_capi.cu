@@ -279,7 +279,7 @@ int dfa3d_msda_backward(const dfa3d_problem *p, const void *value, const int64_t
                 "dfa3d_msda_backward launch");
 }
 
-static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors,
+static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
                                const int32_t *query_offsets, const void *value, const void *dist,
                                const int64_t *shapes3, const int64_t *level_start,
                                const float *ref_points, const float *offsets_uv,
@@ -289,12 +289,14 @@ static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors,
   if (num_anchors <= 0 || p->P % num_anchors != 0)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "num_anchors=%d must be positive and divide P=%d",
                 num_anchors, p->P);
+  if (shape_stride != 2 && shape_stride != 3)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "shape_stride must be 2 or 3 (got %d)", shape_stride);
   if (p->B == 0 || p->Q == 0) return DFA3D_OK;
   REQUIRE_PTR(value); REQUIRE_PTR(dist); REQUIRE_PTR(shapes3); REQUIRE_PTR(level_start);
   REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets_uv); REQUIRE_PTR(offsets_depth); REQUIRE_PTR(logits);
   REQUIRE_PTR(out);
   REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(out);
-  dfa3d::KArgs a = base_args(p, 3, 3);
+  dfa3d::KArgs a = base_args(p, shape_stride, 3);
   a.value = value; a.dist = dist; a.shapes = shapes3; a.lsi = level_start; a.ref = ref_points;
   a.off_uv = offsets_uv; a.off_d = offsets_depth; a.logits = logits; a.Z = num_anchors; a.out = out;
   a.q_off = query_offsets;
@@ -308,7 +310,7 @@ int dfa3d_attn3d_forward(const dfa3d_problem *p, int32_t num_anchors, const void
                          const void *dist, const int64_t *shapes3, const int64_t *level_start,
                          const float *ref_points, const float *offsets_uv, const float *offsets_depth,
                          const float *logits, float *out, void *stream) {
-  return attn3d_forward_impl(p, num_anchors, nullptr, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, nullptr, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
@@ -319,11 +321,11 @@ int dfa3d_attn3d_forward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                 const float *offsets_depth, const float *logits, float *out,
                                 void *stream) {
   REQUIRE_PTR(query_offsets);
-  return attn3d_forward_impl(p, num_anchors, query_offsets, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, query_offsets, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
-static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors,
+static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
                                 const int32_t *query_offsets, const void *value, const void *dist,
                                 const int64_t *shapes3, const int64_t *level_start,
                                 const float *ref_points, const float *offsets_uv,
@@ -334,13 +336,15 @@ static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors,
   if (num_anchors <= 0 || p->P % num_anchors != 0)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "num_anchors=%d must be positive and divide P=%d",
                 num_anchors, p->P);
+  if (shape_stride != 2 && shape_stride != 3)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "shape_stride must be 2 or 3 (got %d)", shape_stride);
   if (p->B == 0 || p->Q == 0) return DFA3D_OK;
   REQUIRE_PTR(value); REQUIRE_PTR(dist); REQUIRE_PTR(shapes3); REQUIRE_PTR(level_start);
   REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets_uv); REQUIRE_PTR(offsets_depth); REQUIRE_PTR(logits);
   REQUIRE_PTR(grad_out); REQUIRE_PTR(grad_value); REQUIRE_PTR(grad_dist); REQUIRE_PTR(grad_offsets_uv);
   REQUIRE_PTR(grad_offsets_depth); REQUIRE_PTR(grad_logits);
   REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(grad_out); REQUIRE_ALIGNED(grad_value);
-  dfa3d::KArgs a = base_args(p, 3, 3);
+  dfa3d::KArgs a = base_args(p, shape_stride, 3);
   a.value = value; a.dist = dist; a.shapes = shapes3; a.lsi = level_start; a.ref = ref_points;
   a.off_uv = offsets_uv; a.off_d = offsets_depth; a.logits = logits; a.Z = num_anchors;
   a.grad_out = grad_out; a.grad_value = grad_value; a.grad_dist = grad_dist;
@@ -358,7 +362,7 @@ int dfa3d_attn3d_backward(const dfa3d_problem *p, int32_t num_anchors, const voi
                           const float *offsets_depth, const float *logits, const float *grad_out,
                           float *grad_value, float *grad_dist, float *grad_offsets_uv,
                           float *grad_offsets_depth, float *grad_logits, void *stream) {
-  return attn3d_backward_impl(p, num_anchors, nullptr, value, dist, shapes3, level_start, ref_points,
+  return attn3d_backward_impl(p, num_anchors, 3, nullptr, value, dist, shapes3, level_start, ref_points,
                               offsets_uv, offsets_depth, logits, grad_out, grad_value, grad_dist,
                               grad_offsets_uv, grad_offsets_depth, grad_logits, stream);
 }
@@ -371,9 +375,82 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                  float *grad_value, float *grad_dist, float *grad_offsets_uv,
                                  float *grad_offsets_depth, float *grad_logits, void *stream) {
   REQUIRE_PTR(query_offsets);
-  return attn3d_backward_impl(p, num_anchors, query_offsets, value, dist, shapes3, level_start,
+  return attn3d_backward_impl(p, num_anchors, 3, query_offsets, value, dist, shapes3, level_start,
                               ref_points, offsets_uv, offsets_depth, logits, grad_out, grad_value,
                               grad_dist, grad_offsets_uv, grad_offsets_depth, grad_logits, stream);
+}
+
+int dfa3d_attn3d_forward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                                const int32_t *query_offsets, const void *value, const void *dist,
+                                const int64_t *shapes, const int64_t *level_start, const float *ref_points,
+                                const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
+                                void *stream) {
+  return attn3d_forward_impl(p, num_anchors, shape_stride, query_offsets, value, dist, shapes, level_start, ref_points,
+                             offsets_uv, offsets_depth, logits, out, stream);
+}
+
+int dfa3d_attn3d_backward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                                 const int32_t *query_offsets, const void *value, const void *dist,
+                                 const int64_t *shapes, const int64_t *level_start, const float *ref_points,
+                                 const float *offsets_uv, const float *offsets_depth, const float *logits,
+                                 const float *grad_out, float *grad_value, float *grad_dist, float *grad_offsets_uv,
+                                 float *grad_offsets_depth, float *grad_logits, void *stream) {
+  return attn3d_backward_impl(p, num_anchors, shape_stride, query_offsets, value, dist, shapes, level_start, ref_points,
+                              offsets_uv, offsets_depth, logits, grad_out, grad_value, grad_dist, grad_offsets_uv,
+                              grad_offsets_depth, grad_logits, stream);
+}
+
+// ---- 2-D attention from offsets and logits ----------------------------------------------------------
+int dfa3d_attn2d_supported(const dfa3d_problem *p, int32_t num_maps) {
+  return check_problem(p, true, false) == DFA3D_OK && num_maps > 0 && p->value_dtype == DFA3D_DTYPE_F32 &&
+         (long long)p->L * num_maps <= DFA3D_MAX_LEVELS && (long long)p->L * p->P <= 16 &&
+         (long long)num_maps * p->N * p->H * p->C < (1LL << 31) && num_maps <= 16 &&
+         dfa3d::attn2d_supported(p->C, p->L * p->P, num_maps);
+}
+
+static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+                       const int64_t *level_start, const float *ref_points, const float *offsets,
+                       const float *logits, dfa3d::KArgs &a) {
+  if (int rc = check_problem(p, true, false)) return rc;
+  if (!dfa3d_attn2d_supported(p, num_maps))
+    return fail(DFA3D_ERR_UNSUPPORTED, "2-D attention from offsets: fp32 value, C of 16, 32 or 64, 4, 8 or 16 points per "
+                "item in maps of a power of two (got C=%d, L*P=%d, maps=%d)", p->C, p->L * p->P, num_maps);
+  REQUIRE_PTR(value); REQUIRE_PTR(shapes2); REQUIRE_PTR(level_start); REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets);
+  REQUIRE_PTR(logits);
+  REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(ref_points); REQUIRE_ALIGNED(offsets);
+  dfa3d_problem q = *p;
+  q.N *= num_maps;
+  q.L *= num_maps;
+  a = base_args(&q, 2, 2);
+  a.value = value; a.shapes = shapes2; a.lsi = level_start; a.ref = ref_points; a.off_uv = offsets; a.logits = logits;
+  a.maps = num_maps;
+  return DFA3D_OK;
+}
+
+int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+                         const int64_t *level_start, const float *ref_points, const float *offsets,
+                         const float *logits, float *out, void *stream) {
+  if (p && (p->B == 0 || p->Q == 0)) return check_problem(p, true, false);
+  dfa3d::KArgs a;
+  if (int rc = attn2d_args(p, num_maps, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
+  REQUIRE_PTR(out); REQUIRE_ALIGNED(out);
+  a.out = out;
+  return finish(dfa3d::launch_forward(a, p->value_dtype, DFA3D_DTYPE_F32, dfa3d::kCallerFused2D, (cudaStream_t)stream),
+                "dfa3d_attn2d_forward launch");
+}
+
+int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+                          const int64_t *level_start, const float *ref_points, const float *offsets,
+                          const float *logits, const float *grad_out, float *grad_value, float *grad_offsets,
+                          float *grad_logits, void *stream) {
+  if (p && (p->B == 0 || p->Q == 0)) return check_problem(p, true, false);
+  dfa3d::KArgs a;
+  if (int rc = attn2d_args(p, num_maps, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
+  REQUIRE_PTR(grad_out); REQUIRE_PTR(grad_value); REQUIRE_PTR(grad_offsets); REQUIRE_PTR(grad_logits);
+  REQUIRE_ALIGNED(grad_out); REQUIRE_ALIGNED(grad_value);
+  a.grad_out = grad_out; a.grad_value = grad_value; a.grad_off_uv = grad_offsets; a.grad_logits = grad_logits;
+  return finish(dfa3d::launch_backward(a, p->value_dtype, DFA3D_DTYPE_F32, dfa3d::kCallerFused2D, (cudaStream_t)stream),
+                "dfa3d_attn2d_backward launch");
 }
 
 // ---- per-camera re-batching -----------------------------------------------------------------
@@ -534,6 +611,30 @@ int dfa3d_column_sum(const float *src, int64_t rows, int32_t cols, float *dst, v
   REQUIRE_PTR(src); REQUIRE_PTR(dst);
   REQUIRE_ALIGNED(src); REQUIRE_ALIGNED(dst);
   return finish(dfa3d::launch_column_sum(src, rows, cols, dst, (cudaStream_t)stream), "dfa3d_column_sum launch");
+}
+
+int dfa3d_add_layer_norm_infer(const float *x, const float *residual, const float *gamma, const float *beta,
+                               int64_t rows, int32_t E, float eps, float *y, void *stream) {
+  if (int rc = check_rows(rows, E)) return rc;
+  if (!(eps >= 0.f)) return fail(DFA3D_ERR_INVALID_ARGUMENT, "eps must be >= 0");
+  if (rows == 0) return DFA3D_OK;
+  REQUIRE_PTR(x); REQUIRE_PTR(gamma); REQUIRE_PTR(beta); REQUIRE_PTR(y);
+  REQUIRE_ALIGNED(x); REQUIRE_ALIGNED(residual); REQUIRE_ALIGNED(gamma); REQUIRE_ALIGNED(beta); REQUIRE_ALIGNED(y);
+  return finish(dfa3d::launch_add_layer_norm_forward(x, residual, gamma, beta, rows, E, eps, nullptr, y, nullptr, nullptr,
+                                                     (cudaStream_t)stream),
+                "dfa3d_add_layer_norm_infer launch");
+}
+
+int dfa3d_relu_backward_column_sum(const float *grad_y, const float *y, int64_t rows, int32_t cols, float *grad_in,
+                                   float *dst, void *stream) {
+  if (rows < 0 || cols < 0)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "rows and cols must be >= 0 (got %lld, %d)", (long long)rows, cols);
+  if (cols % 4 != 0) return fail(DFA3D_ERR_UNSUPPORTED, "cols=%d must be a multiple of 4", cols);
+  if (rows == 0 || cols == 0) return DFA3D_OK;
+  REQUIRE_PTR(grad_y); REQUIRE_PTR(y); REQUIRE_PTR(grad_in); REQUIRE_PTR(dst);
+  REQUIRE_ALIGNED(grad_y); REQUIRE_ALIGNED(y); REQUIRE_ALIGNED(grad_in); REQUIRE_ALIGNED(dst);
+  return finish(dfa3d::launch_relu_backward(grad_y, y, rows, cols, grad_in, dst, (cudaStream_t)stream),
+                "dfa3d_relu_backward_column_sum launch");
 }
 
 int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream) {

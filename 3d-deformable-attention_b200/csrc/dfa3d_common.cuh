@@ -29,10 +29,14 @@ constexpr int kMaxLevels = 32;
 //   kCallerFused      reference point + raw offsets + raw attention logits: the caller's location
 //                     assembly and softmax (BEVFormer_DFA3D/projects/mmdet3d_plugin/bevformer/modules/
 //                     spatial_cross_attention.py:498-538) happen in the prologue; depth scores from dist
-enum Mode { kFused = 0, kGivenDepthScore = 1, kCallerFused = 2 };
+//   kCallerFused2D    the same for the plain 2-D operator (…/bevformer/modules/temporal_self_attention.py:224-262,
+//                     decoder.py:283-318): `maps` value maps per batch element are read as that many times the
+//                     levels, the logits are normalised map by map, the maps' results averaged
+enum Mode { kFused = 0, kGivenDepthScore = 1, kCallerFused = 2, kCallerFused2D = 3 };
 // Storage type codes = DFA3D_DTYPE_F32 / _BF16 / _F16 of the C header.
 enum StorageType { kDtypeF32 = 0, kDtypeBF16 = 1, kDtypeF16 = 3 };
-__host__ __device__ constexpr bool mode_has_depth(int m) { return m != kGivenDepthScore; }
+__host__ __device__ constexpr bool mode_has_depth(int m) { return m == kFused || m == kCallerFused; }
+__host__ __device__ constexpr bool mode_from_offsets(int m) { return m == kCallerFused || m == kCallerFused2D; }
 constexpr int kWarpsPerCta = 8;
 constexpr int kThreads = kWarpsPerCta * 32;
 
@@ -75,7 +79,7 @@ struct KArgs {
   const float *ds_in;      // (B,Q,H,L,P,4) given depth score (two-stage attention)
   const float *grad_out;   // (B,Q,H*C)
   // caller-fused mode: locations and attention weights are formed inside the kernel
-  const float *ref;        // (B,Q,Z,3) reference points
+  const float *ref;        // (B,Q,Z,3) reference points; 2-D: (B*maps,Q,L/maps,2)
   const float *off_uv;     // (B,Q,H,L,P,2) raw x/y offsets in pixels
   const float *off_d;      // (B,Q,H,L,P) raw depth offsets in bins
   const float *logits;     // (B,Q,H,L*P) raw attention logits
@@ -83,6 +87,7 @@ struct KArgs {
   float *grad_off_d;       // (B,Q,H,L,P), overwritten
   float *grad_logits;      // (B,Q,H,L*P), overwritten
   int Z;                   // reference points (pillar anchors) per query
+  int maps;                // 2-D: value maps per batch element; N and L count all of them.  0 elsewhere
   // ragged queries: camera b owns the packed query rows [q_off[b], q_off[b+1]) of every per-query
   // tensor; Q is then only the bound the grid is sized for.  Null = every camera has Q queries.
   const int32_t *q_off;
@@ -115,11 +120,13 @@ struct LevelTable {
 };
 
 __device__ __forceinline__ void stage_levels(LevelTable &t, const KArgs &a) {
+  const int per_map = a.maps > 1 ? a.L / a.maps : a.L;      // every map has the same level table
   for (int l = threadIdx.x; l < a.L; l += blockDim.x) {
-    t.h[l] = (int)a.shapes[l * a.shape_stride];
-    t.w[l] = (int)a.shapes[l * a.shape_stride + 1];
-    t.d[l] = a.shape_stride == 3 ? (int)a.shapes[l * 3 + 2] : a.D;
-    t.start[l] = (int)a.lsi[l];
+    const int sl = l % per_map;
+    t.h[l] = (int)a.shapes[sl * a.shape_stride];
+    t.w[l] = (int)a.shapes[sl * a.shape_stride + 1];
+    t.d[l] = a.shape_stride == 3 ? (int)a.shapes[sl * 3 + 2] : a.D;
+    t.start[l] = (int)a.lsi[sl] + (l == sl ? 0 : l / per_map * (a.N / a.maps));
     // the resize's scale, formed in fp32 from the two sizes as torch's nearest interpolation forms it
     t.map_sy[l] = a.dmap_h > 0 ? (float)a.dmap_h / (float)t.h[l] : 1.f;
     t.map_sx[l] = a.dmap_w > 0 ? (float)a.dmap_w / (float)t.w[l] : 1.f;
@@ -212,6 +219,16 @@ __device__ __forceinline__ void read_point(const KArgs &a, const LevelTable &lv,
     y = __fadd_rn(__ldg(r + 1), __fdiv_rn(__ldg(o + 1), (float)lv.h[l]));
     z = __fadd_rn(__ldg(r + 2), __fdiv_rn(__ldg(a.off_d + c.pt0 + j), (float)a.D));
     aw = __fdiv_rn(expf(__ldg(a.logits + c.pt0 + j) - sm.mx), sm.sum);
+  } else if (MODE == kCallerFused2D) {
+    const int per_map = a.L / a.maps, map = l / per_map;
+    const long long q = c.bq - (long long)c.b * a.Q;
+    const float2 r = __ldg(reinterpret_cast<const float2 *>(a.ref) +
+                           ((((long long)c.b * a.maps + map) * a.Q + q) * per_map + (l - map * per_map)));
+    const float2 o = __ldg(reinterpret_cast<const float2 *>(a.off_uv) + (c.pt0 + j));
+    x = __fadd_rn(r.x, __fdiv_rn(o.x, (float)lv.w[l]));
+    y = __fadd_rn(r.y, __fdiv_rn(o.y, (float)lv.h[l]));
+    z = 0.f;
+    aw = __fdiv_rn(expf(__ldg(a.logits + c.pt0 + j) - sm.mx), sm.sum * (float)a.maps);
   } else {
     const float *lp = c.loc + j * a.loc_stride;
     x = __ldg(lp);

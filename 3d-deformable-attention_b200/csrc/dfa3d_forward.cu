@@ -300,14 +300,13 @@ dfa3d_forward_packed_kernel(const KArgs a) {
       c.attn = a.attn + c.pt0;
       const int j = lane % LP;
       SoftmaxStats sm{0.f, 1.f};
-      if (MODE == kCallerFused) {                // softmax over the item's LP logits: its own LP lanes
+      if (mode_from_offsets(MODE)) {             // softmax over the item's LP logits (2-D: of each map): its own lanes
+        const int half = (MODE == kCallerFused2D ? LP / a.maps : LP) / 2;
         const float lg = live ? __ldg(a.logits + c.pt0 + j) : -INFINITY;
         float mx = lg;
-#pragma unroll
-        for (int s = LP / 2; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+        for (int s = half; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
         float sum = live ? expf(lg - mx) : 0.f;
-#pragma unroll
-        for (int s = LP / 2; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+        for (int s = half; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
         sm = SoftmaxStats{mx, sum};
       }
       float ds[4], wgt[4];
@@ -404,7 +403,7 @@ static bool launch_forward_packed(const KArgs &a, int cams, cudaStream_t s) {
   if (a.LP != 4 && a.LP != 8 && a.LP != 16) return false;
   const int per_cta = kWarpsPerCta * kPackedRounds * (32 / a.LP);
   const dim3 grid((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
-  constexpr bool kCanWriteDs = MODE != kCallerFused;          // the caller-fused entry points return no depth score
+  constexpr bool kCanWriteDs = !mode_from_offsets(MODE);      // the caller-fused entry points return no depth score
   if (kCanWriteDs && a.ds_out) {
     if (a.LP == 4) return launch_forward_packed_c<MODE, kCanWriteDs, 4>(a, grid, s);
     if (a.LP == 8) return launch_forward_packed_c<MODE, kCanWriteDs, 8>(a, grid, s);
@@ -461,6 +460,14 @@ cudaError_t launch_forward(const KArgs &a, int value_dtype, int dist_dtype, int 
     if (value_dtype == kDtypeF16) return launch_forward_vd<__half, float, kGivenDepthScore>(a, s);
     return value_dtype == kDtypeBF16 ? launch_forward_vd<__nv_bfloat16, float, kGivenDepthScore>(a, s)
                                      : launch_forward_vd<float, float, kGivenDepthScore>(a, s);
+  }
+  if (mode == kCallerFused2D) {     // packed kernels only (attn2d_supported)
+    for (int b0 = 0; b0 < a.B; b0 += 65535) {
+      KArgs c = a;
+      c.b0 = b0;
+      if (!launch_forward_packed<kCallerFused2D>(c, min(65535, a.B - b0), s)) return cudaErrorNotSupported;
+    }
+    return cudaGetLastError();
   }
   if (mode == kCallerFused) return launch_forward_m<kCallerFused>(a, value_dtype, dist_dtype, s);
   return launch_forward_m<kFused>(a, value_dtype, dist_dtype, s);

@@ -11,6 +11,12 @@ cudaError_t launch_forward(const KArgs &a, int value_dtype, int dist_dtype, int 
 cudaError_t launch_depth_score_forward(const KArgs &a, int dist_dtype, cudaStream_t s);
 cudaError_t launch_backward(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s);
 cudaError_t launch_depth_score_backward(const KArgs &a, int dist_dtype, cudaStream_t s);
+// 2-D operator from offsets and logits (kCallerFused2D): the sizes its kernels exist for
+inline bool attn2d_supported(int C, int points_per_map, int maps) {
+  const int all = points_per_map * maps;
+  return (C == 16 || C == 32 || C == 64) && (all == 4 || all == 8 || all == 16) &&
+         (points_per_map & (points_per_map - 1)) == 0;
+}
 // per-camera re-batching (dfa3d_rebatch.cu)
 cudaError_t launch_rebatch_plan(const uint8_t *mask, int cams, int bs, int Q, int Z, int32_t *counts,
                                 int32_t *offsets, int32_t *op_offsets, int32_t *packed_query,
@@ -62,5 +68,7 @@ cudaError_t launch_layer_norm_backward(const float *grad_y, const float *in, con
                                        float *grad_in, float *grad_gamma, float *grad_beta,
                                        cudaStream_t s);
 cudaError_t launch_column_sum(const float *src, long long rows, int cols, float *dst, cudaStream_t s);
+cudaError_t launch_relu_backward(const float *grad_y, const float *y, long long rows, int cols, float *grad_in, float *dst,
+                                 cudaStream_t s);
 cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cudaStream_t s);
 }  // namespace dfa3d

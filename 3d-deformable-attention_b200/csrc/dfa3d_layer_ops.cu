@@ -91,7 +91,7 @@ add_layer_norm_forward_kernel(const float *__restrict__ x, const float *__restri
       o.w = (v[j].w - mean) * rstd * g.w + b.w;
       st4(y + row * E + c, o);
     }
-    if (lane == 0) {
+    if (lane == 0 && mean_out) {        // no backward will ask for them otherwise
       mean_out[row] = mean;
       rstd_out[row] = rstd;
     }
@@ -235,6 +235,48 @@ column_sum_kernel(const float *__restrict__ src, long long rows, int cols, float
   }
 }
 
+// Backward of relu(x W^T + b) up to the products: grad_in = y > 0 ? grad_y : 0 and its column sums (the bias gradient)
+// in one pass over both operands.  Split and accumulation as in column_sum_kernel.
+__global__ void __launch_bounds__(kCsThreads)
+relu_backward_kernel(const float *grad_y, const float *__restrict__ y, long long rows, int cols,
+                     float *grad_in, float *__restrict__ dst) {
+  __shared__ float4 part[kCsLanes][kCsGroups];
+  const int grp = threadIdx.x % kCsGroups, rl = threadIdx.x / kCsGroups;
+  const int col = (blockIdx.y * kCsGroups + grp) * 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (col < cols) {
+    const long long step = (long long)gridDim.x * kCsLanes;
+    constexpr int U = 4;
+    for (long long r = (long long)blockIdx.x * kCsLanes + rl; r < rows; r += U * step) {
+      float4 g[U], v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (r + u * step < rows) {
+          g[u] = ld4_stream(grad_y + (r + u * step) * cols + col);
+          v[u] = ld4_stream(y + (r + u * step) * cols + col);
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (r + u * step < rows) {
+          const float4 t = make_float4(v[u].x > 0.f ? g[u].x : 0.f, v[u].y > 0.f ? g[u].y : 0.f,
+                                       v[u].z > 0.f ? g[u].z : 0.f, v[u].w > 0.f ? g[u].w : 0.f);
+          st4(grad_in + (r + u * step) * cols + col, t);
+          acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+        }
+    }
+  }
+  part[rl][grp] = acc;
+  __syncthreads();
+  if (rl == 0 && col < cols) {
+    float4 t = part[0][grp];
+#pragma unroll
+    for (int i = 1; i < kCsLanes; ++i) {
+      t.x += part[i][grp].x; t.y += part[i][grp].y; t.z += part[i][grp].z; t.w += part[i][grp].w;
+    }
+    red_add_v4(dst + col, t);
+  }
+}
+
 // Zeroes two buffers with one launch (a backward zeroes the two gradients it accumulates into; for a small
 // problem a second fill is a launch gap longer than the fill).  16-byte stores, the ragged ends one by one.
 __global__ void __launch_bounds__(256) zero_two_kernel(float *a, long long na, float *b, long long nb) {
@@ -309,6 +351,18 @@ cudaError_t launch_column_sum(const float *src, long long rows, int cols, float 
   if (gx > most) gx = most;
   if (gx < 1) gx = 1;
   column_sum_kernel<<<dim3((unsigned)gx, bands, 1), kCsThreads, 0, s>>>(src, rows, cols, dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_relu_backward(const float *grad_y, const float *y, long long rows, int cols, float *grad_in, float *dst,
+                                 cudaStream_t s) {
+  if (rows == 0 || cols == 0) return cudaSuccess;
+  const unsigned bands = (unsigned)((cols / 4 + kCsGroups - 1) / kCsGroups);
+  long long gx = (long long)kSms * 2 / bands;                            // as launch_column_sum
+  const long long most = (rows + kCsLanes * 8 - 1) / (kCsLanes * 8);
+  if (gx > most) gx = most;
+  if (gx < 1) gx = 1;
+  relu_backward_kernel<<<dim3((unsigned)gx, bands, 1), kCsThreads, 0, s>>>(grad_y, y, rows, cols, grad_in, dst);
   return cudaGetLastError();
 }
 

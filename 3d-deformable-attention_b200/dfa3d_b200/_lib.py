@@ -66,6 +66,11 @@ ENTRY_POINTS_WITH_ANCHORS = {
 _I32, _I64 = ctypes.c_int32, ctypes.c_int64
 # entry points without a problem descriptor: explicit argument types
 PLAIN_ENTRY_POINTS = {
+    "dfa3d_attn2d_supported": [_P, _I32],
+    "dfa3d_attn2d_forward": [_P, _I32] + [_V] * 8,
+    "dfa3d_attn2d_backward": [_P, _I32] + [_V] * 11,
+    "dfa3d_attn3d_forward_levels": [_P, _I32, _I32] + [_V] * 11,
+    "dfa3d_attn3d_backward_levels": [_P, _I32, _I32] + [_V] * 16,
     "dfa3d_rebatch_plan": [ctypes.c_void_p, _I32, _I32, _I32, _I32] + [ctypes.c_void_p] * 8,
     "dfa3d_rebatch_gather": [ctypes.c_void_p] * 4 + [_I32] * 4 + [_I64, _I64] + [ctypes.c_void_p] * 2
                             + [_I64, ctypes.c_void_p],
@@ -80,6 +85,8 @@ PLAIN_ENTRY_POINTS = {
     "dfa3d_add_layer_norm_forward": [ctypes.c_void_p] * 4 + [_I64, _I32, ctypes.c_float] + [ctypes.c_void_p] * 5,
     "dfa3d_layer_norm_backward": [ctypes.c_void_p] * 5 + [_I64, _I32] + [ctypes.c_void_p] * 4,
     "dfa3d_column_sum": [ctypes.c_void_p, _I64, _I32, ctypes.c_void_p, ctypes.c_void_p],
+    "dfa3d_add_layer_norm_infer": [ctypes.c_void_p] * 4 + [_I64, _I32, ctypes.c_float] + [ctypes.c_void_p] * 2,
+    "dfa3d_relu_backward_column_sum": [ctypes.c_void_p] * 2 + [_I64, _I32] + [ctypes.c_void_p] * 3,
     "dfa3d_zero_two": [ctypes.c_void_p, _I64, ctypes.c_void_p, _I64, ctypes.c_void_p],
 }
 ACT_SOFTMAX, ACT_SIGMOID = 0, 1
@@ -143,6 +150,33 @@ def native():
         mod.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in mod.entries()})
         _native = mod
     return _native
+
+
+def native_apply(name):
+    """Class decorator: ``apply`` first offers the call to the native host path (csrc/binding),
+    which takes the plain case -- CUDA tensors of the usual types and layouts, no autocast, no functorch -- and
+    answers NotImplemented to anything else; the Python Function then runs, with its checks and messages.
+    Measured on 512 queries, forward + backward: 190 us a pass through the Python Function, of which 34 us are
+    kernels."""
+
+    def wrap(cls):
+        python_apply = cls.apply.__func__
+        fast = None
+
+        def apply(c, *args):
+            nonlocal fast
+            if c is cls:                        # a subclass may have overridden forward or backward
+                if fast is None:
+                    fast = getattr(native(), name)
+                out = fast(*args)
+                if out is not NotImplemented:
+                    return out
+            return python_apply(c, *args)
+
+        cls.apply = classmethod(apply)
+        return cls
+
+    return wrap
 
 
 def call_plain(name, *args):

@@ -27,35 +27,9 @@ that recomputes the depth scores instead of re-reading them.
 import torch
 from torch.autograd.function import Function, once_differentiable
 
-from . import _lib
 from . import ext as ext_module
-
-
-def _native_apply(name):
-    """Class decorator: ``apply`` first offers the call to the native host path (csrc/binding/dfa3d_torch.cpp),
-    which takes the plain case -- CUDA tensors of the usual types and layouts, no autocast, no functorch -- and
-    answers NotImplemented to anything else; the Python Function then runs, with its checks and messages.
-    Measured on 512 queries, forward + backward: 190 us a pass through the Python Function, of which 34 us are
-    kernels."""
-
-    def wrap(cls):
-        python_apply = cls.apply.__func__
-        fast = None
-
-        def apply(c, *args):
-            nonlocal fast
-            if c is cls:                        # a subclass may have overridden forward or backward
-                if fast is None:
-                    fast = getattr(_lib.native(), name)
-                out = fast(*args)
-                if out is not NotImplemented:
-                    return out
-            return python_apply(c, *args)
-
-        cls.apply = classmethod(apply)
-        return cls
-
-    return wrap
+from . import _lib
+from ._lib import native_apply as _native_apply
 
 
 def _grad_dtype(t):
@@ -161,8 +135,22 @@ class MultiScale3DDeformableAttnFunction(Function):
         return grad_value, grad_dist, None, None, grad_sampling_loc, grad_attn_weight, None, None, None
 
 
+class _FromOffsets2D(Function):
+    @classmethod
+    def from_offsets(cls, value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps, heads,
+                     points):
+        """The operator with what its callers do around it (temporal_self_attention.py:224-262, decoder.py:283-318)
+        inside the kernels: softmax of the logits map by map, locations from reference points and offsets, mean over
+        the `maps` value maps of a batch element.  value (bs*maps, N, H*C); reference_points (bs*maps, Q, L, 2) without
+        gradient; offsets (bs, Q, H*maps*L*P*2) and logits (bs, Q, H*maps*L*P) as the Linear layers leave them.
+        Returns (bs, Q, H*C), or NotImplemented where only the separate steps do it (sizes the kernels do not have,
+        other dtypes, autocast)."""
+        return _lib.native().attn2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps,
+                                    heads, points)
+
+
 @_native_apply("msda")
-class MultiScaleDeformableAttnFunction(Function):
+class MultiScaleDeformableAttnFunction(_FromOffsets2D):
     """Plain 2-D multi-scale deformable attention with the call signature BEVFormer_DFA3D uses for its
     temporal self-attention and decoder (…/bevformer/modules/multi_scale_deformable_attn_function.py:
     MultiScaleDeformableAttnFunction_fp32.forward :97-131, backward :133-163; there the kernels come
@@ -314,8 +302,8 @@ def _fp32_variant(cls, name, native):
     """Same Function with inputs cast to float32 when autocast is active."""
     fwd = torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float32)(cls.forward)
     bwd = torch.amp.custom_bwd(device_type="cuda")(cls.backward)
-    return _native_apply(native)(
-        type(name, (Function,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)}))
+    base = _FromOffsets2D if issubclass(cls, _FromOffsets2D) else Function
+    return _native_apply(native)(type(name, (base,), {"forward": staticmethod(fwd), "backward": staticmethod(bwd)}))
 
 
 MultiScaleDepthScoreSampleFunction_fp32 = _fp32_variant(

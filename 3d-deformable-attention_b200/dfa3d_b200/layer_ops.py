@@ -43,6 +43,7 @@ def column_sum(src):
     return dst
 
 
+@_lib.native_apply("add_layer_norm")
 class AddLayerNormFunction(Function):
     @staticmethod
     @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float32)
@@ -124,6 +125,7 @@ def weight_gradient(grad_out2, x2):
     return w
 
 
+@_lib.native_apply("linear")
 class LinearFunction(Function):
     @staticmethod
     @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.float32)
@@ -158,6 +160,33 @@ class Linear(nn.Linear):
         if self.bias is None or self.out_features % 4 != 0:
             return super().forward(x)
         return LinearFunction.apply(x, self.weight, self.bias)
+
+
+def _plain_linear(m):
+    """A Linear whose forward is LinearFunction and nothing else: no hooks that calling it would run."""
+    return (type(m) is Linear and m.bias is not None and m.out_features % 4 == 0 and not m._forward_hooks
+            and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
+
+
+def linear3(x, a, b, c):
+    """(a(x), b(x), c(x)) for three Linear layers; as one operation where they are plain, so that the gradient of x is
+    accumulated inside the matrix products instead of by two additions of its size."""
+    if _plain_linear(a) and _plain_linear(b) and _plain_linear(c):
+        out = _lib.native().linear3(x, a.weight, a.bias, b.weight, b.bias, c.weight, c.bias)
+        if out is not NotImplemented:
+            return out
+    return a(x), b(x), c(x)
+
+
+def linear_relu(x, linear, relu):
+    """relu(linear(x)); as one operation where both are plain: the ReLU is the product's epilogue, its backward and the
+    bias gradient are one kernel."""
+    if _plain_linear(linear) and type(relu) is nn.ReLU and not relu._forward_hooks and not relu._forward_pre_hooks \
+            and not relu._backward_hooks and not relu._backward_pre_hooks:
+        out = _lib.native().linear_relu(x, linear.weight, linear.bias)
+        if out is not NotImplemented:
+            return out
+    return relu(linear(x))
 
 
 def _time_ms(fn, launches=200):

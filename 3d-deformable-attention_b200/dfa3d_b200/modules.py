@@ -33,9 +33,9 @@ from .functions import (MultiScaleDeformableAttnFunction_fp32,
                         DeformableAttn3DFromOffsetsRaggedFunction_fp32,
                         MultiScale3DDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnRaggedFunction_fp32)
-from .layer_ops import AddLayerNorm, Linear
-from .rebatch import (CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan,
-                      gather_per_camera)
+from . import _lib
+from .layer_ops import AddLayerNorm, Linear, linear3, linear_relu
+from .rebatch import CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan
 
 
 def bev_reference_points(bev_h, bev_w, pillar_height=8, num_points_in_pillar=4, dim="3d", bs=1,
@@ -158,7 +158,7 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
 
     def forward(self, query, value, value_dpt_dist, reference_points, spatial_shapes, level_start_index,
                 query_pos=None, key_padding_mask=None, query_offsets=None, max_queries=None,
-                dist_map=None):
+                dist_map=None, value_projected=False):
         """query (bs, Q, E); value (bs, N, E); value_dpt_dist (bs, N, D); reference_points
         (bs, Q, Z, 3); spatial_shapes (L, 2) int64; level_start_index (L) int64.
         Returns (output (bs, Q, E), weight_update (bs, Q, H, 1))  -- :428-583.
@@ -169,7 +169,8 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
         (R, E) and (R, H, 1).  value / value_dpt_dist are batch-first in this mode.
 
         ``dist_map=(h, w)``: value_dpt_dist is one h x w map per camera, (bs, h*w, D), that every level
-        reads with nearest-neighbour indexing (instead of one resized copy per level)."""
+        reads with nearest-neighbour indexing (instead of one resized copy per level).
+        ``value_projected``: value went through ``value_proj`` already."""
         ragged = query_offsets is not None
         if query_pos is not None:
             query = query + query_pos
@@ -179,17 +180,28 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
         bs, N, _ = value.shape
         H, L, P = self.num_heads, self.num_levels, self.num_points
         D = value_dpt_dist.shape[-1]
-        value = self.value_proj(value)
+        if not value_projected:
+            value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
         value = value.view(bs, N, H, -1)
         if reference_points.shape[-1] != 3:
             raise ValueError("Last dim of reference_points must be 3 (x, y, depth), but got "
                              f"{reference_points.shape[-1]} instead.")
+        off_uv, off_d, logits = linear3(query, self.sampling_offsets, self.sampling_offsets_depth,
+                                        self.attention_weights)
+        off_uv = off_uv.view(*lead, H, L, P, 2)
+        off_d = off_d.view(*lead, H, L, P, 1)
+        logits = logits.view(*lead, H, L * P)
+        if self.fuse_input_ops and not self.compute_weight_update:
+            # the kernels take the (L, 2) table as it is: D bins in every level
+            args = (value.contiguous(), value_dpt_dist.contiguous(), spatial_shapes, level_start_index,
+                    reference_points.contiguous(), off_uv, off_d, logits)
+            output = _lib.native().attn3d_ragged_flat(*args, query_offsets, max_queries, dist_map) if ragged else \
+                _lib.native().attn3d_flat(*args, dist_map)
+            if output is not NotImplemented:
+                return (output if ragged or self.batch_first else output.permute(1, 0, 2)), None
         shapes3 = torch.cat([spatial_shapes, torch.full_like(spatial_shapes[:, :1], D)], -1).contiguous()
-        off_uv = self.sampling_offsets(query).view(*lead, H, L, P, 2)
-        off_d = self.sampling_offsets_depth(query).view(*lead, H, L, P, 1)
-        logits = self.attention_weights(query).view(*lead, H, L * P)
         if self.fuse_input_ops and not self.compute_weight_update:
             if ragged:
                 output = DeformableAttn3DFromOffsetsRaggedFunction_fp32.apply(
@@ -261,15 +273,21 @@ class SpatialCrossAttention_DFA3D(nn.Module):
         plan = rebatch_plan if rebatch_plan is not None else RebatchPlan(bev_mask)
         if (plan.cams, plan.bs, plan.Q) != (cams, bs, Q):
             raise RuntimeError("rebatch_plan does not belong to this bev_mask / query")
-        q_rows = GatherQueriesFunction.apply(query.float(), plan)                 # (bs*T, E)
-        ref_rows = gather_per_camera(reference_points_cam.float(), plan)          # (bs*T, Z, 3)
         N = value.shape[1]
         value = value.permute(2, 0, 1, 3).reshape(bs * cams, N, E)                # element j*cams + i
         dist = value_dpt_dist.permute(2, 0, 1, 3).reshape(bs * cams, N, -1)
-        out_rows, update_weight = self.deformable_attention(
+        # the value projection does not need the plan's row count: queued first, it keeps the device busy while the
+        # count is read back
+        attention, kw = self.deformable_attention, {}
+        if type(attention) is MSDeformableAttention3D_DFA3D and not attention._forward_hooks \
+                and not attention._forward_pre_hooks:
+            value, kw = attention.value_proj(value), {"value_projected": True}
+        q_rows = GatherQueriesFunction.apply(query.float(), plan)                 # (bs*T, E)
+        ref_rows = plan.reference_rows(reference_points_cam.float())              # (bs*T, Z, 3)
+        out_rows, update_weight = attention(
             query=q_rows, value=value, value_dpt_dist=dist, reference_points=ref_rows,
             spatial_shapes=spatial_shapes, level_start_index=level_start_index,
-            query_offsets=plan.op_offsets, max_queries=plan.max_queries, dist_map=dist_map)
+            query_offsets=plan.op_offsets, max_queries=plan.max_queries, dist_map=dist_map, **kw)
         if self.use_empty:
             # :721-722, :739-740 -- rows whose depth-weighted attention found little get the learned
             # per-(BEV cell, head) empty embedding instead
@@ -279,6 +297,17 @@ class SpatialCrossAttention_DFA3D(nn.Module):
         slots = CombineCamerasFunction.apply(out_rows, plan)                      # sum over cameras / count
         slots = self.dropout(self.output_proj(slots))
         return (slots, inp_residual) if return_residual else slots + inp_residual
+
+
+def _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps, heads, points):
+    """The 2-D operator with its callers' softmax, location assembly and mean over the maps inside the kernels, or None
+    where the separate steps have to do it (box reference points, sizes the kernels do not have)."""
+    fused = getattr(MultiScaleDeformableAttnFunction_fp32, "from_offsets", None)
+    if fused is None or reference_points.shape[-1] != 2:
+        return None
+    out = fused(value.contiguous(), spatial_shapes, level_start_index, reference_points.contiguous(), offsets, logits,
+                maps, heads, points)
+    return None if out is NotImplemented else out
 
 
 class TemporalSelfAttention(nn.Module):
@@ -348,9 +377,23 @@ class TemporalSelfAttention(nn.Module):
         value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
-        value = value.reshape(bs * NQ, N, H, -1)
-        offsets = self.sampling_offsets(query).view(bs, Q, H, NQ, L, P, 2)
-        attn = self.attention_weights(query).view(bs, Q, H, NQ, L * P).softmax(-1).view(bs, Q, H, NQ, L, P)
+        offsets, logits = self.sampling_offsets(query), self.attention_weights(query)
+        out = _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, NQ, H, P)
+        if out is None:
+            out = self._attention_in_steps(value.reshape(bs * NQ, N, H, -1), offsets, logits, reference_points,
+                                           spatial_shapes, level_start_index)
+        out = self.output_proj(out)
+        if not self.batch_first:
+            out = out.permute(1, 0, 2)
+        out = self.dropout(out)
+        return (out, identity) if return_residual else out + identity
+
+    def _attention_in_steps(self, value, offsets, logits, reference_points, spatial_shapes, level_start_index):
+        """:205-262 one operation after the other, for what `_attention_2d` does not cover."""
+        bs, Q, _ = offsets.shape
+        H, L, P, NQ = self.num_heads, self.num_levels, self.num_points, self.num_bev_queue
+        offsets = offsets.view(bs, Q, H, NQ, L, P, 2)
+        attn = logits.view(bs, Q, H, NQ, L * P).softmax(-1).view(bs, Q, H, NQ, L, P)
         attn = attn.permute(0, 3, 1, 2, 4, 5).reshape(bs * NQ, Q, H, L, P).contiguous()
         offsets = offsets.permute(0, 3, 1, 2, 4, 5, 6).reshape(bs * NQ, Q, H, L, P, 2)
         if reference_points.shape[-1] == 2:
@@ -365,12 +408,15 @@ class TemporalSelfAttention(nn.Module):
         out = MultiScaleDeformableAttnFunction_fp32.apply(value.contiguous(), spatial_shapes, level_start_index,
                                                           loc.contiguous(), attn, self.im2col_step)
         # mean over the previous and the current BEV (:257-262); batch element j owns rows j*NQ .. j*NQ+NQ-1
-        out = out.view(bs, NQ, Q, E).mean(1)
-        out = self.output_proj(out)
-        if not self.batch_first:
-            out = out.permute(1, 0, 2)
-        out = self.dropout(out)
-        return (out, identity) if return_residual else out + identity
+        return out.view(bs, NQ, Q, -1).mean(1)
+
+
+def _run_ffn(ffn, x):
+    """The feed-forward block (Linear, ReLU, Dropout, Linear, Dropout) with the first Linear and the ReLU as one
+    operation."""
+    if ffn._forward_hooks or ffn._forward_pre_hooks or ffn._backward_hooks or ffn._backward_pre_hooks:
+        return ffn(x)
+    return ffn[4](ffn[3](ffn[2](linear_relu(x, ffn[0], ffn[1]))))
 
 
 class SCAEncoderLayer(nn.Module):
@@ -390,7 +436,7 @@ class SCAEncoderLayer(nn.Module):
 
     def forward(self, query, **kw):
         query = self.norm1(*self.cross_attn(query, return_residual=True, **kw))     # norm(branch + residual)
-        return self.norm2(self.ffn(query), query)
+        return self.norm2(_run_ffn(self.ffn, query), query)
 
 
 class CustomMSDeformableAttention(nn.Module):
@@ -448,9 +494,22 @@ class CustomMSDeformableAttention(nn.Module):
         value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
-        value = value.view(bs, N, H, -1)
-        offsets = self.sampling_offsets(query).view(bs, Q, H, L, P, 2)
-        attn = self.attention_weights(query).view(bs, Q, H, L * P).softmax(-1).view(bs, Q, H, L, P)
+        offsets, logits = self.sampling_offsets(query), self.attention_weights(query)
+        out = _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, 1, H, P)
+        if out is None:
+            out = self._attention_in_steps(value.view(bs, N, H, -1), offsets, logits, reference_points,
+                                           spatial_shapes, level_start_index)
+        out = self.output_proj(out)
+        if not self.batch_first:
+            out = out.permute(1, 0, 2)
+        return self.dropout(out) + identity
+
+    def _attention_in_steps(self, value, offsets, logits, reference_points, spatial_shapes, level_start_index):
+        """:283-318 one operation after the other, for what `_attention_2d` does not cover."""
+        bs, Q, _ = offsets.shape
+        H, L, P = self.num_heads, self.num_levels, self.num_points
+        offsets = offsets.view(bs, Q, H, L, P, 2)
+        attn = logits.view(bs, Q, H, L * P).softmax(-1).view(bs, Q, H, L, P)
         if reference_points.shape[-1] == 2:
             normalizer = torch.stack([spatial_shapes[..., 1], spatial_shapes[..., 0]], -1).to(offsets.dtype)
             loc = reference_points[:, :, None, :, None, :] + offsets / normalizer[None, None, None, :, None, :]
@@ -460,12 +519,8 @@ class CustomMSDeformableAttention(nn.Module):
         else:
             raise ValueError("Last dim of reference_points must be 2 or 4, but get "
                              f"{reference_points.shape[-1]} instead.")
-        out = MultiScaleDeformableAttnFunction_fp32.apply(value.contiguous(), spatial_shapes, level_start_index,
-                                                          loc.contiguous(), attn.contiguous(), self.im2col_step)
-        out = self.output_proj(out)
-        if not self.batch_first:
-            out = out.permute(1, 0, 2)
-        return self.dropout(out) + identity
+        return MultiScaleDeformableAttnFunction_fp32.apply(value.contiguous(), spatial_shapes, level_start_index,
+                                                           loc.contiguous(), attn.contiguous(), self.im2col_step)
 
 
 class BEVFormerEncoderLayer(nn.Module):
@@ -477,6 +532,7 @@ class BEVFormerEncoderLayer(nn.Module):
                  bev_h=200, bev_w=200, dropout=0.1):
         super().__init__()
         self.bev_h, self.bev_w = bev_h, bev_w
+        self._tables = None
         self.self_attn = TemporalSelfAttention(embed_dims, num_heads, num_levels=1, num_points=4,
                                                dropout=dropout)
         self.norm0 = AddLayerNorm(embed_dims)
@@ -489,20 +545,29 @@ class BEVFormerEncoderLayer(nn.Module):
                                  Linear(ffn_dims, embed_dims), nn.Dropout(dropout))
         self.norm2 = AddLayerNorm(embed_dims)
 
+    def _bev_tables(self, device, dtype):
+        """Level table of the BEV and the centres of its cells (1, Q, 1, 2): constants of the layer, made once per device
+        and dtype (making them takes a synchronising copy and a dozen small kernels)."""
+        key = (device, dtype, self.bev_h, self.bev_w)
+        if getattr(self, "_tables", None) is None or self._tables[0] != key:
+            self._tables = (key, torch.tensor([[self.bev_h, self.bev_w]], dtype=torch.int64, device=device),
+                            torch.zeros(1, dtype=torch.int64, device=device),
+                            bev_reference_points(self.bev_h, self.bev_w, dim="2d", device=device, dtype=dtype))
+        return self._tables[1:]
+
     def forward(self, query, prev_bev=None, bev_pos=None, ref_2d=None, **cross_kw):
         """query (bs, bev_h*bev_w, E); prev_bev: None or (bs*2, Q, E) = [previous, current] BEV per batch
         element (encoder.py:519-528 stacks them); ref_2d (bs*2, Q, 1, 2) (`bev_reference_points(dim="2d")`,
         shifted for the previous BEV by the caller); cross_kw: the spatial cross-attention's inputs."""
-        dev = query.device
+        if cross_kw.get("rebatch_plan") is None:    # started before the self-attention, whose work hides its read-back
+            cross_kw["rebatch_plan"] = RebatchPlan(cross_kw["bev_mask"])
+        shapes, lsi, cells = self._bev_tables(query.device, query.dtype)
         if ref_2d is None:
-            ref_2d = bev_reference_points(self.bev_h, self.bev_w, dim="2d", bs=query.shape[0] * 2, device=dev,
-                                          dtype=query.dtype)
-        shapes = torch.tensor([[self.bev_h, self.bev_w]], dtype=torch.int64, device=dev)
-        lsi = torch.zeros(1, dtype=torch.int64, device=dev)
+            ref_2d = cells.expand(query.shape[0] * 2, -1, -1, -1)
         query = self.norm0(*self.self_attn(query, value=prev_bev, query_pos=bev_pos, reference_points=ref_2d,
                                            spatial_shapes=shapes, level_start_index=lsi, return_residual=True))
         query = self.norm1(*self.cross_attn(query, return_residual=True, **cross_kw))
-        return self.norm2(self.ffn(query), query)
+        return self.norm2(_run_ffn(self.ffn, query), query)
 
 
 class SCAEncoderStack(nn.Module):

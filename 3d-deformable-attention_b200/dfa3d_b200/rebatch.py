@@ -10,8 +10,9 @@ tensors built by one call (``dfa3d_rebatch_plan``), the rows are PACKED (exactly
 per-camera row offsets so that cameras of different length share one launch.
 
 A plan depends only on ``bev_mask``, which is geometry: build it once per frame and hand it to every
-encoder layer.  Building reads one integer back (the packed row count, needed to size tensors); nothing
-after that synchronises.
+encoder layer.  The packed row count, needed to size tensors, is read back from the device: the copy is queued with
+the plan's kernels, and whoever first asks for ``rows`` waits for it -- so work that does not need the count should be
+queued in between.  Nothing after that synchronises.
 """
 import torch
 from torch.autograd.function import Function, once_differentiable
@@ -54,12 +55,53 @@ class RebatchPlan:
                             self.offsets.data_ptr(), self.op_offsets.data_ptr(), packed_query.data_ptr(),
                             packed_camera.data_ptr(), self.row_of.data_ptr(), self.inv_count.data_ptr(),
                             _stream(mask))
-        counts = self.counts.tolist()            # the one read-back: sizes of the packed tensors
-        self.rows = int(sum(counts))
-        self.max_queries = int(max(counts)) if counts else 0
-        self.packed_query = packed_query[:self.rows]
-        self.packed_camera = packed_camera[:self.rows]
-        self._pq, self._pc = packed_query, packed_camera     # keep the full buffers alive
+        self._pq, self._pc = packed_query, packed_camera
+        # the one read-back: sizes of the packed tensors
+        self._host_counts = torch.empty(cams, dtype=torch.int32, pin_memory=True)
+        self._host_counts.copy_(self.counts, non_blocking=True)
+        self._counted = torch.cuda.Event()
+        self._counted.record(torch.cuda.current_stream(dev))
+        self._sizes = None
+        self._reference = None
+
+    def _resolve(self):
+        if self._sizes is None:
+            self._counted.synchronize()
+            counts = self._host_counts.tolist()
+            self._sizes = (int(sum(counts)), int(max(counts)) if counts else 0)
+            self._native_args = (self._pq, self._pc, self.offsets, self.row_of, self.inv_count, self.cams, self.bs, self.Q,
+                                 self._sizes[0])
+        return self._sizes
+
+    @property
+    def rows(self):
+        return self._resolve()[0]
+
+    @property
+    def max_queries(self):
+        return self._resolve()[1]
+
+    @property
+    def packed_query(self):
+        return self._pq[:self.rows]
+
+    @property
+    def packed_camera(self):
+        return self._pc[:self.rows]
+
+    def reference_rows(self, reference_points_cam):
+        """``gather_per_camera(reference_points_cam, self)``, kept for the other layers of the frame: they are handed
+        the same tensor, which is geometry like the mask."""
+        key = (reference_points_cam, reference_points_cam._version)
+        if self._reference is None or self._reference[0] is not key[0] or self._reference[1] != key[1]:
+            self._reference = key + (gather_per_camera(reference_points_cam, self),)
+        return self._reference[2]
+
+    @property
+    def native_args(self):
+        """The plan as the native host path takes it."""
+        self._resolve()
+        return self._native_args
 
     @property
     def device(self):
@@ -98,6 +140,14 @@ class GatherQueriesFunction(Function):
     """(bs, Q, W) in BEV order -> (bs*T, W) packed rows: row j*T + p holds query packed_query[p] of
     batch element j (spatial_cross_attention.py:714-717).  Backward: sum over the cameras of a query."""
 
+    @classmethod
+    def apply(cls, src, plan):
+        if cls is GatherQueriesFunction:
+            out = _lib.native().gather_queries(src, *plan.native_args)
+            if out is not NotImplemented:
+                return out
+        return super().apply(src, plan)
+
     @staticmethod
     def forward(ctx, src, plan):
         src = _check(src, "src")
@@ -133,6 +183,9 @@ class GatherSharedRowsFunction(Function):
 def gather_per_camera(src, plan):
     """(cams, bs, Q, ...) per-camera rows (the projected reference points, spatial_cross_attention.py:
     718-719) -> (bs*T, ...) packed rows.  No gradient (the reference points come from fixed geometry)."""
+    out = _lib.native().gather_per_camera(src, *plan.native_args)
+    if out is not NotImplemented:
+        return out
     src = _check(src.detach(), "src")
     if tuple(src.shape[:3]) != (plan.cams, plan.bs, plan.Q):
         raise RuntimeError(f"src must be (cams, bs, Q, ...), got {tuple(src.shape)}")
@@ -147,6 +200,14 @@ class CombineCamerasFunction(Function):
     """(bs*T, W) packed per-camera results -> (bs, Q, W): sum over the cameras that see a query, divided
     by their number (at least 1), zeros where no camera sees it (spatial_cross_attention.py:741-748).
     Backward: each packed row receives its query's gradient times the same factor."""
+
+    @classmethod
+    def apply(cls, src, plan):
+        if cls is CombineCamerasFunction:
+            out = _lib.native().combine_cameras(src, *plan.native_args)
+            if out is not NotImplemented:
+                return out
+        return super().apply(src, plan)
 
     @staticmethod
     def forward(ctx, packed, plan):

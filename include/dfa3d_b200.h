@@ -171,6 +171,24 @@ int dfa3d_attn3d_backward(const dfa3d_problem *p, int32_t num_anchors, const voi
                           float *grad_value, float *grad_dist, float *grad_offsets_uv,
                           float *grad_offsets_depth, float *grad_logits, void *stream);
 
+/* The same for the plain 2-D operator, with what BEVFormer's temporal self-attention and decoder do around it
+ * (…/bevformer/modules/temporal_self_attention.py:224-262, decoder.py:283-318):
+ *   loc[b*maps+m,q,h,l,p]  = ref_points[b*maps+m,q,l] + offsets[b,q,h,m,l,p] / (w_l, h_l)
+ *   attn[b*maps+m,q,h,:,:] = softmax over the L*P logits[b,q,h,m,:]
+ *   out[b,q]               = mean over the maps of the 2-D operator on value[b*maps+m]
+ * p describes one map: B batch elements, N pixels, L levels; value (B*maps,N,H,C), ref_points (B*maps,Q,L,2), offsets
+ * (B,Q,H,maps,L,P,2), logits (B,Q,H,maps,L*P), out (B,Q,H*C), all fp32.  dfa3d_attn2d_supported(): 1 for the sizes the
+ * kernels exist for (C of 16, 32 or 64; 4, 8 or 16 points over all maps, a power of two in each), else 0.  Backward:
+ * grad_value is ACCUMULATED into; grad_offsets and grad_logits are overwritten; the reference points get none. */
+int dfa3d_attn2d_supported(const dfa3d_problem *p, int32_t num_maps);
+int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+                         const int64_t *level_start, const float *ref_points, const float *offsets,
+                         const float *logits, float *out, void *stream);
+int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+                          const int64_t *level_start, const float *ref_points, const float *offsets,
+                          const float *logits, const float *grad_out, float *grad_value, float *grad_offsets,
+                          float *grad_logits, void *stream);
+
 /* The one-stage and the offsets/logits entry points for cameras with DIFFERENT numbers of queries
  * (BEVFormer: every camera sees its own subset of the BEV queries; the reference pads all of them to the
  * longest list, spatial_cross_attention.py:707-722).  query_offsets (B+1 int32, device) gives camera b
@@ -200,6 +218,20 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                  const float *ref_points, const float *offsets_uv,
                                  const float *offsets_depth, const float *logits, const float *grad_out,
                                  float *grad_value, float *grad_dist, float *grad_offsets_uv,
+                                 float *grad_offsets_depth, float *grad_logits, void *stream);
+
+/* dfa3d_attn3d_forward / _backward for either form of the queries (query_offsets null: dense) and either form of the level
+ * table: shapes (L, shape_stride) with shape_stride 3 = (h, w, d), or 2 = (h, w) where every level has p->D bins. */
+int dfa3d_attn3d_forward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                                const int32_t *query_offsets, const void *value, const void *dist,
+                                const int64_t *shapes, const int64_t *level_start, const float *ref_points,
+                                const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
+                                void *stream);
+int dfa3d_attn3d_backward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                                 const int32_t *query_offsets, const void *value, const void *dist,
+                                 const int64_t *shapes, const int64_t *level_start, const float *ref_points,
+                                 const float *offsets_uv, const float *offsets_depth, const float *logits,
+                                 const float *grad_out, float *grad_value, float *grad_dist, float *grad_offsets_uv,
                                  float *grad_offsets_depth, float *grad_logits, void *stream);
 
 /* Per-camera re-batching of the BEV queries.  Replaces the host loops of
@@ -328,6 +360,16 @@ int dfa3d_layer_norm_backward(const float *grad_y, const float *in, const float 
  * grad_output.sum(0)).  cols a multiple of 4; dst accumulated into, zeroed by the caller, 16-byte
  * aligned like src. */
 int dfa3d_column_sum(const float *src, int64_t rows, int32_t cols, float *dst, void *stream);
+
+/* y = LayerNorm(x + residual) * gamma + beta where no backward follows: neither the sum nor the statistics are
+ * written.  residual may be null. */
+int dfa3d_add_layer_norm_infer(const float *x, const float *residual, const float *gamma, const float *beta,
+                               int64_t rows, int32_t E, float eps, float *y, void *stream);
+
+/* grad_in = y > 0 ? grad_y : 0 and dst[c] += sum over rows of grad_in[r, c]: the backward of a Linear layer followed by
+ * a ReLU up to the matrix products.  Conditions of dfa3d_column_sum; grad_in may be grad_y. */
+int dfa3d_relu_backward_column_sum(const float *grad_y, const float *y, int64_t rows, int32_t cols, float *grad_in,
+                                   float *dst, void *stream);
 
 /* a[0..na) = 0 and b[0..nb) = 0 with one launch: the two gradients a backward accumulates into.  Either
  * count may be 0 (its pointer is then not looked at); pointers 16-byte aligned. */
