@@ -113,7 +113,7 @@ Tensor attn3d_forward(const Extra &x, const Tensor &value, const Tensor &dist, c
   Tensor out = ragged ? empty_f32({uv.size(0), (int64_t)p.H * p.C}, value)
                       : empty_f32({uv.size(0), uv.size(1), (int64_t)p.H * p.C}, value);
   void *s = stream_of(value);
-  check(lib.dfa3d_attn3d_forward_levels(&p, (int32_t)x.Z, (int32_t)shapes.size(1), ragged ? ip(q_off) : nullptr,
+  check(lib.dfa3d_attn3d_forward_rows(&p, (int32_t)x.Z, (int32_t)shapes.size(1), 0, 0, ragged ? ip(q_off) : nullptr,
                                         value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(uv),
                                         fp(od), fp(logits), fpm(out), s),
         "dfa3d_attn3d_forward");
@@ -141,12 +141,55 @@ struct Attn3dFn : torch::autograd::Function<Attn3dFn> {
     Tensor guv = at::empty_like(uv), god = at::empty_like(od), gl = at::empty_like(logits);
     void *s = stream_of(value);
     zero_two(gv, gd, s);
-    check(lib.dfa3d_attn3d_backward_levels(&x->p, (int32_t)x->Z, (int32_t)v[2].size(1), q_off.defined() ? ip(q_off) : nullptr,
+    check(lib.dfa3d_attn3d_backward_rows(&x->p, (int32_t)x->Z, (int32_t)v[2].size(1), 0, 0, q_off.defined() ? ip(q_off) : nullptr,
                                            value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(v[4]),
                                            fp(uv), fp(od), fp(logits), fp(go), fpm(gv), fpm(gd), fpm(guv), fpm(god), fpm(gl),
                                            s),
           "dfa3d_attn3d_backward");
     return once({gv, gd, Tensor(), Tensor(), Tensor(), guv, god, gl, Tensor(), Tensor()}, grads);
+  }
+};
+
+// ---- the same with offsets, depth offsets and logits side by side in one row per query --------------------
+Tensor attn3d_joint_forward(const Extra &x, const Tensor &value, const Tensor &dist, const Tensor &shapes, const Tensor &lsi,
+                            const Tensor &ref, const Tensor &joint, const Tensor &q_off) {
+  c10::cuda::CUDAGuard guard(value.device());
+  std::vector<int64_t> sz(joint.sizes().begin(), joint.sizes().end());
+  const int64_t row = sz.back(), part = row / 4;
+  sz.back() = (int64_t)x.p.H * x.p.C;
+  Tensor out = empty_f32(sz, value);
+  check(lib.dfa3d_attn3d_forward_rows(&x.p, (int32_t)x.Z, (int32_t)shapes.size(1), row, row, q_off.defined() ? ip(q_off) : nullptr,
+                                      value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(joint),
+                                      fp(joint) + 2 * part, fp(joint) + 3 * part, fpm(out), stream_of(value)),
+        "dfa3d_attn3d_forward");
+  return out;
+}
+
+struct Attn3dJointFn : torch::autograd::Function<Attn3dJointFn> {
+  static Tensor forward(AutogradContext *ctx, const Tensor &value, const Tensor &dist, const Tensor &shapes,
+                        const Tensor &lsi, const Tensor &ref, const Tensor &joint, const std::optional<Tensor> &offsets,
+                        c10::intrusive_ptr<Extra> x) {
+    const Tensor q_off = offsets.value_or(Tensor());
+    ctx->save_for_backward({value, dist, shapes, lsi, ref, joint, q_off});
+    keep(ctx, x);
+    return attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off);
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const auto v = ctx->get_saved_variables();
+    const Tensor &value = v[0], &dist = v[1], &joint = v[5], &q_off = v[6];
+    const auto x = extra_of(ctx);
+    c10::cuda::CUDAGuard guard(value.device());
+    const Tensor go = f32(grads[0]);
+    Tensor gv = empty_f32(value.sizes(), value), gd = empty_f32(dist.sizes(), dist), gj = at::empty_like(joint);
+    const int64_t row = joint.size(-1), part = row / 4;
+    void *s = stream_of(value);
+    zero_two(gv, gd, s);
+    check(lib.dfa3d_attn3d_backward_rows(&x->p, (int32_t)x->Z, (int32_t)v[2].size(1), row, row,
+                                         q_off.defined() ? ip(q_off) : nullptr, value.const_data_ptr(), dist.const_data_ptr(),
+                                         lp(v[2]), lp(v[3]), fp(v[4]), fp(joint), fp(joint) + 2 * part, fp(joint) + 3 * part,
+                                         fp(go), fpm(gv), fpm(gd), fpm(gj), fpm(gj) + 2 * part, fpm(gj) + 3 * part, s),
+          "dfa3d_attn3d_backward");
+    return once({gv, gd, Tensor(), Tensor(), Tensor(), gj, Tensor(), Tensor()}, grads);
   }
 };
 
@@ -281,9 +324,6 @@ struct DistFn : torch::autograd::Function<DistFn> {
 // ------------------------------------------------------------------------------------------------
 // Python entry points (METH_FASTCALL: no tuple, no keyword parsing)
 // ------------------------------------------------------------------------------------------------
-// torch::autograd::Function takes tensors that may be absent as optionals
-std::optional<Tensor> given(const Tensor &t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; }
-
 // (out, score or None)
 PyObject *pair(const variable_list &r) {
   PyObject *res = PyTuple_New(2);
@@ -367,8 +407,7 @@ PyObject *run_fused(PyObject *const *a, Py_ssize_t n, bool ragged, bool fp16) {
   return pair(r);
 }
 
-// flat: the level table may also be (L, 2), D bins in every level (what the attention module holds)
-PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged, bool flat) {
+PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged) {
   // value, dist, shapes, lsi, ref, off_uv, off_d, logits [, q_off, max_queries] [, dist_map]
   const Py_ssize_t fixed = ragged ? 10 : 8;
   if (n < fixed || n > fixed + 1 || !plain_mode()) return not_plain();
@@ -386,7 +425,8 @@ PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged, bool flat) {
   const int64_t B = value.size(0), H = value.size(2), L = uv.size(k + 1), P = uv.size(k + 2), Z = ref.size(k);
   const int64_t pts = uv.numel() / 2;
   if (uv.size(-1) != 2 || uv.size(k) != H || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 ||
-      !(sizes_are(shapes, {L, 3}) || (flat && sizes_are(shapes, {L, 2}))) || lsi.size(0) != L || od.numel() != pts || logits.numel() != pts || ref.size(0) != uv.size(0))
+      !sizes_are(shapes, {L, 3}) || lsi.size(0) != L ||
+      od.numel() != pts || logits.numel() != pts || ref.size(0) != uv.size(0))
     return not_plain();
   auto x = c10::make_intrusive<Extra>();
   dfa3d_problem &p = x->p;
@@ -412,6 +452,52 @@ PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged, bool flat) {
     r = wants_grad(value, dist, uv, od, logits)
             ? Attn3dFn::apply(value, dist, shapes, lsi, ref, uv, od, logits, given(q_off), x)
             : attn3d_forward(*x, value, dist, shapes, lsi, ref, uv, od, logits, q_off);
+  }
+  return THPVariable_Wrap(r);
+}
+
+PyObject *run_attn3d_joint(PyObject *const *a, Py_ssize_t n) {
+  // value (B, N, H*C), dist (B, Nd, D), shapes (L, 2), lsi, ref (.., Z, 3), joint (.., 4*H*L*P), heads, points,
+  // q_off or None, max_queries, dist_map; ".." is B, Q or, with q_off, R
+  int64_t H, P, max_q = 0, mh, mw;
+  if (n != 11 || !plain_mode() || !integer(a[6], H) || !integer(a[7], P) || !map_argument(a[10], mh, mw)) return not_plain();
+  const bool ragged = a[8] != Py_None;
+  const int64_t k = ragged ? 1 : 2;
+  Tensor value, dist, shapes, lsi, ref, joint, q_off;
+  if (!plain_tensor(a[0], value) || value.dim() != 3 || !plain_tensor(a[1], dist) || dist.dim() != 3 ||
+      !long_tensor(a[2], shapes, 2) || !long_tensor(a[3], lsi, 1) || !float_tensor(a[4], ref, k + 2) ||
+      !float_tensor(a[5], joint, k + 1))
+    return not_plain();
+  if (H <= 0 || P <= 0 || value.size(2) % H != 0 || !storage_type(value.scalar_type()) || !storage_type(dist.scalar_type()) ||
+      !small(value) || !small(dist) || !small(joint) || !one_device(value, dist, shapes, lsi, ref, joint) ||
+      ref.requires_grad())
+    return not_plain();
+  const int64_t B = value.size(0), L = shapes.size(0), Z = ref.size(k);
+  if (shapes.size(1) != 2 || lsi.size(0) != L || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 || ref.size(0) != joint.size(0) ||
+      joint.size(-1) != 4 * H * L * P)
+    return not_plain();
+  auto x = c10::make_intrusive<Extra>();
+  dfa3d_problem &p = x->p;
+  memset(&p, 0, sizeof p);
+  p.B = (int32_t)B; p.N = (int32_t)value.size(1); p.H = (int32_t)H; p.C = (int32_t)(value.size(2) / H);
+  p.value_dtype = dtype_code(value);
+  if (!describe_dist(dist, B, value.size(1), H, mh, mw, p)) return not_plain();
+  if (ragged) {
+    if (!plain_tensor(a[8], q_off) || q_off.scalar_type() != at::kInt || q_off.numel() != B + 1 || !one_device(value, q_off) ||
+        !integer(a[9], max_q) || max_q < 0 || max_q >= (int64_t(1) << 31))
+      return not_plain();
+    p.Q = (int32_t)max_q;
+  } else {
+    if (joint.size(0) != B || ref.size(1) != joint.size(1)) return not_plain();
+    p.Q = (int32_t)joint.size(1);
+  }
+  p.L = (int32_t)L; p.P = (int32_t)P;
+  x->Z = Z;
+  Tensor r;
+  {
+    pybind11::gil_scoped_release nogil;
+    r = wants_grad(value, dist, joint) ? Attn3dJointFn::apply(value, dist, shapes, lsi, ref, joint, given(q_off), x)
+                                       : attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off);
   }
   return THPVariable_Wrap(r);
 }
@@ -542,10 +628,9 @@ PyObject *py_calls(PyObject *, PyObject *) { return PyLong_FromLongLong(calls.lo
 FAST(fused, run_fused(a, n, false, false))
 FAST(fused_fp16, run_fused(a, n, false, true))
 FAST(fused_ragged, run_fused(a, n, true, false))
-FAST(attn3d, run_attn3d(a, n, false, false))
-FAST(attn3d_ragged, run_attn3d(a, n, true, false))
-FAST(attn3d_flat, run_attn3d(a, n, false, true))
-FAST(attn3d_ragged_flat, run_attn3d(a, n, true, true))
+FAST(attn3d, run_attn3d(a, n, false))
+FAST(attn3d_ragged, run_attn3d(a, n, true))
+FAST(attn3d_joint, run_attn3d_joint(a, n))
 FAST(wms, run_attn2d(a, n, true, false))
 FAST(wms_fp16, run_attn2d(a, n, true, true))
 FAST(msda, run_attn2d(a, n, false, false))
@@ -559,7 +644,8 @@ PyMethodDef methods[] = {
     {"bind", py_bind, METH_O, nullptr},
     {"entries", py_entries, METH_NOARGS, nullptr},
     {"calls", py_calls, METH_NOARGS, nullptr},
-    FAST(fused), FAST(fused_fp16), FAST(fused_ragged), FAST(attn3d), FAST(attn3d_ragged), FAST(attn3d_flat), FAST(attn3d_ragged_flat), FAST(wms), FAST(wms_fp16),
+    FAST(fused), FAST(fused_fp16), FAST(fused_ragged), FAST(attn3d), FAST(attn3d_ragged), FAST(attn3d_joint),
+    FAST(wms), FAST(wms_fp16),
     FAST(msda), FAST(msda_fp16), FAST(depth_score), FAST(dist_from_logits),
     {nullptr, nullptr, 0, nullptr},
 };

@@ -31,13 +31,13 @@ using torch::autograd::variable_list;
 #define DFA3D_ENTRIES(X)                                                                                 \
   X(dfa3d_last_error) X(dfa3d_depth_score_forward) X(dfa3d_depth_score_backward)                         \
   X(dfa3d_wms_attn_forward) X(dfa3d_wms_attn_backward) X(dfa3d_fused_forward) X(dfa3d_fused_backward)    \
-  X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward_levels) X(dfa3d_attn3d_backward_levels)          \
+  X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward_rows) X(dfa3d_attn3d_backward_rows) \
   X(dfa3d_fused_forward_ragged) X(dfa3d_fused_backward_ragged) \
   X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward_typed)           \
   X(dfa3d_zero_two) X(dfa3d_attn2d_supported) X(dfa3d_attn2d_forward) X(dfa3d_attn2d_backward)           \
   X(dfa3d_rebatch_gather) X(dfa3d_rebatch_combine) X(dfa3d_add_layer_norm_forward)                       \
   X(dfa3d_add_layer_norm_infer) X(dfa3d_layer_norm_backward) X(dfa3d_column_sum)                         \
-  X(dfa3d_relu_backward_column_sum)
+  X(dfa3d_relu_backward_column_sum) X(dfa3d_slice_sum) X(dfa3d_copy_segments)
 
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
@@ -203,6 +203,9 @@ template <typename... T>
 bool wants_grad(const T &...t) {
   return at::GradMode::is_enabled() && (t.requires_grad() || ...);
 }
+
+// torch::autograd::Function takes tensors that may be absent as optionals
+inline std::optional<Tensor> given(const Tensor &t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; }
 
 inline PyObject *not_plain() { Py_RETURN_NOTIMPLEMENTED; }
 

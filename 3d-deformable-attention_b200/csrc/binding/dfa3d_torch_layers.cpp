@@ -10,40 +10,32 @@ namespace {
 // ------------------------------------------------------------------------------------------------
 // Linear
 // ------------------------------------------------------------------------------------------------
-constexpr int64_t kSplitRows = 16384;
-
-// grad_out (rows, out)^T x (rows, in).  Many rows into a small result is one long reduction that cuBLAS gives to few
-// CTAs; as a batch of row slices and a sum it takes a third of the time (layer_ops.weight_gradient).  A number of
-// slices that divides the rows saves the product of what is left over.
-Tensor weight_gradient(const Tensor &g, const Tensor &x) {
-  const int64_t rows = g.size(0);
-  if (rows < kSplitRows) return at::mm(g.t(), x);
-  int64_t splits = 16;
-  for (int64_t s : {16, 18, 15, 20, 14, 12, 21, 10, 22, 24})
-    if (rows % s == 0) {
-      splits = s;
-      break;
-    }
-  const int64_t k = rows / splits, head = k * splits;
-  Tensor w = at::bmm(g.narrow(0, 0, head).view({splits, k, -1}).transpose(1, 2), x.narrow(0, 0, head).view({splits, k, -1}))
-                 .sum(0);
-  if (head < rows) w.addmm_(g.narrow(0, head, rows - head).t(), x.narrow(0, head, rows - head));
-  return w;
-}
-
 Tensor rows_of(const Tensor &t) { return t.view({-1, t.size(-1)}); }
 
-Tensor zeros_f32(int64_t n, const Tensor &like, void *s) {
-  Tensor t = empty_f32({n}, like);
-  zero_two(t, Tensor(), s);
-  return t;
-}
+constexpr int64_t kSplitRows = 16384, kSplits = 16;
 
-Tensor bias_gradient(const Tensor &g) {
+// Weight gradient g^T x of g (rows, out) and x (rows, in), and bias gradient: the column sums of g.  Many rows into a small
+// product is one long reduction that cuBLAS gives to few CTAs; as a batch of 16 row slices, summed by a kernel of our own
+// that also takes the rows left over and zeroes the bias gradient, it takes a third of the time.
+void parameter_gradients(const Tensor &g, const Tensor &x, bool weight, bool bias, Tensor &gw, Tensor &gb) {
+  const int64_t rows = g.size(0), out = g.size(1), in = x.size(1);
   void *s = stream_of(g);
-  Tensor b = zeros_f32(g.size(1), g, s);
-  check(lib.dfa3d_column_sum(fp(g), g.size(0), (int32_t)g.size(1), fpm(b), s), "dfa3d_column_sum");
-  return b;
+  if (bias) gb = empty_f32({out}, g);
+  bool zeroed = false;
+  if (weight && (rows < kSplitRows || in % 4 != 0)) {
+    gw = at::mm(g.t(), x);
+  } else if (weight) {
+    const int64_t k = rows / kSplits, head = k * kSplits;
+    const Tensor part = at::bmm(g.as_strided({kSplits, out, k}, {k * out, 1, out}), x.as_strided({kSplits, k, in}, {k * in, in, 1}));
+    gw = empty_f32({out, in}, g);
+    check(lib.dfa3d_slice_sum(fp(part), (int32_t)kSplits, (int32_t)out, (int32_t)in, fp(g) + head * out, fp(x) + head * in,
+                              (int32_t)(rows - head), fpm(gw), bias ? fpm(gb) : nullptr, s),
+          "dfa3d_slice_sum");
+    zeroed = true;
+  }
+  if (!bias) return;
+  if (!zeroed) zero_two(gb, Tensor(), s);
+  check(lib.dfa3d_column_sum(fp(g), rows, (int32_t)out, fpm(gb), s), "dfa3d_column_sum");
 }
 
 Tensor linear_forward(const Tensor &x, const Tensor &w, const Tensor &b, bool relu) {
@@ -70,46 +62,72 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const Tensor &x = v[0], &w = v[1];
     c10::cuda::CUDAGuard guard(x.device());
     Tensor g = rows_of(f32(grads[0])), gx, gw, gb;
-    if (ctx->saved_data["relu"].toBool()) {
+    const bool relu = ctx->saved_data["relu"].toBool();
+    if (relu) {
       void *s = stream_of(g);
       Tensor masked = at::empty_like(g);
-      gb = zeros_f32(g.size(1), g, s);
+      gb = empty_f32({g.size(1)}, g);
+      zero_two(gb, Tensor(), s);
       check(lib.dfa3d_relu_backward_column_sum(fp(g), fp(v[2]), g.size(0), (int32_t)g.size(1), fpm(masked), fpm(gb), s),
             "dfa3d_relu_backward_column_sum");
       g = masked;
-    } else if (ctx->needs_input_grad(2)) {
-      gb = bias_gradient(g);
     }
     if (ctx->needs_input_grad(0)) gx = at::mm(g, w).view(x.sizes());
-    if (ctx->needs_input_grad(1)) gw = weight_gradient(g, rows_of(x));
+    Tensor none;
+    parameter_gradients(g, rows_of(x), ctx->needs_input_grad(1), !relu && ctx->needs_input_grad(2), gw, relu ? none : gb);
     return once({gx, gw, gb, Tensor()}, grads);
   }
 };
 
-// Three Linear layers of one input: the input's gradient is accumulated inside the products.
-struct Linear3Fn : torch::autograd::Function<Linear3Fn> {
-  static variable_list forward(AutogradContext *ctx, const Tensor &x, const Tensor &w0, const Tensor &b0, const Tensor &w1,
-                               const Tensor &b1, const Tensor &w2, const Tensor &b2) {
+// Two or three Linear layers of one input, run as one with their weights one below the other: y = [y0 | y1 | y2].  One
+// product instead of three each way, one pass over y's gradient for the bias, and the input's gradient is not summed up
+// from parts.
+struct JointLinearFn : torch::autograd::Function<JointLinearFn> {
+  static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w0, const Tensor &b0, const Tensor &w1,
+                        const Tensor &b1, const std::optional<Tensor> &w2, const std::optional<Tensor> &b2) {
     c10::cuda::CUDAGuard guard(x.device());
-    ctx->save_for_backward({x, w0, w1, w2});
-    return {linear_forward(x, w0, b0, false), linear_forward(x, w1, b1, false), linear_forward(x, w2, b2, false)};
+    const Tensor *w[3] = {&w0, &w1, w2 ? &*w2 : nullptr}, *b[3] = {&b0, &b1, b2 ? &*b2 : nullptr};
+    const int n = w2 ? 3 : 2;
+    int64_t out = 0, counts[6];
+    std::vector<int64_t> split;
+    for (int i = 0; i < n; ++i) {
+      split.push_back(w[i]->size(0));
+      out += w[i]->size(0);
+    }
+    Tensor W = at::empty({out, x.size(-1)}, x.options()), B = at::empty({out}, x.options());
+    const float *src[6];
+    float *dst[6], *wd = fpm(W), *bd = fpm(B);
+    for (int i = 0; i < n; ++i) {
+      src[i] = fp(*w[i]); dst[i] = wd; counts[i] = w[i]->numel();
+      src[n + i] = fp(*b[i]); dst[n + i] = bd; counts[n + i] = b[i]->numel();
+      wd += counts[i]; bd += counts[n + i];
+    }
+    check(lib.dfa3d_copy_segments(src, dst, counts, 2 * n, stream_of(x)), "dfa3d_copy_segments");
+    ctx->save_for_backward({x, W});
+    ctx->saved_data["split"] = split;
+    return linear_forward(x, W, B, false);
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const auto v = ctx->get_saved_variables();
-    const Tensor &x = v[0];
+    const Tensor &x = v[0], &W = v[1];
     c10::cuda::CUDAGuard guard(x.device());
-    Tensor gx;
+    const Tensor g = rows_of(f32(grads[0]));
+    const auto split = ctx->saved_data["split"].toIntVector();
     variable_list out(7);
-    for (int i = 0; i < 3; ++i) {
-      const Tensor g = rows_of(f32(grads[i]));
-      if (ctx->needs_input_grad(0)) {
-        if (gx.defined()) gx.addmm_(g, v[1 + i]);
-        else gx = at::mm(g, v[1 + i]);
-      }
-      if (ctx->needs_input_grad(1 + 2 * i)) out[1 + 2 * i] = weight_gradient(g, rows_of(x));
-      if (ctx->needs_input_grad(2 + 2 * i)) out[2 + 2 * i] = bias_gradient(g);
+    bool weight = false, bias = false;
+    for (size_t i = 0; i < split.size(); ++i) {
+      weight |= ctx->needs_input_grad(1 + 2 * i);
+      bias |= ctx->needs_input_grad(2 + 2 * i);
     }
-    if (gx.defined()) out[0] = gx.view(x.sizes());
+    if (ctx->needs_input_grad(0)) out[0] = at::mm(g, W).view(x.sizes());
+    Tensor gw, gb;
+    parameter_gradients(g, rows_of(x), weight, bias, gw, gb);
+    int64_t at = 0;
+    for (size_t i = 0; i < split.size(); ++i) {
+      if (ctx->needs_input_grad(1 + 2 * i)) out[1 + 2 * i] = gw.narrow(0, at, split[i]);
+      if (ctx->needs_input_grad(2 + 2 * i)) out[2 + 2 * i] = gb.narrow(0, at, split[i]);
+      at += split[i];
+    }
     return once(std::move(out), grads);
   }
 };
@@ -136,26 +154,19 @@ PyObject *run_linear(PyObject *const *a, Py_ssize_t n, bool relu) {
   return THPVariable_Wrap(y);
 }
 
-PyObject *run_linear3(PyObject *const *a, Py_ssize_t n) {
-  if (n != 7 || !plain_mode()) return not_plain();
+PyObject *run_joint_linear(PyObject *const *a, Py_ssize_t n) {
+  // x, w0, b0, w1, b1 [, w2, b2]
+  if ((n != 5 && n != 7) || !plain_mode()) return not_plain();
   Tensor x, w[3], b[3];
   if (!float_tensor(a[0], x, -1) || x.dim() < 1 || x.numel() == 0) return not_plain();
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < (n - 1) / 2; ++i)
     if (!linear_arguments(a + 1 + 2 * i, x, w[i], b[i])) return not_plain();
-  variable_list y;
+  Tensor y;
   {
     pybind11::gil_scoped_release nogil;
-    if (wants_grad(x, w[0], b[0], w[1], b[1], w[2], b[2])) {
-      y = Linear3Fn::apply(x, w[0], b[0], w[1], b[1], w[2], b[2]);
-    } else {
-      c10::cuda::CUDAGuard guard(x.device());
-      for (int i = 0; i < 3; ++i) y.push_back(linear_forward(x, w[i], b[i], false));
-    }
+    y = JointLinearFn::apply(x, w[0], b[0], w[1], b[1], given(w[2]), given(b[2]));
   }
-  PyObject *res = PyTuple_New(3);
-  if (!res) throw python_error();
-  for (int i = 0; i < 3; ++i) PyTuple_SET_ITEM(res, i, THPVariable_Wrap(y[i]));
-  return res;
+  return THPVariable_Wrap(y);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -351,61 +362,62 @@ PyObject *run_gather_per_camera(PyObject *const *a, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// 2-D attention from offsets and logits
+// 2-D attention from offsets and logits side by side in one row per query
 // ------------------------------------------------------------------------------------------------
 struct Attn2dExtra : torch::CustomClassHolder {
   dfa3d_problem p;
   int32_t maps = 1;
 };
 
+// Rows of `joint`: offsets, then logits.
 Tensor attn2d_forward(const Attn2dExtra &x, const Tensor &value, const Tensor &shapes, const Tensor &lsi, const Tensor &ref,
-                      const Tensor &off, const Tensor &logits) {
+                      const Tensor &joint) {
   c10::cuda::CUDAGuard guard(value.device());
+  const int64_t row = joint.size(-1);
   Tensor out = empty_f32({x.p.B, x.p.Q, (int64_t)x.p.H * x.p.C}, value);
-  check(lib.dfa3d_attn2d_forward(&x.p, x.maps, value.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(off), fp(logits),
-                                 fpm(out), stream_of(value)),
+  check(lib.dfa3d_attn2d_forward(&x.p, x.maps, row, row, value.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(joint),
+                                 fp(joint) + row / 3 * 2, fpm(out), stream_of(value)),
         "dfa3d_attn2d_forward");
   return out;
 }
 
 struct Attn2dFn : torch::autograd::Function<Attn2dFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &value, const Tensor &shapes, const Tensor &lsi,
-                        const Tensor &ref, const Tensor &off, const Tensor &logits, c10::intrusive_ptr<Attn2dExtra> x) {
-    ctx->save_for_backward({value, shapes, lsi, ref, off, logits});
+                        const Tensor &ref, const Tensor &joint, c10::intrusive_ptr<Attn2dExtra> x) {
+    ctx->save_for_backward({value, shapes, lsi, ref, joint});
     ctx->saved_data["x"] = c10::IValue::make_capsule(x);
-    return attn2d_forward(*x, value, shapes, lsi, ref, off, logits);
+    return attn2d_forward(*x, value, shapes, lsi, ref, joint);
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const auto v = ctx->get_saved_variables();
-    const Tensor &value = v[0], &off = v[4], &logits = v[5];
+    const Tensor &value = v[0], &joint = v[4];
     const auto x = c10::static_intrusive_pointer_cast<Attn2dExtra>(ctx->saved_data.at("x").toCapsule());
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
-    Tensor gv = at::empty_like(value), goff = at::empty_like(off), gl = at::empty_like(logits);
+    Tensor gv = at::empty_like(value), gj = at::empty_like(joint);
+    const int64_t row = joint.size(-1), logits = row / 3 * 2;
     void *s = stream_of(value);
     zero_two(gv, Tensor(), s);
-    check(lib.dfa3d_attn2d_backward(&x->p, x->maps, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(v[3]), fp(off), fp(logits),
-                                    fp(go), fpm(gv), fpm(goff), fpm(gl), s),
+    check(lib.dfa3d_attn2d_backward(&x->p, x->maps, row, row, value.const_data_ptr(), lp(v[1]), lp(v[2]), fp(v[3]), fp(joint),
+                                    fp(joint) + logits, fp(go), fpm(gv), fpm(gj), fpm(gj) + logits, s),
           "dfa3d_attn2d_backward");
-    return once({gv, Tensor(), Tensor(), Tensor(), goff, gl, Tensor()}, grads);
+    return once({gv, Tensor(), Tensor(), Tensor(), gj, Tensor()}, grads);
   }
 };
 
 PyObject *run_attn2d(PyObject *const *a, Py_ssize_t n) {
-  // value (bs*maps, N, H*C), shapes (L, 2), lsi (L), ref (bs*maps, Q, L, 2), offsets (bs, Q, H*maps*L*P*2),
-  // logits (bs, Q, H*maps*L*P), maps, heads, points
+  // value (bs*maps, N, H*C), shapes (L, 2), lsi (L), ref (bs*maps, Q, L, 2), joint (bs, Q, H*maps*L*P*3), maps, heads, points
   int64_t maps, H, P;
-  if (n != 9 || !plain_mode() || !integer(a[6], maps) || !integer(a[7], H) || !integer(a[8], P)) return not_plain();
-  Tensor value, shapes, lsi, ref, off, logits;
+  if (n != 8 || !plain_mode() || !integer(a[5], maps) || !integer(a[6], H) || !integer(a[7], P)) return not_plain();
+  Tensor value, shapes, lsi, ref, joint;
   if (!float_tensor(a[0], value, 3) || !long_tensor(a[1], shapes, 2) || !long_tensor(a[2], lsi, 1) ||
-      !float_tensor(a[3], ref, 4) || !float_tensor(a[4], off, 3) || !float_tensor(a[5], logits, 3))
+      !float_tensor(a[3], ref, 4) || !float_tensor(a[4], joint, 3))
     return not_plain();
   if (maps <= 0 || H <= 0 || P <= 0 || maps > 16 || value.size(2) % H != 0 || value.size(0) % maps != 0 || !small(value) ||
-      !small(off) || !one_device(value, shapes, lsi, ref, off, logits) || ref.requires_grad())
+      !small(joint) || !one_device(value, shapes, lsi, ref, joint) || ref.requires_grad())
     return not_plain();
-  const int64_t bs = value.size(0) / maps, Q = off.size(1), L = shapes.size(0), pts = H * maps * L * P;
-  if (shapes.size(1) != 2 || lsi.size(0) != L || !sizes_are(ref, {bs * maps, Q, L, 2}) || !sizes_are(off, {bs, Q, pts * 2}) ||
-      !sizes_are(logits, {bs, Q, pts}))
+  const int64_t bs = value.size(0) / maps, Q = joint.size(1), L = shapes.size(0), pts = H * maps * L * P;
+  if (shapes.size(1) != 2 || lsi.size(0) != L || !sizes_are(ref, {bs * maps, Q, L, 2}) || !sizes_are(joint, {bs, Q, pts * 3}))
     return not_plain();
   auto x = c10::make_intrusive<Attn2dExtra>();
   dfa3d_problem &p = x->p;
@@ -418,8 +430,8 @@ PyObject *run_attn2d(PyObject *const *a, Py_ssize_t n) {
   Tensor r;
   {
     pybind11::gil_scoped_release nogil;
-    r = wants_grad(value, off, logits) ? Attn2dFn::apply(value, shapes, lsi, ref, off, logits, x)
-                                       : attn2d_forward(*x, value, shapes, lsi, ref, off, logits);
+    r = wants_grad(value, joint) ? Attn2dFn::apply(value, shapes, lsi, ref, joint, x)
+                                 : attn2d_forward(*x, value, shapes, lsi, ref, joint);
   }
   return THPVariable_Wrap(r);
 }
@@ -432,7 +444,7 @@ PyObject *run_attn2d(PyObject *const *a, Py_ssize_t n) {
   }
 FAST(linear, run_linear(a, n, false))
 FAST(linear_relu, run_linear(a, n, true))
-FAST(linear3, run_linear3(a, n))
+FAST(joint_linear, run_joint_linear(a, n))
 FAST(add_layer_norm, run_add_layer_norm(a, n))
 FAST(gather_queries, run_gather(a, n))
 FAST(combine_cameras, run_combine(a, n))
@@ -445,7 +457,7 @@ FAST(attn2d, run_attn2d(a, n))
 namespace dfa3d_torch {
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef layer_methods[] = {
-    FAST(linear), FAST(linear_relu), FAST(linear3), FAST(add_layer_norm), FAST(gather_queries), FAST(combine_cameras),
+    FAST(linear), FAST(linear_relu), FAST(joint_linear), FAST(add_layer_norm), FAST(gather_queries), FAST(combine_cameras),
     FAST(gather_per_camera), FAST(attn2d), {nullptr, nullptr, 0, nullptr},
 };
 #undef FAST

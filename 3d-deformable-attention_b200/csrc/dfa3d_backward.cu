@@ -121,11 +121,12 @@ __device__ __forceinline__ float bwd_point_epilogue(const KArgs &a, const ItemCt
   if (mode_from_offsets(MODE)) {
     // d loc / d offset = 1 / (W, H, D); the logit gradient needs the whole item's dot product and is
     // finished by finish_logit_grads(): park the attention gradient in its slot for now
-    a.grad_logits[pt] = g_attn;
-    float *gu = a.grad_off_uv + pt * 2;
+    const long long lg = (c.attn - a.attn) + j;
+    a.grad_attn[lg] = g_attn;
+    float *gu = a.grad_loc + (c.loc - a.loc) + j * 2;
     gu[0] = s.live ? __fdiv_rn(g_x, (float)s.g.W) : 0.f;
     gu[1] = s.live ? __fdiv_rn(g_y, (float)s.g.Hh) : 0.f;
-    if (MODE == kCallerFused) a.grad_off_d[pt] = __fdiv_rn(g_z, (float)a.D);
+    if (MODE == kCallerFused) a.grad_off_d[lg] = __fdiv_rn(g_z, (float)a.D);
     return s.aw * g_attn;
   }
   a.grad_attn[pt] = g_attn;
@@ -139,16 +140,16 @@ __device__ __forceinline__ float bwd_point_epilogue(const KArgs &a, const ItemCt
 }
 
 // Softmax backward of the item's logits: grad_logit_j = a_j * (g_j - sum_k a_k g_k).  `partial` is the
-// lane's share of the sum; the g_j were parked in grad_logits by the epilogue (each lane re-reads only
+// lane's share of the sum; the g_j were parked in grad_attn by the epilogue (each lane re-reads only
 // what it wrote itself).
 __device__ __forceinline__ void finish_logit_grads(const KArgs &a, const ItemCtx &c, int lane,
                                                    const SoftmaxStats &sm, float partial) {
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) partial += __shfl_xor_sync(0xffffffffu, partial, s);
   for (int j = lane; j < a.LP; j += 32) {
-    const long long pt = c.pt0 + j;
-    const float aw = __fdiv_rn(expf(__ldg(a.logits + pt) - sm.mx), sm.sum);
-    a.grad_logits[pt] = aw * (a.grad_logits[pt] - partial);
+    float *g = a.grad_attn + (c.attn - a.attn) + j;
+    const float aw = __fdiv_rn(expf(__ldg(c.attn + j) - sm.mx), sm.sum);
+    *g = aw * (*g - partial);
   }
 }
 
@@ -302,7 +303,7 @@ dfa3d_backward_kernel(const KArgs a) {
 #pragma unroll 1
   for (int it = 0; it < DFA3D_BWD_ITEMS_PER_WARP; ++it) {
     ItemCtx c;
-    if (!item_context<DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_BWD_ITEMS_PER_WARP + it, c)) return;
+    if (!item_context<MODE, DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_BWD_ITEMS_PER_WARP + it, c)) return;
     backward_item<VT, DT, C, MODE, FULL>(a, lv, c, rows[warp], dots[warp], lane);
   }
 }
@@ -356,15 +357,13 @@ dfa3d_backward_packed_kernel(const KArgs a) {
       c.bq = q0 + q;
     }
     c.item = q0 * a.H + idx;
-    c.pt0 = c.item * LP;
-    c.loc = a.loc + c.pt0 * a.loc_stride;        // (not dereferenced in caller-fused mode)
-    c.attn = a.attn + c.pt0;
+    item_inputs<MODE>(a, c);
     const int j = live ? lane % LP : a.LP;       // a.LP: no such point, the lane stays idle
     SoftmaxStats sm{0.f, 1.f};
     // lanes of a softmax: the item's LP, in 2-D those of one map
     const int half = (MODE == kCallerFused2D ? LP / a.maps : LP) / 2;
     if (mode_from_offsets(MODE)) {
-      const float lg = live ? __ldg(a.logits + c.pt0 + j) : -INFINITY;
+      const float lg = live ? __ldg(c.attn + j) : -INFINITY;
       float mx = lg;
       for (int s = half; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
       float sum = live ? expf(lg - mx) : 0.f;
@@ -442,10 +441,13 @@ dfa3d_backward_packed_kernel(const KArgs a) {
     float part = bwd_point_epilogue<DT, MODE>(a, c, j, st, tt);
     if (mode_from_offsets(MODE)) {
       // softmax backward, grad_logit_j = a_j * (g_j - sum_k a_k g_k): the sum runs over the softmax's lanes; g_j was
-      // parked in grad_logits by the epilogue.  2-D: the weight in hand is a_j / maps.
+      // parked in grad_attn by the epilogue.  2-D: the weight in hand is a_j / maps.
       for (int s = half; s > 0; s >>= 1) part += __shfl_xor_sync(0xffffffffu, part, s);
       if (MODE == kCallerFused2D) part *= (float)a.maps;
-      if (live) a.grad_logits[c.pt0 + j] = st.aw * (a.grad_logits[c.pt0 + j] - part);
+      if (live) {
+        float *g = a.grad_attn + (c.attn - a.attn) + j;
+        *g = st.aw * (*g - part);
+      }
     }
     __syncwarp();
   }
@@ -463,7 +465,7 @@ dfa3d_backward_generic_kernel(const KArgs a) {
   stage_levels(lv, a);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ItemCtx c;
-  if (!item_context(a, warp, blockIdx.x, c)) return;
+  if (!item_context<MODE>(a, warp, blockIdx.x, c)) return;
   const int C = a.C;
   const long long slice = ((long long)c.b * a.N * a.H + c.h) * C;
   const VT *vbase = reinterpret_cast<const VT *>(a.value) + slice;

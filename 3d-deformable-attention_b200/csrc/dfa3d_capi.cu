@@ -91,6 +91,12 @@ dfa3d::KArgs base_args(const dfa3d_problem *p, int shape_stride, int loc_stride)
   return a;
 }
 
+// Elements from query to query of the offsets and of the logits (and depth offsets); 0: they are contiguous.
+void set_rows(dfa3d::KArgs &a, int64_t offsets_row, int64_t logits_row) {
+  a.row_loc = offsets_row ? offsets_row : (int64_t)a.H * a.LP * 2;
+  a.row_attn = logits_row ? logits_row : (int64_t)a.H * a.LP;
+}
+
 int finish(cudaError_t e, const char *what) {
   if (e != cudaSuccess)
     return fail(DFA3D_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -280,6 +286,7 @@ int dfa3d_msda_backward(const dfa3d_problem *p, const void *value, const int64_t
 }
 
 static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                               int64_t offsets_row, int64_t logits_row,
                                const int32_t *query_offsets, const void *value, const void *dist,
                                const int64_t *shapes3, const int64_t *level_start,
                                const float *ref_points, const float *offsets_uv,
@@ -298,7 +305,8 @@ static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int3
   REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(out);
   dfa3d::KArgs a = base_args(p, shape_stride, 3);
   a.value = value; a.dist = dist; a.shapes = shapes3; a.lsi = level_start; a.ref = ref_points;
-  a.off_uv = offsets_uv; a.off_d = offsets_depth; a.logits = logits; a.Z = num_anchors; a.out = out;
+  a.loc = offsets_uv; a.off_d = offsets_depth; a.attn = logits; a.Z = num_anchors; a.out = out;
+  set_rows(a, offsets_row, logits_row);
   a.q_off = query_offsets;
   return finish(dfa3d::launch_forward(a, p->value_dtype,
                                       p->dist_dtype, dfa3d::kCallerFused,
@@ -310,7 +318,7 @@ int dfa3d_attn3d_forward(const dfa3d_problem *p, int32_t num_anchors, const void
                          const void *dist, const int64_t *shapes3, const int64_t *level_start,
                          const float *ref_points, const float *offsets_uv, const float *offsets_depth,
                          const float *logits, float *out, void *stream) {
-  return attn3d_forward_impl(p, num_anchors, 3, nullptr, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, nullptr, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
@@ -321,11 +329,12 @@ int dfa3d_attn3d_forward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                 const float *offsets_depth, const float *logits, float *out,
                                 void *stream) {
   REQUIRE_PTR(query_offsets);
-  return attn3d_forward_impl(p, num_anchors, 3, query_offsets, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, query_offsets, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
 static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+                               int64_t offsets_row, int64_t logits_row,
                                 const int32_t *query_offsets, const void *value, const void *dist,
                                 const int64_t *shapes3, const int64_t *level_start,
                                 const float *ref_points, const float *offsets_uv,
@@ -346,9 +355,10 @@ static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors, int
   REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(grad_out); REQUIRE_ALIGNED(grad_value);
   dfa3d::KArgs a = base_args(p, shape_stride, 3);
   a.value = value; a.dist = dist; a.shapes = shapes3; a.lsi = level_start; a.ref = ref_points;
-  a.off_uv = offsets_uv; a.off_d = offsets_depth; a.logits = logits; a.Z = num_anchors;
+  a.loc = offsets_uv; a.off_d = offsets_depth; a.attn = logits; a.Z = num_anchors;
+  set_rows(a, offsets_row, logits_row);
   a.grad_out = grad_out; a.grad_value = grad_value; a.grad_dist = grad_dist;
-  a.grad_off_uv = grad_offsets_uv; a.grad_off_d = grad_offsets_depth; a.grad_logits = grad_logits;
+  a.grad_loc = grad_offsets_uv; a.grad_off_d = grad_offsets_depth; a.grad_attn = grad_logits;
   a.q_off = query_offsets;
   return finish(dfa3d::launch_backward(a, p->value_dtype,
                                        p->dist_dtype, dfa3d::kCallerFused,
@@ -362,7 +372,7 @@ int dfa3d_attn3d_backward(const dfa3d_problem *p, int32_t num_anchors, const voi
                           const float *offsets_depth, const float *logits, const float *grad_out,
                           float *grad_value, float *grad_dist, float *grad_offsets_uv,
                           float *grad_offsets_depth, float *grad_logits, void *stream) {
-  return attn3d_backward_impl(p, num_anchors, 3, nullptr, value, dist, shapes3, level_start, ref_points,
+  return attn3d_backward_impl(p, num_anchors, 3, 0, 0, nullptr, value, dist, shapes3, level_start, ref_points,
                               offsets_uv, offsets_depth, logits, grad_out, grad_value, grad_dist,
                               grad_offsets_uv, grad_offsets_depth, grad_logits, stream);
 }
@@ -375,27 +385,29 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                  float *grad_value, float *grad_dist, float *grad_offsets_uv,
                                  float *grad_offsets_depth, float *grad_logits, void *stream) {
   REQUIRE_PTR(query_offsets);
-  return attn3d_backward_impl(p, num_anchors, 3, query_offsets, value, dist, shapes3, level_start,
+  return attn3d_backward_impl(p, num_anchors, 3, 0, 0, query_offsets, value, dist, shapes3, level_start,
                               ref_points, offsets_uv, offsets_depth, logits, grad_out, grad_value,
                               grad_dist, grad_offsets_uv, grad_offsets_depth, grad_logits, stream);
 }
 
-int dfa3d_attn3d_forward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+int dfa3d_attn3d_forward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
+                             int64_t logits_row,
                                 const int32_t *query_offsets, const void *value, const void *dist,
                                 const int64_t *shapes, const int64_t *level_start, const float *ref_points,
                                 const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
                                 void *stream) {
-  return attn3d_forward_impl(p, num_anchors, shape_stride, query_offsets, value, dist, shapes, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, shape_stride, offsets_row, logits_row, query_offsets, value, dist, shapes, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
-int dfa3d_attn3d_backward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+int dfa3d_attn3d_backward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
+                             int64_t logits_row,
                                  const int32_t *query_offsets, const void *value, const void *dist,
                                  const int64_t *shapes, const int64_t *level_start, const float *ref_points,
                                  const float *offsets_uv, const float *offsets_depth, const float *logits,
                                  const float *grad_out, float *grad_value, float *grad_dist, float *grad_offsets_uv,
                                  float *grad_offsets_depth, float *grad_logits, void *stream) {
-  return attn3d_backward_impl(p, num_anchors, shape_stride, query_offsets, value, dist, shapes, level_start, ref_points,
+  return attn3d_backward_impl(p, num_anchors, shape_stride, offsets_row, logits_row, query_offsets, value, dist, shapes, level_start, ref_points,
                               offsets_uv, offsets_depth, logits, grad_out, grad_value, grad_dist, grad_offsets_uv,
                               grad_offsets_depth, grad_logits, stream);
 }
@@ -408,7 +420,7 @@ int dfa3d_attn2d_supported(const dfa3d_problem *p, int32_t num_maps) {
          dfa3d::attn2d_supported(p->C, p->L * p->P, num_maps);
 }
 
-static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                        const int64_t *level_start, const float *ref_points, const float *offsets,
                        const float *logits, dfa3d::KArgs &a) {
   if (int rc = check_problem(p, true, false)) return rc;
@@ -422,33 +434,35 @@ static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, const void *val
   q.N *= num_maps;
   q.L *= num_maps;
   a = base_args(&q, 2, 2);
-  a.value = value; a.shapes = shapes2; a.lsi = level_start; a.ref = ref_points; a.off_uv = offsets; a.logits = logits;
+  a.value = value; a.shapes = shapes2; a.lsi = level_start; a.ref = ref_points; a.loc = offsets; a.attn = logits;
   a.maps = num_maps;
+  set_rows(a, offsets_row, logits_row);
+  if (a.row_loc % 2 != 0) return fail(DFA3D_ERR_INVALID_ARGUMENT, "offsets_row must be even (got %lld)", (long long)a.row_loc);
   return DFA3D_OK;
 }
 
-int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                          const int64_t *level_start, const float *ref_points, const float *offsets,
                          const float *logits, float *out, void *stream) {
   if (p && (p->B == 0 || p->Q == 0)) return check_problem(p, true, false);
   dfa3d::KArgs a;
-  if (int rc = attn2d_args(p, num_maps, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
+  if (int rc = attn2d_args(p, num_maps, offsets_row, logits_row, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
   REQUIRE_PTR(out); REQUIRE_ALIGNED(out);
   a.out = out;
   return finish(dfa3d::launch_forward(a, p->value_dtype, DFA3D_DTYPE_F32, dfa3d::kCallerFused2D, (cudaStream_t)stream),
                 "dfa3d_attn2d_forward launch");
 }
 
-int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                           const int64_t *level_start, const float *ref_points, const float *offsets,
                           const float *logits, const float *grad_out, float *grad_value, float *grad_offsets,
                           float *grad_logits, void *stream) {
   if (p && (p->B == 0 || p->Q == 0)) return check_problem(p, true, false);
   dfa3d::KArgs a;
-  if (int rc = attn2d_args(p, num_maps, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
+  if (int rc = attn2d_args(p, num_maps, offsets_row, logits_row, value, shapes2, level_start, ref_points, offsets, logits, a)) return rc;
   REQUIRE_PTR(grad_out); REQUIRE_PTR(grad_value); REQUIRE_PTR(grad_offsets); REQUIRE_PTR(grad_logits);
   REQUIRE_ALIGNED(grad_out); REQUIRE_ALIGNED(grad_value);
-  a.grad_out = grad_out; a.grad_value = grad_value; a.grad_off_uv = grad_offsets; a.grad_logits = grad_logits;
+  a.grad_out = grad_out; a.grad_value = grad_value; a.grad_loc = grad_offsets; a.grad_attn = grad_logits;
   return finish(dfa3d::launch_backward(a, p->value_dtype, DFA3D_DTYPE_F32, dfa3d::kCallerFused2D, (cudaStream_t)stream),
                 "dfa3d_attn2d_backward launch");
 }
@@ -635,6 +649,32 @@ int dfa3d_relu_backward_column_sum(const float *grad_y, const float *y, int64_t 
   REQUIRE_ALIGNED(grad_y); REQUIRE_ALIGNED(y); REQUIRE_ALIGNED(grad_in); REQUIRE_ALIGNED(dst);
   return finish(dfa3d::launch_relu_backward(grad_y, y, rows, cols, grad_in, dst, (cudaStream_t)stream),
                 "dfa3d_relu_backward_column_sum launch");
+}
+
+int dfa3d_slice_sum(const float *partial, int32_t slices, int32_t out, int32_t in, const float *grad_tail,
+                    const float *x_tail, int32_t tail_rows, float *dst, float *zeroed, void *stream) {
+  if (slices <= 0 || out <= 0 || in <= 0 || tail_rows < 0)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "slices, out, in must be positive and tail_rows >= 0 (got %d %d %d %d)", slices,
+                out, in, tail_rows);
+  if (in % 4 != 0) return fail(DFA3D_ERR_UNSUPPORTED, "in=%d must be a multiple of 4", in);
+  REQUIRE_PTR(partial); REQUIRE_PTR(dst); REQUIRE_ALIGNED(partial); REQUIRE_ALIGNED(dst);
+  if (tail_rows > 0) { REQUIRE_PTR(grad_tail); REQUIRE_PTR(x_tail); REQUIRE_ALIGNED(x_tail); }
+  return finish(dfa3d::launch_slice_sum(partial, slices, out, in, grad_tail, x_tail, tail_rows, dst, zeroed,
+                                        (cudaStream_t)stream),
+                "dfa3d_slice_sum launch");
+}
+
+int dfa3d_copy_segments(const float *const *src, float *const *dst, const int64_t *counts, int32_t n, void *stream) {
+  if (n < 0 || n > 8) return fail(DFA3D_ERR_INVALID_ARGUMENT, "0 to 8 segments (got %d)", n);
+  if (n == 0) return DFA3D_OK;
+  REQUIRE_PTR(src); REQUIRE_PTR(dst); REQUIRE_PTR(counts);
+  long long c[8];
+  for (int i = 0; i < n; ++i) {
+    if (counts[i] < 0) return fail(DFA3D_ERR_INVALID_ARGUMENT, "segment %d: count must be >= 0", i);
+    if (counts[i] > 0) { REQUIRE_PTR(src[i]); REQUIRE_PTR(dst[i]); }
+    c[i] = counts[i];
+  }
+  return finish(dfa3d::launch_copy_segments(src, dst, c, n, (cudaStream_t)stream), "dfa3d_copy_segments launch");
 }
 
 int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream) {

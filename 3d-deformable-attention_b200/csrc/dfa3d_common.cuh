@@ -80,12 +80,12 @@ struct KArgs {
   const float *grad_out;   // (B,Q,H*C)
   // caller-fused mode: locations and attention weights are formed inside the kernel
   const float *ref;        // (B,Q,Z,3) reference points; 2-D: (B*maps,Q,L/maps,2)
-  const float *off_uv;     // (B,Q,H,L,P,2) raw x/y offsets in pixels
-  const float *off_d;      // (B,Q,H,L,P) raw depth offsets in bins
-  const float *logits;     // (B,Q,H,L*P) raw attention logits
-  float *grad_off_uv;      // (B,Q,H,L,P,2), overwritten
+                           //   loc = raw x/y offsets in pixels (B,Q,H,L,P,2), attn = raw logits (B,Q,H,L*P); so
+                           //   are their gradients.  A query's rows of them may lie apart (all three are then
+                           //   parts of one row that a single Linear layer produced)
+  const float *off_d;      // (B,Q,H,L,P) raw depth offsets in bins, rows like those of the logits
   float *grad_off_d;       // (B,Q,H,L,P), overwritten
-  float *grad_logits;      // (B,Q,H,L*P), overwritten
+  long long row_loc, row_attn;  // elements from query to query of loc, and of attn and off_d
   int Z;                   // reference points (pillar anchors) per query
   int maps;                // 2-D: value maps per batch element; N and L count all of them.  0 elsewhere
   // ragged queries: camera b owns the packed query rows [q_off[b], q_off[b+1]) of every per-query
@@ -148,7 +148,20 @@ struct ItemCtx {
 // blockIdx.y (+ b0) selects the camera; the CTA's `group`-th group of kWarpsPerCta items starts at
 // (blockIdx.x * groups_per_cta + group) * kWarpsPerCta, warp w takes item w of it: a (query, head)
 // pair of that camera.  Returns false for the warps past the end of the camera.
-template <bool HEAD_MAJOR = false>
+// Where the item's locations and weights start (a query's rows may lie apart in the caller-fused modes).
+template <int MODE>
+__device__ __forceinline__ void item_inputs(const KArgs &a, ItemCtx &c) {
+  c.pt0 = c.item * a.LP;
+  if (mode_from_offsets(MODE)) {
+    c.loc = a.loc + (c.bq * a.row_loc + c.h * (a.LP * 2));
+    c.attn = a.attn + (c.bq * a.row_attn + c.h * a.LP);
+  } else {
+    c.loc = a.loc + c.pt0 * a.loc_stride;
+    c.attn = a.attn + c.pt0;
+  }
+}
+
+template <int MODE, bool HEAD_MAJOR = false>
 __device__ __forceinline__ bool item_context(const KArgs &a, int warp, unsigned group, ItemCtx &c) {
   const unsigned idx = group * kWarpsPerCta + warp;
   if (idx >= (unsigned)a.items_per_cam) return false;
@@ -178,9 +191,7 @@ __device__ __forceinline__ bool item_context(const KArgs &a, int warp, unsigned 
       c.item = (long long)c.b * a.items_per_cam + idx;
     }
   }
-  c.pt0 = c.item * a.LP;
-  c.loc = a.loc + c.pt0 * a.loc_stride;      // (not dereferenced in caller-fused mode)
-  c.attn = a.attn + c.pt0;
+  item_inputs<MODE>(a, c);
   return true;
 }
 
@@ -191,7 +202,7 @@ struct SoftmaxStats {
 };
 
 __device__ __forceinline__ SoftmaxStats item_softmax_stats(const KArgs &a, const ItemCtx &c, int lane) {
-  const float *lg = a.logits + c.pt0;
+  const float *lg = c.attn;
   float mx = -INFINITY;
   for (int j = lane; j < a.LP; j += 32) mx = fmaxf(mx, __ldg(lg + j));
 #pragma unroll
@@ -214,21 +225,21 @@ __device__ __forceinline__ void read_point(const KArgs &a, const LevelTable &lv,
   if (MODE == kCallerFused) {
     const int zi = (j - l * a.P) % a.Z;
     const float *r = a.ref + (c.bq * a.Z + zi) * 3;
-    const float *o = a.off_uv + (c.pt0 + j) * 2;
+    const float *o = c.loc + j * 2;
     x = __fadd_rn(__ldg(r), __fdiv_rn(__ldg(o), (float)lv.w[l]));
     y = __fadd_rn(__ldg(r + 1), __fdiv_rn(__ldg(o + 1), (float)lv.h[l]));
-    z = __fadd_rn(__ldg(r + 2), __fdiv_rn(__ldg(a.off_d + c.pt0 + j), (float)a.D));
-    aw = __fdiv_rn(expf(__ldg(a.logits + c.pt0 + j) - sm.mx), sm.sum);
+    z = __fadd_rn(__ldg(r + 2), __fdiv_rn(__ldg(a.off_d + (c.attn - a.attn) + j), (float)a.D));
+    aw = __fdiv_rn(expf(__ldg(c.attn + j) - sm.mx), sm.sum);
   } else if (MODE == kCallerFused2D) {
     const int per_map = a.L / a.maps, map = l / per_map;
     const long long q = c.bq - (long long)c.b * a.Q;
     const float2 r = __ldg(reinterpret_cast<const float2 *>(a.ref) +
                            ((((long long)c.b * a.maps + map) * a.Q + q) * per_map + (l - map * per_map)));
-    const float2 o = __ldg(reinterpret_cast<const float2 *>(a.off_uv) + (c.pt0 + j));
+    const float2 o = __ldg(reinterpret_cast<const float2 *>(c.loc) + j);
     x = __fadd_rn(r.x, __fdiv_rn(o.x, (float)lv.w[l]));
     y = __fadd_rn(r.y, __fdiv_rn(o.y, (float)lv.h[l]));
     z = 0.f;
-    aw = __fdiv_rn(expf(__ldg(a.logits + c.pt0 + j) - sm.mx), sm.sum * (float)a.maps);
+    aw = __fdiv_rn(expf(__ldg(c.attn + j) - sm.mx), sm.sum * (float)a.maps);
   } else {
     const float *lp = c.loc + j * a.loc_stride;
     x = __ldg(lp);

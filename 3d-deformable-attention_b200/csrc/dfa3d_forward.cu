@@ -161,7 +161,7 @@ dfa3d_forward_kernel(const KArgs a) {
 #pragma unroll 1
   for (int it = 0; it < DFA3D_FWD_ITEMS_PER_WARP; ++it) {
     ItemCtx c;
-    if (!item_context<DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_FWD_ITEMS_PER_WARP + it, c)) return;
+    if (!item_context<MODE, DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_FWD_ITEMS_PER_WARP + it, c)) return;
     forward_item<VT, DT, C, MODE, WRITE_DS, FULL>(a, lv, c, rows[warp], lane);
   }
 }
@@ -177,7 +177,7 @@ dfa3d_forward_generic_kernel(const KArgs a) {
   stage_levels(lv, a);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ItemCtx c;
-  if (!item_context(a, warp, blockIdx.x, c)) return;
+  if (!item_context<MODE>(a, warp, blockIdx.x, c)) return;
   const int C = a.C;
   const VT *vbase = reinterpret_cast<const VT *>(a.value) + ((long long)c.b * a.N * a.H + c.h) * C;
   RowEntry *my = rows[warp];
@@ -295,14 +295,12 @@ dfa3d_forward_packed_kernel(const KArgs a) {
       c.h = (int)(idx - q * (unsigned)a.H);
       c.bq = q0 + q;
       c.item = q0 * a.H + idx;
-      c.pt0 = c.item * LP;
-      c.loc = a.loc + c.pt0 * a.loc_stride;      // (not dereferenced in caller-fused mode)
-      c.attn = a.attn + c.pt0;
+      item_inputs<MODE>(a, c);
       const int j = lane % LP;
       SoftmaxStats sm{0.f, 1.f};
       if (mode_from_offsets(MODE)) {             // softmax over the item's LP logits (2-D: of each map): its own lanes
         const int half = (MODE == kCallerFused2D ? LP / a.maps : LP) / 2;
-        const float lg = live ? __ldg(a.logits + c.pt0 + j) : -INFINITY;
+        const float lg = live ? __ldg(c.attn + j) : -INFINITY;
         float mx = lg;
         for (int s = half; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
         float sum = live ? expf(lg - mx) : 0.f;

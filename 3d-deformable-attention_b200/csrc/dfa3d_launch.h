@@ -70,5 +70,8 @@ cudaError_t launch_layer_norm_backward(const float *grad_y, const float *in, con
 cudaError_t launch_column_sum(const float *src, long long rows, int cols, float *dst, cudaStream_t s);
 cudaError_t launch_relu_backward(const float *grad_y, const float *y, long long rows, int cols, float *grad_in, float *dst,
                                  cudaStream_t s);
+cudaError_t launch_slice_sum(const float *part, int slices, int out, int in, const float *g_tail, const float *x_tail, int tail,
+                             float *dst, float *zero, cudaStream_t s);
+cudaError_t launch_copy_segments(const float *const *src, float *const *dst, const long long *n, int count, cudaStream_t s);
 cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cudaStream_t s);
 }  // namespace dfa3d

@@ -12,6 +12,8 @@
 // shared memory and added to the caller-zeroed output with one `red.global.add.f32` per column and CTA.
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "dfa3d_launch.h"
 
 namespace dfa3d {
@@ -277,6 +279,58 @@ relu_backward_kernel(const float *grad_y, const float *__restrict__ y, long long
   }
 }
 
+// Last step of a weight gradient formed as a batch of row slices: dst (out, in) = sum of the `slices` partial products,
+// plus the outer products of the few rows that no slice covers.  Zeroes the bias gradient on the way (the column sum that
+// follows accumulates into it): one launch instead of a reduction, a product of 15 rows and a fill.  Bound by reading the
+// slices.
+__global__ void __launch_bounds__(256)
+slice_sum_kernel(const float *__restrict__ part, int slices, int out, int in, const float *__restrict__ g_tail,
+                 const float *__restrict__ x_tail, int tail, float *__restrict__ dst, float *__restrict__ zero) {
+  const long long n4 = (long long)out * in / 4, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (zero && t < out) zero[t] = 0.f;
+  if (t >= n4) return;
+  float4 acc = ld4_stream(part + t * 4);
+  int s = 1;
+  constexpr int U = 5;                       // 16 slices: three rounds of five
+  for (; s + U <= slices; s += U) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = ld4_stream(part + ((s + u) * n4 + t) * 4);
+#pragma unroll
+    for (int u = 0; u < U; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+  }
+  for (; s < slices; ++s) {
+    const float4 v = ld4_stream(part + (s * n4 + t) * 4);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  const int o = (int)(t * 4 / in), i = (int)(t * 4 - (long long)o * in);
+#pragma unroll 5
+  for (int r = 0; r < tail; ++r) {
+    const float g = __ldg(g_tail + (long long)r * out + o);
+    const float4 x = ld4(x_tail + (long long)r * in + i);
+    acc.x = fmaf(g, x.x, acc.x); acc.y = fmaf(g, x.y, acc.y); acc.z = fmaf(g, x.z, acc.z); acc.w = fmaf(g, x.w, acc.w);
+  }
+  st4(dst + t * 4, acc);
+}
+
+// Up to eight buffers, one after the other, into as many places: the weights and biases of Linear layers that are run as
+// one.
+struct Segments {
+  const float *src[8];
+  float *dst[8];
+  long long n[8];
+};
+__global__ void __launch_bounds__(256) copy_segments_kernel(const Segments s) {
+  const float *src = s.src[blockIdx.y];
+  float *dst = s.dst[blockIdx.y];
+  const long long n = s.n[blockIdx.y], step = (long long)gridDim.x * blockDim.x;
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
+  const long long n4 = vec ? n >> 2 : 0;
+  for (long long t = t0; t < n4; t += step) st4(dst + t * 4, ld4(src + t * 4));
+  for (long long t = n4 * 4 + t0; t < n; t += step) dst[t] = __ldg(src + t);
+}
+
 // Zeroes two buffers with one launch (a backward zeroes the two gradients it accumulates into; for a small
 // problem a second fill is a launch gap longer than the fill).  16-byte stores, the ragged ends one by one.
 __global__ void __launch_bounds__(256) zero_two_kernel(float *a, long long na, float *b, long long nb) {
@@ -363,6 +417,26 @@ cudaError_t launch_relu_backward(const float *grad_y, const float *y, long long 
   if (gx > most) gx = most;
   if (gx < 1) gx = 1;
   relu_backward_kernel<<<dim3((unsigned)gx, bands, 1), kCsThreads, 0, s>>>(grad_y, y, rows, cols, grad_in, dst);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_slice_sum(const float *part, int slices, int out, int in, const float *g_tail, const float *x_tail, int tail,
+                             float *dst, float *zero, cudaStream_t s) {
+  const long long n = std::max((long long)out * in / 4, (long long)out);
+  slice_sum_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(part, slices, out, in, g_tail, x_tail, tail, dst, zero);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_copy_segments(const float *const *src, float *const *dst, const long long *n, int count, cudaStream_t s) {
+  Segments g;
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    g.src[i] = src[i]; g.dst[i] = dst[i]; g.n[i] = n[i];
+    most = std::max(most, n[i]);
+  }
+  if (most == 0) return cudaSuccess;
+  const unsigned gx = (unsigned)std::min((most / 4 + 255) / 256 + 1, 148LL * 2);
+  copy_segments_kernel<<<dim3(gx, (unsigned)count), 256, 0, s>>>(g);
   return cudaGetLastError();
 }
 

@@ -67,10 +67,10 @@ _I32, _I64 = ctypes.c_int32, ctypes.c_int64
 # entry points without a problem descriptor: explicit argument types
 PLAIN_ENTRY_POINTS = {
     "dfa3d_attn2d_supported": [_P, _I32],
-    "dfa3d_attn2d_forward": [_P, _I32] + [_V] * 8,
-    "dfa3d_attn2d_backward": [_P, _I32] + [_V] * 11,
-    "dfa3d_attn3d_forward_levels": [_P, _I32, _I32] + [_V] * 11,
-    "dfa3d_attn3d_backward_levels": [_P, _I32, _I32] + [_V] * 16,
+    "dfa3d_attn2d_forward": [_P, _I32, _I64, _I64] + [_V] * 8,
+    "dfa3d_attn2d_backward": [_P, _I32, _I64, _I64] + [_V] * 11,
+    "dfa3d_attn3d_forward_rows": [_P, _I32, _I32, _I64, _I64] + [_V] * 11,
+    "dfa3d_attn3d_backward_rows": [_P, _I32, _I32, _I64, _I64] + [_V] * 16,
     "dfa3d_rebatch_plan": [ctypes.c_void_p, _I32, _I32, _I32, _I32] + [ctypes.c_void_p] * 8,
     "dfa3d_rebatch_gather": [ctypes.c_void_p] * 4 + [_I32] * 4 + [_I64, _I64] + [ctypes.c_void_p] * 2
                             + [_I64, ctypes.c_void_p],
@@ -87,6 +87,8 @@ PLAIN_ENTRY_POINTS = {
     "dfa3d_column_sum": [ctypes.c_void_p, _I64, _I32, ctypes.c_void_p, ctypes.c_void_p],
     "dfa3d_add_layer_norm_infer": [ctypes.c_void_p] * 4 + [_I64, _I32, ctypes.c_float] + [ctypes.c_void_p] * 2,
     "dfa3d_relu_backward_column_sum": [ctypes.c_void_p] * 2 + [_I64, _I32] + [ctypes.c_void_p] * 3,
+    "dfa3d_slice_sum": [ctypes.c_void_p] + [_I32] * 3 + [ctypes.c_void_p] * 2 + [_I32] + [ctypes.c_void_p] * 3,
+    "dfa3d_copy_segments": [ctypes.c_void_p] * 3 + [_I32, ctypes.c_void_p],
     "dfa3d_zero_two": [ctypes.c_void_p, _I64, ctypes.c_void_p, _I64, ctypes.c_void_p],
 }
 ACT_SOFTMAX, ACT_SIGMOID = 0, 1

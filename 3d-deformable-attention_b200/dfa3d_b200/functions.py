@@ -137,16 +137,15 @@ class MultiScale3DDeformableAttnFunction(Function):
 
 class _FromOffsets2D(Function):
     @classmethod
-    def from_offsets(cls, value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps, heads,
-                     points):
+    def from_offsets(cls, value, spatial_shapes, level_start_index, reference_points, joint, maps, heads, points):
         """The operator with what its callers do around it (temporal_self_attention.py:224-262, decoder.py:283-318)
         inside the kernels: softmax of the logits map by map, locations from reference points and offsets, mean over
         the `maps` value maps of a batch element.  value (bs*maps, N, H*C); reference_points (bs*maps, Q, L, 2) without
-        gradient; offsets (bs, Q, H*maps*L*P*2) and logits (bs, Q, H*maps*L*P) as the Linear layers leave them.
+        gradient; joint (bs, Q, H*maps*L*P*3): a query's offsets, then its logits, as the Linear layers leave them.
         Returns (bs, Q, H*C), or NotImplemented where only the separate steps do it (sizes the kernels do not have,
         other dtypes, autocast)."""
-        return _lib.native().attn2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps,
-                                    heads, points)
+        return _lib.native().attn2d(value, spatial_shapes, level_start_index, reference_points, joint, maps, heads,
+                                    points)
 
 
 @_native_apply("msda")

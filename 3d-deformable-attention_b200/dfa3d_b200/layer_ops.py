@@ -168,14 +168,13 @@ def _plain_linear(m):
             and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
 
 
-def linear3(x, a, b, c):
-    """(a(x), b(x), c(x)) for three Linear layers; as one operation where they are plain, so that the gradient of x is
-    accumulated inside the matrix products instead of by two additions of its size."""
-    if _plain_linear(a) and _plain_linear(b) and _plain_linear(c):
-        out = _lib.native().linear3(x, a.weight, a.bias, b.weight, b.bias, c.weight, c.bias)
-        if out is not NotImplemented:
-            return out
-    return a(x), b(x), c(x)
+def joint_linear(x, *linears):
+    """[a(x) | b(x) | ...] of two or three plain Linear layers in one row, as one matrix product each way, or None where
+    they have to be called one by one (hooks on one of them, autocast, other dtypes)."""
+    if not all(_plain_linear(m) for m in linears):
+        return None
+    out = _lib.native().joint_linear(x, *(t for m in linears for t in (m.weight, m.bias)))
+    return None if out is NotImplemented else out
 
 
 def linear_relu(x, linear, relu):

@@ -34,7 +34,7 @@ from .functions import (MultiScaleDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnRaggedFunction_fp32)
 from . import _lib
-from .layer_ops import AddLayerNorm, Linear, linear3, linear_relu
+from .layer_ops import AddLayerNorm, Linear, joint_linear, linear_relu
 from .rebatch import CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan
 
 
@@ -184,23 +184,22 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
             value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
-        value = value.view(bs, N, H, -1)
         if reference_points.shape[-1] != 3:
             raise ValueError("Last dim of reference_points must be 3 (x, y, depth), but got "
                              f"{reference_points.shape[-1]} instead.")
-        off_uv, off_d, logits = linear3(query, self.sampling_offsets, self.sampling_offsets_depth,
-                                        self.attention_weights)
-        off_uv = off_uv.view(*lead, H, L, P, 2)
-        off_d = off_d.view(*lead, H, L, P, 1)
-        logits = logits.view(*lead, H, L * P)
         if self.fuse_input_ops and not self.compute_weight_update:
-            # the kernels take the (L, 2) table as it is: D bins in every level
-            args = (value.contiguous(), value_dpt_dist.contiguous(), spatial_shapes, level_start_index,
-                    reference_points.contiguous(), off_uv, off_d, logits)
-            output = _lib.native().attn3d_ragged_flat(*args, query_offsets, max_queries, dist_map) if ragged else \
-                _lib.native().attn3d_flat(*args, dist_map)
+            # one product for the three projections; the kernels read their parts of a row where it left them, and the
+            # (L, 2) level table as it is: D bins in every level
+            joint = joint_linear(query, self.sampling_offsets, self.sampling_offsets_depth, self.attention_weights)
+            output = NotImplemented if joint is None else _lib.native().attn3d_joint(
+                value.contiguous(), value_dpt_dist.contiguous(), spatial_shapes, level_start_index,
+                reference_points.contiguous(), joint, H, P, query_offsets, max_queries, dist_map)
             if output is not NotImplemented:
                 return (output if ragged or self.batch_first else output.permute(1, 0, 2)), None
+        value = value.view(bs, N, H, -1)
+        off_uv = self.sampling_offsets(query).view(*lead, H, L, P, 2)
+        off_d = self.sampling_offsets_depth(query).view(*lead, H, L, P, 1)
+        logits = self.attention_weights(query).view(*lead, H, L * P)
         shapes3 = torch.cat([spatial_shapes, torch.full_like(spatial_shapes[:, :1], D)], -1).contiguous()
         if self.fuse_input_ops and not self.compute_weight_update:
             if ragged:
@@ -299,14 +298,19 @@ class SpatialCrossAttention_DFA3D(nn.Module):
         return (slots, inp_residual) if return_residual else slots + inp_residual
 
 
-def _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, maps, heads, points):
-    """The 2-D operator with its callers' softmax, location assembly and mean over the maps inside the kernels, or None
-    where the separate steps have to do it (box reference points, sizes the kernels do not have)."""
+def _attention_2d(value, query, module, reference_points, spatial_shapes, level_start_index, maps):
+    """The 2-D operator of `module` (its sampling_offsets, attention_weights, num_heads, num_points) with its callers'
+    softmax, location assembly and mean over the maps inside the kernels, or None where the separate steps have to do it
+    (box reference points, sizes the kernels do not have)."""
     fused = getattr(MultiScaleDeformableAttnFunction_fp32, "from_offsets", None)
-    if fused is None or reference_points.shape[-1] != 2:
+    points = maps * module.num_levels * module.num_points
+    if fused is None or reference_points.shape[-1] != 2 or points not in (4, 8, 16):
         return None
-    out = fused(value.contiguous(), spatial_shapes, level_start_index, reference_points.contiguous(), offsets, logits,
-                maps, heads, points)
+    joint = joint_linear(query, module.sampling_offsets, module.attention_weights)
+    if joint is None:
+        return None
+    out = fused(value.contiguous(), spatial_shapes, level_start_index, reference_points.contiguous(), joint, maps,
+                module.num_heads, module.num_points)
     return None if out is NotImplemented else out
 
 
@@ -377,11 +381,11 @@ class TemporalSelfAttention(nn.Module):
         value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
-        offsets, logits = self.sampling_offsets(query), self.attention_weights(query)
-        out = _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, NQ, H, P)
+        out = _attention_2d(value, query, self, reference_points, spatial_shapes, level_start_index, NQ)
         if out is None:
-            out = self._attention_in_steps(value.reshape(bs * NQ, N, H, -1), offsets, logits, reference_points,
-                                           spatial_shapes, level_start_index)
+            out = self._attention_in_steps(value.reshape(bs * NQ, N, H, -1), self.sampling_offsets(query),
+                                           self.attention_weights(query), reference_points, spatial_shapes,
+                                           level_start_index)
         out = self.output_proj(out)
         if not self.batch_first:
             out = out.permute(1, 0, 2)
@@ -494,11 +498,11 @@ class CustomMSDeformableAttention(nn.Module):
         value = self.value_proj(value)
         if key_padding_mask is not None:
             value = value.masked_fill(key_padding_mask[..., None], 0.0)
-        offsets, logits = self.sampling_offsets(query), self.attention_weights(query)
-        out = _attention_2d(value, spatial_shapes, level_start_index, reference_points, offsets, logits, 1, H, P)
+        out = _attention_2d(value, query, self, reference_points, spatial_shapes, level_start_index, 1)
         if out is None:
-            out = self._attention_in_steps(value.view(bs, N, H, -1), offsets, logits, reference_points,
-                                           spatial_shapes, level_start_index)
+            out = self._attention_in_steps(value.reshape(bs, N, H, -1), self.sampling_offsets(query),
+                                           self.attention_weights(query), reference_points, spatial_shapes,
+                                           level_start_index)
         out = self.output_proj(out)
         if not self.batch_first:
             out = out.permute(1, 0, 2)

@@ -179,12 +179,13 @@ int dfa3d_attn3d_backward(const dfa3d_problem *p, int32_t num_anchors, const voi
  * p describes one map: B batch elements, N pixels, L levels; value (B*maps,N,H,C), ref_points (B*maps,Q,L,2), offsets
  * (B,Q,H,maps,L,P,2), logits (B,Q,H,maps,L*P), out (B,Q,H*C), all fp32.  dfa3d_attn2d_supported(): 1 for the sizes the
  * kernels exist for (C of 16, 32 or 64; 4, 8 or 16 points over all maps, a power of two in each), else 0.  Backward:
- * grad_value is ACCUMULATED into; grad_offsets and grad_logits are overwritten; the reference points get none. */
+ * grad_value is ACCUMULATED into; grad_offsets and grad_logits are overwritten; the reference points get none.
+ * offsets_row, logits_row: elements from query to query of offsets and logits, 0 where these are contiguous. */
 int dfa3d_attn2d_supported(const dfa3d_problem *p, int32_t num_maps);
-int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                          const int64_t *level_start, const float *ref_points, const float *offsets,
                          const float *logits, float *out, void *stream);
-int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, const void *value, const int64_t *shapes2,
+int dfa3d_attn2d_backward(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                           const int64_t *level_start, const float *ref_points, const float *offsets,
                           const float *logits, const float *grad_out, float *grad_value, float *grad_offsets,
                           float *grad_logits, void *stream);
@@ -221,13 +222,17 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                  float *grad_offsets_depth, float *grad_logits, void *stream);
 
 /* dfa3d_attn3d_forward / _backward for either form of the queries (query_offsets null: dense) and either form of the level
- * table: shapes (L, shape_stride) with shape_stride 3 = (h, w, d), or 2 = (h, w) where every level has p->D bins. */
-int dfa3d_attn3d_forward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+ * table: shapes (L, shape_stride) with shape_stride 3 = (h, w, d), or 2 = (h, w) where every level has p->D bins.
+ * offsets_row, logits_row: elements from query to query of offsets_uv, and of offsets_depth and logits (their gradients'
+ * rows alike), 0 where these are contiguous: one Linear layer may produce all three side by side in one row. */
+int dfa3d_attn3d_forward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
+                             int64_t logits_row,
                                 const int32_t *query_offsets, const void *value, const void *dist,
                                 const int64_t *shapes, const int64_t *level_start, const float *ref_points,
                                 const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
                                 void *stream);
-int dfa3d_attn3d_backward_levels(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
+int dfa3d_attn3d_backward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
+                             int64_t logits_row,
                                  const int32_t *query_offsets, const void *value, const void *dist,
                                  const int64_t *shapes, const int64_t *level_start, const float *ref_points,
                                  const float *offsets_uv, const float *offsets_depth, const float *logits,
@@ -370,6 +375,16 @@ int dfa3d_add_layer_norm_infer(const float *x, const float *residual, const floa
  * a ReLU up to the matrix products.  Conditions of dfa3d_column_sum; grad_in may be grad_y. */
 int dfa3d_relu_backward_column_sum(const float *grad_y, const float *y, int64_t rows, int32_t cols, float *grad_in,
                                    float *dst, void *stream);
+
+/* dst (out, in) = sum of `slices` partial products partial (slices, out, in) + grad_tail^T x_tail, with grad_tail
+ * (tail_rows, out) and x_tail (tail_rows, in): the end of a weight gradient that was formed as a batch of row slices.
+ * zeroed (out), if given, is set to 0 (a bias gradient to be accumulated next).  in a multiple of 4; partial, dst and
+ * x_tail 16-byte aligned. */
+int dfa3d_slice_sum(const float *partial, int32_t slices, int32_t out, int32_t in, const float *grad_tail,
+                    const float *x_tail, int32_t tail_rows, float *dst, float *zeroed, void *stream);
+
+/* dst[i][0..counts[i]) = src[i][0..counts[i]) for i < n <= 8 with one launch; the three tables are in HOST memory. */
+int dfa3d_copy_segments(const float *const *src, float *const *dst, const int64_t *counts, int32_t n, void *stream);
 
 /* a[0..na) = 0 and b[0..nb) = 0 with one launch: the two gradients a backward accumulates into.  Either
  * count may be 0 (its pointer is then not looked at); pointers 16-byte aligned. */
