@@ -87,6 +87,7 @@ struct KArgs {
   float *grad_off_d;       // (B,Q,H,L,P), overwritten
   long long row_loc, row_attn;  // elements from query to query of loc, and of attn and off_d
   int Z;                   // reference points (pillar anchors) per query
+  int rounds;              // several items per warp: batches of 32 lanes a warp takes
   int maps;                // 2-D: value maps per batch element; N and L count all of them.  0 elsewhere
   // ragged queries: camera b owns the packed query rows [q_off[b], q_off[b+1]) of every per-query
   // tensor; Q is then only the bound the grid is sized for.  Null = every camera has Q queries.
@@ -195,11 +196,28 @@ __device__ __forceinline__ bool item_context(const KArgs &a, int warp, unsigned 
   return true;
 }
 
+// ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
+// Items of up to 16 points, rows of 16, 32 or 64 channels.
+inline bool packed_covers(int LP, int C) { return LP <= 16 && (C == 16 || C == 32 || C == 64); }
+// Batches of 32 lanes a warp takes before its CTA retires, by the CTA-sized batches of the launch: two once the device is
+// filled twice over (fewer, longer-lived CTAs), one before that, so that a small launch spreads over the SMs and is one
+// chain of latencies deep (900 queries x 8 heads x 4 points forward: 7.9 us at two).
+inline int packed_rounds(long long batches) { return batches >= 148 * 12 ? 2 : 1; }
+
 // Softmax of an item's L*P attention logits (caller-fused mode): maximum and sum of exp(l - max),
 // formed with warp shuffles; lane j later turns its own logit into exp(l_j - max) / sum.
 struct SoftmaxStats {
   float mx, sum;
 };
+
+// The same for an item that has `lanes` consecutive lanes, a power of two, to itself.
+__device__ __forceinline__ SoftmaxStats lanes_softmax_stats(float logit, bool have, int lanes) {
+  float mx = have ? logit : -INFINITY;
+  for (int s = lanes / 2; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+  float sum = have ? expf(logit - mx) : 0.f;
+  for (int s = lanes / 2; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+  return SoftmaxStats{mx, sum};
+}
 
 __device__ __forceinline__ SoftmaxStats item_softmax_stats(const KArgs &a, const ItemCtx &c, int lane) {
   const float *lg = c.attn;

@@ -1,0 +1,209 @@
+// DFA3D forward for items of few points (L*P <= 16): a warp takes several consecutive items at once (sm_100a).
+//
+// With one item per warp an item of 4 points (temporal self-attention and the decoder's cross-attention
+// use 1 level x 4 points) keeps 4 lanes busy in the prologue and costs a whole chain of dependent
+// latencies (locations -> row table -> rows -> sum -> store) for 16 rows.  Here an item has LPP lanes -- 4, 8 or 16,
+// the next of them from L*P on -- and lane j of them owns its point j, so the prologue is (nearly) full and coalesced:
+// the points of consecutive items are consecutive in memory.  A group of G lanes then sums all rows of one item (or,
+// when the warp holds fewer items than groups, a share of them) and writes that item's output itself.
+// Bound like the one-item kernels by the rows that travel from L2 to the SM.  Against one item per warp, 6 cameras x 6000
+// queries x 8 heads of fp32: 3 levels x 4 points of 32 channels 205 -> 142 us, 1 x 5 points of 16 channels 150 -> 64 us.
+#include "dfa3d_forward_point.cuh"
+#include "dfa3d_launch.h"
+
+namespace dfa3d {
+namespace {
+
+// CTAs per SM the kernel is compiled for.  fp32 rows: 6 (48 warps; the kernel waits on chains of dependent loads)
+// measured 1-4 % faster than 5 and 4-8 % faster than 4 -- but not where the depth scores are kept to be written: the
+// 40 registers then spill up to 270 bytes (1 level x 8 points, 6 x 6000 queries: 142 us at 6).  16-bit rows hold eight
+// channels a lane.
+template <typename VT, int MODE, bool WRITE_DS>
+struct PackedCtas { static constexpr int value = RowVec<VT>::kElems == 8 ? 4 : WRITE_DS ? 5 : 6; };
+
+// EXACT: L*P == LPP, the row loop is unrolled; otherwise it ends at the item's last row.
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+__global__ void __launch_bounds__(kThreads, PackedCtas<VT, MODE, WRITE_DS>::value)
+dfa3d_forward_packed_kernel(const KArgs a) {
+  constexpr int V = RowVec<VT>::kElems;
+  constexpr int G = C / V;                      // lanes per row
+  constexpr int R = 32 / G;                     // groups per warp
+  constexpr int K = 32 / LPP;                   // items per warp
+  constexpr int GPI = R > K ? R / K : 1;        // groups sharing one item
+  constexpr int IPG = K > R ? K / R : 1;        // items one group handles in turn
+  constexpr int U = 4;
+  constexpr int kSlots = LPP * 4;               // row slots of one item
+  // Fully unrolled is 1-8 % faster than by 2 -- except where a group has one item of its own and neither softmax nor
+  // dist to wait for: the loads of the whole item are then moved to the front and spill 172 bytes (1 level x 8 points,
+  // 6 x 6000 queries: 122 us fully unrolled, 75 by 2).
+  constexpr int kUnroll = MODE == kGivenDepthScore && GPI == 1 && IPG == 1 ? 2 : kSlots / (GPI * U);
+  static_assert(32 % LPP == 0 && 32 % G == 0 && kSlots % (GPI * U) == 0, "unsupported packing");
+  __shared__ LevelTable lv;
+  __shared__ __align__(16) RowEntry rows[kWarpsPerCta][128];
+  stage_levels(lv, a);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane % G, grp = lane / G;
+  const int b = (int)blockIdx.y + a.b0;
+  const VT *vbase = reinterpret_cast<const VT *>(a.value) + ((long long)b * a.N * a.H * C + sub * V);
+  RowEntry *table = rows[warp];
+  // the camera's queries: rows [q0, q0 + nq) of the per-query tensors
+  const long long q0 = a.q_off ? (long long)__ldg(a.q_off + b) : (long long)b * a.Q;
+  const unsigned nitems = (unsigned)(a.q_off ? __ldg(a.q_off + b + 1) - (int)q0 : a.Q) * (unsigned)a.H;
+  const int nrows = EXACT ? kSlots : a.LP * 4;
+#pragma unroll 1
+  for (int it = 0; it < a.rounds; ++it) {
+    const unsigned first = ((blockIdx.x * a.rounds + it) * kWarpsPerCta + warp) * K;
+    if (first >= nitems) return;
+    {
+      const unsigned idx = first + lane / LPP;
+      const int j = lane % LPP;
+      const bool live = idx < nitems && (EXACT || j < a.LP);
+      ItemCtx c;
+      c.b = b;
+      const unsigned q = idx / (unsigned)a.H;
+      c.h = (int)(idx - q * (unsigned)a.H);
+      c.bq = q0 + q;
+      c.item = q0 * a.H + idx;
+      item_inputs<MODE>(a, c);
+      SoftmaxStats sm{0.f, 1.f};
+      if (mode_from_offsets(MODE))
+        sm = lanes_softmax_stats(live ? __ldg(c.attn + j) : 0.f, live, MODE == kCallerFused2D ? LPP / a.maps : LPP);
+      float ds[4], wgt[4];
+      int off[4];
+      fwd_point<DT, MODE>(a, lv, c, live ? j : a.LP, sm, ds, wgt, off);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (off[k] >= 0) off[k] += c.h * C;     // rows of different heads share the table
+      store_rows(table, lane, off, wgt);
+      if (WRITE_DS && live)
+        reinterpret_cast<float4 *>(a.ds_out)[c.pt0 + j] = make_float4(ds[0], ds[1], ds[2], ds[3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < IPG; ++t) {
+      const int i = grp / GPI + t * (R / GPI);  // item of the warp this group works on
+      const RowEntry *my = table + i * kSlots + (grp % GPI) * U;
+      float acc[V];
+#pragma unroll
+      for (int x = 0; x < V; ++x) acc[x] = 0.f;
+      auto step = [&](int r0) {
+        RowEntry e[U];
+        float v[U][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u) e[u] = my[r0 + u];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (e[u].off >= 0) {
+            RowVec<VT>::load(vbase + e[u].off, v[u]);
+          } else {
+#pragma unroll
+            for (int x = 0; x < V; ++x) v[u][x] = 0.f;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int x = 0; x < V; ++x) acc[x] = fmaf(e[u].wgt, v[u][x], acc[x]);
+      };
+      if (EXACT) {
+#pragma unroll kUnroll
+        for (int r0 = 0; r0 < kSlots; r0 += GPI * U) step(r0);
+      } else {
+#pragma unroll 1
+        for (int r0 = 0; r0 < nrows; r0 += GPI * U) step(r0);
+      }
+#pragma unroll
+      for (int s = G; s < G * GPI; s <<= 1)
+#pragma unroll
+        for (int x = 0; x < V; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], s);
+      const unsigned idx = first + i;
+      if (grp % GPI == 0 && idx < nitems) {
+        float *o = a.out + ((q0 * a.H + idx) * C + sub * V);
+#pragma unroll
+        for (int x = 0; x < V; x += 4)
+          *reinterpret_cast<float4 *>(o + x) = make_float4(acc[x], acc[x + 1], acc[x + 2], acc[x + 3]);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// host-side dispatch
+// ------------------------------------------------------------------------------------------------
+template <typename VT, typename DT, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+void launch_c(const KArgs &a, dim3 grid, cudaStream_t s) {
+  if (a.C == 16) dfa3d_forward_packed_kernel<VT, DT, 16, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
+  else if (a.C == 32) dfa3d_forward_packed_kernel<VT, DT, 32, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
+  else dfa3d_forward_packed_kernel<VT, DT, 64, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
+}
+
+template <typename VT, typename DT, int MODE, bool WRITE_DS>
+void launch_lp(const KArgs &a, dim3 grid, cudaStream_t s) {
+  // the unrolled loop is instantiated where it is the common case: fp32 throughout
+  constexpr bool kFloat = sizeof(VT) == 4 && (sizeof(DT) == 4 || !mode_has_depth(MODE));
+  const int lpp = a.LP <= 4 ? 4 : a.LP <= 8 ? 8 : 16;
+  if constexpr (kFloat) {
+    if (a.LP == lpp) {
+      if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, true>(a, grid, s);
+      else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, true>(a, grid, s);
+      else launch_c<VT, DT, MODE, WRITE_DS, 16, true>(a, grid, s);
+      return;
+    }
+  }
+  if constexpr (MODE != kCallerFused2D) {      // attn2d_supported: fp32, exact
+    if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, false>(a, grid, s);
+    else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, false>(a, grid, s);
+    else launch_c<VT, DT, MODE, WRITE_DS, 16, false>(a, grid, s);
+  }
+}
+
+template <typename VT, typename DT, int MODE>
+cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
+  const int lpp = a0.LP <= 4 ? 4 : a0.LP <= 8 ? 8 : 16;
+  const unsigned batch = kWarpsPerCta * (32 / lpp);                  // items a CTA takes at a time
+  const unsigned batches = ((unsigned)a0.items_per_cam + batch - 1) / batch;
+  for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
+    KArgs a = a0;
+    a.b0 = b0;
+    const unsigned cams = (unsigned)min(65535, a0.B - b0);
+    a.rounds = packed_rounds((long long)batches * cams);
+    const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
+    if constexpr (mode_from_offsets(MODE)) {      // the caller-fused entry points return no depth score
+      launch_lp<VT, DT, MODE, false>(a, grid, s);
+    } else if constexpr (MODE == kFused) {
+      if (a.ds_out) launch_lp<VT, DT, MODE, true>(a, grid, s);
+      else launch_lp<VT, DT, MODE, false>(a, grid, s);
+    } else {
+      launch_lp<VT, DT, MODE, false>(a, grid, s);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+template <int MODE>
+cudaError_t launch_m(const KArgs &a, int value_dtype, int dist_dtype, cudaStream_t s) {
+  if (value_dtype == kDtypeF16) return launch_vd<__half, __half, MODE>(a, s);
+  if (value_dtype == kDtypeBF16)
+    return dist_dtype == kDtypeBF16 ? launch_vd<__nv_bfloat16, __nv_bfloat16, MODE>(a, s)
+                                    : launch_vd<__nv_bfloat16, float, MODE>(a, s);
+  return dist_dtype == kDtypeBF16 ? launch_vd<float, __nv_bfloat16, MODE>(a, s) : launch_vd<float, float, MODE>(a, s);
+}
+
+}  // namespace
+
+cudaError_t launch_forward_packed(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s) {
+  if (mode == kCallerFused2D)
+    return value_dtype == kDtypeF32 ? launch_vd<float, float, kCallerFused2D>(a, s) : cudaErrorNotSupported;
+  if (mode == kGivenDepthScore) {   // dist is not read: its type parameter is irrelevant
+    if (value_dtype == kDtypeF16) return launch_vd<__half, float, kGivenDepthScore>(a, s);
+    return value_dtype == kDtypeBF16 ? launch_vd<__nv_bfloat16, float, kGivenDepthScore>(a, s)
+                                     : launch_vd<float, float, kGivenDepthScore>(a, s);
+  }
+  if (mode == kCallerFused) return launch_m<kCallerFused>(a, value_dtype, dist_dtype, s);
+  return launch_m<kFused>(a, value_dtype, dist_dtype, s);
+}
+
+}  // namespace dfa3d

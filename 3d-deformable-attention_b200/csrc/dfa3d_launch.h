@@ -8,6 +8,9 @@ namespace dfa3d {
 struct KArgs;
 // mode: dfa3d::Mode
 cudaError_t launch_forward(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s);
+// items of few points, several per warp (dfa3d_forward_packed.cu, dfa3d_backward_packed.cu); see packed_covers
+cudaError_t launch_forward_packed(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s);
+cudaError_t launch_backward_packed(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s);
 cudaError_t launch_depth_score_forward(const KArgs &a, int dist_dtype, cudaStream_t s);
 cudaError_t launch_backward(const KArgs &a, int value_dtype, int dist_dtype, int mode, cudaStream_t s);
 cudaError_t launch_depth_score_backward(const KArgs &a, int dist_dtype, cudaStream_t s);
