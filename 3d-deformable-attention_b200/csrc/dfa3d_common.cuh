@@ -196,6 +196,31 @@ __device__ __forceinline__ bool item_context(const KArgs &a, int warp, unsigned 
   return true;
 }
 
+// Asks L2 for the bytes [p, p + bytes), a line per thread of `threads`.
+__device__ __forceinline__ void prefetch_l2(const void *p, long long bytes, int thread, int threads) {
+  const char *c = reinterpret_cast<const char *>(p);
+  for (long long o = (long long)thread * 128; o < bytes; o += (long long)threads * 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(c + o));
+}
+
+// Caller-fused mode: asks L2 for the offsets and logits of items [first, first + count) of camera b (query-major), for a
+// CTA that comes to them one group after the other.  An item's chain of dependent loads is longest here (logits, twice,
+// for the softmax, then offsets, depth bins, rows), and it began with a read from HBM: 6 cameras at the base levels
+// 469 -> 463 us.  With locations and weights given the chain is shorter and the same prefetch cost 1.5 %.
+__device__ __forceinline__ void prefetch_offsets(const KArgs &a, int b, unsigned first, unsigned count) {
+  const long long q0 = a.q_off ? (long long)__ldg(a.q_off + b) : (long long)b * a.Q;
+  const unsigned n = (unsigned)(a.q_off ? __ldg(a.q_off + b + 1) - (int)q0 : a.Q) * (unsigned)a.H;
+  if (first >= n) return;
+  const unsigned last = first + min(count, n - first) - 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long width = (long long)a.H * a.LP * 4;
+  for (unsigned q = first / (unsigned)a.H + warp; q <= last / (unsigned)a.H; q += kWarpsPerCta) {
+    prefetch_l2(a.loc + (q0 + q) * a.row_loc, 2 * width, lane, 32);
+    prefetch_l2(a.off_d + (q0 + q) * a.row_attn, width, lane, 32);
+    prefetch_l2(a.attn + (q0 + q) * a.row_attn, width, lane, 32);
+  }
+}
+
 // ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
 // Items of up to 16 points, rows of 16, 32 or 64 channels.
 inline bool packed_covers(int LP, int C) { return LP <= 16 && (C == 16 || C == 32 || C == 64); }
@@ -365,6 +390,30 @@ __device__ __forceinline__ void store_rows(RowEntry *table, int lane, const int 
   dst[0] = make_uint4((uint32_t)off[0], __float_as_uint(wgt[0]), (uint32_t)off[1], __float_as_uint(wgt[1]));
   dst[1] = make_uint4((uint32_t)off[2], __float_as_uint(wgt[2]), (uint32_t)off[3], __float_as_uint(wgt[3]));
 }
+
+// The same table for readers that take a point's four corners at a time: corners 0,1 of all points, then corners 2,3, so
+// that a lane's two 16-byte stores and a reader's two 16-byte loads meet no bank conflict -- also where the groups of a
+// warp read points 4, 8 or 16 apart, which is what the gap after every eighth point is for.  Two reads where there were
+// four: forward of 1 level x 8 points, 6 x 6000 queries, with depth scores 108 -> 101 us, 4 levels x 5 points 270 -> 259.
+// In the backward, which waits for its reductions, it was no gain (1 % slower at 32 points).
+struct RowTable {
+  static constexpr int kHalf = 36;
+  uint4 slot[2 * kHalf];
+  __device__ static __forceinline__ int at(int point) { return point + (point >> 3); }
+  __device__ __forceinline__ void store(int point, const int (&off)[4], const float (&wgt)[4]) {
+    uint4 *d = slot + at(point);
+    d[0] = make_uint4((uint32_t)off[0], __float_as_uint(wgt[0]), (uint32_t)off[1], __float_as_uint(wgt[1]));
+    d[kHalf] = make_uint4((uint32_t)off[2], __float_as_uint(wgt[2]), (uint32_t)off[3], __float_as_uint(wgt[3]));
+  }
+  __device__ __forceinline__ void load(int point, RowEntry (&e)[4]) const {
+    const uint4 *d = slot + at(point);
+    const uint4 x = d[0], y = d[kHalf];
+    e[0] = RowEntry{(int)x.x, __uint_as_float(x.y)};
+    e[1] = RowEntry{(int)x.z, __uint_as_float(x.w)};
+    e[2] = RowEntry{(int)y.x, __uint_as_float(y.y)};
+    e[3] = RowEntry{(int)y.z, __uint_as_float(y.w)};
+  }
+};
 
 // Two adjacent depth bins p[0], p[1] that are both in range: one naturally aligned 8-byte (fp32) or
 // 4-byte (bf16) load when the pair happens to be aligned, two scalar loads otherwise (the second then

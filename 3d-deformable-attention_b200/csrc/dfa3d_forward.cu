@@ -30,15 +30,14 @@ namespace dfa3d {
 // of the row table in shared memory.
 template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
 __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &lv, const ItemCtx &c,
-                                             RowEntry *table, int lane) {
+                                             RowTable &table, int lane) {
   constexpr int V = RowVec<VT>::kElems;   // channels per lane
   constexpr int G = C / V;                // lanes per row
   constexpr int R = 32 / G;               // rows per warp-wide request
-  constexpr int U = 4;                    // requests in flight per lane
+  constexpr int U = 4;                    // requests in flight per lane: the corners of a group's point
   static_assert(G >= 1 && G <= 32 && (G & (G - 1)) == 0, "C/V must be a power of two <= 32");
   const VT *vbase = reinterpret_cast<const VT *>(a.value) + (((long long)c.b * a.N * a.H + c.h) * C +
                                                              (lane % G) * V);
-  const RowEntry *my = table + lane / G;
 
   float acc[V];
 #pragma unroll
@@ -50,18 +49,19 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
     float ds[4], wgt[4];
     int off[4];
     fwd_point<DT, MODE>(a, lv, c, chunk + lane, sm, ds, wgt, off);
-    store_rows(table, lane, off, wgt);
+    table.store(lane, off, wgt);
     if (WRITE_DS && chunk + lane < a.LP)
       reinterpret_cast<float4 *>(a.ds_out)[c.pt0 + chunk + lane] = make_float4(ds[0], ds[1], ds[2], ds[3]);
     __syncwarp();
-    // R*U rows per step: U independent row-fragment loads in flight per lane, then U fused multiply-adds.
-    auto step = [&](int r0, int nrows) {
+    // R points per step: U independent row-fragment loads in flight per lane, then U fused multiply-adds.
+    auto step = [&](int p0, int n) {
       RowEntry e[U];
       float v[U][V];
+      if (FULL || p0 + lane / G < n) {
+        table.load(p0 + lane / G, e);
+      } else {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int r = r0 + u * R;
-        e[u] = (FULL || r + lane / G < nrows) ? my[r] : RowEntry{-1, 0.f};
+        for (int u = 0; u < U; ++u) e[u] = RowEntry{-1, 0.f};
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -77,13 +77,13 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] = fmaf(e[u].wgt, v[u][i], acc[i]);
     };
-    if (FULL) {          // 128 rows: compile-time trip count, table offsets become immediates
+    if (FULL) {          // compile-time trip count, table offsets become immediates
 #pragma unroll
-      for (int r0 = 0; r0 < 128; r0 += R * U) step(r0, 128);
+      for (int p0 = 0; p0 < 32; p0 += R) step(p0, 32);
     } else {
-      const int nrows = min(32, a.LP - chunk) * 4;
+      const int n = min(32, a.LP - chunk);
 #pragma unroll 1
-      for (int r0 = 0; r0 < nrows; r0 += R * U) step(r0, nrows);
+      for (int p0 = 0; p0 < n; p0 += R) step(p0, n);
     }
     __syncwarp();
   }
@@ -106,8 +106,10 @@ template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
 __global__ void __launch_bounds__(kThreads, DFA3D_FWD_MIN_CTAS)
 dfa3d_forward_kernel(const KArgs a) {
   __shared__ LevelTable lv;
-  __shared__ __align__(16) RowEntry rows[kWarpsPerCta][128];
+  __shared__ RowTable rows[kWarpsPerCta];
   stage_levels(lv, a);
+  constexpr unsigned kItems = kWarpsPerCta * DFA3D_FWD_ITEMS_PER_WARP;
+  if (MODE == kCallerFused) prefetch_offsets(a, (int)blockIdx.y + a.b0, blockIdx.x * kItems, kItems);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int it = 0; it < DFA3D_FWD_ITEMS_PER_WARP; ++it) {

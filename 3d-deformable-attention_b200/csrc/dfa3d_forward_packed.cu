@@ -32,24 +32,24 @@ dfa3d_forward_packed_kernel(const KArgs a) {
   constexpr int GPI = R > K ? R / K : 1;        // groups sharing one item
   constexpr int IPG = K > R ? K / R : 1;        // items one group handles in turn
   constexpr int U = 4;
-  constexpr int kSlots = LPP * 4;               // row slots of one item
-  // Fully unrolled is 1-8 % faster than by 2 -- except where a group has one item of its own and neither softmax nor
-  // dist to wait for: the loads of the whole item are then moved to the front and spill 172 bytes (1 level x 8 points,
-  // 6 x 6000 queries: 122 us fully unrolled, 75 by 2).
-  constexpr int kUnroll = MODE == kGivenDepthScore && GPI == 1 && IPG == 1 ? 2 : kSlots / (GPI * U);
-  static_assert(32 % LPP == 0 && 32 % G == 0 && kSlots % (GPI * U) == 0, "unsupported packing");
+  // Fully unrolled is 1-8 % faster than by 2 -- except where a group has one item of its own and no dist to wait for: the
+  // loads of the whole item are then moved to the front and spill 170 to 240 bytes (1 level x 8 points, 6 x 6000
+  // queries: 122 us fully unrolled, 75 by 2; 2-D from offsets, 22500 queries: 88, 63 by 2, 62 by 4).
+  constexpr bool kShort = !mode_has_depth(MODE) && GPI == 1 && IPG == 1;
+  constexpr int kUnroll = !kShort ? LPP / GPI : MODE == kCallerFused2D ? 4 : 2;
+  static_assert(32 % LPP == 0 && 32 % G == 0 && LPP % GPI == 0, "unsupported packing");
   __shared__ LevelTable lv;
-  __shared__ __align__(16) RowEntry rows[kWarpsPerCta][128];
+  __shared__ RowTable rows[kWarpsPerCta];
   stage_levels(lv, a);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % G, grp = lane / G;
   const int b = (int)blockIdx.y + a.b0;
   const VT *vbase = reinterpret_cast<const VT *>(a.value) + ((long long)b * a.N * a.H * C + sub * V);
-  RowEntry *table = rows[warp];
+  RowTable &table = rows[warp];
   // the camera's queries: rows [q0, q0 + nq) of the per-query tensors
   const long long q0 = a.q_off ? (long long)__ldg(a.q_off + b) : (long long)b * a.Q;
   const unsigned nitems = (unsigned)(a.q_off ? __ldg(a.q_off + b + 1) - (int)q0 : a.Q) * (unsigned)a.H;
-  const int nrows = EXACT ? kSlots : a.LP * 4;
+  const int n = EXACT ? LPP : a.LP;
 #pragma unroll 1
   for (int it = 0; it < a.rounds; ++it) {
     const unsigned first = ((blockIdx.x * a.rounds + it) * kWarpsPerCta + warp) * K;
@@ -74,23 +74,22 @@ dfa3d_forward_packed_kernel(const KArgs a) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (off[k] >= 0) off[k] += c.h * C;     // rows of different heads share the table
-      store_rows(table, lane, off, wgt);
+      table.store(lane, off, wgt);
       if (WRITE_DS && live)
         reinterpret_cast<float4 *>(a.ds_out)[c.pt0 + j] = make_float4(ds[0], ds[1], ds[2], ds[3]);
     }
     __syncwarp();
-#pragma unroll
+#pragma unroll 1                               // unrolled too, 4 points an item spilled 70 to 140 bytes
     for (int t = 0; t < IPG; ++t) {
       const int i = grp / GPI + t * (R / GPI);  // item of the warp this group works on
-      const RowEntry *my = table + i * kSlots + (grp % GPI) * U;
+      const int base = i * LPP + grp % GPI;     // its first point
       float acc[V];
 #pragma unroll
       for (int x = 0; x < V; ++x) acc[x] = 0.f;
-      auto step = [&](int r0) {
+      auto step = [&](int p0) {
         RowEntry e[U];
         float v[U][V];
-#pragma unroll
-        for (int u = 0; u < U; ++u) e[u] = my[r0 + u];
+        table.load(base + p0, e);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (e[u].off >= 0) {
@@ -107,10 +106,10 @@ dfa3d_forward_packed_kernel(const KArgs a) {
       };
       if (EXACT) {
 #pragma unroll kUnroll
-        for (int r0 = 0; r0 < kSlots; r0 += GPI * U) step(r0);
+        for (int p0 = 0; p0 < LPP; p0 += GPI) step(p0);
       } else {
 #pragma unroll 1
-        for (int r0 = 0; r0 < nrows; r0 += GPI * U) step(r0);
+        for (int p0 = 0; p0 < n; p0 += GPI) step(p0);
       }
 #pragma unroll
       for (int s = G; s < G * GPI; s <<= 1)
