@@ -113,7 +113,7 @@ Tensor attn3d_forward(const Extra &x, const Tensor &value, const Tensor &dist, c
   Tensor out = ragged ? empty_f32({uv.size(0), (int64_t)p.H * p.C}, value)
                       : empty_f32({uv.size(0), uv.size(1), (int64_t)p.H * p.C}, value);
   void *s = stream_of(value);
-  check(lib.dfa3d_attn3d_forward_rows(&p, (int32_t)x.Z, (int32_t)shapes.size(1), 0, 0, ragged ? ip(q_off) : nullptr,
+  check(lib.dfa3d_attn3d_forward_rows(&p, (int32_t)x.Z, (int32_t)shapes.size(1), 0, 0, ragged ? ip(q_off) : nullptr, nullptr,
                                         value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(uv),
                                         fp(od), fp(logits), fpm(out), s),
         "dfa3d_attn3d_forward");
@@ -152,13 +152,15 @@ struct Attn3dFn : torch::autograd::Function<Attn3dFn> {
 
 // ---- the same with offsets, depth offsets and logits side by side in one row per query --------------------
 Tensor attn3d_joint_forward(const Extra &x, const Tensor &value, const Tensor &dist, const Tensor &shapes, const Tensor &lsi,
-                            const Tensor &ref, const Tensor &joint, const Tensor &q_off) {
+                            const Tensor &ref, const Tensor &joint, const Tensor &q_off, const Tensor &q_row) {
   c10::cuda::CUDAGuard guard(value.device());
   std::vector<int64_t> sz(joint.sizes().begin(), joint.sizes().end());
   const int64_t row = sz.back(), part = row / 4;
+  sz.front() = ref.size(0);
   sz.back() = (int64_t)x.p.H * x.p.C;
   Tensor out = empty_f32(sz, value);
-  check(lib.dfa3d_attn3d_forward_rows(&x.p, (int32_t)x.Z, (int32_t)shapes.size(1), row, row, q_off.defined() ? ip(q_off) : nullptr,
+  check(lib.dfa3d_attn3d_forward_rows(&x.p, (int32_t)x.Z, (int32_t)shapes.size(1), row, row,
+                                      q_off.defined() ? ip(q_off) : nullptr, q_row.defined() ? ip(q_row) : nullptr,
                                       value.const_data_ptr(), dist.const_data_ptr(), lp(shapes), lp(lsi), fp(ref), fp(joint),
                                       fp(joint) + 2 * part, fp(joint) + 3 * part, fpm(out), stream_of(value)),
         "dfa3d_attn3d_forward");
@@ -172,7 +174,7 @@ struct Attn3dJointFn : torch::autograd::Function<Attn3dJointFn> {
     const Tensor q_off = offsets.value_or(Tensor());
     ctx->save_for_backward({value, dist, shapes, lsi, ref, joint, q_off});
     keep(ctx, x);
-    return attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off);
+    return attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off, Tensor());
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const auto v = ctx->get_saved_variables();
@@ -458,12 +460,12 @@ PyObject *run_attn3d(PyObject *const *a, Py_ssize_t n, bool ragged) {
 
 PyObject *run_attn3d_joint(PyObject *const *a, Py_ssize_t n) {
   // value (B, N, H*C), dist (B, Nd, D), shapes (L, 2), lsi, ref (.., Z, 3), joint (.., 4*H*L*P), heads, points,
-  // q_off or None, max_queries, dist_map; ".." is B, Q or, with q_off, R
+  // q_off or None, max_queries, dist_map, q_row or None; ".." is B, Q or, with q_off, R -- of joint, with q_row, any number
   int64_t H, P, max_q = 0, mh, mw;
-  if (n != 11 || !plain_mode() || !integer(a[6], H) || !integer(a[7], P) || !map_argument(a[10], mh, mw)) return not_plain();
+  if (n != 12 || !plain_mode() || !integer(a[6], H) || !integer(a[7], P) || !map_argument(a[10], mh, mw)) return not_plain();
   const bool ragged = a[8] != Py_None;
   const int64_t k = ragged ? 1 : 2;
-  Tensor value, dist, shapes, lsi, ref, joint, q_off;
+  Tensor value, dist, shapes, lsi, ref, joint, q_off, q_row;
   if (!plain_tensor(a[0], value) || value.dim() != 3 || !plain_tensor(a[1], dist) || dist.dim() != 3 ||
       !long_tensor(a[2], shapes, 2) || !long_tensor(a[3], lsi, 1) || !float_tensor(a[4], ref, k + 2) ||
       !float_tensor(a[5], joint, k + 1))
@@ -473,8 +475,7 @@ PyObject *run_attn3d_joint(PyObject *const *a, Py_ssize_t n) {
       ref.requires_grad())
     return not_plain();
   const int64_t B = value.size(0), L = shapes.size(0), Z = ref.size(k);
-  if (shapes.size(1) != 2 || lsi.size(0) != L || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 || ref.size(0) != joint.size(0) ||
-      joint.size(-1) != 4 * H * L * P)
+  if (shapes.size(1) != 2 || lsi.size(0) != L || ref.size(-1) != 3 || Z <= 0 || P % Z != 0 || joint.size(-1) != 4 * H * L * P)
     return not_plain();
   auto x = c10::make_intrusive<Extra>();
   dfa3d_problem &p = x->p;
@@ -487,8 +488,15 @@ PyObject *run_attn3d_joint(PyObject *const *a, Py_ssize_t n) {
         !integer(a[9], max_q) || max_q < 0 || max_q >= (int64_t(1) << 31))
       return not_plain();
     p.Q = (int32_t)max_q;
+    if (a[11] != Py_None) {                      // no backward
+      if (!plain_tensor(a[11], q_row) || q_row.scalar_type() != at::kInt || q_row.numel() < ref.size(0) ||
+          !one_device(value, q_row) || wants_grad(value, dist, joint))
+        return not_plain();
+    } else if (ref.size(0) != joint.size(0)) {
+      return not_plain();
+    }
   } else {
-    if (joint.size(0) != B || ref.size(1) != joint.size(1)) return not_plain();
+    if (a[11] != Py_None || ref.size(0) != B || joint.size(0) != B || ref.size(1) != joint.size(1)) return not_plain();
     p.Q = (int32_t)joint.size(1);
   }
   p.L = (int32_t)L; p.P = (int32_t)P;
@@ -497,7 +505,7 @@ PyObject *run_attn3d_joint(PyObject *const *a, Py_ssize_t n) {
   {
     pybind11::gil_scoped_release nogil;
     r = wants_grad(value, dist, joint) ? Attn3dJointFn::apply(value, dist, shapes, lsi, ref, joint, given(q_off), x)
-                                       : attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off);
+                                       : attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off, q_row);
   }
   return THPVariable_Wrap(r);
 }

@@ -287,7 +287,7 @@ int dfa3d_msda_backward(const dfa3d_problem *p, const void *value, const int64_t
 
 static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride,
                                int64_t offsets_row, int64_t logits_row,
-                               const int32_t *query_offsets, const void *value, const void *dist,
+                               const int32_t *query_offsets, const int32_t *query_rows, const void *value, const void *dist,
                                const int64_t *shapes3, const int64_t *level_start,
                                const float *ref_points, const float *offsets_uv,
                                const float *offsets_depth, const float *logits, float *out,
@@ -298,6 +298,8 @@ static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int3
                 num_anchors, p->P);
   if (shape_stride != 2 && shape_stride != 3)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "shape_stride must be 2 or 3 (got %d)", shape_stride);
+  if (query_rows && !query_offsets)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "query_rows goes with query_offsets");
   if (p->B == 0 || p->Q == 0) return DFA3D_OK;
   REQUIRE_PTR(value); REQUIRE_PTR(dist); REQUIRE_PTR(shapes3); REQUIRE_PTR(level_start);
   REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets_uv); REQUIRE_PTR(offsets_depth); REQUIRE_PTR(logits);
@@ -308,6 +310,7 @@ static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int3
   a.loc = offsets_uv; a.off_d = offsets_depth; a.attn = logits; a.Z = num_anchors; a.out = out;
   set_rows(a, offsets_row, logits_row);
   a.q_off = query_offsets;
+  a.q_row = query_rows;
   return finish(dfa3d::launch_forward(a, p->value_dtype,
                                       p->dist_dtype, dfa3d::kCallerFused,
                                       (cudaStream_t)stream),
@@ -318,7 +321,7 @@ int dfa3d_attn3d_forward(const dfa3d_problem *p, int32_t num_anchors, const void
                          const void *dist, const int64_t *shapes3, const int64_t *level_start,
                          const float *ref_points, const float *offsets_uv, const float *offsets_depth,
                          const float *logits, float *out, void *stream) {
-  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, nullptr, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, nullptr, nullptr, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
@@ -329,7 +332,7 @@ int dfa3d_attn3d_forward_ragged(const dfa3d_problem *p, int32_t num_anchors,
                                 const float *offsets_depth, const float *logits, float *out,
                                 void *stream) {
   REQUIRE_PTR(query_offsets);
-  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, query_offsets, value, dist, shapes3, level_start, ref_points,
+  return attn3d_forward_impl(p, num_anchors, 3, 0, 0, query_offsets, nullptr, value, dist, shapes3, level_start, ref_points,
                              offsets_uv, offsets_depth, logits, out, stream);
 }
 
@@ -391,13 +394,12 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
 }
 
 int dfa3d_attn3d_forward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
-                             int64_t logits_row,
-                                const int32_t *query_offsets, const void *value, const void *dist,
-                                const int64_t *shapes, const int64_t *level_start, const float *ref_points,
-                                const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
-                                void *stream) {
-  return attn3d_forward_impl(p, num_anchors, shape_stride, offsets_row, logits_row, query_offsets, value, dist, shapes, level_start, ref_points,
-                             offsets_uv, offsets_depth, logits, out, stream);
+                              int64_t logits_row, const int32_t *query_offsets, const int32_t *query_rows,
+                              const void *value, const void *dist, const int64_t *shapes, const int64_t *level_start,
+                              const float *ref_points, const float *offsets_uv, const float *offsets_depth,
+                              const float *logits, float *out, void *stream) {
+  return attn3d_forward_impl(p, num_anchors, shape_stride, offsets_row, logits_row, query_offsets, query_rows, value, dist,
+                             shapes, level_start, ref_points, offsets_uv, offsets_depth, logits, out, stream);
 }
 
 int dfa3d_attn3d_backward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,

@@ -92,6 +92,8 @@ struct KArgs {
   // ragged queries: camera b owns the packed query rows [q_off[b], q_off[b+1]) of every per-query
   // tensor; Q is then only the bound the grid is sized for.  Null = every camera has Q queries.
   const int32_t *q_off;
+  // caller-fused forward: packed query row r reads its offsets and logits from row q_row[r] of theirs.  Null = row r
+  const int32_t *q_row;
   const float *grad_ds_in; // (B,Q,H,L,P,4) incoming depth-score gradient (two-stage depth backward)
   float *out;              // (B,Q,H*C)
   float *ds_out;           // (B,Q,H,L,P,4) or null
@@ -154,8 +156,10 @@ template <int MODE>
 __device__ __forceinline__ void item_inputs(const KArgs &a, ItemCtx &c) {
   c.pt0 = c.item * a.LP;
   if (mode_from_offsets(MODE)) {
-    c.loc = a.loc + (c.bq * a.row_loc + c.h * (a.LP * 2));
-    c.attn = a.attn + (c.bq * a.row_attn + c.h * a.LP);
+    unsigned row = (unsigned)c.bq;       // (64 bits spill and cost the base levels' forward 463 -> 495 us)
+    if (MODE == kCallerFused && a.q_row) row = (unsigned)__ldg(a.q_row + row);
+    c.loc = a.loc + (row * a.row_loc + c.h * (a.LP * 2));
+    c.attn = a.attn + (row * a.row_attn + c.h * a.LP);
   } else {
     c.loc = a.loc + c.pt0 * a.loc_stride;
     c.attn = a.attn + c.pt0;
@@ -215,9 +219,10 @@ __device__ __forceinline__ void prefetch_offsets(const KArgs &a, int b, unsigned
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long width = (long long)a.H * a.LP * 4;
   for (unsigned q = first / (unsigned)a.H + warp; q <= last / (unsigned)a.H; q += kWarpsPerCta) {
-    prefetch_l2(a.loc + (q0 + q) * a.row_loc, 2 * width, lane, 32);
-    prefetch_l2(a.off_d + (q0 + q) * a.row_attn, width, lane, 32);
-    prefetch_l2(a.attn + (q0 + q) * a.row_attn, width, lane, 32);
+    const long long row = a.q_row ? (long long)__ldg(a.q_row + q0 + q) : q0 + q;
+    prefetch_l2(a.loc + row * a.row_loc, 2 * width, lane, 32);
+    prefetch_l2(a.off_d + row * a.row_attn, width, lane, 32);
+    prefetch_l2(a.attn + row * a.row_attn, width, lane, 32);
   }
 }
 

@@ -60,10 +60,11 @@ dfa3d_forward_packed_kernel(const KArgs a) {
       const bool live = idx < nitems && (EXACT || j < a.LP);
       ItemCtx c;
       c.b = b;
-      const unsigned q = idx / (unsigned)a.H;
-      c.h = (int)(idx - q * (unsigned)a.H);
+      const unsigned inside = min(idx, nitems - 1);           // (past the end: the last item, which is there to read)
+      const unsigned q = inside / (unsigned)a.H;
+      c.h = (int)(inside - q * (unsigned)a.H);
       c.bq = q0 + q;
-      c.item = q0 * a.H + idx;
+      c.item = q0 * a.H + inside;
       item_inputs<MODE>(a, c);
       SoftmaxStats sm{0.f, 1.f};
       if (mode_from_offsets(MODE))

@@ -69,7 +69,7 @@ PLAIN_ENTRY_POINTS = {
     "dfa3d_attn2d_supported": [_P, _I32],
     "dfa3d_attn2d_forward": [_P, _I32, _I64, _I64] + [_V] * 8,
     "dfa3d_attn2d_backward": [_P, _I32, _I64, _I64] + [_V] * 11,
-    "dfa3d_attn3d_forward_rows": [_P, _I32, _I32, _I64, _I64] + [_V] * 11,
+    "dfa3d_attn3d_forward_rows": [_P, _I32, _I32, _I64, _I64] + [_V] * 12,
     "dfa3d_attn3d_backward_rows": [_P, _I32, _I32, _I64, _I64] + [_V] * 16,
     "dfa3d_rebatch_plan": [ctypes.c_void_p, _I32, _I32, _I32, _I32] + [ctypes.c_void_p] * 8,
     "dfa3d_rebatch_gather": [ctypes.c_void_p] * 4 + [_I32] * 4 + [_I64, _I64] + [ctypes.c_void_p] * 2

@@ -158,7 +158,7 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
 
     def forward(self, query, value, value_dpt_dist, reference_points, spatial_shapes, level_start_index,
                 query_pos=None, key_padding_mask=None, query_offsets=None, max_queries=None,
-                dist_map=None, value_projected=False):
+                dist_map=None, value_projected=False, query_rows=None):
         """query (bs, Q, E); value (bs, N, E); value_dpt_dist (bs, N, D); reference_points
         (bs, Q, Z, 3); spatial_shapes (L, 2) int64; level_start_index (L) int64.
         Returns (output (bs, Q, E), weight_update (bs, Q, H, 1))  -- :428-583.
@@ -170,7 +170,9 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
 
         ``dist_map=(h, w)``: value_dpt_dist is one h x w map per camera, (bs, h*w, D), that every level
         reads with nearest-neighbour indexing (instead of one resized copy per level).
-        ``value_projected``: value went through ``value_proj`` already."""
+        ``value_projected``: value went through ``value_proj`` already.  ``query_rows`` (int32, CUDA, at least R;
+        packed rows and no gradients only): packed row r stands for row query_rows[r] of query, whose
+        projections the cameras that see it then share."""
         ragged = query_offsets is not None
         if query_pos is not None:
             query = query + query_pos
@@ -193,9 +195,12 @@ class MSDeformableAttention3D_DFA3D(nn.Module):
             joint = joint_linear(query, self.sampling_offsets, self.sampling_offsets_depth, self.attention_weights)
             output = NotImplemented if joint is None else _lib.native().attn3d_joint(
                 value.contiguous(), value_dpt_dist.contiguous(), spatial_shapes, level_start_index,
-                reference_points.contiguous(), joint, H, P, query_offsets, max_queries, dist_map)
+                reference_points.contiguous(), joint, H, P, query_offsets, max_queries, dist_map, query_rows)
             if output is not NotImplemented:
                 return (output if ragged or self.batch_first else output.permute(1, 0, 2)), None
+        if query_rows is not None:
+            query = query[query_rows[:reference_points.shape[0]].long()]
+            lead = query.shape[:-1]
         value = value.view(bs, N, H, -1)
         off_uv = self.sampling_offsets(query).view(*lead, H, L, P, 2)
         off_d = self.sampling_offsets_depth(query).view(*lead, H, L, P, 1)
@@ -281,7 +286,12 @@ class SpatialCrossAttention_DFA3D(nn.Module):
         if type(attention) is MSDeformableAttention3D_DFA3D and not attention._forward_hooks \
                 and not attention._forward_pre_hooks:
             value, kw = attention.value_proj(value), {"value_projected": True}
-        q_rows = GatherQueriesFunction.apply(query.float(), plan)                 # (bs*T, E)
+        if kw and bs == 1 and not torch.is_grad_enabled():
+            # with gradients a row for each camera: they are summed over cameras at E values a query, before the
+            # projections, instead of at the projections' 4*H*L*P
+            q_rows, kw["query_rows"] = query.float()[0], plan.all_queries
+        else:
+            q_rows = GatherQueriesFunction.apply(query.float(), plan)             # (bs*T, E)
         ref_rows = plan.reference_rows(reference_points_cam.float())              # (bs*T, Z, 3)
         out_rows, update_weight = attention(
             query=q_rows, value=value, value_dpt_dist=dist, reference_points=ref_rows,

@@ -86,6 +86,11 @@ class RebatchPlan:
         return self._pq[:self.rows]
 
     @property
+    def all_queries(self):
+        """packed_query with its unused tail: no need to know how many rows there are."""
+        return self._pq
+
+    @property
     def packed_camera(self):
         return self._pc[:self.rows]
 

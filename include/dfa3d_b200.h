@@ -224,13 +224,14 @@ int dfa3d_attn3d_backward_ragged(const dfa3d_problem *p, int32_t num_anchors,
 /* dfa3d_attn3d_forward / _backward for either form of the queries (query_offsets null: dense) and either form of the level
  * table: shapes (L, shape_stride) with shape_stride 3 = (h, w, d), or 2 = (h, w) where every level has p->D bins.
  * offsets_row, logits_row: elements from query to query of offsets_uv, and of offsets_depth and logits (their gradients'
- * rows alike), 0 where these are contiguous: one Linear layer may produce all three side by side in one row. */
+ * rows alike), 0 where these are contiguous: one Linear layer may produce all three side by side in one row.
+ * query_rows: null, or (with query_offsets) for each packed query row the row of offsets_uv, offsets_depth and logits that it
+ * reads, an index the caller keeps inside these tensors: the cameras that see one query then share its row. */
 int dfa3d_attn3d_forward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
-                             int64_t logits_row,
-                                const int32_t *query_offsets, const void *value, const void *dist,
-                                const int64_t *shapes, const int64_t *level_start, const float *ref_points,
-                                const float *offsets_uv, const float *offsets_depth, const float *logits, float *out,
-                                void *stream);
+                              int64_t logits_row, const int32_t *query_offsets, const int32_t *query_rows,
+                              const void *value, const void *dist, const int64_t *shapes, const int64_t *level_start,
+                              const float *ref_points, const float *offsets_uv, const float *offsets_depth,
+                              const float *logits, float *out, void *stream);
 int dfa3d_attn3d_backward_rows(const dfa3d_problem *p, int32_t num_anchors, int32_t shape_stride, int64_t offsets_row,
                              int64_t logits_row,
                                  const int32_t *query_offsets, const void *value, const void *dist,
