@@ -770,7 +770,7 @@ def report(a, w, world, launches_per_step, value, ms_per_step, fwd_ms, bwd_ms, c
     }
     if a.impl == "ours":
         # items of 4 / 8 / 16 points (fp32, 16 / 32 / 64 channels) take the kernels in which a warp holds several
-        packed = w.L * w.P in (4, 8, 16) and w.C in (16, 32, 64) and w.value_dtype == "fp32"
+        packed = w.L * w.P <= 16 and w.C in (16, 32, 64)
         line["roofline"] = {
             "kernel": "dfa3d_backward_packed_kernel" if packed else "dfa3d_backward_kernel", "bound": "hbm",
             "achieved": bwd_b / (bwd_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
