@@ -70,9 +70,7 @@ struct FusedFn : torch::autograd::Function<FusedFn> {
     ctx->set_materialize_grads(false);
     const Tensor q_off = offsets.value_or(Tensor());
     auto out = fused_forward(x->p, value, dist, shapes, lsi, loc, attn, q_off, need_score);
-    if (x->half)
-      for (auto &t : out)
-        if (t.defined()) t = t.to(at::kHalf);
+    if (x->half) narrow_two(out[0], at::kHalf, out[1], at::kHalf);
     ctx->save_for_backward({value, dist, shapes, lsi, loc, attn, q_off});
     keep(ctx, x);
     if (!need_score) out.pop_back();
@@ -99,6 +97,9 @@ struct FusedFn : torch::autograd::Function<FusedFn> {
       check(lib.dfa3d_fused_backward(&x->p, value.const_data_ptr(), dist.const_data_ptr(), lp(v[2]), lp(v[3]), fp(loc),
                                      fp(attn), fp(go), fpm(gv), fpm(gd), fpm(gl), fpm(ga), s),
             "dfa3d_fused_backward");
+    // what autograd would convert after this node
+    narrow_two(gv, ctx->needs_input_grad(0) ? value.scalar_type() : at::kFloat, gd,
+               ctx->needs_input_grad(1) ? dist.scalar_type() : at::kFloat);
     return once({gv, gd, Tensor(), Tensor(), gl, ga, Tensor(), Tensor(), Tensor()}, grads);
   }
 };
@@ -401,9 +402,7 @@ PyObject *run_fused(PyObject *const *a, Py_ssize_t n, bool ragged, bool fp16) {
       r = FusedFn::apply(value, dist, shapes, lsi, loc, attn, given(q_off), need_score, x);
     } else {
       r = fused_forward(p, value, dist, shapes, lsi, loc, attn, q_off, need_score);
-      if (half.on)
-        for (auto &t : r)
-          if (t.defined()) t = t.to(at::kHalf);
+      if (half.on) narrow_two(r[0], at::kHalf, r[1], at::kHalf);
     }
   }
   return pair(r);

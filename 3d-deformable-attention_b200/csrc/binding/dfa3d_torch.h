@@ -34,7 +34,7 @@ using torch::autograd::variable_list;
   X(dfa3d_msda_forward) X(dfa3d_msda_backward) X(dfa3d_attn3d_forward_rows) X(dfa3d_attn3d_backward_rows) \
   X(dfa3d_fused_forward_ragged) X(dfa3d_fused_backward_ragged) \
   X(dfa3d_dist_from_logits) X(dfa3d_dist_from_logits_backward_typed)           \
-  X(dfa3d_zero_two) X(dfa3d_attn2d_supported) X(dfa3d_attn2d_forward) X(dfa3d_attn2d_backward)           \
+  X(dfa3d_zero_two) X(dfa3d_convert_two) X(dfa3d_attn2d_supported) X(dfa3d_attn2d_forward) X(dfa3d_attn2d_backward)           \
   X(dfa3d_rebatch_gather) X(dfa3d_rebatch_combine) X(dfa3d_add_layer_norm_forward)                       \
   X(dfa3d_add_layer_norm_infer) X(dfa3d_layer_norm_backward) X(dfa3d_column_sum)                         \
   X(dfa3d_relu_backward_column_sum) X(dfa3d_slice_sum) X(dfa3d_copy_segments)
@@ -170,7 +170,41 @@ inline const int64_t *lp(const Tensor &t) { return static_cast<const int64_t *>(
 inline const int32_t *ip(const Tensor &t) { return static_cast<const int32_t *>(t.const_data_ptr()); }
 
 // float32 and contiguous, whatever the consumer of the result handed back
-inline Tensor f32(const Tensor &g) { return (g.scalar_type() == at::kFloat ? g : g.to(at::kFloat)).contiguous(); }
+inline bool aligned16(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0; }
+
+inline Tensor f32(const Tensor &g) {
+  if (g.scalar_type() == at::kFloat) return g.contiguous();
+  if ((g.scalar_type() != at::kHalf && g.scalar_type() != at::kBFloat16) || !g.is_cuda() || !g.is_contiguous() || !aligned16(g))
+    return g.to(at::kFloat).contiguous();
+  c10::cuda::CUDAGuard guard(g.device());
+  Tensor w = empty_f32(g.sizes(), g);
+  check(lib.dfa3d_convert_two(dtype_code(g), 1, const_cast<void *>(g.const_data_ptr()), w.mutable_data_ptr(), g.numel(), nullptr,
+                              nullptr, 0, stream_of(g)),
+        "dfa3d_convert_two");
+  return w;
+}
+
+// fp32 results in the types that the caller gets them in (kFloat: as they are), both 16-bit ones with one launch; undefined
+// tensors stay so.
+inline void narrow_two(Tensor &a, at::ScalarType ta, Tensor &b, at::ScalarType tb) {
+  const bool na = a.defined() && ta != at::kFloat, nb = b.defined() && tb != at::kFloat;
+  if (!na && !nb) return;
+  if (na && nb && ta != tb) {
+    a = a.to(ta);
+    b = b.to(tb);
+    return;
+  }
+  c10::cuda::CUDAGuard guard((na ? a : b).device());
+  Tensor ra, rb;
+  if (na) ra = at::empty(a.sizes(), a.options().dtype(ta));
+  if (nb) rb = at::empty(b.sizes(), b.options().dtype(tb));
+  check(lib.dfa3d_convert_two(dtype_code(na ? ra : rb), 0, na ? ra.mutable_data_ptr() : nullptr,
+                              na ? a.mutable_data_ptr() : nullptr, na ? a.numel() : 0, nb ? rb.mutable_data_ptr() : nullptr,
+                              nb ? b.mutable_data_ptr() : nullptr, nb ? b.numel() : 0, stream_of(na ? a : b)),
+        "dfa3d_convert_two");
+  if (na) a = ra;
+  if (nb) b = rb;
+}
 
 // Gradients of a backward that must not be differentiated again: with create_graph the results get a node that
 // says so when it is reached (torch.autograd.function.once_differentiable does the same).

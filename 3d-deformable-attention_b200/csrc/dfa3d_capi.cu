@@ -679,6 +679,19 @@ int dfa3d_copy_segments(const float *const *src, float *const *dst, const int64_
   return finish(dfa3d::launch_copy_segments(src, dst, c, n, (cudaStream_t)stream), "dfa3d_copy_segments launch");
 }
 
+int dfa3d_convert_two(int32_t narrow_dtype, int32_t widen, void *narrow0, void *wide0, int64_t count0, void *narrow1,
+                      void *wide1, int64_t count1, void *stream) {
+  if (narrow_dtype != DFA3D_DTYPE_F16 && narrow_dtype != DFA3D_DTYPE_BF16)
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "narrow_dtype %d is not a 16-bit DFA3D_DTYPE_*", narrow_dtype);
+  if (count0 < 0 || count1 < 0) return fail(DFA3D_ERR_INVALID_ARGUMENT, "counts must be >= 0");
+  if (count0 > 0) { REQUIRE_PTR(narrow0); REQUIRE_PTR(wide0); }
+  if (count1 > 0) { REQUIRE_PTR(narrow1); REQUIRE_PTR(wide1); }
+  REQUIRE_ALIGNED(narrow0); REQUIRE_ALIGNED(wide0); REQUIRE_ALIGNED(narrow1); REQUIRE_ALIGNED(wide1);
+  return finish(dfa3d::launch_convert_two(narrow_dtype == DFA3D_DTYPE_F16, widen != 0, narrow0, wide0, count0, narrow1, wide1,
+                                          count1, (cudaStream_t)stream),
+                "dfa3d_convert_two launch");
+}
+
 int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream) {
   if (na < 0 || nb < 0)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "element counts must be >= 0 (got %lld, %lld)", (long long)na, (long long)nb);

@@ -76,5 +76,7 @@ cudaError_t launch_relu_backward(const float *grad_y, const float *y, long long 
 cudaError_t launch_slice_sum(const float *part, int slices, int out, int in, const float *g_tail, const float *x_tail, int tail,
                              float *dst, float *zero, cudaStream_t s);
 cudaError_t launch_copy_segments(const float *const *src, float *const *dst, const long long *n, int count, cudaStream_t s);
+cudaError_t launch_convert_two(bool half, bool widen, void *n0, void *w0, long long c0, void *n1, void *w1, long long c1,
+                               cudaStream_t s);
 cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cudaStream_t s);
 }  // namespace dfa3d

@@ -14,6 +14,9 @@
 
 #include <algorithm>
 
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
 #include "dfa3d_launch.h"
 
 namespace dfa3d {
@@ -342,6 +345,51 @@ __global__ void __launch_bounds__(256) zero_two_kernel(float *a, long long na, f
   if (t0 < (nb & 3)) b[vb * 4 + t0] = 0.f;
 }
 
+// Converts up to two buffers between fp32 and a 16-bit type with one launch, eight elements (16 bytes of the narrow type) a
+// thread at a time, the ragged ends one by one.  Bound by HBM and L2.  The five conversions of an fp16 operator call and its
+// backward (outputs 6.9 M elements, gradients 4.2 M, grad_out 1.5 M), one launch of torch's each: 20.7 us; as three 14.4.
+template <typename T> struct Narrow;
+template <> struct Narrow<__half> {
+  __device__ static __forceinline__ __half of(float x) { return __float2half_rn(x); }
+  __device__ static __forceinline__ float wide(__half x) { return __half2float(x); }
+};
+template <> struct Narrow<__nv_bfloat16> {
+  __device__ static __forceinline__ __nv_bfloat16 of(float x) { return __float2bfloat16_rn(x); }
+  __device__ static __forceinline__ float wide(__nv_bfloat16 x) { return __bfloat162float(x); }
+};
+
+template <typename T, bool WIDEN>
+__global__ void __launch_bounds__(256)
+convert_two_kernel(void *n0, void *w0, long long c0, void *n1, void *w1, long long c1) {
+  const long long v0 = c0 >> 3, v1 = c1 >> 3, step = (long long)gridDim.x * blockDim.x;
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long t = t0; t < v0 + v1; t += step) {
+    T *n = t < v0 ? static_cast<T *>(n0) + t * 8 : static_cast<T *>(n1) + (t - v0) * 8;
+    float *w = t < v0 ? static_cast<float *>(w0) + t * 8 : static_cast<float *>(w1) + (t - v0) * 8;
+    __align__(16) T x[8];
+    if (WIDEN) {
+      *reinterpret_cast<uint4 *>(x) = *reinterpret_cast<const uint4 *>(n);
+#pragma unroll
+      for (int i = 0; i < 8; i += 4)
+        st4(w + i, make_float4(Narrow<T>::wide(x[i]), Narrow<T>::wide(x[i + 1]), Narrow<T>::wide(x[i + 2]),
+                               Narrow<T>::wide(x[i + 3])));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i += 4) {
+        const float4 f = *reinterpret_cast<const float4 *>(w + i);
+        x[i] = Narrow<T>::of(f.x); x[i + 1] = Narrow<T>::of(f.y); x[i + 2] = Narrow<T>::of(f.z); x[i + 3] = Narrow<T>::of(f.w);
+      }
+      *reinterpret_cast<uint4 *>(n) = *reinterpret_cast<const uint4 *>(x);
+    }
+  }
+  auto one = [&](void *n, void *w, long long i) {
+    if (WIDEN) static_cast<float *>(w)[i] = Narrow<T>::wide(static_cast<const T *>(n)[i]);
+    else static_cast<T *>(n)[i] = Narrow<T>::of(static_cast<const float *>(w)[i]);
+  };
+  if (t0 < (c0 & 7)) one(n0, w0, v0 * 8 + t0);
+  if (t0 < (c1 & 7)) one(n1, w1, v1 * 8 + t0);
+}
+
 unsigned row_grid(long long rows) {
   const long long want = (rows + kLnWarps - 1) / kLnWarps;
   const long long cap = (long long)kSms * kCtasPerSm;
@@ -444,6 +492,18 @@ cudaError_t launch_zero_two(float *a, long long na, float *b, long long nb, cuda
   const long long groups = (na + nb + 3) / 4, want = (groups + 255) / 256, cap = (long long)kSms * 8;
   if (na + nb == 0) return cudaSuccess;
   zero_two_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(a, na, b, nb);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_convert_two(bool half, bool widen, void *n0, void *w0, long long c0, void *n1, void *w1, long long c1,
+                               cudaStream_t s) {
+  if (c0 + c1 == 0) return cudaSuccess;
+  const long long want = ((c0 + c1 + 7) / 8 + 255) / 256, cap = (long long)kSms * 8;
+  const unsigned grid = (unsigned)(want < cap ? want : cap);
+  if (half && widen) convert_two_kernel<__half, true><<<grid, 256, 0, s>>>(n0, w0, c0, n1, w1, c1);
+  else if (half) convert_two_kernel<__half, false><<<grid, 256, 0, s>>>(n0, w0, c0, n1, w1, c1);
+  else if (widen) convert_two_kernel<__nv_bfloat16, true><<<grid, 256, 0, s>>>(n0, w0, c0, n1, w1, c1);
+  else convert_two_kernel<__nv_bfloat16, false><<<grid, 256, 0, s>>>(n0, w0, c0, n1, w1, c1);
   return cudaGetLastError();
 }
 

@@ -89,6 +89,7 @@ PLAIN_ENTRY_POINTS = {
     "dfa3d_relu_backward_column_sum": [ctypes.c_void_p] * 2 + [_I64, _I32] + [ctypes.c_void_p] * 3,
     "dfa3d_slice_sum": [ctypes.c_void_p] + [_I32] * 3 + [ctypes.c_void_p] * 2 + [_I32] + [ctypes.c_void_p] * 3,
     "dfa3d_copy_segments": [ctypes.c_void_p] * 3 + [_I32, ctypes.c_void_p],
+    "dfa3d_convert_two": [_I32, _I32, _V, _V, _I64, _V, _V, _I64, _V],
     "dfa3d_zero_two": [ctypes.c_void_p, _I64, ctypes.c_void_p, _I64, ctypes.c_void_p],
 }
 ACT_SOFTMAX, ACT_SIGMOID = 0, 1

@@ -391,6 +391,11 @@ int dfa3d_copy_segments(const float *const *src, float *const *dst, const int64_
  * count may be 0 (its pointer is then not looked at); pointers 16-byte aligned. */
 int dfa3d_zero_two(float *a, int64_t na, float *b, int64_t nb, void *stream);
 
+/* Converts one or two buffers (count1 may be 0) between fp32 and a 16-bit type: wide -> narrow rounded to nearest, or with
+ * `widen` narrow -> wide.  All addresses 16-byte aligned. */
+int dfa3d_convert_two(int32_t narrow_dtype, int32_t widen, void *narrow0, void *wide0, int64_t count0, void *narrow1,
+                      void *wide1, int64_t count1, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
