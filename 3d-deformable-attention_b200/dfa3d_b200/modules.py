@@ -35,7 +35,8 @@ from .functions import (MultiScaleDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnRaggedFunction_fp32)
 from . import _lib
 from .layer_ops import AddLayerNorm, Linear, joint_linear, linear_relu
-from .rebatch import CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan
+from .rebatch import (CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan,
+                      gather_per_camera)
 
 
 def bev_reference_points(bev_h, bev_w, pillar_height=8, num_points_in_pillar=4, dim="3d", bs=1,
@@ -292,7 +293,7 @@ class SpatialCrossAttention_DFA3D(nn.Module):
             q_rows, kw["query_rows"] = query.float()[0], plan.all_queries
         else:
             q_rows = GatherQueriesFunction.apply(query.float(), plan)             # (bs*T, E)
-        ref_rows = plan.reference_rows(reference_points_cam.float())              # (bs*T, Z, 3)
+        ref_rows = gather_per_camera(reference_points_cam.float(), plan)          # (bs*T, Z, 3)
         out_rows, update_weight = attention(
             query=q_rows, value=value, value_dpt_dist=dist, reference_points=ref_rows,
             spatial_shapes=spatial_shapes, level_start_index=level_start_index,

@@ -62,7 +62,6 @@ class RebatchPlan:
         self._counted = torch.cuda.Event()
         self._counted.record(torch.cuda.current_stream(dev))
         self._sizes = None
-        self._reference = None
 
     def _resolve(self):
         if self._sizes is None:
@@ -93,14 +92,6 @@ class RebatchPlan:
     @property
     def packed_camera(self):
         return self._pc[:self.rows]
-
-    def reference_rows(self, reference_points_cam):
-        """``gather_per_camera(reference_points_cam, self)``, kept for the other layers of the frame: they are handed
-        the same tensor, which is geometry like the mask."""
-        key = (reference_points_cam, reference_points_cam._version)
-        if self._reference is None or self._reference[0] is not key[0] or self._reference[1] != key[1]:
-            self._reference = key + (gather_per_camera(reference_points_cam, self),)
-        return self._reference[2]
 
     @property
     def native_args(self):
