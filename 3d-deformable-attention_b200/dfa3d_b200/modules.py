@@ -547,7 +547,7 @@ class BEVFormerEncoderLayer(nn.Module):
                  bev_h=200, bev_w=200, dropout=0.1):
         super().__init__()
         self.bev_h, self.bev_w = bev_h, bev_w
-        self._tables = None
+        self._tables = {}
         self.self_attn = TemporalSelfAttention(embed_dims, num_heads, num_levels=1, num_points=4,
                                                dropout=dropout)
         self.norm0 = AddLayerNorm(embed_dims)
@@ -561,14 +561,26 @@ class BEVFormerEncoderLayer(nn.Module):
         self.norm2 = AddLayerNorm(embed_dims)
 
     def _bev_tables(self, device, dtype):
-        """Level table of the BEV and the centres of its cells (1, Q, 1, 2): constants of the layer, made once per device
-        and dtype (making them takes a synchronising copy and a dozen small kernels)."""
+        """Level table of the BEV and the centres of its cells (1, Q, 1, 2): constants of the layer, made once per size,
+        device and dtype (making them takes a synchronising copy and a dozen small kernels).  They are ordinary tensors
+        also when the first pass is made in inference mode, because a later training pass saves them for its backward;
+        complete before they are kept, because the next pass may come on another stream; and not part of the layer's
+        pickled state, which may be loaded for another device."""
+        if not isinstance(self.__dict__.get("_tables"), dict):              # a layer pickled without them
+            self._tables = {}
         key = (device, dtype, self.bev_h, self.bev_w)
-        if getattr(self, "_tables", None) is None or self._tables[0] != key:
-            self._tables = (key, torch.tensor([[self.bev_h, self.bev_w]], dtype=torch.int64, device=device),
-                            torch.zeros(1, dtype=torch.int64, device=device),
-                            bev_reference_points(self.bev_h, self.bev_w, dim="2d", device=device, dtype=dtype))
-        return self._tables[1:]
+        if key not in self._tables:
+            with torch.inference_mode(False):
+                made = (torch.tensor([[self.bev_h, self.bev_w]], dtype=torch.int64, device=device),
+                        torch.zeros(1, dtype=torch.int64, device=device),
+                        bev_reference_points(self.bev_h, self.bev_w, dim="2d", device=device, dtype=dtype))
+            if device.type == "cuda":
+                torch.cuda.current_stream(device).synchronize()
+            self._tables[key] = made
+        return self._tables[key]
+
+    def __getstate__(self):
+        return dict(self.__dict__, _tables={})
 
     def forward(self, query, prev_bev=None, bev_pos=None, ref_2d=None, **cross_kw):
         """query (bs, bev_h*bev_w, E); prev_bev: None or (bs*2, Q, E) = [previous, current] BEV per batch

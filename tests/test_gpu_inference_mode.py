@@ -43,3 +43,32 @@ def test_reference_points_are_read_in_every_pass(lib_built):
         got = stack(d["query"], **kw)
         want = stack(d["query"], **dict(kw, reference_points_cam=d["reference_points_cam"].clone()))
     assert torch.equal(got, want)
+
+
+def _full_layer():
+    torch.manual_seed(1)
+    return modules.BEVFormerEncoderLayer(embed_dims=32, ffn_dims=64, num_cams=3, num_heads=2, num_levels=2, num_points=8,
+                                         bev_h=5, bev_w=10, dropout=0.0).to(DEV)
+
+
+def test_layer_trains_after_it_has_served(lib_built):
+    layer, d = _full_layer(), _inputs(5)
+    with torch.inference_mode():
+        served = layer(d["query"], **_keywords(d)).clone()
+    out = layer(d["query"].requires_grad_(True), **_keywords(d))
+    assert torch.equal(out, served)
+    out.sum().backward()
+    assert all(torch.isfinite(p.grad).all() for p in layer.parameters())
+
+
+def test_layer_saved_after_a_pass_runs_where_it_is_loaded(lib_built, tmp_path):
+    layer, d = _full_layer(), _inputs(6)
+    with torch.no_grad():
+        want = layer(d["query"], **_keywords(d))
+        torch.save(layer, tmp_path / "layer.pt")
+        loaded = torch.load(tmp_path / "layer.pt", map_location="cpu", weights_only=False).to(DEV)
+        assert torch.equal(loaded(d["query"], **_keywords(d)), want)
+        layer.bev_h, layer.bev_w = 10, 5                                     # another size of the same layer
+        other = layer(d["query"], **_keywords(d))
+        layer.bev_h, layer.bev_w = 5, 10
+        assert torch.equal(layer(d["query"], **_keywords(d)), want) and not torch.equal(other, want)
