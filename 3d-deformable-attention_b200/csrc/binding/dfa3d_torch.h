@@ -5,6 +5,7 @@
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <ATen/ATen.h>
@@ -65,9 +66,10 @@ inline void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(
 // ------------------------------------------------------------------------------------------------
 // arguments
 // ------------------------------------------------------------------------------------------------
-// Modes in which the Python Function does something of its own.
+// Modes in which the Python Function does something of its own.  (Under jit.trace it becomes an operation of the graph; of a
+// call made here the tracer would see the allocation of the result and not the kernel that fills it.)
 inline bool plain_mode() {
-  return bound && !at::autocast::is_autocast_enabled(at::kCUDA) &&
+  return bound && !torch::jit::tracer::isTracing() && !at::autocast::is_autocast_enabled(at::kCUDA) &&
          !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
          !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
