@@ -171,12 +171,12 @@ inline float *fpm(const Tensor &t) { return static_cast<float *>(t.mutable_data_
 inline const int64_t *lp(const Tensor &t) { return static_cast<const int64_t *>(t.const_data_ptr()); }
 inline const int32_t *ip(const Tensor &t) { return static_cast<const int32_t *>(t.const_data_ptr()); }
 
-// float32 and contiguous, whatever the consumer of the result handed back
-inline bool aligned16(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0; }
+inline bool aligned(const Tensor &t, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % bytes == 0; }
 
+// float32 and contiguous, whatever the consumer of the result handed back
 inline Tensor f32(const Tensor &g) {
   if (g.scalar_type() == at::kFloat) return g.contiguous();
-  if ((g.scalar_type() != at::kHalf && g.scalar_type() != at::kBFloat16) || !g.is_cuda() || !g.is_contiguous() || !aligned16(g))
+  if ((g.scalar_type() != at::kHalf && g.scalar_type() != at::kBFloat16) || !g.is_cuda() || !g.is_contiguous() || !aligned(g, 16))
     return g.to(at::kFloat).contiguous();
   c10::cuda::CUDAGuard guard(g.device());
   Tensor w = empty_f32(g.sizes(), g);

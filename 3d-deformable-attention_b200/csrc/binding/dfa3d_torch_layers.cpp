@@ -28,9 +28,11 @@ void parameter_gradients(const Tensor &g, const Tensor &x, bool weight, bool bia
     const int64_t k = rows / kSplits, head = k * kSplits;
     const Tensor part = at::bmm(g.as_strided({kSplits, out, k}, {k * out, 1, out}), x.as_strided({kSplits, k, in}, {k * in, in, 1}));
     gw = empty_f32({out, in}, g);
+    const bool own_tail = aligned(x, 16);             // the kernel reads x's last rows in 16-byte words
     check(lib.dfa3d_slice_sum(fp(part), (int32_t)kSplits, (int32_t)out, (int32_t)in, fp(g) + head * out, fp(x) + head * in,
-                              (int32_t)(rows - head), fpm(gw), bias ? fpm(gb) : nullptr, s),
+                              own_tail ? (int32_t)(rows - head) : 0, fpm(gw), bias ? fpm(gb) : nullptr, s),
           "dfa3d_slice_sum");
+    if (!own_tail && head < rows) gw.addmm_(g.narrow(0, head, rows - head).t(), x.narrow(0, head, rows - head));
     zeroed = true;
   }
   if (!bias) return;
@@ -65,6 +67,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const bool relu = ctx->saved_data["relu"].toBool();
     if (relu) {
       void *s = stream_of(g);
+      if (!aligned(g, 16)) g = g.clone();
       Tensor masked = at::empty_like(g);
       gb = empty_f32({g.size(1)}, g);
       zero_two(gb, Tensor(), s);
@@ -416,6 +419,7 @@ PyObject *run_attn2d(PyObject *const *a, Py_ssize_t n) {
   if (maps <= 0 || H <= 0 || P <= 0 || maps > 16 || value.size(2) % H != 0 || value.size(0) % maps != 0 || !small(value) ||
       !small(joint) || !one_device(value, shapes, lsi, ref, joint) || ref.requires_grad())
     return not_plain();
+  if (!aligned(value, 16) || !aligned(ref, 8) || !aligned(joint, 8)) return not_plain();
   const int64_t bs = value.size(0) / maps, Q = joint.size(1), L = shapes.size(0), pts = H * maps * L * P;
   if (shapes.size(1) != 2 || lsi.size(0) != L || !sizes_are(ref, {bs * maps, Q, L, 2}) || !sizes_are(joint, {bs, Q, pts * 3}))
     return not_plain();

@@ -22,6 +22,7 @@ int fail(int code, const char *fmt, ...) {
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
 // Checks the descriptor; `need_value` / `need_dist` say which tensors the call reads.
 int check_problem(const dfa3d_problem *p, bool need_value, bool need_dist) {
@@ -73,6 +74,10 @@ int check_problem(const dfa3d_problem *p, bool need_value, bool need_dist) {
 #define REQUIRE_ALIGNED(ptr)                                                                          \
   do {                                                                                                 \
     if (!aligned16(ptr)) return fail(DFA3D_ERR_INVALID_ARGUMENT, "`%s` must be 16-byte aligned", #ptr); \
+  } while (0)
+#define REQUIRE_ALIGNED8(ptr)                                                                         \
+  do {                                                                                                 \
+    if (!aligned8(ptr)) return fail(DFA3D_ERR_INVALID_ARGUMENT, "`%s` must be 8-byte aligned", #ptr); \
   } while (0)
 
 dfa3d::KArgs base_args(const dfa3d_problem *p, int shape_stride, int loc_stride) {
@@ -431,7 +436,8 @@ static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, int64_t offsets
                 "item in maps of a power of two (got C=%d, L*P=%d, maps=%d)", p->C, p->L * p->P, num_maps);
   REQUIRE_PTR(value); REQUIRE_PTR(shapes2); REQUIRE_PTR(level_start); REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets);
   REQUIRE_PTR(logits);
-  REQUIRE_ALIGNED(value); REQUIRE_ALIGNED(ref_points); REQUIRE_ALIGNED(offsets);
+  REQUIRE_ALIGNED(value);
+  REQUIRE_ALIGNED8(ref_points); REQUIRE_ALIGNED8(offsets);      // read as pairs
   dfa3d_problem q = *p;
   q.N *= num_maps;
   q.L *= num_maps;

@@ -180,7 +180,8 @@ int dfa3d_attn3d_backward(const dfa3d_problem *p, int32_t num_anchors, const voi
  * (B,Q,H,maps,L,P,2), logits (B,Q,H,maps,L*P), out (B,Q,H*C), all fp32.  dfa3d_attn2d_supported(): 1 for the sizes the
  * kernels exist for (C of 16, 32 or 64; 4, 8 or 16 points over all maps, a power of two in each), else 0.  Backward:
  * grad_value is ACCUMULATED into; grad_offsets and grad_logits are overwritten; the reference points get none.
- * offsets_row, logits_row: elements from query to query of offsets and logits, 0 where these are contiguous. */
+ * offsets_row, logits_row: elements from query to query of offsets and logits, 0 where these are contiguous.
+ * ref_points and offsets 8-byte aligned, offsets_row even; value, out, grad_out and grad_value 16-byte aligned. */
 int dfa3d_attn2d_supported(const dfa3d_problem *p, int32_t num_maps);
 int dfa3d_attn2d_forward(const dfa3d_problem *p, int32_t num_maps, int64_t offsets_row, int64_t logits_row, const void *value, const int64_t *shapes2,
                          const int64_t *level_start, const float *ref_points, const float *offsets,
