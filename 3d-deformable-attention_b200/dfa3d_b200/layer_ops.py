@@ -16,6 +16,7 @@ Functions); like the rest of the package there is no fallback path.
 """
 import torch
 import torch.nn as nn
+import torch.nn.modules.module as _module
 from torch.autograd.function import Function, once_differentiable
 
 from . import _lib
@@ -162,10 +163,17 @@ class Linear(nn.Linear):
         return LinearFunction.apply(x, self.weight, self.bias)
 
 
+def runs_forward_only(m):
+    """Whether calling module `m` does nothing but run its class's ``forward``, so that an operation that does the same
+    work may stand in for the call: no hooks of its own, no hooks for all modules, no ``forward`` set on the instance."""
+    return not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks
+                or _module._global_backward_hooks or _module._global_backward_pre_hooks or "forward" in m.__dict__)
+
+
 def _plain_linear(m):
-    """A Linear whose forward is LinearFunction and nothing else: no hooks that calling it would run."""
-    return (type(m) is Linear and m.bias is not None and m.out_features % 4 == 0 and not m._forward_hooks
-            and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks)
+    """A Linear whose call is LinearFunction and nothing else."""
+    return type(m) is Linear and m.bias is not None and m.out_features % 4 == 0 and runs_forward_only(m)
 
 
 def joint_linear(x, *linears):
@@ -180,8 +188,7 @@ def joint_linear(x, *linears):
 def linear_relu(x, linear, relu):
     """relu(linear(x)); as one operation where both are plain: the ReLU is the product's epilogue, its backward and the
     bias gradient are one kernel."""
-    if _plain_linear(linear) and type(relu) is nn.ReLU and not relu._forward_hooks and not relu._forward_pre_hooks \
-            and not relu._backward_hooks and not relu._backward_pre_hooks:
+    if _plain_linear(linear) and type(relu) is nn.ReLU and runs_forward_only(relu):
         out = _lib.native().linear_relu(x, linear.weight, linear.bias)
         if out is not NotImplemented:
             return out

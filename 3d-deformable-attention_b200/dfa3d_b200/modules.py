@@ -34,7 +34,7 @@ from .functions import (MultiScaleDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnFunction_fp32,
                         MultiScale3DDeformableAttnRaggedFunction_fp32)
 from . import _lib
-from .layer_ops import AddLayerNorm, Linear, joint_linear, linear_relu
+from .layer_ops import AddLayerNorm, Linear, joint_linear, linear_relu, runs_forward_only
 from .rebatch import (CombineCamerasFunction, GatherQueriesFunction, GatherSharedRowsFunction, RebatchPlan,
                       gather_per_camera)
 
@@ -284,8 +284,7 @@ class SpatialCrossAttention_DFA3D(nn.Module):
         # the value projection does not need the plan's row count: queued first, it keeps the device busy while the
         # count is read back
         attention, kw = self.deformable_attention, {}
-        if type(attention) is MSDeformableAttention3D_DFA3D and not attention._forward_hooks \
-                and not attention._forward_pre_hooks:
+        if type(attention) is MSDeformableAttention3D_DFA3D and runs_forward_only(attention):
             value, kw = attention.value_proj(value), {"value_projected": True}
         if kw and bs == 1 and not torch.is_grad_enabled():
             # with gradients a row for each camera: they are summed over cameras at E values a query, before the
@@ -427,11 +426,15 @@ class TemporalSelfAttention(nn.Module):
 
 
 def _run_ffn(ffn, x):
-    """The feed-forward block (Linear, ReLU, Dropout, Linear, Dropout) with the first Linear and the ReLU as one
-    operation."""
-    if ffn._forward_hooks or ffn._forward_pre_hooks or ffn._backward_hooks or ffn._backward_pre_hooks:
+    """``ffn(x)``; where it is a plain Sequential that begins with a Linear and a ReLU, as the layers build it, these two
+    are one operation."""
+    if type(ffn) is not nn.Sequential or len(ffn) < 2 or not runs_forward_only(ffn):
         return ffn(x)
-    return ffn[4](ffn[3](ffn[2](linear_relu(x, ffn[0], ffn[1]))))
+    first, second, *rest = ffn
+    x = linear_relu(x, first, second)
+    for m in rest:
+        x = m(x)
+    return x
 
 
 class SCAEncoderLayer(nn.Module):
