@@ -589,7 +589,8 @@ class BEVFormerEncoderLayer(nn.Module):
         """query (bs, bev_h*bev_w, E); prev_bev: None or (bs*2, Q, E) = [previous, current] BEV per batch
         element (encoder.py:519-528 stacks them); ref_2d (bs*2, Q, 1, 2) (`bev_reference_points(dim="2d")`,
         shifted for the previous BEV by the caller); cross_kw: the spatial cross-attention's inputs."""
-        if cross_kw.get("rebatch_plan") is None:    # started before the self-attention, whose work hides its read-back
+        if cross_kw.get("rebatch_plan") is None and type(self.cross_attn) is SpatialCrossAttention_DFA3D:
+            # started before the self-attention, whose work hides its read-back
             cross_kw["rebatch_plan"] = RebatchPlan(cross_kw["bev_mask"])
         shapes, lsi, cells = self._bev_tables(query.device, query.dtype)
         if ref_2d is None:

@@ -80,3 +80,18 @@ def test_a_forward_set_on_an_instance_is_called(lib_built):
         layer(d["query"], **{k: d[k] for k in KEYS})
     assert sorted(called) == sorted(["ffn.0", "ffn.1", "ffn", "cross_attn.deformable_attention", "self_attn.sampling_offsets",
                                      "cross_attn.deformable_attention.attention_weights"])
+
+
+class _OtherCrossAttention(nn.Module):
+    """A user's block with the layer's inputs and no more."""
+
+    def forward(self, query, value, value_dpt_dist, reference_points_cam, bev_mask, spatial_shapes, level_start_index,
+                return_residual):
+        return query * 0.5, query
+
+
+def test_replaced_cross_attention_gets_what_the_caller_gave(lib_built):
+    layer, d = _layer(), _inputs(9)
+    layer.cross_attn = _OtherCrossAttention()
+    with torch.no_grad():
+        assert layer(d["query"], **{k: d[k] for k in KEYS}).shape == d["query"].shape
