@@ -2,10 +2,12 @@
 measurement code) and _native.so (host path of the autograd Functions) in-tree, for sm_100a.
 
 The library is plain CUDA C++ behind an ``extern "C"`` interface (include/dfa3d_b200.h) without torch
-headers; only _native.so, which contains no kernels, is compiled against torch.  The results are written
+headers; only _native.so, which contains no kernels, is compiled against torch, and carries the version of
+the torch it was compiled against: with another one installed it is built anew.  The results are written
 next to the Python package (``dfa3d_b200/``) so that they are found without any install step.
 """
 import os
+import shutil
 import subprocess
 import sys
 
@@ -30,16 +32,30 @@ def _nvcc():
     return "nvcc"
 
 
+def _cuda_include():
+    """The headers of the toolkit that `_nvcc` belongs to."""
+    nvcc = shutil.which(_nvcc()) or "/usr/local/cuda/bin/nvcc"
+    return os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+
+
+def _built_for():
+    """What _native.so is compiled against; it holds this text."""
+    import sysconfig
+    import torch
+    return f"torch {torch.__version__} python {sysconfig.get_config_var('SOABI')}"
+
+
 def _native_command():
     """g++ command of the torch binding: header and library folders come from the installed torch."""
     import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+           sysconfig.get_paths()["include"], _cuda_include()]
     lib = os.path.join(root, "lib")
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE,
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DDFA3D_BUILT_FOR="{_built_for()}"',
+            "-I", INCLUDE,
             *[a for i in inc for a in ("-isystem", i)], *NATIVE_SRC, "-o", NATIVE_OUT, "-L", lib,
             "-Wl,-rpath," + lib, "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
@@ -48,6 +64,9 @@ def needs_build():
     outs = (OUT, RATES_OUT, NATIVE_OUT)
     if not all(os.path.exists(o) for o in outs):
         return True
+    with open(NATIVE_OUT, "rb") as f:
+        if _built_for().encode() not in f.read():
+            return True
     t = min(os.path.getmtime(o) for o in outs)
     deps = [os.path.join(d, f) for d, _, fs in os.walk(CSRC) for f in fs]
     deps.append(os.path.join(HERE, "..", "include", "dfa3d_b200.h"))

@@ -664,7 +664,9 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nu
 
 PyMODINIT_FUNC PyInit__native(void) {
   PyObject *m = PyModule_Create(&module);
-  if (m && PyModule_AddFunctions(m, dfa3d_torch::layer_methods) != 0) {
+  // the headers this was compiled against: another torch may lay its classes out differently
+  if (m && (PyModule_AddFunctions(m, dfa3d_torch::layer_methods) != 0 ||
+            PyModule_AddStringConstant(m, "built_for", DFA3D_BUILT_FOR) != 0)) {
     Py_DECREF(m);
     return nullptr;
   }

@@ -144,12 +144,15 @@ def native():
     """The native host path (csrc/binding): built beside the library, bound to the library's entry points."""
     global _native
     if _native is None:
+        import torch
         lib = load()
+        how = "build it with `python 3d-deformable-attention_b200/build.py`. dfa3d_b200 has no fallback implementation."
         try:
             from . import _native as mod
         except ImportError as e:
-            raise ImportError(f"{e}: build it with `python 3d-deformable-attention_b200/build.py`. dfa3d_b200 has no "
-                              "fallback implementation.") from e
+            raise ImportError(f"{e}: {how}") from e
+        if mod.built_for.split()[1] != str(torch.__version__):
+            raise ImportError(f"{mod.__file__} was built for {mod.built_for}, this is torch {torch.__version__}: {how}")
         mod.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in mod.entries()})
         _native = mod
     return _native
