@@ -50,6 +50,10 @@ Tensor linear_forward(const Tensor &x, const Tensor &w, const Tensor &b, bool re
   return y;
 }
 
+// The products of a backward are of the forward's kind, float32, wherever backward() is called: autograd carries the caller's
+// autocast state into the node, where a product in 16 bits would be taken for a float32 one.
+using NoAutocast = c10::impl::ExcludeDispatchKeyGuard;
+
 struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const Tensor &b, bool relu) {
     c10::cuda::CUDAGuard guard(x.device());
@@ -60,6 +64,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     return y;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const NoAutocast no_autocast(c10::autocast_dispatch_keyset);
     const auto v = ctx->get_saved_variables();
     const Tensor &x = v[0], &w = v[1];
     c10::cuda::CUDAGuard guard(x.device());
@@ -111,6 +116,7 @@ struct JointLinearFn : torch::autograd::Function<JointLinearFn> {
     return linear_forward(x, W, B, false);
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    const NoAutocast no_autocast(c10::autocast_dispatch_keyset);
     const auto v = ctx->get_saved_variables();
     const Tensor &x = v[0], &W = v[1];
     c10::cuda::CUDAGuard guard(x.device());
