@@ -20,20 +20,13 @@ using namespace dfa3d_torch;
 namespace {
 
 // ------------------------------------------------------------------------------------------------
-// autograd nodes; what they keep beside their tensors travels in one capsule
+// autograd nodes; what they keep beside their tensors travels with them in one capsule
 // ------------------------------------------------------------------------------------------------
-struct Extra : torch::CustomClassHolder {
+struct Extra : Kept {
   dfa3d_problem p;
   int64_t Z = 0;
   bool half = false;
 };
-
-c10::intrusive_ptr<Extra> extra_of(AutogradContext *ctx) {
-  return c10::static_intrusive_pointer_cast<Extra>(ctx->saved_data.at("x").toCapsule());
-}
-void keep(AutogradContext *ctx, const c10::intrusive_ptr<Extra> &x) {
-  ctx->saved_data["x"] = c10::IValue::make_capsule(x);
-}
 
 // ---- one-stage operator, dense and ragged ----------------------------------------------------------
 // Result tensors of the forward: out and, when asked for, the depth scores.
@@ -71,8 +64,7 @@ struct FusedFn : torch::autograd::Function<FusedFn> {
     const Tensor q_off = offsets.value_or(Tensor());
     auto out = fused_forward(x->p, value, dist, shapes, lsi, loc, attn, q_off, need_score);
     if (x->half) narrow_two(out[0], at::kHalf, out[1], at::kHalf);
-    ctx->save_for_backward({value, dist, shapes, lsi, loc, attn, q_off});
-    keep(ctx, x);
+    keep(ctx, x, {value, dist, shapes, lsi, loc, attn, q_off});
     if (!need_score) out.pop_back();
     return out;
   }
@@ -80,9 +72,9 @@ struct FusedFn : torch::autograd::Function<FusedFn> {
     variable_list none(9);
     if (grads.size() > 1) refuse_score_gradient(grads[1]);
     if (!grads[0].defined()) return none;
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Extra>(ctx, v);
     const Tensor &value = v[0], &dist = v[1], &loc = v[4], &attn = v[5], &q_off = v[6];
-    const auto x = extra_of(ctx);
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
     Tensor gv = empty_f32(value.sizes(), value), gd = empty_f32(dist.sizes(), dist);
@@ -128,14 +120,13 @@ struct Attn3dFn : torch::autograd::Function<Attn3dFn> {
                         c10::intrusive_ptr<Extra> x) {
     const Tensor q_off = offsets.value_or(Tensor());
     Tensor out = attn3d_forward(*x, value, dist, shapes, lsi, ref, uv, od, logits, q_off);
-    ctx->save_for_backward({value, dist, shapes, lsi, ref, uv, od, logits, q_off});
-    keep(ctx, x);
+    keep(ctx, x, {value, dist, shapes, lsi, ref, uv, od, logits, q_off});
     return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Extra>(ctx, v);
     const Tensor &value = v[0], &dist = v[1], &uv = v[5], &od = v[6], &logits = v[7], &q_off = v[8];
-    const auto x = extra_of(ctx);
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
     Tensor gv = empty_f32(value.sizes(), value), gd = empty_f32(dist.sizes(), dist);
@@ -173,14 +164,13 @@ struct Attn3dJointFn : torch::autograd::Function<Attn3dJointFn> {
                         const Tensor &lsi, const Tensor &ref, const Tensor &joint, const std::optional<Tensor> &offsets,
                         c10::intrusive_ptr<Extra> x) {
     const Tensor q_off = offsets.value_or(Tensor());
-    ctx->save_for_backward({value, dist, shapes, lsi, ref, joint, q_off});
-    keep(ctx, x);
+    keep(ctx, x, {value, dist, shapes, lsi, ref, joint, q_off});
     return attn3d_joint_forward(*x, value, dist, shapes, lsi, ref, joint, q_off, Tensor());
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Extra>(ctx, v);
     const Tensor &value = v[0], &dist = v[1], &joint = v[5], &q_off = v[6];
-    const auto x = extra_of(ctx);
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
     Tensor gv = empty_f32(value.sizes(), value), gd = empty_f32(dist.sizes(), dist), gj = at::empty_like(joint);
@@ -219,14 +209,13 @@ struct Attn2dFn : torch::autograd::Function<Attn2dFn> {
     const Tensor score = scores.value_or(Tensor());
     Tensor out = attn2d_forward(x->p, value, shapes, lsi, loc, attn, score);
     if (x->half) out = out.to(at::kHalf);
-    ctx->save_for_backward({value, shapes, lsi, loc, attn, score});
-    keep(ctx, x);
+    keep(ctx, x, {value, shapes, lsi, loc, attn, score});
     return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Extra>(ctx, v);
     const Tensor &value = v[0], &loc = v[3], &attn = v[4], &score = v[5];
-    const auto x = extra_of(ctx);
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
     Tensor gv = empty_f32(value.sizes(), value), gl = at::empty_like(loc), ga = at::empty_like(attn), gs;
@@ -263,14 +252,13 @@ struct DepthScoreFn : torch::autograd::Function<DepthScoreFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &dist, const Tensor &shapes, const Tensor &lsi,
                         const Tensor &loc, c10::intrusive_ptr<Extra> x) {
     Tensor out = depth_score_forward(x->p, dist, shapes, lsi, loc);
-    ctx->save_for_backward({dist, shapes, lsi, loc});
-    keep(ctx, x);
+    keep(ctx, x, {dist, shapes, lsi, loc});
     return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Extra>(ctx, v);
     const Tensor &dist = v[0], &loc = v[3];
-    const auto x = extra_of(ctx);
     c10::cuda::CUDAGuard guard(dist.device());
     const Tensor go = f32(grads[0]);
     Tensor gd = empty_f32(dist.sizes(), dist), gl = at::empty_like(loc);
@@ -284,7 +272,7 @@ struct DepthScoreFn : torch::autograd::Function<DepthScoreFn> {
 };
 
 // ---- depth distribution from logits -------------------------------------------------------------------
-struct DistArgs : torch::CustomClassHolder {
+struct DistArgs : Kept {
   int32_t N = 0, act = 0, dtype = 0;
 };
 
@@ -304,14 +292,13 @@ struct DistFn : torch::autograd::Function<DistFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &logits, const Tensor &shapes, const Tensor &lsi,
                         c10::intrusive_ptr<DistArgs> a, int64_t type) {
     Tensor dist = dist_forward(*a, logits, shapes, lsi, static_cast<at::ScalarType>(type));
-    ctx->save_for_backward({logits, shapes, lsi});
-    ctx->saved_data["x"] = c10::IValue::make_capsule(a);
+    keep(ctx, a, {logits, shapes, lsi});
     return dist;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto a = kept<DistArgs>(ctx, v);
     const Tensor &logits = v[0];
-    const auto a = c10::static_intrusive_pointer_cast<DistArgs>(ctx->saved_data.at("x").toCapsule());
     c10::cuda::CUDAGuard guard(logits.device());
     const Tensor go = storage_type(grads[0].scalar_type()) ? grads[0].contiguous() : f32(grads[0]);
     Tensor gl = at::empty_like(logits);

@@ -208,6 +208,43 @@ inline void narrow_two(Tensor &a, at::ScalarType ta, Tensor &b, at::ScalarType t
   if (nb) b = rb;
 }
 
+// What a node keeps from its forward: the tensors, which pass through the saved-tensor hooks in force, and beside them what
+// they were.  The kernels read them by address, so what a hook hands back has to be of the same type, size and device; its
+// layout may be another.
+struct Kept : torch::CustomClassHolder {
+  struct Was {
+    int64_t numel;
+    at::ScalarType type;
+    c10::Device device;
+  };
+  c10::SmallVector<Was, 9> was;
+};
+
+template <typename X>
+void keep(AutogradContext *ctx, const c10::intrusive_ptr<X> &x, variable_list tensors) {
+  for (const Tensor &t : tensors) {
+    if (t.defined()) x->was.push_back({t.numel(), t.scalar_type(), t.device()});
+    else x->was.push_back({-1, at::kFloat, at::kCPU});
+  }
+  ctx->save_for_backward(std::move(tensors));
+  ctx->saved_data["x"] = c10::IValue::make_capsule(x);
+}
+
+template <typename X>
+c10::intrusive_ptr<X> kept(AutogradContext *ctx, variable_list &tensors) {
+  const auto x = c10::static_intrusive_pointer_cast<X>(ctx->saved_data.at("x").toCapsule());
+  tensors = ctx->get_saved_variables();
+  TORCH_CHECK(tensors.size() == x->was.size(), "saved tensors are missing");
+  for (size_t i = 0; i < tensors.size(); ++i) {
+    Tensor &t = tensors[i];
+    const Kept::Was &w = x->was[i];
+    TORCH_CHECK(t.defined() ? t.numel() == w.numel && t.scalar_type() == w.type && t.device() == w.device : w.numel < 0,
+                "a saved-tensor hook returned a tensor of another type, size or device than it was given");
+    if (t.defined()) t = t.contiguous();
+  }
+  return x;
+}
+
 // Gradients of a backward that must not be differentiated again: with create_graph the results get a node that
 // says so when it is reached (torch.autograd.function.once_differentiable does the same).
 inline variable_list once(variable_list out, const variable_list &grads) {

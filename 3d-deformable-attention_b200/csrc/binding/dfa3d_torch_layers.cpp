@@ -58,18 +58,17 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &w, const Tensor &b, bool relu) {
     c10::cuda::CUDAGuard guard(x.device());
     Tensor y = linear_forward(x, w, b, relu);
-    ctx->saved_data["relu"] = relu;
-    if (relu) ctx->save_for_backward({x, w, y});
-    else ctx->save_for_backward({x, w});
+    keep(ctx, c10::make_intrusive<Kept>(), {x, w, relu ? y : Tensor()});
     return y;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const NoAutocast no_autocast(c10::autocast_dispatch_keyset);
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    kept<Kept>(ctx, v);
     const Tensor &x = v[0], &w = v[1];
     c10::cuda::CUDAGuard guard(x.device());
     Tensor g = rows_of(f32(grads[0])), gx, gw, gb;
-    const bool relu = ctx->saved_data["relu"].toBool();
+    const bool relu = v[2].defined();
     if (relu) {
       void *s = stream_of(g);
       if (!aligned(g, 16)) g = g.clone();
@@ -111,13 +110,14 @@ struct JointLinearFn : torch::autograd::Function<JointLinearFn> {
       wd += counts[i]; bd += counts[n + i];
     }
     check(lib.dfa3d_copy_segments(src, dst, counts, 2 * n, stream_of(x)), "dfa3d_copy_segments");
-    ctx->save_for_backward({x, W});
+    keep(ctx, c10::make_intrusive<Kept>(), {x, W});
     ctx->saved_data["split"] = split;
     return linear_forward(x, W, B, false);
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const NoAutocast no_autocast(c10::autocast_dispatch_keyset);
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    kept<Kept>(ctx, v);
     const Tensor &x = v[0], &W = v[1];
     c10::cuda::CUDAGuard guard(x.device());
     const Tensor g = rows_of(f32(grads[0]));
@@ -192,12 +192,13 @@ struct AddLayerNormFn : torch::autograd::Function<AddLayerNormFn> {
     check(lib.dfa3d_add_layer_norm_forward(fp(x), res ? fp(*res) : nullptr, fp(w), fp(b), rows, (int32_t)E, (float)eps,
                                            res ? fpm(sum) : nullptr, fpm(y), mean, rstd, stream_of(x)),
           "dfa3d_add_layer_norm_forward");
-    ctx->save_for_backward({res ? sum : x, w, stats});
+    keep(ctx, c10::make_intrusive<Kept>(), {res ? sum : x, w, stats});
     ctx->saved_data["res"] = res.has_value();
     return y;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    kept<Kept>(ctx, v);
     const Tensor &in = v[0], &w = v[1], &stats = v[2];
     c10::cuda::CUDAGuard guard(in.device());
     const int64_t E = in.size(-1), rows = in.numel() / E;
@@ -373,7 +374,7 @@ PyObject *run_gather_per_camera(PyObject *const *a, Py_ssize_t n) {
 // ------------------------------------------------------------------------------------------------
 // 2-D attention from offsets and logits side by side in one row per query
 // ------------------------------------------------------------------------------------------------
-struct Attn2dExtra : torch::CustomClassHolder {
+struct Attn2dExtra : Kept {
   dfa3d_problem p;
   int32_t maps = 1;
 };
@@ -393,14 +394,13 @@ Tensor attn2d_forward(const Attn2dExtra &x, const Tensor &value, const Tensor &s
 struct Attn2dFn : torch::autograd::Function<Attn2dFn> {
   static Tensor forward(AutogradContext *ctx, const Tensor &value, const Tensor &shapes, const Tensor &lsi,
                         const Tensor &ref, const Tensor &joint, c10::intrusive_ptr<Attn2dExtra> x) {
-    ctx->save_for_backward({value, shapes, lsi, ref, joint});
-    ctx->saved_data["x"] = c10::IValue::make_capsule(x);
+    keep(ctx, x, {value, shapes, lsi, ref, joint});
     return attn2d_forward(*x, value, shapes, lsi, ref, joint);
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
-    const auto v = ctx->get_saved_variables();
+    variable_list v;
+    const auto x = kept<Attn2dExtra>(ctx, v);
     const Tensor &value = v[0], &joint = v[4];
-    const auto x = c10::static_intrusive_pointer_cast<Attn2dExtra>(ctx->saved_data.at("x").toCapsule());
     c10::cuda::CUDAGuard guard(value.device());
     const Tensor go = f32(grads[0]);
     Tensor gv = at::empty_like(value), gj = at::empty_like(joint);
