@@ -275,7 +275,7 @@ class SpatialCrossAttention_DFA3D(nn.Module):
             query = query + query_pos
         bs, Q, E = query.shape
         cams = self.num_cams
-        plan = rebatch_plan if rebatch_plan is not None else RebatchPlan(bev_mask)
+        plan = rebatch_plan if rebatch_plan is not None else RebatchPlan(bev_mask, wait=False)
         if (plan.cams, plan.bs, plan.Q) != (cams, bs, Q):
             raise RuntimeError("rebatch_plan does not belong to this bev_mask / query")
         N = value.shape[1]
@@ -591,7 +591,7 @@ class BEVFormerEncoderLayer(nn.Module):
         shifted for the previous BEV by the caller); cross_kw: the spatial cross-attention's inputs."""
         if cross_kw.get("rebatch_plan") is None and type(self.cross_attn) is SpatialCrossAttention_DFA3D:
             # started before the self-attention, whose work hides its read-back
-            cross_kw["rebatch_plan"] = RebatchPlan(cross_kw["bev_mask"])
+            cross_kw["rebatch_plan"] = RebatchPlan(cross_kw["bev_mask"], wait=False)
         shapes, lsi, cells = self._bev_tables(query.device, query.dtype)
         if ref_2d is None:
             ref_2d = cells.expand(query.shape[0] * 2, -1, -1, -1)
@@ -608,7 +608,7 @@ class SCAEncoderStack(nn.Module):
 
     def forward(self, query, **kw):
         if kw.get("rebatch_plan") is None:          # bev_mask is the same for every layer: one plan
-            kw = dict(kw, rebatch_plan=RebatchPlan(kw["bev_mask"]))
+            kw = dict(kw, rebatch_plan=RebatchPlan(kw["bev_mask"], wait=False))
         for layer in self.layers:
             query = layer(query, **kw)
         return query

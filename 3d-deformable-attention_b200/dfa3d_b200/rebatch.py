@@ -10,9 +10,10 @@ tensors built by one call (``dfa3d_rebatch_plan``), the rows are PACKED (exactly
 per-camera row offsets so that cameras of different length share one launch.
 
 A plan depends only on ``bev_mask``, which is geometry: build it once per frame and hand it to every
-encoder layer.  The packed row count, needed to size tensors, is read back from the device: the copy is queued with
-the plan's kernels, and whoever first asks for ``rows`` waits for it -- so work that does not need the count should be
-queued in between.  Nothing after that synchronises.
+encoder layer.  The packed row count, needed to size tensors, is read back from the device, which is what the
+constructor waits for.  Nothing after that synchronises.  With ``wait=False``, for a plan that is used up by the code
+that makes it, the copy is only queued with the plan's kernels and whoever first asks for ``rows`` waits for it, so that
+work that does not need the count can be queued in between.
 """
 import torch
 from torch.autograd.function import Function, once_differentiable
@@ -30,9 +31,13 @@ class RebatchPlan:
     counts (cams), offsets (cams+1), op_offsets (bs*cams+1) int32; packed_query / packed_camera (T)
     int32; row_of (cams, Q) int32 (-1 = not seen); inv_count (bs, Q) float32; ``rows`` = T = packed rows
     of one batch element, ``max_queries`` = longest camera list (both Python ints).
+
+    A plan is complete once constructed: any stream or thread may use it, also while a CUDA graph is captured, and it
+    can be copied and pickled.  With ``wait=False`` only after ``rows`` was asked for; until then its tables belong to
+    the stream that was current.
     """
 
-    def __init__(self, bev_mask):
+    def __init__(self, bev_mask, wait=True):
         if bev_mask.dim() != 4:
             raise RuntimeError("bev_mask must be (num_cams, bs, Q, Z)")
         if not bev_mask.is_cuda:
@@ -62,14 +67,18 @@ class RebatchPlan:
         self._counted = torch.cuda.Event()
         self._counted.record(torch.cuda.current_stream(dev))
         self._sizes = None
+        if wait:
+            self._resolve()
 
     def _resolve(self):
         if self._sizes is None:
             self._counted.synchronize()
             counts = self._host_counts.tolist()
-            self._sizes = (int(sum(counts)), int(max(counts)) if counts else 0)
+            rows = int(sum(counts))
             self._native_args = (self._pq, self._pc, self.offsets, self.row_of, self.inv_count, self.cams, self.bs, self.Q,
-                                 self._sizes[0])
+                                 rows)
+            self._sizes = (rows, int(max(counts)) if counts else 0)
+            self._counted = self._host_counts = None
         return self._sizes
 
     @property
