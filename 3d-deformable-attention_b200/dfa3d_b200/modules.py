@@ -311,10 +311,11 @@ class SpatialCrossAttention_DFA3D(nn.Module):
 def _attention_2d(value, query, module, reference_points, spatial_shapes, level_start_index, maps):
     """The 2-D operator of `module` (its sampling_offsets, attention_weights, num_heads, num_points) with its callers'
     softmax, location assembly and mean over the maps inside the kernels, or None where the separate steps have to do it
-    (box reference points, sizes the kernels do not have)."""
+    (box reference points, sizes the kernels do not have) or to refuse it (a batch that im2col_step does not divide)."""
     fused = getattr(MultiScaleDeformableAttnFunction_fp32, "from_offsets", None)
-    points = maps * module.num_levels * module.num_points
-    if fused is None or reference_points.shape[-1] != 2 or points not in (4, 8, 16):
+    points, batch, step = maps * module.num_levels * module.num_points, value.shape[0], module.im2col_step
+    if fused is None or reference_points.shape[-1] != 2 or points not in (4, 8, 16) \
+            or batch > 0 and (step <= 0 or batch % min(batch, step) != 0):
         return None
     joint = joint_linear(query, module.sampling_offsets, module.attention_weights)
     if joint is None:

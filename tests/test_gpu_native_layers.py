@@ -15,6 +15,7 @@ DEV = "cuda"
 
 def _close(got, want, rtol=2e-4):
     for a, b in zip(got, want):
+        a, b = a.detach(), b.detach()
         assert a.shape == b.shape
         scale = float(b.abs().max()) + 1e-30
         assert float((a - b).abs().max()) <= rtol * scale
@@ -100,3 +101,17 @@ def test_attention_2d_from_offsets_leaves_other_sizes_alone(lib_built):
         out = fused(torch.zeros(1, 16, C, device=DEV), shapes, lsi, torch.zeros(1, 5, 1, 2, device=DEV),
                     torch.zeros(1, 5, P * 3, device=DEV), 1, 1, P)
         assert out is NotImplemented
+
+
+@pytest.mark.parametrize("bs,step,accepted", [(3, 4, False), (3, 2, True), (3, 64, True), (2, 3, False), (1, 0, False)])
+def test_attention_2d_refuses_a_batch_that_im2col_step_does_not_divide(lib_built, bs, step, accepted):
+    """The step has no use here but the reference's check on it; the joint form makes it like the separate one."""
+    att = modules.TemporalSelfAttention(64, 4, 1, 4, im2col_step=step, dropout=0.0).to(DEV)
+    query, value = torch.randn(bs, 12, 64, device=DEV), torch.randn(2 * bs, 12, 64, device=DEV)
+    kw = dict(value=value, reference_points=torch.rand(2 * bs, 12, 1, 2, device=DEV),
+              spatial_shapes=torch.tensor([[3, 4]], device=DEV), level_start_index=torch.zeros(1, dtype=torch.int64, device=DEV))
+    if accepted:
+        assert att(query, **kw).shape == query.shape
+    else:
+        with pytest.raises(RuntimeError, match="must divide im2col_step"):
+            att(query, **kw)
