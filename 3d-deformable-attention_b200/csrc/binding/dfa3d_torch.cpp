@@ -653,7 +653,8 @@ PyMODINIT_FUNC PyInit__native(void) {
   PyObject *m = PyModule_Create(&module);
   // the headers this was compiled against: another torch may lay its classes out differently
   if (m && (PyModule_AddFunctions(m, dfa3d_torch::layer_methods) != 0 ||
-            PyModule_AddStringConstant(m, "built_for", DFA3D_BUILT_FOR) != 0)) {
+            PyModule_AddStringConstant(m, "built_for", DFA3D_BUILT_FOR) != 0 ||
+            PyModule_AddIntConstant(m, "split_rows", kSplitRows) != 0 || PyModule_AddIntConstant(m, "splits", kSplits) != 0)) {
     Py_DECREF(m);
     return nullptr;
   }

@@ -282,6 +282,10 @@ inline std::optional<Tensor> given(const Tensor &t) { return t.defined() ? std::
 
 inline PyObject *not_plain() { Py_RETURN_NOTIMPLEMENTED; }
 
+// A weight gradient of at least so many rows is formed as so many slices of them (dfa3d_torch_layers.cpp; the Python
+// Function does the same, layer_ops.py)
+constexpr int64_t kSplitRows = 16384, kSplits = 16;
+
 extern PyMethodDef layer_methods[];      // dfa3d_torch_layers.cpp, ends in a null entry
 
 }  // namespace dfa3d_torch

@@ -12,8 +12,6 @@ namespace {
 // ------------------------------------------------------------------------------------------------
 Tensor rows_of(const Tensor &t) { return t.view({-1, t.size(-1)}); }
 
-constexpr int64_t kSplitRows = 16384, kSplits = 16;
-
 // Weight gradient g^T x of g (rows, out) and x (rows, in), and bias gradient: the column sums of g.  Many rows into a small
 // product is one long reduction that cuBLAS gives to few CTAs; as a batch of 16 row slices, summed by a kernel of our own
 // that also takes the rows left over and zeroes the bias gradient, it takes a third of the time.
