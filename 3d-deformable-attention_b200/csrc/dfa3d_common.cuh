@@ -148,9 +148,6 @@ struct ItemCtx {
   long long pt0;            // index of the item's first point: item * LP
 };
 
-// blockIdx.y (+ b0) selects the camera; the CTA's `group`-th group of kWarpsPerCta items starts at
-// (blockIdx.x * groups_per_cta + group) * kWarpsPerCta, warp w takes item w of it: a (query, head)
-// pair of that camera.  Returns false for the warps past the end of the camera.
 // Where the item's locations and weights start (a query's rows may lie apart in the caller-fused modes).
 template <int MODE>
 __device__ __forceinline__ void item_inputs(const KArgs &a, ItemCtx &c) {
@@ -166,6 +163,9 @@ __device__ __forceinline__ void item_inputs(const KArgs &a, ItemCtx &c) {
   }
 }
 
+// blockIdx.y (+ b0) selects the camera; the CTA's `group`-th group of kWarpsPerCta items starts at
+// (blockIdx.x * groups_per_cta + group) * kWarpsPerCta, warp w takes item w of it: a (query, head)
+// pair of that camera.  Returns false for the warps past the end of the camera.
 template <int MODE, bool HEAD_MAJOR = false>
 __device__ __forceinline__ bool item_context(const KArgs &a, int warp, unsigned group, ItemCtx &c) {
   const unsigned idx = group * kWarpsPerCta + warp;
@@ -307,9 +307,6 @@ struct PointGeo {
   bool ok2, ok3;
 };
 
-// `has_z`: the location carries a depth coordinate (3-D range test applies to ok3).
-// Corner pixels are additionally bounded by N so that inconsistent shape tables cannot make the
-// kernels touch memory outside the tensors (such corners are treated as outside the image).
 // Row of the dist map that pixel (y, x) of a level reads: nearest-neighbour resize,
 // src = min(floor(dst * scale), size - 1) with scale = (float)map size / (float)level size.
 __device__ __forceinline__ int map_row(int y, int x, float sy, float sx, int mh, int mw) {
@@ -326,6 +323,9 @@ __device__ __forceinline__ DistMap dist_map_of(const KArgs &a, const LevelTable 
   return DistMap{a.dmap_h, a.dmap_w, lv.map_sy[l], lv.map_sx[l]};
 }
 
+// `has_z`: the location carries a depth coordinate (3-D range test applies to ok3).
+// Corner pixels are additionally bounded by N so that inconsistent shape tables cannot make the
+// kernels touch memory outside the tensors (such corners are treated as outside the image).
 __device__ __forceinline__ PointGeo point_geometry(float x, float y, float z, bool has_z, int Hh,
                                                    int W, int Dd, int start, int N,
                                                    const DistMap dm = DistMap{0, 0, 1.f, 1.f}) {

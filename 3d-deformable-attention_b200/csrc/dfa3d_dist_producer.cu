@@ -197,8 +197,11 @@ __device__ __forceinline__ void normalised_bins(const float *tile, int stride, c
 }
 
 // Forward: a CTA owns kTile map pixels, normalises each once and writes the rows of every level pixel that reads one
-// of them, from registers.  Bound by the writes of dist.  (A CTA per 32 output rows, which normalised every level
-// pixel anew, took 53 us at 6 x 58 x 100 x 64 -> 30 825 rows; about 9 us of that is HBM time.)
+// of them, from registers.  (A CTA per 32 output rows, which normalised every level pixel anew, took 53 us at
+// 6 x 58 x 100 x 64 -> 30 825 rows; this takes 16.5 with the operands in L2, 18.6 cold.)  Bound by instructions and the
+// tail, not by memory: issue slots 63 % busy, DRAM 6 % (dist stays in L2), stores 27 % of the path to L2; six CTAs are
+// resident on an SM (registers), so that 1392 are 1.57 waves, and the CTA of a map row's last 4 columns takes as long as
+// a full one: widths 96, 100, 128 14.5, 16.5, 16.5 us, widths 33 and 64 both 10.4.
 template <typename OT, int V, int NC>
 __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];
@@ -228,8 +231,10 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const Pr
 
 // Backward: the same ownership.  A pixel's eight lanes sum the incoming gradient over the level pixels that read it, in
 // the order of the levels, rows and columns, and form p * (G - <p, G>) (softmax) or p * (1 - p) * G (sigmoid), stored
-// along x through shared memory.  Bound by the reads of grad_dist.  (A warp per map pixel, one level pixel after the
-// other: 87 us at the shape above; this takes 26, about 10 of them HBM time.)
+// along x through shared memory.  (A warp per map pixel, one level pixel after the other: 87 us at the shape above; this
+// takes 18.9 with the operands in L2, 25.5 cold.)  Bound by the latency of the gradient's rows (a third of the stalls, the
+// barrier behind them another fifth), issue slots (53 % busy) and the same tail; DRAM 27 %.  Widths 96, 100, 128 take 16.8,
+// 18.9, 20.6 us, widths 33 and 64 both 12.4.
 template <typename GT, int V, int NC>
 __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];

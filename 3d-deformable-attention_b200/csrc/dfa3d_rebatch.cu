@@ -53,7 +53,7 @@ __device__ __forceinline__ int block_exclusive_count(bool flag, int &total, int 
 // A camera's queries are shared out over a cluster of CTAs in consecutive ranges; a CTA goes over its range 1024 queries
 // at a time.  The CTAs' counts meet in distributed shared memory.  (One CTA per camera, two barriers and a scan for every
 // 1024 queries, took 46 + 56 us for 6 x 40 000 queries; a thread per consecutive chunk, without them, 10 + 47: its stores
-// do not coalesce.)
+// do not coalesce.  Both kernels like this: 18.6 us back to back, 7.8 + 15.0 cold.)
 constexpr int kCluster = 8;
 
 // Queries of this CTA's range that the camera sees.

@@ -3,11 +3,10 @@
 ``libdfa3d_rates.so`` (csrc/rates/dfa3d_rates.cu) replays the address stream of one operator launch --
 the four 128-byte corner rows per sampling point in ``value`` / ``grad_value`` and the (z0, z0+1) pairs
 of the four corner pixels in ``dist`` / ``grad_dist`` -- with pseudo-random uniform positions and none of
-the arithmetic.  Timing each primitive alone and the ones a kernel needs together gives a lower bound
-for that kernel that does not depend on how its arithmetic is written:
-
-  forward  >= time(GATHER_ROWS + dist gathers)
-  backward >= time(GATHER_ROWS + dist gathers + RED_ROWS + dist reductions)
+the arithmetic.  The reductions alone (RED_ROWS + dist reductions) are a lower bound of the backward: they are
+done in L2, whoever issues them.  The streams of gathers are not bounds, only measures of comparison: the probe
+overlaps its accesses in its own way, and the forward kernel (0.54 ms at the BEVFormer-base shape) runs faster
+than GATHER_ROWS + dist gathers replayed (0.77 ms).
 
     python -m dfa3d_b200.rates [--workload cfg2] [--cameras 6] [--reps 20] [--json]
 
@@ -134,7 +133,8 @@ def measure(levels, P, D, Q, B, reps=20, per_level=True):
 
 
 def floors(levels, P, D, Q, B, reps=10):
-    """Lower bounds (ms) of the forward and the backward of this shape from their memory streams."""
+    """Times (ms) of the forward's and the backward's address streams of this shape, and of the backward's reductions
+    alone, which are its lower bound."""
     pb = Prober(levels, P, D, Q, B, cells=False)
     return {"forward_ms": pb.time_ms(GATHER_ROWS | GATHER_PAIRS, reps=reps),
             "backward_ms": pb.time_ms(GATHER_ROWS | GATHER_PAIRS | RED_ROWS | RED_PAIRS, reps=reps),

@@ -477,7 +477,7 @@ def main():
     ap.add_argument("--e2e-steps", type=int, default=16)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-extras", action="store_true",
-                    help="skip the side measurements (cfg3, Function-level step, memory-stream floor)")
+                    help="skip the side measurements (cfg3, Function-level step, memory-stream probe)")
     ap.add_argument("--scaling", choices=("weak", "strong"), default="weak",
                     help="weak: 6 cameras per GPU (default, the headline); strong: one batch, queries "
                          "split over the GPUs with an all-reduce of the value/dist gradients")
@@ -617,7 +617,7 @@ def main():
             except AssertionError as e:
                 extra["query_blocks"] = {"error": f"adjoint identity violated: {e}"}
         if rank == 0 and w.L * w.P == 32 and w.H == 8 and w.C == 32 and w.value_dtype == "fp32":
-            extra["memory_stream_floor"] = memory_stream_floor(w)
+            extra["memory_stream_probe"] = memory_stream_probe(w)
         if w.name == "cfg2":
             # the training configuration: 6-layer spatial-cross-attention encoder stack, one frame per GPU
             extra["encoder_stack"] = measure_encoder_stack(rank, world, dev, 5, 2)
@@ -732,15 +732,16 @@ def measure_few_points(dev, world, barrier):
     return out
 
 
-def memory_stream_floor(w):
-    """Lower bounds of the two kernels from the measured rates of the memory primitives they are made
-    of (dfa3d_b200.rates replays a launch's address stream without the arithmetic)."""
+def memory_stream_probe(w):
+    """The two kernels' address streams replayed without the arithmetic (dfa3d_b200.rates).  Only the reductions' time
+    is a lower bound; the probe overlaps its gathers no better than the kernels do, and the forward runs faster than it."""
     try:
         from dfa3d_b200 import rates
         f = rates.floors(w.levels, w.P, w.D, w.Q, w.B)
         f["what"] = ("probe launches with this workload's address stream: forward = value-row gathers + "
                      "dist-pair gathers; backward = the same gathers + grad_value row reductions + "
-                     "grad_dist pair reductions; reductions only = what the L2 reduction units alone need")
+                     "grad_dist pair reductions (neither is a lower bound); reductions only = what the L2 reduction "
+                     "units alone need (one)")
         return f
     except Exception as e:          # measurement aid only: never fail the bench over it
         return {"unavailable": str(e)}
@@ -769,7 +770,7 @@ def report(a, w, world, launches_per_step, value, ms_per_step, fwd_ms, bwd_ms, c
         "e2e": e2e,
     }
     if a.impl == "ours":
-        # items of 4 / 8 / 16 points (fp32, 16 / 32 / 64 channels) take the kernels in which a warp holds several
+        # items of up to 16 points (16 / 32 / 64 channels, every storage type) share a warp in kernels of their own
         packed = w.L * w.P <= 16 and w.C in (16, 32, 64)
         line["roofline"] = {
             "kernel": "dfa3d_backward_packed_kernel" if packed else "dfa3d_backward_kernel", "bound": "hbm",
@@ -783,15 +784,15 @@ def report(a, w, world, launches_per_step, value, ms_per_step, fwd_ms, bwd_ms, c
             "algorithmic_bytes": fwd_b}
         line["roofline_step"] = {"frac": (fwd_b + bwd_b) / (ms_per_step * 1e-3) / 1e9 / peak,
                                  "algorithmic_bytes": fwd_b + bwd_b}
-        floor = (extra or {}).get("memory_stream_floor") or {}
-        if "backward_ms" in floor:
+        probe = (extra or {}).get("memory_stream_probe") or {}
+        if "backward_ms" in probe:
             # floor_ms: the launch's reductions alone at the measured L2 reduction rate (nothing the
-            # kernel does can make them cheaper); stream_ms: all of its gathers and reductions replayed
-            # without arithmetic
-            line["roofline"]["floor_ms"] = floor["backward_reductions_only_ms"]
-            line["roofline"]["frac_of_floor"] = floor["backward_reductions_only_ms"] / bwd_ms
-            line["roofline"]["stream_ms"] = floor["backward_ms"]
-            line["roofline_forward"]["stream_ms"] = floor["forward_ms"]
+            # kernel does can make them cheaper); stream_probe_ms: all of its gathers and reductions replayed
+            # without arithmetic, for comparison
+            line["roofline"]["floor_ms"] = probe["backward_reductions_only_ms"]
+            line["roofline"]["frac_of_floor"] = probe["backward_reductions_only_ms"] / bwd_ms
+            line["roofline"]["stream_probe_ms"] = probe["backward_ms"]
+            line["roofline_forward"]["stream_probe_ms"] = probe["forward_ms"]
         if extra:
             line["extra"] = extra
         if world == 1 and not a.no_cpu_baseline:
