@@ -240,8 +240,8 @@ column_sum_kernel(const float *__restrict__ src, long long rows, int cols, float
   }
 }
 
-// Backward of relu(x W^T + b) up to the products: grad_in = y > 0 ? grad_y : 0 and its column sums (the bias gradient)
-// in one pass over both operands.  Split and accumulation as in column_sum_kernel.
+// Backward of relu(x W^T + b) up to the products: grad_in = y <= 0 ? 0 : grad_y (a NaN lets its gradient pass, as in
+// torch) and its column sums (the bias gradient) in one pass over both operands.  Split and accumulation as in column_sum_kernel.
 __global__ void __launch_bounds__(kCsThreads)
 relu_backward_kernel(const float *grad_y, const float *__restrict__ y, long long rows, int cols,
                      float *grad_in, float *__restrict__ dst) {
@@ -263,8 +263,8 @@ relu_backward_kernel(const float *grad_y, const float *__restrict__ y, long long
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (r + u * step < rows) {
-          const float4 t = make_float4(v[u].x > 0.f ? g[u].x : 0.f, v[u].y > 0.f ? g[u].y : 0.f,
-                                       v[u].z > 0.f ? g[u].z : 0.f, v[u].w > 0.f ? g[u].w : 0.f);
+          const float4 t = make_float4(v[u].x <= 0.f ? 0.f : g[u].x, v[u].y <= 0.f ? 0.f : g[u].y,
+                                       v[u].z <= 0.f ? 0.f : g[u].z, v[u].w <= 0.f ? 0.f : g[u].w);
           st4(grad_in + (r + u * step) * cols + col, t);
           acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
         }

@@ -373,7 +373,7 @@ int dfa3d_column_sum(const float *src, int64_t rows, int32_t cols, float *dst, v
 int dfa3d_add_layer_norm_infer(const float *x, const float *residual, const float *gamma, const float *beta,
                                int64_t rows, int32_t E, float eps, float *y, void *stream);
 
-/* grad_in = y > 0 ? grad_y : 0 and dst[c] += sum over rows of grad_in[r, c]: the backward of a Linear layer followed by
+/* grad_in = y <= 0 ? 0 : grad_y and dst[c] += sum over rows of grad_in[r, c]: the backward of a Linear layer followed by
  * a ReLU up to the matrix products.  Conditions of dfa3d_column_sum; grad_in may be grad_y. */
 int dfa3d_relu_backward_column_sum(const float *grad_y, const float *y, int64_t rows, int32_t cols, float *grad_in,
                                    float *dst, void *stream);
