@@ -96,6 +96,15 @@ dfa3d::KArgs base_args(const dfa3d_problem *p, int shape_stride, int loc_stride)
   return a;
 }
 
+// Rows of offsets and logits hold a query's values of all `maps` maps, with or without something between them.
+int check_row_strides(const dfa3d_problem *p, int maps, int64_t offsets_row, int64_t logits_row) {
+  const int64_t values = (int64_t)p->H * p->L * p->P * maps;
+  if ((offsets_row != 0 && offsets_row < 2 * values) || (logits_row != 0 && logits_row < values))
+    return fail(DFA3D_ERR_INVALID_ARGUMENT, "offsets_row and logits_row must be 0 or hold a query's %lld and %lld values (got "
+                "%lld, %lld)", (long long)(2 * values), (long long)values, (long long)offsets_row, (long long)logits_row);
+  return DFA3D_OK;
+}
+
 // Elements from query to query of the offsets and of the logits (and depth offsets); 0: they are contiguous.
 void set_rows(dfa3d::KArgs &a, int64_t offsets_row, int64_t logits_row) {
   a.row_loc = offsets_row ? offsets_row : (int64_t)a.H * a.LP * 2;
@@ -303,6 +312,7 @@ static int attn3d_forward_impl(const dfa3d_problem *p, int32_t num_anchors, int3
                 num_anchors, p->P);
   if (shape_stride != 2 && shape_stride != 3)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "shape_stride must be 2 or 3 (got %d)", shape_stride);
+  if (int rc = check_row_strides(p, 1, offsets_row, logits_row)) return rc;
   if (query_rows && !query_offsets)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "query_rows goes with query_offsets");
   if (p->B == 0 || p->Q == 0) return DFA3D_OK;
@@ -355,6 +365,7 @@ static int attn3d_backward_impl(const dfa3d_problem *p, int32_t num_anchors, int
                 num_anchors, p->P);
   if (shape_stride != 2 && shape_stride != 3)
     return fail(DFA3D_ERR_INVALID_ARGUMENT, "shape_stride must be 2 or 3 (got %d)", shape_stride);
+  if (int rc = check_row_strides(p, 1, offsets_row, logits_row)) return rc;
   if (p->B == 0 || p->Q == 0) return DFA3D_OK;
   REQUIRE_PTR(value); REQUIRE_PTR(dist); REQUIRE_PTR(shapes3); REQUIRE_PTR(level_start);
   REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets_uv); REQUIRE_PTR(offsets_depth); REQUIRE_PTR(logits);
@@ -434,6 +445,7 @@ static int attn2d_args(const dfa3d_problem *p, int32_t num_maps, int64_t offsets
   if (!dfa3d_attn2d_supported(p, num_maps))
     return fail(DFA3D_ERR_UNSUPPORTED, "2-D attention from offsets: fp32 value, C of 16, 32 or 64, 4, 8 or 16 points per "
                 "item in maps of a power of two (got C=%d, L*P=%d, maps=%d)", p->C, p->L * p->P, num_maps);
+  if (int rc = check_row_strides(p, num_maps, offsets_row, logits_row)) return rc;
   REQUIRE_PTR(value); REQUIRE_PTR(shapes2); REQUIRE_PTR(level_start); REQUIRE_PTR(ref_points); REQUIRE_PTR(offsets);
   REQUIRE_PTR(logits);
   REQUIRE_ALIGNED(value);
