@@ -6,8 +6,8 @@ fused forward / backward.  All of them validate their tensors like the reference
 (contiguous, CUDA, ``batch % min(batch, im2col_step) == 0`` -- DFA3D/dfa3D/ops/csrc/cuda/
 wms_deform_attn_cuda.cu:220-253) and then call the C ABI on the current CUDA stream.
 
-Narrowing with respect to the reference: tensors are float32 (the reference also instantiates
-float64), plus bfloat16 storage for ``value`` / ``dist`` which the reference lacks.
+Tensors are float32 or, all of a call's floating-point ones together, float64, as in the reference; added is
+bfloat16 and float16 storage of ``value`` / ``dist``.
 """
 import torch
 
