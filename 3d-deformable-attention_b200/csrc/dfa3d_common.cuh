@@ -478,7 +478,9 @@ template <> struct RowVec<__nv_bfloat16> {
   // Forward: 8 elements (16 bytes) per lane -- half the requests and row-table reads per point.
   static constexpr int kElems = 8;
   __device__ static __forceinline__ void load(const __nv_bfloat16 *p, float (&v)[8]) {
-    const uint4 t = __ldg(reinterpret_cast<const uint4 *>(p));
+    widen(__ldg(reinterpret_cast<const uint4 *>(p)), v);
+  }
+  __device__ static __forceinline__ void widen(uint4 t, float (&v)[8]) {
     const uint32_t u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {           // bf16 -> fp32 is a 16-bit shift
@@ -491,7 +493,9 @@ template <> struct RowVec<__nv_bfloat16> {
 template <> struct RowVec<__half> {
   static constexpr int kElems = 8;
   __device__ static __forceinline__ void load(const __half *p, float (&v)[8]) {
-    const uint4 t = __ldg(reinterpret_cast<const uint4 *>(p));
+    widen(__ldg(reinterpret_cast<const uint4 *>(p)), v);
+  }
+  __device__ static __forceinline__ void widen(uint4 t, float (&v)[8]) {
     const uint32_t u[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {

@@ -10,7 +10,7 @@
 //                16-byte loads (4 fp32 or 8 bf16 channels per lane), so one warp-wide request fetches
 //                32/G rows, and every lane
 //                accumulates weight * row fragment;
-//   epilogue  -- the 32/G partial sums are folded with xor-shuffles and G lanes store the output row.
+//   epilogue  -- the 32/G partial sums are folded with xor-shuffles and the output row is stored.
 // This replaces the reference's pair of kernels (one thread per (b,q,h) for the depth scores,
 // ms_depth_score_sample_cuda_kernel.cuh:94-148; one thread per output channel for the attention,
 // wms_deform_attn_cuda_kernel.cuh:240-303) and the depth_score round trip through HBM between them.
@@ -77,7 +77,36 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] = fmaf(e[u].wgt, v[u][i], acc[i]);
     };
-    if (FULL) {          // compile-time trip count, table offsets become immediates
+    if constexpr (FULL && V == 8) {
+      // 16-bit rows stay packed until they are summed, so that a lane's next row can be asked for as soon as the last one in
+      // its place is used up: bf16, 6 cameras of the base levels, uniform locations 504 -> 491 us, fp16 with depth scores
+      // 288 -> 275 (fp32 rows, which take as many registers packed or not: no gain)
+      RowEntry e[U], next[U];
+      uint4 v[U];
+      auto fetch = [&](int off, uint4 &r) {
+        r = make_uint4(0, 0, 0, 0);
+        if (off >= 0) r = __ldg(reinterpret_cast<const uint4 *>(vbase + off));
+      };
+      table.load(lane / G, e);
+#pragma unroll
+      for (int u = 0; u < U; ++u) fetch(e[u].off, v[u]);
+#pragma unroll
+      for (int p0 = 0; p0 < 32; p0 += R) {
+        const bool more = p0 + R < 32;
+        if (more) table.load(p0 + R + lane / G, next);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float t[V];
+          RowVec<VT>::widen(v[u], t);
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[i] = fmaf(e[u].wgt, t[i], acc[i]);
+          if (more) {
+            fetch(next[u].off, v[u]);
+            e[u] = next[u];
+          }
+        }
+      }
+    } else if constexpr (FULL) {          // compile-time trip count, table offsets become immediates
 #pragma unroll
       for (int p0 = 0; p0 < 32; p0 += R) step(p0, 32);
     } else {
@@ -87,16 +116,7 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
     }
     __syncwarp();
   }
-#pragma unroll
-  for (int s = G; s < 32; s <<= 1)
-#pragma unroll
-    for (int i = 0; i < V; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], s);
-  if (lane < G) {
-    float *o = a.out + (c.item * C + lane * V);
-#pragma unroll
-    for (int i = 0; i < V; i += 4)
-      *reinterpret_cast<float4 *>(o + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-  }
+  fold_and_store<V, G, R>(acc, lane, a.out + (c.item * C + lane % G * V), true);
 }
 
 // 5 CTAs (40 warps) per SM: measured best; at 6+ the register cap starts to cost more than the

@@ -112,17 +112,8 @@ dfa3d_forward_packed_kernel(const KArgs a) {
 #pragma unroll 1
         for (int p0 = 0; p0 < n; p0 += GPI) step(p0);
       }
-#pragma unroll
-      for (int s = G; s < G * GPI; s <<= 1)
-#pragma unroll
-        for (int x = 0; x < V; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], s);
       const unsigned idx = first + i;
-      if (grp % GPI == 0 && idx < nitems) {
-        float *o = a.out + ((q0 * a.H + idx) * C + sub * V);
-#pragma unroll
-        for (int x = 0; x < V; x += 4)
-          *reinterpret_cast<float4 *>(o + x) = make_float4(acc[x], acc[x + 1], acc[x + 2], acc[x + 3]);
-      }
+      fold_and_store<V, G, GPI>(acc, lane, a.out + ((q0 * a.H + idx) * C + sub * V), idx < nitems);
     }
     __syncwarp();
   }
