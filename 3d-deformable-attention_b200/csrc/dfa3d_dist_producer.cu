@@ -21,7 +21,7 @@
 namespace dfa3d {
 namespace {
 
-constexpr int kTile = 32;          // map pixels of one map row per CTA
+constexpr int kTile = 32;          // map pixels per CTA, consecutive in memory: they may run over several map rows
 constexpr int kMaxBins = 256;      // D limit of the shared-memory tile
 constexpr int kProdThreads = 256;
 constexpr int kProdLevels = DFA3D_MAX_LEVELS;
@@ -86,38 +86,52 @@ __device__ __forceinline__ int first_at(int s, float scale, int n, int size) {
   return d;
 }
 
-// Which level pixels read the CTA's map pixels (row sy, columns sx0 .. sx0 + kTile - 1): per level the rows
-// [y0, y1) and, per map pixel i, the columns [x[i], x[i+1]).
+// Which level pixels read the CTA's map pixels p0 .. p0 + kTile - 1 (row-major): per level, x[i] is the first column that
+// reads pixel i's map column, and y[r] the first row that reads the r-th map row of the tile.
 struct Footprint {
-  int4 level[kProdLevels];           // y0, y1, width, first row of dist
+  int2 level[kProdLevels];           // width, first row of dist
   int x[kProdLevels][kTile + 1];
+  int y[kProdLevels][kTile + 1];
 };
 
-__device__ __forceinline__ void stage_footprint(Footprint &f, const ProdArgs &a, int sy, int sx0) {
-  for (int t = threadIdx.x; t < a.L * (kTile + 2); t += kProdThreads) {
-    const int l = t / (kTile + 2), i = t - l * (kTile + 2);
-    const int w = (int)a.shapes[l * a.shape_stride + 1];
+__device__ __forceinline__ void stage_footprint(Footprint &f, const ProdArgs &a, int p0, int rows) {
+  const int sy0 = p0 / a.ws, each = kTile + 1 + rows + 1;
+  for (int t = threadIdx.x; t < a.L * each; t += kProdThreads) {
+    const int l = t / each, i = t - l * each;
+    const int h = (int)a.shapes[l * a.shape_stride], w = (int)a.shapes[l * a.shape_stride + 1];
     if (i <= kTile) {
-      f.x[l][i] = first_at(min(sx0 + i, a.ws), (float)a.ws / (float)w, w, a.ws);
+      f.x[l][i] = first_at((int)((unsigned)(p0 + i) % (unsigned)a.ws), (float)a.ws / (float)w, w, a.ws);
+      if (i == 0) f.level[l] = make_int2(w, (int)a.lsi[l]);
     } else {
-      const int h = (int)a.shapes[l * a.shape_stride];
-      const float scale = (float)a.hs / (float)h;
-      f.level[l] = make_int4(first_at(sy, scale, h, a.hs), first_at(sy + 1, scale, h, a.hs), w, (int)a.lsi[l]);
+      const int r = i - (kTile + 1);
+      f.y[l][r] = first_at(sy0 + r, (float)a.hs / (float)h, h, a.hs);
     }
   }
 }
 
-// Calls row(n) for every row n of dist that reads map pixel i of the CTA, levels, rows and columns in order.
-template <typename F>
-__device__ __forceinline__ void for_each_row(const Footprint &f, const ProdArgs &a, int i, F row) {
+// Calls rows(n) with the rows n[0..K) of dist that read map pixel i of the CTA, K at a time and -1 where there is none,
+// levels, rows and columns in order.
+template <int K, typename F>
+__device__ __forceinline__ void for_each_row(const Footprint &f, const ProdArgs &a, int p0, int i, F rows) {
+  const int sy = (p0 + i) / a.ws, r = sy - p0 / a.ws;
+  const bool last = p0 + i + 1 == (sy + 1) * a.ws;          // the map row's last pixel: up to the level's edge
   for (int l = 0; l < a.L; ++l) {
-    const int x0 = f.x[l][i], nx = f.x[l][i + 1] - x0;
-    const int4 v = f.level[l];
-    if (nx == 0) continue;
-    for (int y = v.x; y < v.y; ++y) {
-      const int n = v.w + y * v.z + x0;
-      for (int x = 0; x < nx; ++x)
-        if ((unsigned)(n + x) < (unsigned)a.N) row(n + x);
+    const int2 v = f.level[l];
+    const int x0 = f.x[l][i], nx = (last ? v.x : f.x[l][i + 1]) - x0;
+    if (nx <= 0) continue;
+    const int y0 = f.y[l][r], count = (f.y[l][r + 1] - y0) * nx;
+    int first = v.y + y0 * v.x + x0, x = 0;
+    for (int k = 0; k < count; k += K) {
+      int n[K];
+#pragma unroll
+      for (int u = 0; u < K; ++u) {
+        n[u] = k + u < count && (unsigned)(first + x) < (unsigned)a.N ? first + x : -1;
+        if (++x == nx) {
+          x = 0;
+          first += v.x;
+        }
+      }
+      rows(n);
     }
   }
 }
@@ -128,18 +142,31 @@ __host__ __device__ __forceinline__ int padded(int D) { return (D + 3) & ~3; }
 __host__ __device__ __forceinline__ int tile_stride(int D) { return (padded(D) + 31) / 32 * 32 + 4; }
 
 // Logits of the CTA's map pixels into the tile (padding: -inf, so that it vanishes in the softmax).  A thread takes
-// four bins of one pixel: four loads along the map's x axis, one 16-byte store.
-__device__ __forceinline__ void load_tile(float *tile, int stride, const ProdArgs &a, const float *lg, int npix) {
-  const long long plane = (long long)a.hs * a.ws;
-  const int i = threadIdx.x % kTile;
-  if (i >= npix) return;
-  for (int q = threadIdx.x / kTile; q * 4 < a.D; q += kProdThreads / kTile) {
-    float v[4];
+// four bins of one pixel Q times: four loads along the map each, one 16-byte store.  They are asked for first and stored
+// after the footprint is worked out, which hides the one behind the other.
+template <int Q>
+struct TileLoad {
+  float v[Q][4];
+  __device__ __forceinline__ void ask(const ProdArgs &a, const float *lg, int npix) {
+    const long long plane = (long long)a.hs * a.ws;
+    const int i = threadIdx.x % kTile;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = q * 4 + k < a.D ? __ldg(lg + (q * 4 + k) * plane + i) : -INFINITY;
-    *reinterpret_cast<float4 *>(tile + i * stride + q * 4) = make_float4(v[0], v[1], v[2], v[3]);
+    for (int j = 0; j < Q; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int d = (threadIdx.x / kTile + j * (kProdThreads / kTile)) * 4 + k;
+        v[j][k] = i < npix && d < a.D ? __ldg(lg + d * plane + i) : -INFINITY;
+      }
   }
-}
+  __device__ __forceinline__ void store(float *tile, int stride, const ProdArgs &a) const {
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+      const int d = (threadIdx.x / kTile + j * (kProdThreads / kTile)) * 4;
+      if (d < a.D)
+        *reinterpret_cast<float4 *>(tile + threadIdx.x % kTile * stride + d) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+    }
+  }
+};
 
 constexpr int kLanes = 8;          // lanes that share a map pixel: a warp normalises four pixels at once
 
@@ -198,19 +225,20 @@ __device__ __forceinline__ void normalised_bins(const float *tile, int stride, c
 
 // Forward: a CTA owns kTile map pixels, normalises each once and writes the rows of every level pixel that reads one
 // of them, from registers.  (A CTA per 32 output rows, which normalised every level pixel anew, took 53 us at
-// 6 x 58 x 100 x 64 -> 30 825 rows; this takes 16.5 with the operands in L2, 18.6 cold.)  Bound by instructions and the
-// tail, not by memory: issue slots 63 % busy, DRAM 6 % (dist stays in L2), stores 27 % of the path to L2; six CTAs are
-// resident on an SM (registers), so that 1392 are 1.57 waves, and the CTA of a map row's last 4 columns takes as long as
-// a full one: widths 96, 100, 128 14.5, 16.5, 16.5 us, widths 33 and 64 both 10.4.
+// 6 x 58 x 100 x 64 -> 30 825 rows; tiles that ended with their map row, 3 1/8 of them for 100 columns, 17.1; this 15.1;
+// a 29 x 50 map 14.7 -> 10.8, 118 bins 28.9 -> 26.2.)  Bound by instructions and the tail, not by memory: 1092 CTAs of
+// which six are resident on an SM are 1.23 waves; held to 32 registers for eight it took 13.9, but bf16 12.4 -> 13.2, 59
+// bins 6.9 -> 8.0.
 template <typename OT, int V, int NC>
 __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];
   __shared__ Footprint f;
-  const int tiles = (a.ws + kTile - 1) / kTile, b = blockIdx.y, sy = blockIdx.x / tiles;
-  const int sx0 = (blockIdx.x - sy * tiles) * kTile, npix = min(kTile, a.ws - sx0);
+  const int pixels = a.hs * a.ws, b = blockIdx.y, p0 = blockIdx.x * kTile, npix = min(kTile, pixels - p0);
   const int stride = tile_stride(a.D);
-  load_tile(tile, stride, a, a.logits + ((long long)b * a.D * a.hs + sy) * a.ws + sx0, npix);
-  stage_footprint(f, a, sy, sx0);
+  TileLoad<(V * NC + 3) / 4> load;
+  load.ask(a, a.logits + (long long)b * a.D * pixels + p0, npix);
+  stage_footprint(f, a, p0, (p0 + npix - 1) / a.ws - p0 / a.ws + 1);
+  load.store(tile, stride, a);
   __syncthreads();
   float p[NC][V];
   normalised_bins<V, NC>(tile, stride, a, p);
@@ -221,8 +249,9 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const Pr
   OT *out = reinterpret_cast<OT *>(a.dist) + (long long)b * a.N * a.D + threadIdx.x % kLanes * V;
   const int room = a.D - threadIdx.x % kLanes * V, i = threadIdx.x / kLanes;
   if (i >= npix) return;
-  for_each_row(f, a, i, [&](int n) {
-    OT *dst = out + (long long)n * a.D;
+  for_each_row<1>(f, a, p0, i, [&](const int (&n)[1]) {
+    if (n[0] < 0) return;
+    OT *dst = out + (long long)n[0] * a.D;
 #pragma unroll
     for (int j = 0; j < NC; ++j)
       if (j * kLanes * V < room) *reinterpret_cast<W *>(dst + j * kLanes * V) = w[j];
@@ -231,19 +260,21 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const Pr
 
 // Backward: the same ownership.  A pixel's eight lanes sum the incoming gradient over the level pixels that read it, in
 // the order of the levels, rows and columns, and form p * (G - <p, G>) (softmax) or p * (1 - p) * G (sigmoid), stored
-// along x through shared memory.  (A warp per map pixel, one level pixel after the other: 87 us at the shape above; this
-// takes 18.9 with the operands in L2, 25.5 cold.)  Bound by the latency of the gradient's rows (a third of the stalls, the
-// barrier behind them another fifth), issue slots (53 % busy) and the same tail; DRAM 27 %.  Widths 96, 100, 128 take 16.8,
-// 18.9, 20.6 us, widths 33 and 64 both 12.4.
+// along the map through shared memory.  (A warp per map pixel, one level pixel after the other: 87 us at the shape above;
+// tiles that ended with their map row 24.5; this 22.6; a 29 x 50 map 33.4 -> 22.1, 118 bins 38.5 -> 33.8.)  Bound by the
+// latency of the gradient's rows at the CTAs that the registers leave room for.
 template <typename GT, int V, int NC>
 __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];
   __shared__ Footprint f;
-  const int tiles = (a.ws + kTile - 1) / kTile, b = blockIdx.y, sy = blockIdx.x / tiles;
-  const int sx0 = (blockIdx.x - sy * tiles) * kTile, npix = min(kTile, a.ws - sx0);
+  const int pixels = a.hs * a.ws, b = blockIdx.y, p0 = blockIdx.x * kTile, npix = min(kTile, pixels - p0);
   const int stride = tile_stride(a.D), sub = threadIdx.x % kLanes, pixel = threadIdx.x / kLanes;
-  stage_footprint(f, a, sy, sx0);
-  load_tile(tile, stride, a, a.logits + ((long long)b * a.D * a.hs + sy) * a.ws + sx0, npix);
+  {
+    TileLoad<(V * NC + 3) / 4> load;
+    load.ask(a, a.logits + (long long)b * a.D * pixels + p0, npix);
+    stage_footprint(f, a, p0, (p0 + npix - 1) / a.ws - p0 / a.ws + 1);
+    load.store(tile, stride, a);
+  }
   __syncthreads();
   float G[NC][V];
 #pragma unroll
@@ -252,20 +283,26 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel
     for (int k = 0; k < V; ++k) G[j][k] = 0.f;
   const GT *grad = reinterpret_cast<const GT *>(a.grad_dist) + (long long)b * a.N * a.D + sub * V;
   const int room = a.D - sub * V;
+  // rows asked for at a time: a second one costs registers, and so CTAs, that few bins cannot spare (118 bins 39.5 us at one
+  // row, 33.8 at two; 64 bins 22.6, 23.5)
+  constexpr int K = V * NC <= 8 ? 1 : 2;
   if (pixel < npix)
-    for_each_row(f, a, pixel, [&](int n) {
-      const GT *g = grad + (long long)n * a.D;
-      float v[NC][V];
+    for_each_row<K>(f, a, p0, pixel, [&](const int (&n)[K]) {
+      float v[K][NC][V];
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
+      for (int u = 0; u < K; ++u)
 #pragma unroll
-        for (int k = 0; k < V; ++k) v[j][k] = 0.f;
-        if (j * kLanes * V < room) load_bins<V>(g + j * kLanes * V, v[j]);
-      }
+        for (int j = 0; j < NC; ++j) {
 #pragma unroll
-      for (int j = 0; j < NC; ++j)
+          for (int k = 0; k < V; ++k) v[u][j][k] = 0.f;
+          if (n[u] >= 0 && j * kLanes * V < room) load_bins<V>(grad + (long long)n[u] * a.D + j * kLanes * V, v[u][j]);
+        }
 #pragma unroll
-        for (int k = 0; k < V; ++k) G[j][k] += v[j][k];
+      for (int u = 0; u < K; ++u)
+#pragma unroll
+        for (int j = 0; j < NC; ++j)
+#pragma unroll
+          for (int k = 0; k < V; ++k) G[j][k] += v[u][j][k];
     });
   float p[NC][V], pg = 0.f;
   normalised_bins<V, NC>(tile, stride, a, p);
@@ -283,7 +320,7 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel
         row[j * kLanes * V + k] = a.sigmoid ? p[j][k] * (1.f - p[j][k]) * G[j][k] : p[j][k] * (G[j][k] - pg);
   __syncthreads();
   const long long plane = (long long)a.hs * a.ws;
-  float *gl = a.grad_logits + ((long long)b * a.D * a.hs + sy) * a.ws + sx0;
+  float *gl = a.grad_logits + (long long)b * a.D * pixels + p0;
   const int i = threadIdx.x % kTile;
   if (i < npix)
     for (int q = threadIdx.x / kTile; q * 4 < a.D; q += kProdThreads / kTile) {
@@ -339,7 +376,7 @@ cudaError_t launch_dist_from_logits(const float *logits, const int64_t *shapes, 
     ProdArgs c = a;
     c.logits = logits + (long long)b0 * D * hs * ws;
     c.dist = static_cast<char *>(dist) + (long long)b0 * N * D * (dist_dtype == 0 ? 4 : 2);
-    const dim3 grid((unsigned)((ws + kTile - 1) / kTile) * (unsigned)hs, (unsigned)min(65535, B - b0), 1);
+    const dim3 grid((unsigned)(((long long)hs * ws + kTile - 1) / kTile), (unsigned)min(65535, B - b0), 1);
     const cudaError_t e = dist_dtype == 3   ? launch<__half>(c, false, grid, s)
                           : dist_dtype == 1 ? launch<__nv_bfloat16>(c, false, grid, s)
                                             : launch<float>(c, false, grid, s);
@@ -362,7 +399,7 @@ cudaError_t launch_dist_from_logits_backward(const float *logits, const int64_t 
     c.logits = logits + (long long)b0 * D * hs * ws;
     c.grad_logits = grad_logits + (long long)b0 * D * hs * ws;
     c.grad_dist = static_cast<const char *>(grad_dist) + (long long)b0 * N * D * (grad_dtype == 0 ? 4 : 2);
-    const dim3 grid((unsigned)((ws + kTile - 1) / kTile) * (unsigned)hs, (unsigned)min(65535, B - b0), 1);
+    const dim3 grid((unsigned)(((long long)hs * ws + kTile - 1) / kTile), (unsigned)min(65535, B - b0), 1);
     const cudaError_t e = grad_dtype == 3   ? launch<__half>(c, true, grid, s)
                           : grad_dtype == 1 ? launch<__nv_bfloat16>(c, true, grid, s)
                                             : launch<float>(c, true, grid, s);

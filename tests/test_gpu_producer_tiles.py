@@ -29,3 +29,21 @@ def test_tile_edges_match_softmax_and_nearest_resize(lib_built, map_w, D, dtype)
     got.backward(gd)
     want.backward(gd.float())
     assert_close("grad_logits", logits.grad, ref.grad, rtol=1e-4, atol_frac=2e-6)
+
+
+@pytest.mark.parametrize("map_h,map_w", [(70, 1), (33, 3), (9, 11), (2, 47), (3, 64)])
+def test_tiles_that_run_over_map_rows(lib_built, map_h, map_w):
+    """A tile is 32 consecutive map pixels: of one row, the end of one and the start of the next, or of up to 32 rows."""
+    from dfa3d_b200.dist_producer import depth_distribution
+    g = torch.Generator().manual_seed(map_h)
+    levels = ((2 * map_h + 1, 2 * map_w), (map_h, map_w), (map_h // 3 + 1, map_w // 2 + 1))
+    logits = torch.randn(2, 20, map_h, map_w, generator=g).to(DEV).requires_grad_(True)
+    shapes, lsi, N = level_tensors(levels)
+    ref = logits.detach().clone().requires_grad_(True)
+    want = reference_dist(ref, levels, "softmax")
+    got = depth_distribution(logits, shapes, lsi, N)
+    assert ((got - want.detach()).abs() <= want.detach().abs() * 2e-6 + 2 ** -24).all()
+    gd = torch.randn(2, N, 20, generator=g).to(DEV)
+    got.backward(gd)
+    want.backward(gd)
+    assert_close("grad_logits", logits.grad, ref.grad, rtol=1e-4, atol_frac=2e-6)
