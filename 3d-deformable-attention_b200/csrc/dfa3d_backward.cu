@@ -69,13 +69,13 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
     bwd_point<DT, MODE>(a, lv, c, chunk + lane, sm, st, wgt, off);
     store_rows(table, lane, off, wgt);
     __syncwarp();
-    auto step = [&](int r0, int nrows) {
+    auto step = [&](int r0) {
       RowEntry e[U];
       float v[U][V];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int r = r0 + u * R;
-        e[u] = (FULL || r + grp < nrows) ? my[r] : RowEntry{-1, 0.f};
+        e[u] = my[r];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -97,7 +97,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
         int u_mine;
         const float f = fold_four_dots<G>(d, sub, u_mine);
         const int r = r0 + u_mine * R;
-        if (u_mine >= 0 && (FULL || r + grp < nrows)) myd[r] = f;
+        if (u_mine >= 0) myd[r] = f;
       } else {
         // groups of 2 lanes (8 channels): a group's first lane stores its four totals one by one
 #pragma unroll
@@ -106,7 +106,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
 #pragma unroll
           for (int s = 1; s < G; s <<= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
           const int r = r0 + u * R;
-          if (sub == 0 && (FULL || r + grp < nrows)) myd[r] = t;
+          if (sub == 0) myd[r] = t;
         }
       }
 #pragma unroll
@@ -120,9 +120,10 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
         }
       }
     };
+    // (the table's slots past the last point hold no rows: a step may run over it)
     const int nrows = FULL ? 128 : min(32, a.LP - chunk) * 4;
 #pragma unroll 1
-    for (int r0 = 0; r0 < nrows; r0 += R * U) step(r0, nrows);
+    for (int r0 = 0; r0 < nrows; r0 += R * U) step(r0);
     __syncwarp();
     const float4 tq = reinterpret_cast<const float4 *>(dot_slots)[lane];
     const float t[4] = {tq.x, tq.y, tq.z, tq.w};
@@ -136,7 +137,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
 // fused / given-depth-score backward, C/4 a power of two
 // ------------------------------------------------------------------------------------------------
 // 4 CTAs (32 warps) per SM is the measured optimum (64 registers, a few bytes of spill); a CTA walks
-// DFA3D_BWD_ITEMS_PER_WARP consecutive groups of 8 items before it retires.
+// up to DFA3D_BWD_ITEMS_PER_WARP consecutive groups of 8 items before it retires (walk_rounds).
 template <typename VT, typename DT, int C, int MODE, bool FULL>
 __global__ void __launch_bounds__(kThreads, DFA3D_BWD_MIN_CTAS)
 dfa3d_backward_kernel(const KArgs a) {
@@ -146,9 +147,9 @@ dfa3d_backward_kernel(const KArgs a) {
   stage_levels(lv, a);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int it = 0; it < DFA3D_BWD_ITEMS_PER_WARP; ++it) {
+  for (int it = 0; it < a.rounds; ++it) {
     ItemCtx c;
-    if (!item_context<MODE, DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_BWD_ITEMS_PER_WARP + it, c)) return;
+    if (!item_context<MODE, DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * a.rounds + it, c)) return;
     backward_item<VT, DT, C, MODE, FULL>(a, lv, c, rows[warp], dots[warp], lane);
   }
 }
@@ -278,9 +279,11 @@ static cudaError_t launch_backward_vd(const KArgs &a0, cudaStream_t s) {
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
-    constexpr int kPerCta = kWarpsPerCta * DFA3D_BWD_ITEMS_PER_WARP;
-    const dim3 grid((unsigned)((a.items_per_cam + kPerCta - 1) / kPerCta),
-                    (unsigned)min(65535, a0.B - b0), 1);
+    const int cams = min(65535, a0.B - b0);
+    a.rounds = walk_rounds((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, DFA3D_BWD_ITEMS_PER_WARP,
+                           DFA3D_BWD_MIN_CTAS);
+    const int per_cta = kWarpsPerCta * a.rounds;
+    const dim3 grid((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
     if (full) launch_backward_g<VT, DT, MODE, true>(a, grid, s);
     else launch_backward_g<VT, DT, MODE, false>(a, grid, s);
     const cudaError_t e = cudaGetLastError();

@@ -162,7 +162,7 @@ cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
     KArgs a = a0;
     a.b0 = b0;
     const unsigned cams = (unsigned)min(65535, a0.B - b0);
-    a.rounds = packed_rounds((long long)batches * cams);
+    a.rounds = walk_rounds(batches, (int)cams, kPackedRounds, DFA3D_BWD_MIN_CTAS);
     const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
     if (lpp == 4) launch_c<VT, DT, MODE, 4>(a, grid, s);
     else if (lpp == 8) launch_c<VT, DT, MODE, 8>(a, grid, s);

@@ -41,8 +41,8 @@ constexpr int kWarpsPerCta = 8;
 constexpr int kThreads = kWarpsPerCta * 32;
 
 // Compile-time tuning knobs (defaults = the measured optimum on B200 at the BEVFormer-base shape).
-//   *_ITEMS_PER_WARP  consecutive CTA-sized groups of items a CTA works through before it retires:
-//                     fewer, longer-lived CTAs (a CTA that handles one item per warp lives ~2 us)
+//   *_ITEMS_PER_WARP  consecutive CTA-sized groups of items a CTA works through before it retires, at most
+//                     (walk_rounds): fewer, longer-lived CTAs (a CTA that handles one item per warp lives ~2 us)
 //   *_MIN_CTAS        __launch_bounds__ residency target, i.e. the register cap
 #ifndef DFA3D_FWD_ITEMS_PER_WARP
 #define DFA3D_FWD_ITEMS_PER_WARP 8
@@ -87,7 +87,7 @@ struct KArgs {
   float *grad_off_d;       // (B,Q,H,L,P), overwritten
   long long row_loc, row_attn;  // elements from query to query of loc, and of attn and off_d
   int Z;                   // reference points (pillar anchors) per query
-  int rounds;              // several items per warp: batches of 32 lanes a warp takes
+  int rounds;              // items, or batches of 32 lanes where several items share a warp, that a warp takes in turn
   int maps;                // 2-D: value maps per batch element; N and L count all of them.  0 elsewhere
   // ragged queries: camera b owns the packed query rows [q_off[b], q_off[b+1]) of every per-query
   // tensor; Q is then only the bound the grid is sized for.  Null = every camera has Q queries.
@@ -226,13 +226,33 @@ __device__ __forceinline__ void prefetch_offsets(const KArgs &a, int b, unsigned
   }
 }
 
+// How many CTA-sized groups of items (`groups` of them a camera) a CTA walks before it retires: up to `most`, fewer where
+// that many would leave the last wave of CTAs nearly empty, or the device (`resident` CTAs fit an SM); starting a CTA costs
+// about a third of a group.  From six waves on the last one counts little.  Forward, 32 points an item, us at eight groups /
+// with this rule: 6 cameras x 1000 queries x 8 heads 95 / 70, 1 x 1000 29 / 15, 1 x 300 28 / 7.5, 6 x 6000 and more the same.
+inline int walk_rounds(long long groups, int cams, int most, int resident) {
+  const long long slots = 148LL * resident;
+  if ((groups + most - 1) / most * cams >= 6 * slots) return most;
+  int best = most;
+  long long cost = 0;
+  for (int r = most; r >= 1; --r) {
+    const long long ctas = (groups + r - 1) / r * cams;
+    const long long c = (ctas + slots - 1) / slots * (3 * r + 1);
+    if (r == most || c < cost) {
+      best = r;
+      cost = c;
+    }
+  }
+  return best;
+}
+
 // ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
 // Items of up to 16 points, rows of 16, 32 or 64 channels.
 inline bool packed_covers(int LP, int C) { return LP <= 16 && (C == 16 || C == 32 || C == 64); }
-// Batches of 32 lanes a warp takes before its CTA retires, by the CTA-sized batches of the launch: two once the device is
-// filled twice over (fewer, longer-lived CTAs), one before that, so that a small launch spreads over the SMs and is one
-// chain of latencies deep (900 queries x 8 heads x 4 points forward: 7.9 us at two).
-inline int packed_rounds(long long batches) { return batches >= 148 * 12 ? 2 : 1; }
+// Batches of 32 lanes a warp takes before its CTA retires, at most (walk_rounds): two, for fewer, longer-lived CTAs; a small
+// launch spreads over the SMs with one and is one chain of latencies deep (900 queries x 8 heads x 4 points forward: 7.9 us
+// at two, 5.1 at one).
+constexpr int kPackedRounds = 2;
 
 // Softmax of an item's L*P attention logits (caller-fused mode): maximum and sum of exp(l - max),
 // formed with warp shuffles; lane j later turns its own logit into exp(l_j - max) / sum.

@@ -54,15 +54,10 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
       reinterpret_cast<float4 *>(a.ds_out)[c.pt0 + chunk + lane] = make_float4(ds[0], ds[1], ds[2], ds[3]);
     __syncwarp();
     // R points per step: U independent row-fragment loads in flight per lane, then U fused multiply-adds.
-    auto step = [&](int p0, int n) {
+    auto step = [&](int p0) {
       RowEntry e[U];
       float v[U][V];
-      if (FULL || p0 + lane / G < n) {
-        table.load(p0 + lane / G, e);
-      } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u) e[u] = RowEntry{-1, 0.f};
-      }
+      table.load(p0 + lane / G, e);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (e[u].off >= 0) {
@@ -108,11 +103,11 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
       }
     } else if constexpr (FULL) {          // compile-time trip count, table offsets become immediates
 #pragma unroll
-      for (int p0 = 0; p0 < 32; p0 += R) step(p0, 32);
+      for (int p0 = 0; p0 < 32; p0 += R) step(p0);
     } else {
-      const int n = min(32, a.LP - chunk);
+      const int n = min(32, a.LP - chunk);         // (the table's slots past the last point hold no rows)
 #pragma unroll 1
-      for (int p0 = 0; p0 < n; p0 += R) step(p0, n);
+      for (int p0 = 0; p0 < n; p0 += R) step(p0);
     }
     __syncwarp();
   }
@@ -120,7 +115,7 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
 }
 
 // 5 CTAs (40 warps) per SM: measured best; at 6+ the register cap starts to cost more than the
-// extra warps hide.  A CTA walks DFA3D_FWD_ITEMS_PER_WARP consecutive groups of 8 items (the grid's
+// extra warps hide.  A CTA walks up to DFA3D_FWD_ITEMS_PER_WARP consecutive groups of 8 items (the grid's
 // ~60 000 CTAs per camera otherwise live ~2 us each and their turnover shows: measured -7 % at 8).
 template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
 __global__ void __launch_bounds__(kThreads, DFA3D_FWD_MIN_CTAS)
@@ -128,13 +123,15 @@ dfa3d_forward_kernel(const KArgs a) {
   __shared__ LevelTable lv;
   __shared__ RowTable rows[kWarpsPerCta];
   stage_levels(lv, a);
-  constexpr unsigned kItems = kWarpsPerCta * DFA3D_FWD_ITEMS_PER_WARP;
-  if (MODE == kCallerFused) prefetch_offsets(a, (int)blockIdx.y + a.b0, blockIdx.x * kItems, kItems);
+  if (MODE == kCallerFused) {
+    const unsigned items = kWarpsPerCta * (unsigned)a.rounds;
+    prefetch_offsets(a, (int)blockIdx.y + a.b0, blockIdx.x * items, items);
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int it = 0; it < DFA3D_FWD_ITEMS_PER_WARP; ++it) {
+  for (int it = 0; it < a.rounds; ++it) {
     ItemCtx c;
-    if (!item_context<MODE, DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * DFA3D_FWD_ITEMS_PER_WARP + it, c)) return;
+    if (!item_context<MODE, DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * a.rounds + it, c)) return;
     forward_item<VT, DT, C, MODE, WRITE_DS, FULL>(a, lv, c, rows[warp], lane);
   }
 }
@@ -243,7 +240,10 @@ static cudaError_t launch_forward_vd(const KArgs &a0, cudaStream_t s) {
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
-    const dim3 grid = item_grid(a, min(65535, a0.B - b0), DFA3D_FWD_ITEMS_PER_WARP);
+    const int cams = min(65535, a0.B - b0);
+    a.rounds = walk_rounds((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, DFA3D_FWD_ITEMS_PER_WARP,
+                           DFA3D_FWD_MIN_CTAS);
+    const dim3 grid = item_grid(a, cams, a.rounds);
     if (a.ds_out) {
       if (full) launch_forward_g<VT, DT, MODE, true, true>(a, grid, s);
       else launch_forward_g<VT, DT, MODE, true, false>(a, grid, s);

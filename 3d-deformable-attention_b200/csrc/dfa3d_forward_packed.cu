@@ -158,7 +158,8 @@ cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
     KArgs a = a0;
     a.b0 = b0;
     const unsigned cams = (unsigned)min(65535, a0.B - b0);
-    a.rounds = packed_rounds((long long)batches * cams);
+    const int resident = RowVec<VT>::kElems == 8 ? 4 : MODE == kFused && a.ds_out ? 5 : 6;       // see PackedCtas
+    a.rounds = walk_rounds(batches, (int)cams, kPackedRounds, resident);
     const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
     if constexpr (mode_from_offsets(MODE)) {      // the caller-fused entry points return no depth score
       launch_lp<VT, DT, MODE, false>(a, grid, s);
