@@ -1,6 +1,6 @@
 // DFA3D backward for items of few points (L*P <= 16): a warp takes several consecutive items at once (sm_100a).
 //
-// An item has LPP lanes -- 4, 8 or 16, the next of them from L*P on -- and lane j of them owns its point j (full or nearly
+// An item has LPP lanes -- 4, 8 or 16 (packed_lanes) -- and lane j of them owns its point j (full or nearly
 // full, coalesced prologue and epilogue); a group of G lanes walks the rows of one item -- or a share of them when the warp
 // holds fewer items than groups -- with that item's grad_out fragment.  Same row phase as the one-item kernels otherwise,
 // and the same bound: the row reductions, in L2 and on the way to it.
@@ -155,7 +155,7 @@ void launch_c(const KArgs &a, dim3 grid, cudaStream_t s) {
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
-  const int lpp = a0.LP <= 4 ? 4 : a0.LP <= 8 ? 8 : 16;
+  const int lpp = packed_lanes(a0, MODE);
   const unsigned batch = kWarpsPerCta * (32 / lpp);                  // items a CTA takes at a time
   const unsigned batches = ((unsigned)a0.items_per_cam + batch - 1) / batch;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit

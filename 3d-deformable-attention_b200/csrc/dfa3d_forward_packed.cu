@@ -130,10 +130,9 @@ void launch_c(const KArgs &a, dim3 grid, cudaStream_t s) {
 }
 
 template <typename VT, typename DT, int MODE, bool WRITE_DS>
-void launch_lp(const KArgs &a, dim3 grid, cudaStream_t s) {
+void launch_lp(const KArgs &a, int lpp, dim3 grid, cudaStream_t s) {
   // the unrolled loop is instantiated where it is the common case: fp32 throughout
   constexpr bool kFloat = sizeof(VT) == 4 && (sizeof(DT) == 4 || !mode_has_depth(MODE));
-  const int lpp = a.LP <= 4 ? 4 : a.LP <= 8 ? 8 : 16;
   if constexpr (kFloat) {
     if (a.LP == lpp) {
       if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, true>(a, grid, s);
@@ -151,7 +150,7 @@ void launch_lp(const KArgs &a, dim3 grid, cudaStream_t s) {
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
-  const int lpp = a0.LP <= 4 ? 4 : a0.LP <= 8 ? 8 : 16;
+  const int lpp = packed_lanes(a0, MODE);
   const unsigned batch = kWarpsPerCta * (32 / lpp);                  // items a CTA takes at a time
   const unsigned batches = ((unsigned)a0.items_per_cam + batch - 1) / batch;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
@@ -162,12 +161,12 @@ cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
     a.rounds = walk_rounds(batches, (int)cams, kPackedRounds, resident);
     const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
     if constexpr (mode_from_offsets(MODE)) {      // the caller-fused entry points return no depth score
-      launch_lp<VT, DT, MODE, false>(a, grid, s);
+      launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
     } else if constexpr (MODE == kFused) {
-      if (a.ds_out) launch_lp<VT, DT, MODE, true>(a, grid, s);
-      else launch_lp<VT, DT, MODE, false>(a, grid, s);
+      if (a.ds_out) launch_lp<VT, DT, MODE, true>(a, lpp, grid, s);
+      else launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
     } else {
-      launch_lp<VT, DT, MODE, false>(a, grid, s);
+      launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -1,6 +1,6 @@
-"""CTAs that walk several groups of items: launches of a few groups, of some waves of CTAs and of sizes in between, item
-counts that do not fill the last group, with one item and with several items per warp, and cameras of different numbers of
-queries.  Checked against the CPU oracle."""
+"""CTAs that walk several groups of items, and items that get more lanes in a small launch: launches of a few groups, of some
+waves of CTAs and of sizes in between, item counts that do not fill the last group, with one item and with several items
+per warp, and cameras of different numbers of queries.  Checked against the CPU oracle."""
 import numpy as np
 import pytest
 import torch
@@ -13,7 +13,7 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("Q", [7, 211, 803, 2401])
-@pytest.mark.parametrize("P,C", [(17, 8), (3, 16)])
+@pytest.mark.parametrize("P,C", [(17, 8), (3, 16), (2, 64), (4, 32), (7, 64), (8, 32)])
 def test_every_item_is_walked(lib_built, P, C, Q):
     from dfa3d_b200 import ext
     w = wl.WORKLOADS["tiny"].with_(B=5, H=7, C=C, D=6, Q=Q, levels=((6, 9),), P=P, seed=Q + P)
