@@ -2,8 +2,8 @@
 //
 // With one item per warp an item of 4 points (temporal self-attention and the decoder's cross-attention
 // use 1 level x 4 points) keeps 4 lanes busy in the prologue and costs a whole chain of dependent
-// latencies (locations -> row table -> rows -> sum -> store) for 16 rows.  Here an item has LPP lanes -- 4, 8 or 16,
-// the next of them from L*P on -- and lane j of them owns its point j, so the prologue is (nearly) full and coalesced:
+// latencies (locations -> row table -> rows -> sum -> store) for 16 rows.  Here an item has LPP lanes -- 4, 8 or 16
+// (packed_lanes) -- and lane j of them owns its point j, so the prologue is (nearly) full and coalesced:
 // the points of consecutive items are consecutive in memory.  A group of G lanes then sums all rows of one item (or,
 // when the warp holds fewer items than groups, a share of them) and writes that item's output itself.
 // Bound like the one-item kernels by the rows that travel from L2 to the SM.  Against one item per warp, 6 cameras x 6000
