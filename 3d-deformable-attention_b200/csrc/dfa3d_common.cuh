@@ -252,7 +252,7 @@ inline bool packed_covers(int LP, int C) { return LP <= 16 && (C == 16 || C == 3
 // Lanes of an item: 4, 8 or 16, the next from L*P on -- or more of them where the launch would have fewer than two CTAs for
 // every SM: it then takes as long as one warp's chain of loads, which is shorter with fewer items to a group.  2-D, one
 // 200 x 200 map, 4 points, forward / backward: 300 queries 10.5 / 8.9 -> 5.3 / 4.9 us, 900 11.4 / 10.3 -> 6.5 / 6.8 (warm 5.1
-// -> 4.6); 8 points of 23 x 40 and 512 queries 4.9 / 10.5 -> 4.9 / 8.5.  Up to four CTAs an SM: 1500 queries of 2 x 4 points
+// -> 4.5); 8 points of 23 x 40 and 512 queries 4.9 / 10.5 -> 4.9 / 8.5.  Up to four CTAs an SM: 1500 queries of 2 x 4 points
 // 7.3 -> 8.9.  (From offsets in 2-D, the kernels are made for the lanes of a map.)
 inline int packed_lanes(const KArgs &a, int mode) {
   int lanes = a.LP <= 4 ? 4 : a.LP <= 8 ? 8 : 16;
