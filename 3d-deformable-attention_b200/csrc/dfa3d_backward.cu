@@ -41,6 +41,13 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
   constexpr int G = C / V;
   constexpr int R = 32 / G;
   constexpr int U = 4;
+  // The table's slots past the last point hold no rows, and the dots of those are read by no one: a step may run over the
+  // last point.  Conditions stand where the kernel comes out faster with them (20 points, 6 x 6000 queries x 8 heads, us
+  // without / with): on the dots (from offsets, bf16 dist 906 / 892; two-stage of 16 channels 194 / 187) unless 16-bit rows
+  // come with locations (648 / 666), on the rows for 16-bit rows with fp32 dist from offsets (831 / 806, 64 channels
+  // 1236 / 1194; other types lose up to 5 %).
+  constexpr bool kGuardDots = !FULL && !(MODE == kFused && sizeof(VT) == 2);
+  constexpr bool kGuardRows = !FULL && MODE == kCallerFused && sizeof(VT) == 2 && sizeof(DT) == 4;
   const int sub = lane % G, grp = lane / G;
   const long long slice = ((long long)c.b * a.N * a.H + c.h) * C + sub * V;
   const VT *vbase = reinterpret_cast<const VT *>(a.value) + slice;
@@ -69,13 +76,14 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
     bwd_point<DT, MODE>(a, lv, c, chunk + lane, sm, st, wgt, off);
     store_rows(table, lane, off, wgt);
     __syncwarp();
+    const int nrows = FULL ? 128 : min(32, a.LP - chunk) * 4;
     auto step = [&](int r0) {
       RowEntry e[U];
       float v[U][V];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int r = r0 + u * R;
-        e[u] = my[r];
+        e[u] = !kGuardRows || r + grp < nrows ? my[r] : RowEntry{-1, 0.f};
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -97,7 +105,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
         int u_mine;
         const float f = fold_four_dots<G>(d, sub, u_mine);
         const int r = r0 + u_mine * R;
-        if (u_mine >= 0) myd[r] = f;
+        if (u_mine >= 0 && (!kGuardDots || r + grp < nrows)) myd[r] = f;
       } else {
         // groups of 2 lanes (8 channels): a group's first lane stores its four totals one by one
 #pragma unroll
@@ -106,7 +114,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
 #pragma unroll
           for (int s = 1; s < G; s <<= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
           const int r = r0 + u * R;
-          if (sub == 0) myd[r] = t;
+          if (sub == 0 && (!kGuardDots || r + grp < nrows)) myd[r] = t;
         }
       }
 #pragma unroll
@@ -120,8 +128,6 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
         }
       }
     };
-    // (the table's slots past the last point hold no rows: a step may run over it)
-    const int nrows = FULL ? 128 : min(32, a.LP - chunk) * 4;
 #pragma unroll 1
     for (int r0 = 0; r0 < nrows; r0 += R * U) step(r0);
     __syncwarp();
@@ -137,19 +143,20 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
 // fused / given-depth-score backward, C/4 a power of two
 // ------------------------------------------------------------------------------------------------
 // 4 CTAs (32 warps) per SM is the measured optimum (64 registers, a few bytes of spill); a CTA walks
-// up to DFA3D_BWD_ITEMS_PER_WARP consecutive groups of 8 items before it retires (walk_rounds).
-template <typename VT, typename DT, int C, int MODE, bool FULL>
+// up to DFA3D_BWD_ITEMS_PER_WARP consecutive groups of 8 items before it retires.  WALK: that number; 0: a.rounds
+// (walk_rounds), which costs registers that the kernel does not have (from offsets with bf16 dist 1202 us, 1194 as a constant).
+template <typename VT, typename DT, int C, int MODE, bool FULL, int WALK>
 __global__ void __launch_bounds__(kThreads, DFA3D_BWD_MIN_CTAS)
 dfa3d_backward_kernel(const KArgs a) {
   __shared__ LevelTable lv;
   __shared__ __align__(16) RowEntry rows[kWarpsPerCta][128];
   __shared__ __align__(16) float dots[kWarpsPerCta][128];
   stage_levels(lv, a);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rounds = WALK ? WALK : a.rounds, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int it = 0; it < a.rounds; ++it) {
+  for (int it = 0; it < rounds; ++it) {
     ItemCtx c;
-    if (!item_context<MODE, DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * a.rounds + it, c)) return;
+    if (!item_context<MODE, DFA3D_BWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * rounds + it, c)) return;
     backward_item<VT, DT, C, MODE, FULL>(a, lv, c, rows[warp], dots[warp], lane);
   }
 }
@@ -256,15 +263,15 @@ dfa3d_depth_score_backward_kernel(const KArgs a) {
 // ------------------------------------------------------------------------------------------------
 // host-side dispatch
 // ------------------------------------------------------------------------------------------------
-template <typename VT, typename DT, int MODE, bool FULL>
+template <typename VT, typename DT, int MODE, bool FULL, int WALK>
 static void launch_backward_g(const KArgs &a, dim3 grid, cudaStream_t s) {
   constexpr int V = RowVec4<VT>::kElems;
   switch ((a.C % V == 0) ? a.C / V : 0) {
-    case 2:  dfa3d_backward_kernel<VT, DT, 2 * V, MODE, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 4:  dfa3d_backward_kernel<VT, DT, 4 * V, MODE, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 8:  dfa3d_backward_kernel<VT, DT, 8 * V, MODE, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 16: dfa3d_backward_kernel<VT, DT, 16 * V, MODE, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 32: dfa3d_backward_kernel<VT, DT, 32 * V, MODE, FULL><<<grid, kThreads, 0, s>>>(a); break;
+    case 2:  dfa3d_backward_kernel<VT, DT, 2 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
+    case 4:  dfa3d_backward_kernel<VT, DT, 4 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
+    case 8:  dfa3d_backward_kernel<VT, DT, 8 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
+    case 16: dfa3d_backward_kernel<VT, DT, 16 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
+    case 32: dfa3d_backward_kernel<VT, DT, 32 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
     default: {
       const dim3 g1((unsigned)((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta), grid.y, 1);
       dfa3d_backward_generic_kernel<VT, DT, MODE><<<g1, kThreads, 0, s>>>(a);
@@ -284,8 +291,14 @@ static cudaError_t launch_backward_vd(const KArgs &a0, cudaStream_t s) {
                            DFA3D_BWD_MIN_CTAS);
     const int per_cta = kWarpsPerCta * a.rounds;
     const dim3 grid((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
-    if (full) launch_backward_g<VT, DT, MODE, true>(a, grid, s);
-    else launch_backward_g<VT, DT, MODE, false>(a, grid, s);
+    constexpr int kMost = DFA3D_BWD_ITEMS_PER_WARP;
+    if (a.rounds == kMost) {
+      if (full) launch_backward_g<VT, DT, MODE, true, kMost>(a, grid, s);
+      else launch_backward_g<VT, DT, MODE, false, kMost>(a, grid, s);
+    } else {
+      if (full) launch_backward_g<VT, DT, MODE, true, 0>(a, grid, s);
+      else launch_backward_g<VT, DT, MODE, false, 0>(a, grid, s);
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

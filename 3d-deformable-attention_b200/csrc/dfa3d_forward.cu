@@ -117,21 +117,27 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
 // 5 CTAs (40 warps) per SM: measured best; at 6+ the register cap starts to cost more than the
 // extra warps hide.  A CTA walks up to DFA3D_FWD_ITEMS_PER_WARP consecutive groups of 8 items (the grid's
 // ~60 000 CTAs per camera otherwise live ~2 us each and their turnover shows: measured -7 % at 8).
-template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
+// WALK: that number, as every launch of some size has it; 0: a.rounds of them (walk_rounds).  As a run-time number it costs
+// registers that most kernels do not have: 6 cameras of the base levels, us at run time / as a constant: bf16 of 32 channels
+// 524 / 519, of 64 from offsets 503 / 491, fp32 of 64 535 / 521, fp16 of 20 points 363 / 350.  Unrolled, fp32 rows of up to 32
+// channels were faster with the run-time number (base 565 / 569, 8 channels from offsets 348 / 371, bf16 dist from offsets
+// 435 / 459), as were bf16 rows of 32 with fp32 dist (6000 queries 330 / 341).
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL, int WALK>
 __global__ void __launch_bounds__(kThreads, DFA3D_FWD_MIN_CTAS)
 dfa3d_forward_kernel(const KArgs a) {
   __shared__ LevelTable lv;
   __shared__ RowTable rows[kWarpsPerCta];
   stage_levels(lv, a);
+  const int rounds = WALK ? WALK : a.rounds;
   if (MODE == kCallerFused) {
-    const unsigned items = kWarpsPerCta * (unsigned)a.rounds;
+    const unsigned items = kWarpsPerCta * (unsigned)rounds;
     prefetch_offsets(a, (int)blockIdx.y + a.b0, blockIdx.x * items, items);
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-  for (int it = 0; it < a.rounds; ++it) {
+  for (int it = 0; it < rounds; ++it) {
     ItemCtx c;
-    if (!item_context<MODE, DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * a.rounds + it, c)) return;
+    if (!item_context<MODE, DFA3D_FWD_HEAD_MAJOR != 0>(a, warp, blockIdx.x * rounds + it, c)) return;
     forward_item<VT, DT, C, MODE, WRITE_DS, FULL>(a, lv, c, rows[warp], lane);
   }
 }
@@ -219,24 +225,40 @@ static dim3 item_grid(const KArgs &a, int cams, int items_per_warp) {
   return dim3((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
 }
 
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
+static void launch_forward_c(const KArgs &a, dim3 grid, cudaStream_t s) {
+  // unrolled, fp32 rows of up to 32 channels or bf16 rows of 32 with fp32 dist: one kernel for every launch (see the kernel)
+  constexpr bool kOne = FULL && (RowVec<VT>::kElems == 4 ? C <= 32 : C == 32 && MODE == kFused && sizeof(DT) == 4 && !WRITE_DS);
+  constexpr int kMost = DFA3D_FWD_ITEMS_PER_WARP;
+  if (!kOne && a.rounds == kMost)
+    dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, kOne ? 0 : kMost><<<grid, kThreads, 0, s>>>(a);
+  else
+    dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, 0><<<grid, kThreads, 0, s>>>(a);
+}
+
 template <typename VT, typename DT, int MODE, bool WRITE_DS, bool FULL>
 static void launch_forward_g(const KArgs &a, dim3 grid, cudaStream_t s) {
   constexpr int V = RowVec<VT>::kElems;
   switch ((a.C % V == 0) ? a.C / V : 0) {
-    case 2:  dfa3d_forward_kernel<VT, DT, 2 * V, MODE, WRITE_DS, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 4:  dfa3d_forward_kernel<VT, DT, 4 * V, MODE, WRITE_DS, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 8:  dfa3d_forward_kernel<VT, DT, 8 * V, MODE, WRITE_DS, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 16: dfa3d_forward_kernel<VT, DT, 16 * V, MODE, WRITE_DS, FULL><<<grid, kThreads, 0, s>>>(a); break;
-    case 32: dfa3d_forward_kernel<VT, DT, 32 * V, MODE, WRITE_DS, FULL><<<grid, kThreads, 0, s>>>(a); break;
+    case 2:  launch_forward_c<VT, DT, 2 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
+    case 4:  launch_forward_c<VT, DT, 4 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
+    case 8:  launch_forward_c<VT, DT, 8 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
+    case 16: launch_forward_c<VT, DT, 16 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
+    case 32: launch_forward_c<VT, DT, 32 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
     default:
       dfa3d_forward_generic_kernel<VT, DT, MODE, WRITE_DS><<<item_grid(a, (int)grid.y, 1), kThreads, 0, s>>>(a);
       break;
   }
 }
 
+template <typename VT, typename DT, int MODE, bool WRITE_DS>
+static void launch_forward_ds(const KArgs &a, dim3 grid, cudaStream_t s) {
+  if (a.LP % 32 == 0) launch_forward_g<VT, DT, MODE, WRITE_DS, true>(a, grid, s);
+  else launch_forward_g<VT, DT, MODE, WRITE_DS, false>(a, grid, s);
+}
+
 template <typename VT, typename DT, int MODE>
 static cudaError_t launch_forward_vd(const KArgs &a0, cudaStream_t s) {
-  const bool full = a0.LP % 32 == 0;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
@@ -244,12 +266,11 @@ static cudaError_t launch_forward_vd(const KArgs &a0, cudaStream_t s) {
     a.rounds = walk_rounds((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, DFA3D_FWD_ITEMS_PER_WARP,
                            DFA3D_FWD_MIN_CTAS);
     const dim3 grid = item_grid(a, cams, a.rounds);
-    if (a.ds_out) {
-      if (full) launch_forward_g<VT, DT, MODE, true, true>(a, grid, s);
-      else launch_forward_g<VT, DT, MODE, true, false>(a, grid, s);
+    if constexpr (MODE == kFused) {               // the other modes' entry points return no depth score
+      if (a.ds_out) launch_forward_ds<VT, DT, MODE, true>(a, grid, s);
+      else launch_forward_ds<VT, DT, MODE, false>(a, grid, s);
     } else {
-      if (full) launch_forward_g<VT, DT, MODE, false, true>(a, grid, s);
-      else launch_forward_g<VT, DT, MODE, false, false>(a, grid, s);
+      launch_forward_ds<VT, DT, MODE, false>(a, grid, s);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
