@@ -37,6 +37,11 @@ dfa3d_forward_packed_kernel(const KArgs a) {
   // queries: 122 us fully unrolled, 75 by 2; 2-D from offsets, 22500 queries: 88, 63 by 2, 62 by 4).
   constexpr bool kShort = !mode_has_depth(MODE) && GPI == 1 && IPG == 1;
   constexpr int kUnroll = !kShort ? LPP / GPI : MODE == kCallerFused2D ? 4 : 2;
+  // fold_and_store where there is something to halve (16-bit rows whose item is shared), and for fp32 rows where the kernel is
+  // faster with it: 5 points of 64 channels, locations given and no scores 113.7 us without, 106.9 with (6 x 6000 queries);
+  // 2-D from offsets, 900 x 16 points 8.80 / 8.61.  It cost the others registers: 2-D from offsets, 40000 queries x 4 points
+  // 51.8 / 53.8, 4 x 900 13.2 / 13.7; 16 points of 16 channels with scores 165.8 / 173.3; fp16, 8 points of 64 channels 126 / 133.
+  constexpr bool kFold = V == 8 || MODE == kCallerFused2D ? GPI > 1 : !EXACT && MODE == kFused && !WRITE_DS;
   static_assert(32 % LPP == 0 && 32 % G == 0 && LPP % GPI == 0, "unsupported packing");
   __shared__ LevelTable lv;
   __shared__ RowTable rows[kWarpsPerCta];
@@ -113,7 +118,20 @@ dfa3d_forward_packed_kernel(const KArgs a) {
         for (int p0 = 0; p0 < n; p0 += GPI) step(p0);
       }
       const unsigned idx = first + i;
-      fold_and_store<V, G, GPI>(acc, lane, a.out + ((q0 * a.H + idx) * C + sub * V), idx < nitems);
+      if constexpr (kFold) {
+        fold_and_store<V, G, GPI>(acc, lane, a.out + ((q0 * a.H + idx) * C + sub * V), idx < nitems);
+      } else {
+#pragma unroll
+        for (int s = G; s < G * GPI; s <<= 1)
+#pragma unroll
+          for (int x = 0; x < V; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], s);
+        if (grp % GPI == 0 && idx < nitems) {
+          float *o = a.out + ((q0 * a.H + idx) * C + sub * V);
+#pragma unroll
+          for (int x = 0; x < V; x += 4)
+            *reinterpret_cast<float4 *>(o + x) = make_float4(acc[x], acc[x + 1], acc[x + 2], acc[x + 3]);
+        }
+      }
     }
     __syncwarp();
   }
