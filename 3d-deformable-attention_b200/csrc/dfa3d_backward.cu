@@ -144,7 +144,7 @@ __device__ __forceinline__ void backward_item(const KArgs &a, const LevelTable &
 // ------------------------------------------------------------------------------------------------
 // 4 CTAs (32 warps) per SM is the measured optimum (64 registers, a few bytes of spill); a CTA walks
 // up to DFA3D_BWD_ITEMS_PER_WARP consecutive groups of 8 items before it retires.  WALK: that number; 0: a.rounds
-// (walk_rounds), which costs registers that the kernel does not have (from offsets with bf16 dist 1202 us, 1194 as a constant).
+// (dfa3d_walk.h), which costs registers that the kernel does not have (from offsets with bf16 dist 1202 us, 1194 as a constant).
 template <typename VT, typename DT, int C, int MODE, bool FULL, int WALK>
 __global__ void __launch_bounds__(kThreads, DFA3D_BWD_MIN_CTAS)
 dfa3d_backward_kernel(const KArgs a) {
@@ -263,17 +263,29 @@ dfa3d_depth_score_backward_kernel(const KArgs a) {
 // ------------------------------------------------------------------------------------------------
 // host-side dispatch
 // ------------------------------------------------------------------------------------------------
-template <typename VT, typename DT, int MODE, bool FULL, int WALK>
-static void launch_backward_g(const KArgs &a, dim3 grid, cudaStream_t s) {
+template <typename VT, typename DT, int C, int MODE, bool FULL>
+static void launch_backward_c(KArgs &a, int cams, cudaStream_t s) {
+  constexpr int kMost = DFA3D_BWD_ITEMS_PER_WARP;
+  constexpr auto kLong = dfa3d_backward_kernel<VT, DT, C, MODE, FULL, kMost>;
+  constexpr auto kShort = dfa3d_backward_kernel<VT, DT, C, MODE, FULL, 0>;
+  a.rounds = walk_backward((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, kMost, resident_ctas<kLong>(), sm_count());
+  const int per_cta = kWarpsPerCta * a.rounds;
+  const dim3 grid((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
+  if (a.rounds == kMost) kLong<<<grid, kThreads, 0, s>>>(a);
+  else kShort<<<grid, kThreads, 0, s>>>(a);
+}
+
+template <typename VT, typename DT, int MODE, bool FULL>
+static void launch_backward_g(KArgs &a, int cams, cudaStream_t s) {
   constexpr int V = RowVec4<VT>::kElems;
   switch ((a.C % V == 0) ? a.C / V : 0) {
-    case 2:  dfa3d_backward_kernel<VT, DT, 2 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
-    case 4:  dfa3d_backward_kernel<VT, DT, 4 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
-    case 8:  dfa3d_backward_kernel<VT, DT, 8 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
-    case 16: dfa3d_backward_kernel<VT, DT, 16 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
-    case 32: dfa3d_backward_kernel<VT, DT, 32 * V, MODE, FULL, WALK><<<grid, kThreads, 0, s>>>(a); break;
+    case 2:  launch_backward_c<VT, DT, 2 * V, MODE, FULL>(a, cams, s); break;
+    case 4:  launch_backward_c<VT, DT, 4 * V, MODE, FULL>(a, cams, s); break;
+    case 8:  launch_backward_c<VT, DT, 8 * V, MODE, FULL>(a, cams, s); break;
+    case 16: launch_backward_c<VT, DT, 16 * V, MODE, FULL>(a, cams, s); break;
+    case 32: launch_backward_c<VT, DT, 32 * V, MODE, FULL>(a, cams, s); break;
     default: {
-      const dim3 g1((unsigned)((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta), grid.y, 1);
+      const dim3 g1((unsigned)((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta), (unsigned)cams, 1);
       dfa3d_backward_generic_kernel<VT, DT, MODE><<<g1, kThreads, 0, s>>>(a);
       break;
     }
@@ -282,23 +294,12 @@ static void launch_backward_g(const KArgs &a, dim3 grid, cudaStream_t s) {
 
 template <typename VT, typename DT, int MODE>
 static cudaError_t launch_backward_vd(const KArgs &a0, cudaStream_t s) {
-  const bool full = a0.LP % 32 == 0;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
     const int cams = min(65535, a0.B - b0);
-    a.rounds = walk_rounds((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, DFA3D_BWD_ITEMS_PER_WARP,
-                           DFA3D_BWD_MIN_CTAS);
-    const int per_cta = kWarpsPerCta * a.rounds;
-    const dim3 grid((unsigned)((a.items_per_cam + per_cta - 1) / per_cta), (unsigned)cams, 1);
-    constexpr int kMost = DFA3D_BWD_ITEMS_PER_WARP;
-    if (a.rounds == kMost) {
-      if (full) launch_backward_g<VT, DT, MODE, true, kMost>(a, grid, s);
-      else launch_backward_g<VT, DT, MODE, false, kMost>(a, grid, s);
-    } else {
-      if (full) launch_backward_g<VT, DT, MODE, true, 0>(a, grid, s);
-      else launch_backward_g<VT, DT, MODE, false, 0>(a, grid, s);
-    }
+    if (a.LP % 32 == 0) launch_backward_g<VT, DT, MODE, true>(a, cams, s);
+    else launch_backward_g<VT, DT, MODE, false>(a, cams, s);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

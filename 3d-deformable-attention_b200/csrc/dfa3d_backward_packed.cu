@@ -146,27 +146,32 @@ dfa3d_backward_packed_kernel(const KArgs a) {
 // ------------------------------------------------------------------------------------------------
 // host-side dispatch
 // ------------------------------------------------------------------------------------------------
+template <typename VT, typename DT, int C, int MODE, int LPP>
+void launch_k(KArgs &a, int cams, cudaStream_t s) {
+  constexpr auto kernel = dfa3d_backward_packed_kernel<VT, DT, C, MODE, LPP>;
+  constexpr unsigned kBatch = kWarpsPerCta * (32 / LPP);             // items a CTA takes at a time
+  const unsigned batches = ((unsigned)a.items_per_cam + kBatch - 1) / kBatch;
+  a.rounds = walk_backward(batches, cams, kPackedRounds, resident_ctas<kernel>(), sm_count());
+  kernel<<<dim3((batches + a.rounds - 1) / a.rounds, (unsigned)cams, 1), kThreads, 0, s>>>(a);
+}
+
 template <typename VT, typename DT, int MODE, int LPP>
-void launch_c(const KArgs &a, dim3 grid, cudaStream_t s) {
-  if (a.C == 16) dfa3d_backward_packed_kernel<VT, DT, 16, MODE, LPP><<<grid, kThreads, 0, s>>>(a);
-  else if (a.C == 32) dfa3d_backward_packed_kernel<VT, DT, 32, MODE, LPP><<<grid, kThreads, 0, s>>>(a);
-  else dfa3d_backward_packed_kernel<VT, DT, 64, MODE, LPP><<<grid, kThreads, 0, s>>>(a);
+void launch_c(KArgs &a, int cams, cudaStream_t s) {
+  if (a.C == 16) launch_k<VT, DT, 16, MODE, LPP>(a, cams, s);
+  else if (a.C == 32) launch_k<VT, DT, 32, MODE, LPP>(a, cams, s);
+  else launch_k<VT, DT, 64, MODE, LPP>(a, cams, s);
 }
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
   const int lpp = packed_lanes(a0, MODE);
-  const unsigned batch = kWarpsPerCta * (32 / lpp);                  // items a CTA takes at a time
-  const unsigned batches = ((unsigned)a0.items_per_cam + batch - 1) / batch;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
-    const unsigned cams = (unsigned)min(65535, a0.B - b0);
-    a.rounds = walk_rounds(batches, (int)cams, kPackedRounds, DFA3D_BWD_MIN_CTAS);
-    const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
-    if (lpp == 4) launch_c<VT, DT, MODE, 4>(a, grid, s);
-    else if (lpp == 8) launch_c<VT, DT, MODE, 8>(a, grid, s);
-    else launch_c<VT, DT, MODE, 16>(a, grid, s);
+    const int cams = min(65535, a0.B - b0);
+    if (lpp == 4) launch_c<VT, DT, MODE, 4>(a, cams, s);
+    else if (lpp == 8) launch_c<VT, DT, MODE, 8>(a, cams, s);
+    else launch_c<VT, DT, MODE, 16>(a, cams, s);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -18,6 +18,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
+#include "dfa3d_walk.h"
+
 namespace dfa3d {
 
 constexpr int kMaxLevels = 32;
@@ -42,7 +46,7 @@ constexpr int kThreads = kWarpsPerCta * 32;
 
 // Compile-time tuning knobs (defaults = the measured optimum on B200 at the BEVFormer-base shape).
 //   *_ITEMS_PER_WARP  consecutive CTA-sized groups of items a CTA works through before it retires, at most
-//                     (walk_rounds): fewer, longer-lived CTAs (a CTA that handles one item per warp lives ~2 us)
+//                     (dfa3d_walk.h): fewer, longer-lived CTAs (a CTA that handles one item per warp lives ~2 us)
 //   *_MIN_CTAS        __launch_bounds__ residency target, i.e. the register cap
 #ifndef DFA3D_FWD_ITEMS_PER_WARP
 #define DFA3D_FWD_ITEMS_PER_WARP 8
@@ -226,24 +230,28 @@ __device__ __forceinline__ void prefetch_offsets(const KArgs &a, int b, unsigned
   }
 }
 
-// How many CTA-sized groups of items (`groups` of them a camera) a CTA walks before it retires: up to `most`, fewer where
-// that many would leave the last wave of CTAs nearly empty, or the device (`resident` CTAs fit an SM); starting a CTA costs
-// about a third of a group.  From six waves on the last one counts little.  Forward, 32 points an item, us at eight groups /
-// with this rule: 6 cameras x 1000 queries x 8 heads 95 / 70, 1 x 1000 29 / 15, 1 x 300 28 / 7.5, 6 x 6000 and more the same.
-inline int walk_rounds(long long groups, int cams, int most, int resident) {
-  const long long slots = 148LL * resident;
-  if ((groups + most - 1) / most * cams >= 6 * slots) return most;
-  int best = most;
-  long long cost = 0;
-  for (int r = most; r >= 1; --r) {
-    const long long ctas = (groups + r - 1) / r * cams;
-    const long long c = (ctas + slots - 1) / slots * (3 * r + 1);
-    if (r == most || c < cost) {
-      best = r;
-      cost = c;
-    }
+// CTAs of kThreads threads that an SM holds of a kernel, and the SMs of the device: what walk_forward and walk_backward
+// (dfa3d_walk.h) share the groups out over.  Asked of the runtime once; the devices of a process are taken to be alike.
+template <void (*Kernel)(KArgs)>
+inline int resident_ctas() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, kThreads, 0) != cudaSuccess || n < 1) return 4;
+    known.store(n, std::memory_order_relaxed);
   }
-  return best;
+  return n;
+}
+inline int sm_count() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed), device = 0;
+  if (n == 0) {
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n < 1)
+      return 148;
+    known.store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 // ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
@@ -260,7 +268,7 @@ inline int packed_lanes(const KArgs &a, int mode) {
   while (lanes < 16 && (long long)a.items_per_cam * lanes / kThreads * a.B < 148 * 2) lanes *= 2;
   return lanes;
 }
-// Batches of 32 lanes a warp takes before its CTA retires, at most (walk_rounds): two, for fewer, longer-lived CTAs; a small
+// Batches of 32 lanes a warp takes before its CTA retires, at most (dfa3d_walk.h): two, for fewer, longer-lived CTAs; a small
 // launch spreads over the SMs with one and is one chain of latencies deep (900 queries x 8 heads x 4 points forward: 7.9 us
 // at two, 5.1 at one).
 constexpr int kPackedRounds = 2;

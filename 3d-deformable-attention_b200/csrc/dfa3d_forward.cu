@@ -117,7 +117,7 @@ __device__ __forceinline__ void forward_item(const KArgs &a, const LevelTable &l
 // 5 CTAs (40 warps) per SM: measured best; at 6+ the register cap starts to cost more than the
 // extra warps hide.  A CTA walks up to DFA3D_FWD_ITEMS_PER_WARP consecutive groups of 8 items (the grid's
 // ~60 000 CTAs per camera otherwise live ~2 us each and their turnover shows: measured -7 % at 8).
-// WALK: that number, as every launch of some size has it; 0: a.rounds of them (walk_rounds).  As a run-time number it costs
+// WALK: that number, as every launch of some size has it; 0: a.rounds of them (dfa3d_walk.h).  As a run-time number it costs
 // registers that most kernels do not have: 6 cameras of the base levels, us at run time / as a constant: bf16 of 32 channels
 // 524 / 519, of 64 from offsets 503 / 491, fp32 of 64 535 / 521, fp16 of 20 points 363 / 350.  Unrolled, fp32 rows of up to 32
 // channels were faster with the run-time number (base 565 / 569, 8 channels from offsets 348 / 371, bf16 dist from offsets
@@ -226,35 +226,39 @@ static dim3 item_grid(const KArgs &a, int cams, int items_per_warp) {
 }
 
 template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, bool FULL>
-static void launch_forward_c(const KArgs &a, dim3 grid, cudaStream_t s) {
+static void launch_forward_c(KArgs &a, int cams, cudaStream_t s) {
   // unrolled, fp32 rows of up to 32 channels or bf16 rows of 32 with fp32 dist: one kernel for every launch (see the kernel)
   constexpr bool kOne = FULL && (RowVec<VT>::kElems == 4 ? C <= 32 : C == 32 && MODE == kFused && sizeof(DT) == 4 && !WRITE_DS);
   constexpr int kMost = DFA3D_FWD_ITEMS_PER_WARP;
-  if (!kOne && a.rounds == kMost)
-    dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, kOne ? 0 : kMost><<<grid, kThreads, 0, s>>>(a);
-  else
-    dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, 0><<<grid, kThreads, 0, s>>>(a);
+  constexpr auto kLong = dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, kOne ? 0 : kMost>;
+  constexpr auto kShort = dfa3d_forward_kernel<VT, DT, C, MODE, WRITE_DS, FULL, 0>;
+  // a group of 32 points is long beside the start of a CTA; a chain of loads weighs as much as a resident CTA's share
+  a.rounds = walk_forward((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, kMost, resident_ctas<kLong>(), sm_count(),
+                          WalkCost{2, 8});
+  const dim3 grid = item_grid(a, cams, a.rounds);
+  if (a.rounds == kMost) kLong<<<grid, kThreads, 0, s>>>(a);
+  else kShort<<<grid, kThreads, 0, s>>>(a);
 }
 
 template <typename VT, typename DT, int MODE, bool WRITE_DS, bool FULL>
-static void launch_forward_g(const KArgs &a, dim3 grid, cudaStream_t s) {
+static void launch_forward_g(KArgs &a, int cams, cudaStream_t s) {
   constexpr int V = RowVec<VT>::kElems;
   switch ((a.C % V == 0) ? a.C / V : 0) {
-    case 2:  launch_forward_c<VT, DT, 2 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
-    case 4:  launch_forward_c<VT, DT, 4 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
-    case 8:  launch_forward_c<VT, DT, 8 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
-    case 16: launch_forward_c<VT, DT, 16 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
-    case 32: launch_forward_c<VT, DT, 32 * V, MODE, WRITE_DS, FULL>(a, grid, s); break;
+    case 2:  launch_forward_c<VT, DT, 2 * V, MODE, WRITE_DS, FULL>(a, cams, s); break;
+    case 4:  launch_forward_c<VT, DT, 4 * V, MODE, WRITE_DS, FULL>(a, cams, s); break;
+    case 8:  launch_forward_c<VT, DT, 8 * V, MODE, WRITE_DS, FULL>(a, cams, s); break;
+    case 16: launch_forward_c<VT, DT, 16 * V, MODE, WRITE_DS, FULL>(a, cams, s); break;
+    case 32: launch_forward_c<VT, DT, 32 * V, MODE, WRITE_DS, FULL>(a, cams, s); break;
     default:
-      dfa3d_forward_generic_kernel<VT, DT, MODE, WRITE_DS><<<item_grid(a, (int)grid.y, 1), kThreads, 0, s>>>(a);
+      dfa3d_forward_generic_kernel<VT, DT, MODE, WRITE_DS><<<item_grid(a, cams, 1), kThreads, 0, s>>>(a);
       break;
   }
 }
 
 template <typename VT, typename DT, int MODE, bool WRITE_DS>
-static void launch_forward_ds(const KArgs &a, dim3 grid, cudaStream_t s) {
-  if (a.LP % 32 == 0) launch_forward_g<VT, DT, MODE, WRITE_DS, true>(a, grid, s);
-  else launch_forward_g<VT, DT, MODE, WRITE_DS, false>(a, grid, s);
+static void launch_forward_ds(KArgs &a, int cams, cudaStream_t s) {
+  if (a.LP % 32 == 0) launch_forward_g<VT, DT, MODE, WRITE_DS, true>(a, cams, s);
+  else launch_forward_g<VT, DT, MODE, WRITE_DS, false>(a, cams, s);
 }
 
 template <typename VT, typename DT, int MODE>
@@ -263,14 +267,11 @@ static cudaError_t launch_forward_vd(const KArgs &a0, cudaStream_t s) {
     KArgs a = a0;
     a.b0 = b0;
     const int cams = min(65535, a0.B - b0);
-    a.rounds = walk_rounds((a.items_per_cam + kWarpsPerCta - 1) / kWarpsPerCta, cams, DFA3D_FWD_ITEMS_PER_WARP,
-                           DFA3D_FWD_MIN_CTAS);
-    const dim3 grid = item_grid(a, cams, a.rounds);
     if constexpr (MODE == kFused) {               // the other modes' entry points return no depth score
-      if (a.ds_out) launch_forward_ds<VT, DT, MODE, true>(a, grid, s);
-      else launch_forward_ds<VT, DT, MODE, false>(a, grid, s);
+      if (a.ds_out) launch_forward_ds<VT, DT, MODE, true>(a, cams, s);
+      else launch_forward_ds<VT, DT, MODE, false>(a, cams, s);
     } else {
-      launch_forward_ds<VT, DT, MODE, false>(a, grid, s);
+      launch_forward_ds<VT, DT, MODE, false>(a, cams, s);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -140,51 +140,56 @@ dfa3d_forward_packed_kernel(const KArgs a) {
 // ------------------------------------------------------------------------------------------------
 // host-side dispatch
 // ------------------------------------------------------------------------------------------------
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+void launch_k(KArgs &a, int cams, cudaStream_t s) {
+  constexpr auto kernel = dfa3d_forward_packed_kernel<VT, DT, C, MODE, WRITE_DS, LPP, EXACT>;
+  constexpr unsigned kBatch = kWarpsPerCta * (32 / LPP);             // items a CTA takes at a time
+  const unsigned batches = ((unsigned)a.items_per_cam + kBatch - 1) / kBatch;
+  // unrolled, a batch takes nearly as long alone as beside others, and a CTA's start counts more
+  a.rounds = walk_forward(batches, cams, kPackedRounds, resident_ctas<kernel>(), sm_count(), EXACT ? WalkCost{8, 24} : WalkCost{6, 8});
+  kernel<<<dim3((batches + a.rounds - 1) / a.rounds, (unsigned)cams, 1), kThreads, 0, s>>>(a);
+}
+
 template <typename VT, typename DT, int MODE, bool WRITE_DS, int LPP, bool EXACT>
-void launch_c(const KArgs &a, dim3 grid, cudaStream_t s) {
-  if (a.C == 16) dfa3d_forward_packed_kernel<VT, DT, 16, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
-  else if (a.C == 32) dfa3d_forward_packed_kernel<VT, DT, 32, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
-  else dfa3d_forward_packed_kernel<VT, DT, 64, MODE, WRITE_DS, LPP, EXACT><<<grid, kThreads, 0, s>>>(a);
+void launch_c(KArgs &a, int cams, cudaStream_t s) {
+  if (a.C == 16) launch_k<VT, DT, 16, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
+  else if (a.C == 32) launch_k<VT, DT, 32, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
+  else launch_k<VT, DT, 64, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
 }
 
 template <typename VT, typename DT, int MODE, bool WRITE_DS>
-void launch_lp(const KArgs &a, int lpp, dim3 grid, cudaStream_t s) {
+void launch_lp(KArgs &a, int lpp, int cams, cudaStream_t s) {
   // the unrolled loop is instantiated where it is the common case: fp32 throughout
   constexpr bool kFloat = sizeof(VT) == 4 && (sizeof(DT) == 4 || !mode_has_depth(MODE));
   if constexpr (kFloat) {
     if (a.LP == lpp) {
-      if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, true>(a, grid, s);
-      else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, true>(a, grid, s);
-      else launch_c<VT, DT, MODE, WRITE_DS, 16, true>(a, grid, s);
+      if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, true>(a, cams, s);
+      else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, true>(a, cams, s);
+      else launch_c<VT, DT, MODE, WRITE_DS, 16, true>(a, cams, s);
       return;
     }
   }
   if constexpr (MODE != kCallerFused2D) {      // attn2d_supported: fp32, exact
-    if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, false>(a, grid, s);
-    else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, false>(a, grid, s);
-    else launch_c<VT, DT, MODE, WRITE_DS, 16, false>(a, grid, s);
+    if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, false>(a, cams, s);
+    else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, false>(a, cams, s);
+    else launch_c<VT, DT, MODE, WRITE_DS, 16, false>(a, cams, s);
   }
 }
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
   const int lpp = packed_lanes(a0, MODE);
-  const unsigned batch = kWarpsPerCta * (32 / lpp);                  // items a CTA takes at a time
-  const unsigned batches = ((unsigned)a0.items_per_cam + batch - 1) / batch;
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;
-    const unsigned cams = (unsigned)min(65535, a0.B - b0);
-    const int resident = RowVec<VT>::kElems == 8 ? 4 : MODE == kFused && a.ds_out ? 5 : 6;       // see PackedCtas
-    a.rounds = walk_rounds(batches, (int)cams, kPackedRounds, resident);
-    const dim3 grid((batches + a.rounds - 1) / a.rounds, cams, 1);
+    const int cams = min(65535, a0.B - b0);
     if constexpr (mode_from_offsets(MODE)) {      // the caller-fused entry points return no depth score
-      launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
+      launch_lp<VT, DT, MODE, false>(a, lpp, cams, s);
     } else if constexpr (MODE == kFused) {
-      if (a.ds_out) launch_lp<VT, DT, MODE, true>(a, lpp, grid, s);
-      else launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
+      if (a.ds_out) launch_lp<VT, DT, MODE, true>(a, lpp, cams, s);
+      else launch_lp<VT, DT, MODE, false>(a, lpp, cams, s);
     } else {
-      launch_lp<VT, DT, MODE, false>(a, lpp, grid, s);
+      launch_lp<VT, DT, MODE, false>(a, lpp, cams, s);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
