@@ -41,11 +41,12 @@ inline int walk_forward(long long groups, int cams, int most, int resident, int 
 
 // The backward waits for its reductions and pays next to nothing for a CTA's start: one group, but two where one would leave
 // a second wave about half empty (760 groups of 592: 31.3 us at one, 28.6 at two, 40.0 at four; 1400: 44.4, 51.8, 51.5), and
-// from twelve waves on (8900 groups of 64 channels 4 % longer at one).
+// from eleven waves on (8900 groups of 64 channels 4 % longer at one, 7000 batches of 4 points in two stages 3 %; 5000 batches
+// are 2.4 % longer at two).
 inline int walk_backward(long long groups, int cams, int most, int resident, int sms) {
   if (walks_full(groups, cams, most, resident, sms)) return most;
   const long long all = groups * cams * 20, wave = (long long)sms * resident;
-  return (all > 23 * wave && all <= 31 * wave) || all > 240 * wave ? (most < 2 ? most : 2) : 1;
+  return (all > 23 * wave && all <= 31 * wave) || all > 220 * wave ? (most < 2 ? most : 2) : 1;
 }
 
 }  // namespace dfa3d
