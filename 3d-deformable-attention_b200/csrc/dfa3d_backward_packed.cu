@@ -164,7 +164,10 @@ void launch_c(KArgs &a, int cams, cudaStream_t s) {
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
-  const int lpp = packed_lanes(a0, MODE);
+  // (2-D from offsets: the kernels are made for the lanes of a map)
+  const int lpp = MODE == kCallerFused2D ? lanes_of_points(a0.LP)
+                                         : packed_lanes(a0.LP, a0.C, RowVec4<VT>::kElems, a0.items, true, mode_has_depth(MODE),
+                                                        sm_count());
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;

@@ -257,17 +257,6 @@ inline int sm_count() {
 // ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
 // Items of up to 16 points, rows of 16, 32 or 64 channels.
 inline bool packed_covers(int LP, int C) { return LP <= 16 && (C == 16 || C == 32 || C == 64); }
-// Lanes of an item: 4, 8 or 16, the next from L*P on -- or more of them where the launch would have fewer than two CTAs for
-// every SM: it then takes as long as one warp's chain of loads, which is shorter with fewer items to a group.  2-D, one
-// 200 x 200 map, 4 points, forward / backward: 300 queries 10.5 / 8.9 -> 5.3 / 4.9 us, 900 11.4 / 10.3 -> 6.5 / 6.8 (warm 5.1
-// -> 4.5); 8 points of 23 x 40 and 512 queries 4.9 / 10.5 -> 4.9 / 8.5.  Up to four CTAs an SM: 1500 queries of 2 x 4 points
-// 7.3 -> 8.9.  (From offsets in 2-D, the kernels are made for the lanes of a map.)
-inline int packed_lanes(const KArgs &a, int mode) {
-  int lanes = a.LP <= 4 ? 4 : a.LP <= 8 ? 8 : 16;
-  if (mode == kCallerFused2D) return lanes;
-  while (lanes < 16 && (long long)a.items_per_cam * lanes / kThreads * a.B < 148 * 2) lanes *= 2;
-  return lanes;
-}
 // Batches of 32 lanes a warp takes before its CTA retires, at most (dfa3d_walk.h): two, for fewer, longer-lived CTAs; a small
 // launch spreads over the SMs with one and is one chain of latencies deep (900 queries x 8 heads x 4 points forward: 7.9 us
 // at two, 5.1 at one).

@@ -22,7 +22,10 @@ template <typename VT, int MODE, bool WRITE_DS>
 struct PackedCtas { static constexpr int value = RowVec<VT>::kElems == 8 ? 4 : WRITE_DS ? 5 : 6; };
 
 // EXACT: L*P == LPP, the row loop is unrolled; otherwise it ends at the item's last row.
-template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+// TURNS: an item that a small launch gives more lanes than its points need (packed_lanes) has TURNS times the groups.  They
+// read their rows at the same time, but add them up one after the other, in the order in which the fewer groups of another
+// launch do: an item's result does not depend on what else the launch holds.
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT, int TURNS>
 __global__ void __launch_bounds__(kThreads, PackedCtas<VT, MODE, WRITE_DS>::value)
 dfa3d_forward_packed_kernel(const KArgs a) {
   constexpr int V = RowVec<VT>::kElems;
@@ -42,8 +45,10 @@ dfa3d_forward_packed_kernel(const KArgs a) {
   // queries 113.7 / 106.9, 10 of 32 in 2-D, 3 x 6000 57.6 / 54.9, 900 queries of 8 in 16 lanes 9.3 / 7.7, bf16 dist from
   // offsets 68.5 / 66.5); 2-D from offsets, 900 x 16 points 8.80 / 8.61.  It cost the others registers: 2-D from offsets, 40000
   // queries x 4 points 51.8 / 53.8; 16 points of 16 channels with scores 165.8 / 173.3; fp16, 8 points of 64 channels 126 / 133.
-  constexpr bool kFold = V == 8 || MODE == kCallerFused2D ? GPI > 1 : !EXACT && !WRITE_DS;
+  constexpr bool kFold = V == 8 || MODE == kCallerFused2D ? GPI / TURNS > 1 : !EXACT && !WRITE_DS;
+  constexpr int SUMS = GPI / TURNS;             // partial sums of an item
   static_assert(32 % LPP == 0 && 32 % G == 0 && LPP % GPI == 0, "unsupported packing");
+  static_assert(GPI % TURNS == 0 && (TURNS == 1 || (!EXACT && IPG == 1)), "unsupported packing");
   __shared__ LevelTable lv;
   __shared__ RowTable rows[kWarpsPerCta];
   stage_levels(lv, a);
@@ -107,23 +112,31 @@ dfa3d_forward_packed_kernel(const KArgs a) {
           }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int turn = 0; turn < TURNS; ++turn) {
 #pragma unroll
-          for (int x = 0; x < V; ++x) acc[x] = fmaf(e[u].wgt, v[u][x], acc[x]);
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int x = 0; x < V; ++x) acc[x] = fmaf(e[u].wgt, v[u][x], acc[x]);
+          if (TURNS > 1) {                     // all go on from the sum of the group whose turn it was
+#pragma unroll
+            for (int x = 0; x < V; ++x)
+              acc[x] = __shfl_sync(0xffffffffu, acc[x], (grp / GPI * GPI + turn * SUMS + grp % SUMS) * G + sub);
+          }
+        }
       };
       if (EXACT) {
 #pragma unroll kUnroll
         for (int p0 = 0; p0 < LPP; p0 += GPI) step(p0);
       } else {
 #pragma unroll 1
-        for (int p0 = 0; p0 < n; p0 += GPI) step(p0);
+        for (int p0 = 0; p0 < n; p0 += GPI) step(p0);     // (past the last point the table holds no rows)
       }
       const unsigned idx = first + i;
       if constexpr (kFold) {
-        fold_and_store<V, G, GPI>(acc, lane, a.out + ((q0 * a.H + idx) * C + sub * V), idx < nitems);
+        fold_and_store<V, G, SUMS>(acc, lane, a.out + ((q0 * a.H + idx) * C + sub * V), idx < nitems && grp % GPI < SUMS);
       } else {
 #pragma unroll
-        for (int s = G; s < G * GPI; s <<= 1)
+        for (int s = G; s < G * SUMS; s <<= 1)
 #pragma unroll
           for (int x = 0; x < V; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], s);
         if (grp % GPI == 0 && idx < nitems) {
@@ -141,9 +154,10 @@ dfa3d_forward_packed_kernel(const KArgs a) {
 // ------------------------------------------------------------------------------------------------
 // host-side dispatch
 // ------------------------------------------------------------------------------------------------
-template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+template <typename VT, typename DT, int C, int MODE, bool WRITE_DS, int LPP, bool EXACT, int LANES>
 void launch_k(KArgs &a, int cams, cudaStream_t s) {
-  constexpr auto kernel = dfa3d_forward_packed_kernel<VT, DT, C, MODE, WRITE_DS, LPP, EXACT>;
+  constexpr int V = RowVec<VT>::kElems, kTurns = groups_of_item(C, V, LPP) / groups_of_item(C, V, LANES);
+  constexpr auto kernel = dfa3d_forward_packed_kernel<VT, DT, C, MODE, WRITE_DS, LPP, EXACT, kTurns>;
   constexpr unsigned kBatch = kWarpsPerCta * (32 / LPP);             // items a CTA takes at a time
   const unsigned batches = ((unsigned)a.items_per_cam + kBatch - 1) / kBatch;
   // unrolled, a batch takes nearly as long alone as beside others, and a CTA's start counts more
@@ -151,11 +165,12 @@ void launch_k(KArgs &a, int cams, cudaStream_t s) {
   kernel<<<dim3((batches + a.rounds - 1) / a.rounds, (unsigned)cams, 1), kThreads, 0, s>>>(a);
 }
 
-template <typename VT, typename DT, int MODE, bool WRITE_DS, int LPP, bool EXACT>
+// LANES: what the item's points need, LPP: what it gets
+template <typename VT, typename DT, int MODE, bool WRITE_DS, int LPP, bool EXACT, int LANES = LPP>
 void launch_c(KArgs &a, int cams, cudaStream_t s) {
-  if (a.C == 16) launch_k<VT, DT, 16, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
-  else if (a.C == 32) launch_k<VT, DT, 32, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
-  else launch_k<VT, DT, 64, MODE, WRITE_DS, LPP, EXACT>(a, cams, s);
+  if (a.C == 16) launch_k<VT, DT, 16, MODE, WRITE_DS, LPP, EXACT, LANES>(a, cams, s);
+  else if (a.C == 32) launch_k<VT, DT, 32, MODE, WRITE_DS, LPP, EXACT, LANES>(a, cams, s);
+  else launch_k<VT, DT, 64, MODE, WRITE_DS, LPP, EXACT, LANES>(a, cams, s);
 }
 
 template <typename VT, typename DT, int MODE, bool WRITE_DS>
@@ -172,14 +187,23 @@ void launch_lp(KArgs &a, int lpp, int cams, cudaStream_t s) {
   }
   if constexpr (MODE != kCallerFused2D) {      // attn2d_supported: fp32, exact
     if (lpp == 4) launch_c<VT, DT, MODE, WRITE_DS, 4, false>(a, cams, s);
-    else if (lpp == 8) launch_c<VT, DT, MODE, WRITE_DS, 8, false>(a, cams, s);
-    else launch_c<VT, DT, MODE, WRITE_DS, 16, false>(a, cams, s);
+    else if (lpp == 8) {
+      if (a.LP <= 4) launch_c<VT, DT, MODE, WRITE_DS, 8, false, 4>(a, cams, s);
+      else launch_c<VT, DT, MODE, WRITE_DS, 8, false>(a, cams, s);
+    } else {
+      if (a.LP <= 4) launch_c<VT, DT, MODE, WRITE_DS, 16, false, 4>(a, cams, s);
+      else if (a.LP <= 8) launch_c<VT, DT, MODE, WRITE_DS, 16, false, 8>(a, cams, s);
+      else launch_c<VT, DT, MODE, WRITE_DS, 16, false>(a, cams, s);
+    }
   }
 }
 
 template <typename VT, typename DT, int MODE>
 cudaError_t launch_vd(const KArgs &a0, cudaStream_t s) {
-  const int lpp = packed_lanes(a0, MODE);
+  // (2-D from offsets: the kernels are made for the lanes of a map)
+  const int lpp = MODE == kCallerFused2D ? lanes_of_points(a0.LP)
+                                         : packed_lanes(a0.LP, a0.C, RowVec<VT>::kElems, a0.items, false, mode_has_depth(MODE),
+                                                        sm_count());
   for (int b0 = 0; b0 < a0.B; b0 += 65535) {      // grid.y limit
     KArgs a = a0;
     a.b0 = b0;

@@ -1,4 +1,5 @@
-// How many CTA-sized groups of items a CTA of the operator's kernels walks before it retires (host code).
+// How the operator's kernels share the items of a launch out over the device (host code): the groups of items that a CTA
+// walks before it retires, and the lanes that an item gets where a warp takes several.
 //
 // A long walk saves the start of CTAs; a short one fills the device where there are few groups, and leaves less of it idle at
 // the end.  Launches of six waves of full walks and more always take the full walk (`most`); below, a few groups decide.
@@ -47,6 +48,40 @@ inline int walk_backward(long long groups, int cams, int most, int resident, int
   if (walks_full(groups, cams, most, resident, sms)) return most;
   const long long all = groups * cams * 20, wave = (long long)sms * resident;
   return (all > 23 * wave && all <= 31 * wave) || all > 220 * wave ? (most < 2 ? most : 2) : 1;
+}
+
+// ---- kernels in which a warp takes several items (dfa3d_*_packed.cu) ---------------------------------
+// Groups of C / V lanes (a row each, V channels a lane) that share an item of `lanes` lanes, each with every so-maniest point.
+constexpr int groups_of_item(int C, int V, int lanes) { return V * lanes / C > 1 ? V * lanes / C : 1; }
+// Lanes of an item: the next of 4, 8 and 16 from its points on ...
+constexpr int lanes_of_points(int LP) { return LP <= 4 ? 4 : LP <= 8 ? 8 : 16; }
+// ... or more of them in a small launch, which takes as long as one warp's chain of loads: with twice the lanes a group has
+// half the points to walk.  The more it has, the larger the launch that gains by it; one point is no chain.  Where groups of
+// the forward would then share the item, they add up in turns, so that its result stays the same in any launch: less to gain;
+// and less where the scores come from depth bins (`bins`), whose loads come before the rows and are not shortened.
+// 8 heads, us with the points' lanes / 8 / 16: 2-D, 4 points of 32 channels, forward 300 queries 4.9 / 3.8 / 3.4, 900 5.1 / 4.3 /
+// 4.8 (6.6 / 5.3 / 5.3 where the map has to come from HBM), backward 8.4 / 5.4 / 4.3, 8.7 / 6.7 / 6.3; 3-D, bf16, 8 points of 64
+// channels, forward 300 - / 6.4 / 5.8, 1200 - / 9.1 / 11.5, backward - / 14.9 / 10.7, - / 22.7 / 22.9.  Over 2070 sizes (60 to 2000
+// queries, 2-D, 3-D, fp32 and 16-bit, 2 to 8 points of 16 to 64 channels, maps in L2 or not) 0.3 % from the best choice on
+// average, more than 3 % at 85; with one line for all of them, four CTAs an SM, 3.3 % and 536.
+inline int packed_lanes(int LP, int C, int V, long long items, bool backward, bool bins, int sms) {
+  const int least = lanes_of_points(LP);
+  int lanes = least;
+  for (; lanes < 16; lanes *= 2) {
+    const long long walk = (long long)LP * C, group = V * lanes;       // points a group walks: walk / group
+    const long long ctas = (items * 2 * lanes + 255) / 256;
+    const auto few = [&](int per_sm, int per_point, int at_most) {     // CTAs of the launch, in tenths of one an SM
+      const long long limit = per_sm * group + per_point * walk;
+      return 10 * ctas * group <= sms * (limit < at_most * group ? limit : at_most * group);
+    };
+    const bool alike = groups_of_item(C, V, 2 * lanes) == groups_of_item(C, V, least);
+    const bool more = walk > group && (backward ? few(4, 7, 34)
+                                       : alike ? (bins && V == 4 ? few(7, 5, 42) : few(5, 8, 60))
+                                       : V == 8 ? few(5, 2, 20)        // eight channels a lane, 64 registers
+                                       : bins ? few(15, 0, 15) : few(5, 5, 40));
+    if (!more) break;
+  }
+  return lanes;
 }
 
 }  // namespace dfa3d

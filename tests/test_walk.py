@@ -1,5 +1,6 @@
-"""How many groups of items a CTA walks (csrc/dfa3d_walk.h), on the CPU: the choice against times measured on a B200 at sizes
-where the last wave of CTAs is full, just begun, half empty, and against the limits of its range."""
+"""How a launch's items are shared out (csrc/dfa3d_walk.h), on the CPU: the groups of items that a CTA walks against times
+measured on a B200 at sizes where the last wave of CTAs is full, just begun, half empty, the lanes of an item against times of
+small launches, and both against the limits of their range."""
 import ctypes
 import os
 import subprocess
@@ -16,6 +17,9 @@ extern "C" int forward(long long groups, int cams, int most, int resident, int s
 extern "C" int backward(long long groups, int cams, int most, int resident, int sms) {
   return dfa3d::walk_backward(groups, cams, most, resident, sms);
 }
+extern "C" int lanes(int LP, int C, int V, long long items, int backward, int bins, int sms) {
+  return dfa3d::packed_lanes(LP, C, V, items, backward, bins, sms);
+}
 """
 # us at one and two groups; one camera, 8 points an item (fp16 forward: 4 CTAs an SM; fp32 with scores: 5; backward: 4)
 FP16 = {500: (8.43, 9.31), 600: (10.38, 11.15), 650: (10.82, 11.44), 700: (11.34, 11.62), 920: (13.02, 13.97),
@@ -31,6 +35,14 @@ LONG = {100: (5.41, 8.48, 11.58, 14.59, 17.39, 20.35, 23.33, 26.19), 740: (10.85
         850: (14.88, 13.23, 15.20, 18.96, 22.67, 23.74, 27.62, 30.59), 2000: (26.77, 29.26, 26.02, 28.24, 28.79, 32.94, 33.28, 36.63),
         2600: (34.13, 32.67, 36.90, 32.77, 34.05, 33.67, 37.46, 41.35),
         6000: (68.34, 64.00, 62.96, 67.75, 66.45, 74.80, 78.07, 78.53)}
+# Items of several a warp, 8 heads: us at 4, 8 and 16 lanes by (points, channels, channels a lane, queries, backward, depth bins)
+_ = None
+LANES = {(4, 32, 4, 300, 0, 0): (4.88, 3.81, 3.42), (4, 32, 4, 900, 0, 0): (6.62, 5.31, 5.25), (4, 32, 4, 300, 1, 0): (8.35, 5.44, 4.26),
+         (8, 32, 4, 512, 0, 0): (_, 5.23, 4.54), (8, 32, 4, 512, 0, 1): (_, 4.90, 5.17), (8, 32, 4, 900, 0, 1): (_, 6.08, 6.88),
+         (4, 32, 4, 700, 1, 1): (10.56, 8.32, 7.79), (4, 32, 4, 1200, 1, 1): (10.98, 9.76, 10.88), (2, 16, 4, 900, 1, 1): (5.66, 5.55, 7.07),
+         (2, 16, 4, 1200, 1, 1): (6.05, 6.29, 8.59), (5, 16, 4, 1200, 1, 1): (_, 9.07, 10.72), (5, 16, 4, 900, 0, 1): (_, 4.83, 5.47),
+         (8, 64, 8, 300, 1, 1): (_, 14.88, 10.69), (8, 64, 8, 1200, 0, 1): (_, 9.09, 11.49), (2, 32, 8, 900, 0, 1): (4.46, 4.37, 5.42),
+         (2, 16, 8, 700, 0, 1): (4.03, 4.27, 4.87), (2, 16, 8, 60, 0, 1): (3.71, 3.89, 4.00), (4, 64, 4, 900, 0, 0): (17.23, 11.65, 9.41)}
 
 
 @pytest.fixture(scope="module")
@@ -42,6 +54,7 @@ def walk(tmp_path_factory):
     lib = ctypes.CDLL(str(d / "walk.so"))
     lib.forward.argtypes = [ctypes.c_longlong] + [ctypes.c_int] * 6
     lib.backward.argtypes = [ctypes.c_longlong] + [ctypes.c_int] * 4
+    lib.lanes.argtypes = [ctypes.c_int] * 3 + [ctypes.c_longlong] + [ctypes.c_int] * 3
     return lib
 
 
@@ -68,3 +81,19 @@ def test_range(walk, cams, most, resident):
             assert r == [most] * 4
         elif groups * cams <= 148:
             assert r == [1] * 4
+
+
+def test_lanes_are_within_5_percent_of_the_fastest(walk):
+    for (LP, C, V, queries, backward, bins), us in LANES.items():
+        took = us[{4: 0, 8: 1, 16: 2}[walk.lanes(LP, C, V, 8 * queries, backward, bins, 148)]]
+        assert took <= 1.05 * min(t for t in us if t), (LP, C, V, queries, backward, bins)
+
+
+@pytest.mark.parametrize("backward,bins", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("C,V", [(16, 4), (32, 4), (64, 4), (16, 8), (32, 8), (64, 8)])
+def test_lanes_range(walk, C, V, backward, bins):
+    for LP in range(1, 17):
+        least = 4 if LP <= 4 else 8 if LP <= 8 else 16
+        chosen = [walk.lanes(LP, C, V, items, backward, bins, 148) for items in (1, 100, 2400, 7200, 20000, 10 ** 6, 2 ** 40)]
+        assert all(x in (4, 8, 16) and x >= least for x in chosen) and chosen == sorted(chosen, reverse=True)
+        assert chosen[-1] == chosen[-2] == least
