@@ -61,12 +61,13 @@ __device__ __forceinline__ float widen(float v) { return v; }
 __device__ __forceinline__ float widen(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float widen(__half v) { return __half2float(v); }
 
+// adds the bins of a word to V sums
 template <int V, typename T>
-__device__ __forceinline__ void load_bins(const T *p, float (&r)[V]) {
-  union { typename Word<T, V>::type w; T t[V]; } u;
-  u.w = __ldg(reinterpret_cast<const typename Word<T, V>::type *>(p));
+__device__ __forceinline__ void add_bins(typename Word<T, V>::type w, float (&sum)[V]) {
+  T t[V];
+  memcpy(t, &w, sizeof w);
 #pragma unroll
-  for (int i = 0; i < V; ++i) r[i] = widen(u.t[i]);
+  for (int i = 0; i < V; ++i) sum[i] += widen(t[i]);
 }
 // the bins as they are stored, formed once for all the rows that receive them
 template <typename T, int V>
@@ -283,26 +284,28 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel
     for (int k = 0; k < V; ++k) G[j][k] = 0.f;
   const GT *grad = reinterpret_cast<const GT *>(a.grad_dist) + (long long)b * a.N * a.D + sub * V;
   const int room = a.D - sub * V;
-  // rows asked for at a time: a second one costs registers, and so CTAs, that few bins cannot spare (118 bins 39.5 us at one
-  // row, 33.8 at two; 64 bins 22.6, 23.5)
-  constexpr int K = V * NC <= 8 ? 1 : 2;
+  // Rows asked for at a time, kept as they are stored until they are summed: a second one costs registers, and so CTAs, that few
+  // bins cannot spare (118 fp32 bins 39.5 us at one row, 33.8 at two; 64 bins 22.6, 23.5), nor 65 to 128 16-bit bins in words of
+  // one or two, where it takes as many registers as fp32 (bf16, rows widened when they came / kept / kept, one row: 97 bins 42.7
+  // / 32.4 / 28.4 us, 118 bins 43.6 / 26.6 / 26.2; of more than 128 two stay ahead: 130 bins 69.5 / 54.7 / 59.1, 255
+  // bins 131 / 67 / 68; words of four bins have two, 128 bins 37.5 / 26.0).
+  using W = typename Word<GT, V>::type;
+  constexpr int K = V * NC <= 8 || (V * NC == 16 && sizeof(GT) == 2 && V < 4) ? 1 : 2;
   if (pixel < npix)
     for_each_row<K>(f, a, p0, pixel, [&](const int (&n)[K]) {
-      float v[K][NC][V];
+      W w[K][NC];
 #pragma unroll
       for (int u = 0; u < K; ++u)
 #pragma unroll
         for (int j = 0; j < NC; ++j) {
-#pragma unroll
-          for (int k = 0; k < V; ++k) v[u][j][k] = 0.f;
-          if (n[u] >= 0 && j * kLanes * V < room) load_bins<V>(grad + (long long)n[u] * a.D + j * kLanes * V, v[u][j]);
+          memset(&w[u][j], 0, sizeof(W));
+          if (n[u] >= 0 && j * kLanes * V < room)
+            w[u][j] = __ldg(reinterpret_cast<const W *>(grad + (long long)n[u] * a.D + j * kLanes * V));
         }
 #pragma unroll
       for (int u = 0; u < K; ++u)
 #pragma unroll
-        for (int j = 0; j < NC; ++j)
-#pragma unroll
-          for (int k = 0; k < V; ++k) G[j][k] += v[u][j][k];
+        for (int j = 0; j < NC; ++j) add_bins<V, GT>(w[u][j], G[j]);
     });
   float p[NC][V], pg = 0.f;
   normalised_bins<V, NC>(tile, stride, a, p);

@@ -40,18 +40,22 @@ def test_headers_come_from_the_toolkit_of_nvcc(build_py, monkeypatch, tmp_path):
     assert os.path.join(os.path.realpath(tmp_path), "include") in build_py._native_command()
 
 
-def _spill_bytes(build_py, source, kernel):
-    """Bytes that the one kernel whose mangled name holds `kernel` spills, as ptxas reported it when `source` was compiled."""
+def _report(source, kernel, numbers):
+    """What ptxas reported of the one kernel whose mangled name holds `kernel` when `source` was compiled: the numbers that the
+    expression `numbers` finds."""
     import re
     log = os.path.join(PKG_DIR, "build", source + ".log")
     if not os.path.exists(log):
         pytest.skip("the library was not compiled here")
     with open(log) as f:
         text = f.read()
-    found = re.findall(r"Compiling entry function '\S*%s\S*' .*?(\d+) bytes spill stores, (\d+) bytes spill loads"
-                       % re.escape(kernel), text, re.S)
+    found = re.findall(r"Compiling entry function '\S*%s\S*' .*?%s" % (re.escape(kernel), numbers), text, re.S)
     assert len(found) == 1, (kernel, found)
-    return sum(int(x) for x in found[0])
+    return sum(int(x) for x in ([found[0]] if isinstance(found[0], str) else found[0]))
+
+
+def _spill_bytes(build_py, source, kernel):
+    return _report(source, kernel, r"(\d+) bytes spill stores, (\d+) bytes spill loads")
 
 
 # A launch of full size walks its groups of items with a constant bound: as a run-time number it cost these kernels registers
@@ -71,3 +75,11 @@ def test_full_size_launches_have_a_constant_walk(build_py, source, kernel, most)
 @pytest.mark.parametrize("kernel", ["IffLi32ELi3ELb0ELi4ELb1E", "IffLi64ELi3ELb0ELi8ELb1E", "IffLi16ELi0ELb1ELi16ELb1E"])
 def test_fp32_items_that_share_a_warp_spill_nothing(build_py, kernel):
     assert _spill_bytes(build_py, "dfa3d_forward_packed.cu", "dfa3d_forward_packed_kernel" + kernel) == 0
+
+
+# Registers of 256 threads and with them the CTAs on an SM.  Distribution producer, backward: rows of 16-bit gradients that were
+# widened when they came took 76 registers for 65 to 128 bins (three CTAs, now four).
+@pytest.mark.parametrize("words", ["Li2ELi8E", "Li4ELi4E", "Li1ELi16E"])
+@pytest.mark.parametrize("dtype", ["13__nv_bfloat16", "6__half"])
+def test_four_ctas_of_the_16_bit_producer_backward(dtype, words):
+    assert _report("dfa3d_dist_producer.cu", "32dist_from_logits_backward_kernelI" + dtype + words, r"Used (\d+) registers") <= 64

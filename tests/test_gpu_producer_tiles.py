@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("map_w,D", [(1, 1), (31, 4), (32, 64), (33, 65), (64, 3), (100, 256), (7, 255)])
+# bins: one, two and four a word, up to 64, 128 and 256 of them
+@pytest.mark.parametrize("map_w,D", [(1, 1), (31, 4), (32, 64), (33, 65), (64, 3), (100, 256), (7, 255), (50, 66), (33, 128),
+                                     (9, 130), (40, 127)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 def test_tile_edges_match_softmax_and_nearest_resize(lib_built, map_w, D, dtype):
     from dfa3d_b200.dist_producer import depth_distribution
