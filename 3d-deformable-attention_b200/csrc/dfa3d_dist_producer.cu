@@ -225,13 +225,15 @@ __device__ __forceinline__ void normalised_bins(const float *tile, int stride, c
 }
 
 // Forward: a CTA owns kTile map pixels, normalises each once and writes the rows of every level pixel that reads one
-// of them, from registers.  (A CTA per 32 output rows, which normalised every level pixel anew, took 53 us at
-// 6 x 58 x 100 x 64 -> 30 825 rows; tiles that ended with their map row, 3 1/8 of them for 100 columns, 17.1; this 15.1;
-// a 29 x 50 map 14.7 -> 10.8, 118 bins 28.9 -> 26.2.)  Bound by instructions and the tail, not by memory: 1092 CTAs of
-// which six are resident on an SM are 1.23 waves; held to 32 registers for eight it took 13.9, but bf16 12.4 -> 13.2, 59
-// bins 6.9 -> 8.0.
+// of them, from registers.  us, 6 x 58 x 100 maps to 30 825 rows, the operands of three calls in turn: a CTA per 32 output
+// rows, which normalised every level pixel anew, 53; tiles that ended with their map row (3 1/8 of them for 100 columns) / this:
+// 64 bins 17.9 / 15.0, 118 bins 30.0 / 27.0, 6 x 29 x 50 maps of 64 to 7250 rows 6.3 / 5.3.  Bound by instructions and the tail,
+// not by memory: 1092 CTAs of which six are resident on an SM are 1.23 waves; held to 32 registers for eight CTAs 64 bins gain
+// a tenth, bf16 loses 7 % and 59 bins 16 %.  More than 128 bins are held to 64 registers, four CTAs instead of three (75 to 80
+// registers, which 32 logits a thread at once take): 129 bins 42.8 -> 36.8, bf16 49.6 -> 43.0; 256 bins 48.1 -> 43.7, bf16 33.2 ->
+// 30.1 (48 registers 35.9).
 template <typename OT, int V, int NC>
-__global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const ProdArgs a) {
+__global__ void __launch_bounds__(kProdThreads, V * NC == 32 ? 4 : 0) dist_from_logits_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];
   __shared__ Footprint f;
   const int pixels = a.hs * a.ws, b = blockIdx.y, p0 = blockIdx.x * kTile, npix = min(kTile, pixels - p0);
@@ -261,9 +263,9 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_kernel(const Pr
 
 // Backward: the same ownership.  A pixel's eight lanes sum the incoming gradient over the level pixels that read it, in
 // the order of the levels, rows and columns, and form p * (G - <p, G>) (softmax) or p * (1 - p) * G (sigmoid), stored
-// along the map through shared memory.  (A warp per map pixel, one level pixel after the other: 87 us at the shape above;
-// tiles that ended with their map row 24.5; this 22.6; a 29 x 50 map 33.4 -> 22.1, 118 bins 38.5 -> 33.8.)  Bound by the
-// latency of the gradient's rows at the CTAs that the registers leave room for.
+// along the map through shared memory.  us as above: a warp per map pixel, one level pixel after the other, 87; tiles that
+// ended with their map row / this: 64 bins 23.9 / 21.0, 118 bins 34.8 / 31.1, the 29 x 50 maps 7.1 / 6.3.  Bound by the latency of
+// the gradient's rows at the CTAs that the registers leave room for.
 template <typename GT, int V, int NC>
 __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel(const ProdArgs a) {
   extern __shared__ __align__(16) float tile[];
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(kProdThreads) dist_from_logits_backward_kernel
   const GT *grad = reinterpret_cast<const GT *>(a.grad_dist) + (long long)b * a.N * a.D + sub * V;
   const int room = a.D - sub * V;
   // Rows asked for at a time, kept as they are stored until they are summed: a second one costs registers, and so CTAs, that few
-  // bins cannot spare (118 fp32 bins 39.5 us at one row, 33.8 at two; 64 bins 22.6, 23.5), nor 65 to 128 16-bit bins in words of
+  // bins cannot spare (118 fp32 bins gain 14 % by it, 64 lose 4 %), nor 65 to 128 16-bit bins in words of
   // one or two, where it takes as many registers as fp32 (bf16, rows widened when they came / kept / kept, one row: 97 bins 42.7
   // / 32.4 / 28.4 us, 118 bins 43.6 / 26.6 / 26.2; of more than 128 two stay ahead: 130 bins 69.5 / 54.7 / 59.1, 255
   // bins 131 / 67 / 68; words of four bins have two, 128 bins 37.5 / 26.0).

@@ -78,8 +78,14 @@ def test_fp32_items_that_share_a_warp_spill_nothing(build_py, kernel):
 
 
 # Registers of 256 threads and with them the CTAs on an SM.  Distribution producer, backward: rows of 16-bit gradients that were
-# widened when they came took 76 registers for 65 to 128 bins (three CTAs, now four).
+# widened when they came took 76 registers for 65 to 128 bins (three CTAs, now four).  Forward of more than 128 bins: 75 to 80.
 @pytest.mark.parametrize("words", ["Li2ELi8E", "Li4ELi4E", "Li1ELi16E"])
 @pytest.mark.parametrize("dtype", ["13__nv_bfloat16", "6__half"])
 def test_four_ctas_of_the_16_bit_producer_backward(dtype, words):
     assert _report("dfa3d_dist_producer.cu", "32dist_from_logits_backward_kernelI" + dtype + words, r"Used (\d+) registers") <= 64
+
+
+@pytest.mark.parametrize("words", ["Li1ELi32E", "Li2ELi16E", "Li4ELi8E"])
+@pytest.mark.parametrize("dtype", ["f", "13__nv_bfloat16", "6__half"])
+def test_four_ctas_of_the_producer_forward_of_many_bins(dtype, words):
+    assert _report("dfa3d_dist_producer.cu", "23dist_from_logits_kernelI" + dtype + words, r"Used (\d+) registers") <= 64
