@@ -1,6 +1,7 @@
 """Kernels in which a warp takes several items of up to 16 points: point counts below, at and between the lane counts
-4, 8 and 16, last warps that are partly filled, every storage type and width, one and two batches per warp, with and
-without depth scores, one- and two-stage, per-camera query counts.  Checked against the CPU oracle."""
+4, 8 and 16, last warps that are partly filled, every storage type and width, small launches (whose items have 16 lanes) and
+fp32 ones of two batches per warp, with and without depth scores, one- and two-stage, per-camera query counts.  Checked
+against the CPU oracle.  (test_gpu_full_launches.py: the other lane counts.)"""
 import numpy as np
 import pytest
 import torch
@@ -16,7 +17,7 @@ STORAGE = {"fp32": (torch.float32, torch.float32), "bf16": (torch.bfloat16, torc
            "bf16_fp32": (torch.bfloat16, torch.float32)}
 
 
-@pytest.mark.parametrize("Q", [37, 9001])            # 9001 x 3 cameras x 3 heads of 8 lanes: two batches per warp
+@pytest.mark.parametrize("Q", [37, 9001])            # 9001 x 3 cameras x 3 heads of 8 lanes: two batches per warp in some kernels
 @pytest.mark.parametrize("storage", sorted(STORAGE))
 @pytest.mark.parametrize("L,P,C", [(1, 1, 16), (1, 2, 64), (1, 3, 32), (1, 4, 32), (1, 5, 16), (2, 3, 32), (1, 7, 64),
                                    (2, 4, 32), (3, 3, 64), (2, 5, 32), (3, 4, 16), (5, 3, 32), (4, 4, 64)])

@@ -135,7 +135,7 @@ def _per_camera_problem(w, lens, seed):
 def test_ragged_fused_entry_points_match_dense_per_camera(M, lens, packed):
     from dfa3d_b200 import ext
     w = wl.WORKLOADS["odd"].with_(C=32)
-    if packed:                                   # L*P = 8: the kernels in which a warp holds 4 items
+    if packed:                                   # L*P = 8: the kernels in which items share a warp
         w = w.with_(levels=((9, 6), (4, 5)), P=4)
     d, dense, packed, off, _ = _per_camera_problem(w, lens, seed=5)
     t = {k: v.to(DEV) for k, v in d.items()}
@@ -167,7 +167,7 @@ def test_ragged_offsets_entry_points_match_dense_per_camera(M, packed):
     from dfa3d_b200 import ext
     lens, Z = [7, 0, 12], 2
     w = wl.WORKLOADS["odd"].with_(C=32, P=4)
-    if packed:                                   # L*P = 16: the kernels in which a warp holds 2 items
+    if packed:                                   # L*P = 16: the kernels in which items share a warp
         w = w.with_(levels=((9, 6), (4, 5), (2, 2), (1, 1)))
     d, dense, packed, off, g = _per_camera_problem(w, lens, seed=9)
     R = sum(lens)
