@@ -24,8 +24,11 @@ struct WalkCost {
 // The walk whose waves cost the fullest SM least.  Forward, 32 points an item: 6 cameras x 1000 queries x 8 heads 95 us at
 // eight groups, 70 with this rule, 1 x 1000 29 / 15, 1 x 300 28 / 7.5.  Just past a wave (batches of several items a warp, fp16,
 // 8 points): 600 batches 10.4 us at one, 11.2 at two, 920 13.0 / 14.0; fp32, unrolled, with scores takes two there, 16.0 / 15.1.
+// Waves of CTAs run into one another the more of them there are: from six of one group on, two are never slower (with scores,
+// 6 x 6000 queries of 4 points, 6.1 waves, which the costs would give one: 52.9 us at one, 51.2 at two; 5000 to 9000 batches 2 to 4 %).
 inline int walk_forward(long long groups, int cams, int most, int resident, int sms, WalkCost w) {
   if (walks_full(groups, cams, most, resident, sms)) return most;
+  if (most == 2 && groups * cams >= (long long)kFullWaves * sms * resident) return 2;
   int best = most;
   long long least = -1;
   for (int r = most; r >= 1; --r) {
