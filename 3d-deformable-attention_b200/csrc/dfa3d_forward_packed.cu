@@ -43,9 +43,11 @@ dfa3d_forward_packed_kernel(const KArgs a) {
   // fold_and_store where there is something to halve (16-bit rows whose item is shared), and for fp32 rows where the kernel is
   // faster with it: rows in a loop that is not unrolled, no scores (us without / with: 5 points of 64 channels, 6 x 6000
   // queries 113.7 / 106.9, 10 of 32 in 2-D, 3 x 6000 57.6 / 54.9, 900 queries of 8 in 16 lanes 9.3 / 7.7, bf16 dist from
-  // offsets 68.5 / 66.5); 2-D from offsets, 900 x 16 points 8.80 / 8.61.  It cost the others registers: 2-D from offsets, 40000
-  // queries x 4 points 51.8 / 53.8; 16 points of 16 channels with scores 165.8 / 173.3; fp16, 8 points of 64 channels 126 / 133.
-  constexpr bool kFold = V == 8 || MODE == kCallerFused2D ? GPI / TURNS > 1 : !EXACT && !WRITE_DS;
+  // offsets 68.5 / 66.5); 2-D from offsets, 900 x 16 points 8.80 / 8.61; 16 points of 32 channels without scores (6 x 6000
+  // queries, 2-D 126.3 / 124.1, with two levels 139.5 / 136.8, from offsets 174.7 / 173.4; of 16 channels 109.2 / 110.5).  It cost
+  // the others registers: 2-D from offsets, 40000 queries x 4 points 51.8 / 53.8; 16 points of 16 channels with scores 165.8 /
+  // 173.3; fp16, 8 points of 64 channels 126 / 133.
+  constexpr bool kFold = V == 8 || MODE == kCallerFused2D ? GPI / TURNS > 1 : !WRITE_DS && (!EXACT || (GPI == 2 && C == 32));
   constexpr int SUMS = GPI / TURNS;             // partial sums of an item
   static_assert(32 % LPP == 0 && 32 % G == 0 && LPP % GPI == 0, "unsupported packing");
   static_assert(GPI % TURNS == 0 && (TURNS == 1 || (!EXACT && IPG == 1)), "unsupported packing");
