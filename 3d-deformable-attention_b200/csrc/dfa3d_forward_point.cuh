@@ -59,8 +59,9 @@ template <int V, int G, int NG>
 __device__ __forceinline__ void fold_and_store(float (&acc)[V], int lane, float *out, bool live) {
   // 16-bit rows (8 channels a lane): a lane that still holds several values hands half of them over at each exchange, 7
   // shuffles for 32 channels where all of them passed around took 24 (they go through the L1 pipe, which binds), and all
-  // lanes write the row.  The sums are formed in the same order.  bf16, 6 cameras of the base levels: 555 -> 521 us.  For
-  // fp32 rows, 3 shuffles instead of 8, it was no gain: 525 -> 529, from offsets 470 -> 481.
+  // lanes write the row (of 16 channels half of them: the fourth exchange has one value left).  The sums are formed in the
+  // same order.  bf16, 6 cameras of the base levels: 555 -> 521 us.  For fp32 rows, 3 shuffles instead of 8, it was no gain:
+  // 525 -> 529, from offsets 470 -> 481.
   constexpr bool kHalve = V == 8;
   int n = V;
 #pragma unroll
